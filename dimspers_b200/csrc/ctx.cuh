@@ -185,15 +185,61 @@ struct CudaError {
 // levels, reductions, control) shorter than their own launch latency.  With
 // g_pdl set, klaunch gives each launch the programmatic-stream-serialization
 // attribute: the kernel may be scheduled while its predecessor is still
-// running, and waits in grid_dep_wait() (griddepcontrol.wait, which returns
+// running, and waits in grid_dep_sync() (griddepcontrol.wait, which returns
 // once the predecessor grid has completed and its memory is visible) before it
-// touches memory.  Every kernel of the solve path calls grid_dep_wait() first,
-// so a launch with or without the attribute computes the same thing; without
-// the attribute the wait returns at once.
-__device__ __forceinline__ void grid_dep_wait() {
+// touches memory that a kernel of the solve writes.  Every kernel of the solve
+// path first lets its own successor launch (grid_dep_launch: the successor's
+// CTAs take the slots that the last wave leaves, decode their indices, fetch
+// what no kernel of the solve writes -- element blocks, D^-1, coefficients --
+// and then wait), so a launch with or without the attribute computes the same
+// thing; without the attribute the wait returns at once.
+// A kernel completes only after its own wait returned, so waiting for the
+// direct predecessor covers all earlier ones.  Pointers to data that a
+// predecessor writes carry no __restrict__ here: the compiler may move a load
+// it takes for read-only data above the wait.
+__device__ __forceinline__ void grid_dep_launch() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void grid_dep_sync() {
 #if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
   asm volatile("griddepcontrol.wait;" ::: "memory");
 #endif
+}
+__device__ __forceinline__ void grid_dep_wait() {
+  grid_dep_launch();
+  grid_dep_sync();
+}
+
+// Streaming loads of data that is constant during a solve, kept in program
+// order by volatile so that they are issued before the wait that follows.
+__device__ __forceinline__ float4 ld_stream(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 ld_stream(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ld_stream(const double* p) {
+  double v;
+  asm volatile("ld.global.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+// the same through L1, for data whose neighbours the same warp reads next
+__device__ __forceinline__ double ld_early(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_early(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
 }
 
 inline thread_local int g_pdl = 0;

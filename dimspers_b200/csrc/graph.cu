@@ -177,8 +177,8 @@ __global__ void k_guess_select(DevCtl* ctl, double* scal) {
     scal[S_RR] = rz;
   }
 }
-__global__ void k_guess_apply(const DevCtl* ctl, double* __restrict__ U, const double* __restrict__ Uz,
-                              double* __restrict__ r, const double* __restrict__ rz, double* __restrict__ P,
+__global__ void k_guess_apply(const DevCtl* ctl, double* U, const double* Uz,
+                              double* r, const double* rz, double* P,
                               int64_t nU, int64_t nP) {
   grid_dep_wait();
   if (ctl->guess_used) return;
@@ -193,7 +193,7 @@ __global__ void k_guess_apply(const DevCtl* ctl, double* __restrict__ U, const d
 // ---- PCG vector kernels reading their scalars from the table --------------------
 // p = z + beta p with beta = rzn/rz, except p = z on the first iteration
 template <typename T>
-__global__ void k_pcg_dir_g(T* __restrict__ p, const T* __restrict__ z, T* __restrict__ Ap, int64_t n,
+__global__ void k_pcg_dir_g(T* p, const T* z, T* Ap, int64_t n,
                             const double* scal, int rzn, int rz, const int* it) {
   grid_dep_wait();
   const double beta = (*it == 0 || scal[rz] == 0.0) ? 0.0 : scal[rzn] / scal[rz];
@@ -206,7 +206,7 @@ __global__ void k_pcg_dir_g(T* __restrict__ p, const T* __restrict__ z, T* __res
 
 // p = s z32 + beta p (s = ||b||, the FP32 V-cycle ran on r / ||b||), Ap = 0:
 // the mixed-precision form reads the FP32 preconditioned residual directly
-__global__ void k_pcg_dir_f32z(double* __restrict__ p, const float* __restrict__ z32, double* __restrict__ Ap,
+__global__ void k_pcg_dir_f32z(double* p, const float* z32, double* Ap,
                                int64_t n, const double* scal, int yy, int rzn, int rz, const int* it) {
   grid_dep_wait();
   const double beta = (*it == 0 || scal[rz] == 0.0) ? 0.0 : scal[rzn] / scal[rz];
@@ -219,7 +219,7 @@ __global__ void k_pcg_dir_f32z(double* __restrict__ p, const float* __restrict__
 }
 
 // FP64 residual -> FP32 hierarchy input, scaled by 1/sqrt(scal[irr]) (keeps FP32 in range)
-__global__ void k_r_to_f32(const double* __restrict__ r, float* __restrict__ r32, const double* scal, int irr, int64_t n) {
+__global__ void k_r_to_f32(const double* r, float* r32, const double* scal, int irr, int64_t n) {
   grid_dep_wait();
   const double s = 1.0 / sqrt(scal[irr]);
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -227,7 +227,7 @@ __global__ void k_r_to_f32(const double* __restrict__ r, float* __restrict__ r32
 }
 // nodal block Jacobi with an inverse of another precision
 template <typename Td, typename Tv>
-__global__ void k_bj_mixed(const Td* __restrict__ dinv, const Tv* __restrict__ r, Tv* __restrict__ z, int64_t nnod) {
+__global__ void k_bj_mixed(const Td* __restrict__ dinv, const Tv* r, Tv* z, int64_t nnod) {
   grid_dep_wait();
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nnod) return;
@@ -241,7 +241,7 @@ __global__ void k_bj_mixed(const Td* __restrict__ dinv, const Tv* __restrict__ r
 
 // rz = r . z with z = ||b|| z32 (the V-cycle ran on r / ||b||); z itself is
 // never stored: k_pcg_dir_f32z reads z32 again
-__global__ void __launch_bounds__(kRedThreads) k_rz_f32(const float* __restrict__ z32, const double* __restrict__ r,
+__global__ void __launch_bounds__(kRedThreads) k_rz_f32(const float* z32, const double* r,
                                                         double* scal, int yy, int rzn, int64_t n, double* partial,
                                                         unsigned int* counter) {
   grid_dep_wait();
@@ -259,12 +259,12 @@ __global__ void __launch_bounds__(kRedThreads) k_rz_f32(const float* __restrict_
 // ||r||^2 > tol^2 ||b||^2 and it < inner_itmax.  r32 != null (FP64 Krylov on
 // the FP32 hierarchy): also writes the next V-cycle's input r / ||b||.
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_pcg_upd_check(T* __restrict__ x, T* __restrict__ r,
-                                                                const T* __restrict__ p, const T* __restrict__ Ap,
+__global__ void __launch_bounds__(kRedThreads) k_pcg_upd_check(T* x, T* r,
+                                                                const T* p, const T* Ap,
                                                                 int64_t n, double* scal, int rz, int rzn, int pap,
                                                                 int irr, double* partial, unsigned int* counter,
                                                                 cudaGraphConditionalHandle h, DevCtl* ctl, int fp32,
-                                                                float* __restrict__ r32, int yy) {
+                                                                float* r32, int yy) {
   grid_dep_wait();
   const double inv_s = r32 ? 1.0 / sqrt(scal[yy]) : 0.0;
   // a non-positive or non-finite p.Ap (breakdown, e.g. an FP32 operator that
@@ -294,13 +294,13 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_upd_check(T* __restrict__ x
   }
 }
 
-__global__ void k_to_f32_scaled(const double* __restrict__ a, float* __restrict__ b, const double* scal, int64_t n) {
+__global__ void k_to_f32_scaled(const double* a, float* b, const double* scal, int64_t n) {
   grid_dep_wait();
   const double s = 1.0 / sqrt(scal[R_RES2]);
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) b[i] = (float)(s * a[i]);
 }
-__global__ void k_add_f32_scaled(double* __restrict__ z, const float* __restrict__ e, const double* scal, int64_t n) {
+__global__ void k_add_f32_scaled(double* z, const float* e, const double* scal, int64_t n) {
   grid_dep_wait();
   const double s = sqrt(scal[R_RES2]);
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

@@ -297,15 +297,16 @@ __device__ inline void fine_node_weights(int a, int b, int ncrc, int Ac, int Bc,
 // xf += P xc (per fine node, gather); also sets rf = bf (the fine level's
 // residual buffer, from which the next apply subtracts A xf)
 template <typename T>
-__global__ void k_prolong_add(const T* __restrict__ xc, T* __restrict__ xf, const T* __restrict__ bf,
-                              T* __restrict__ rf, int Af, int Bf, int ncrc, int Ac, int Bc, int pin) {
-  grid_dep_wait();
+__global__ void k_prolong_add(const T* xc, T* xf, const T* bf,
+                              T* rf, int Af, int Bf, int ncrc, int Ac, int Bc, int pin) {
+  grid_dep_launch();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= Af * Bf) return;
   const int b = n / Af, a = n - b * Af;
   int cn[6];
   double w[6];
   fine_node_weights(a, b, ncrc, Ac, Bc, cn, w);
+  grid_dep_sync();
   // the 6 nodes of the containing coarse element are always valid: gather them
   // all unconditionally (zero weights included) so the loads issue together
   typedef typename V2<T>::T X2;
@@ -336,10 +337,10 @@ __global__ void k_prolong_add(const T* __restrict__ xc, T* __restrict__ xf, cons
 // (the work of k_cheb_first): rc = bc, dc = xc = coef[0] D^-1 bc, and tc = 0
 // when tc is given (the cluster tail's levels accumulate into t).
 template <typename T, int LPN>
-__global__ void __launch_bounds__(256) k_restrict_g(const T* __restrict__ r, const T* __restrict__ t, T* __restrict__ bc,
+__global__ void __launch_bounds__(256) k_restrict_g(const T* r, const T* t, T* bc,
                                                     int Af, int Bf, int Ac, int Bc, int pin, int first,
-                                                    const T* __restrict__ dinv_c, T* __restrict__ xc, T* __restrict__ rc,
-                                                    T* __restrict__ dc, T* __restrict__ tc,
+                                                    const T* __restrict__ dinv_c, T* xc, T* rc,
+                                                    T* dc, T* tc,
                                                     const double* __restrict__ coef_c) {
   grid_dep_wait();
   const int cls = blockIdx.y;
@@ -410,10 +411,10 @@ __global__ void __launch_bounds__(256) k_restrict_g(const T* __restrict__ r, con
 constexpr int kRTile = 16;
 constexpr int kRPatch = 2 * (kRTile - 1) + 1 + 8;   // 39: stencil offsets reach 4 fine nodes each way
 template <typename T>
-__global__ void __launch_bounds__(256) k_restrict_tile(const T* __restrict__ r, const T* __restrict__ t,
-                                                       T* __restrict__ bc, int Af, int Bf, int Ac, int Bc, int pin,
-                                                       int first, const T* __restrict__ dinv_c, T* __restrict__ xc,
-                                                       T* __restrict__ rc, T* __restrict__ dc, T* __restrict__ tc,
+__global__ void __launch_bounds__(256) k_restrict_tile(const T* r, const T* t,
+                                                       T* bc, int Af, int Bf, int Ac, int Bc, int pin,
+                                                       int first, const T* __restrict__ dinv_c, T* xc,
+                                                       T* rc, T* dc, T* tc,
                                                        const double* __restrict__ coef_c) {
   grid_dep_wait();
   typedef typename V2<T>::T X2;
@@ -496,24 +497,31 @@ __global__ void __launch_bounds__(256) k_restrict_tile(const T* __restrict__ r, 
 // hierarchy) and move each node's pair of components with one 8/16-byte
 // access, all loads issued before the arithmetic.
 template <typename T>
-__device__ __forceinline__ void bj_apply_t(const T* __restrict__ dinv, int64_t n, T r0, T r1, T& z0, T& z1) {
-  const T a = dinv[3 * n], b = dinv[3 * n + 1], c = dinv[3 * n + 2];
-  z0 = a * r0 + b * r1;
-  z1 = b * r0 + c * r1;
-}
+struct NodeInv {
+  T a, b, c;
+  // D^-1 is constant during a solve: the steps fetch it before their wait
+  __device__ __forceinline__ NodeInv(const T* __restrict__ dinv, int64_t n)
+      : a(ld_early(dinv + 3 * n)), b(ld_early(dinv + 3 * n + 1)), c(ld_early(dinv + 3 * n + 2)) {}
+  __device__ __forceinline__ void apply(T r0, T r1, T& z0, T& z1) const {
+    z0 = a * r0 + b * r1;
+    z1 = b * r0 + c * r1;
+  }
+};
 
 // first step from x = 0: r = b, d = (1/theta) D^-1 b, x = d
 template <typename T>
-__global__ void k_cheb_first(const T* __restrict__ b, const T* __restrict__ dinv, T* __restrict__ x,
-                             T* __restrict__ r, T* __restrict__ d, const double* __restrict__ coef, int64_t nnod) {
-  grid_dep_wait();
+__global__ void k_cheb_first(const T* b, const T* __restrict__ dinv, T* x,
+                             T* r, T* d, const double* __restrict__ coef, int64_t nnod) {
+  grid_dep_launch();
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   typedef typename V2<T>::T X2;
+  const NodeInv<T> di(dinv, n);
+  const T it = (T)ld_early(coef);
+  grid_dep_sync();
   const X2 bv = reinterpret_cast<const X2*>(b)[n];
-  const T it = (T)coef[0];
   T z0, z1;
-  bj_apply_t<T>(dinv, n, bv.x, bv.y, z0, z1);
+  di.apply(bv.x, bv.y, z0, z1);
   X2 dv;
   dv.x = it * z0; dv.y = it * z1;
   reinterpret_cast<X2*>(r)[n] = bv;
@@ -522,18 +530,20 @@ __global__ void k_cheb_first(const T* __restrict__ b, const T* __restrict__ dinv
 }
 // first step from a given x (r = b - Ax on entry): d = (1/theta) D^-1 r, x += d
 template <typename T>
-__global__ void k_cheb_first_x(const T* __restrict__ r, const T* __restrict__ dinv, T* __restrict__ x,
-                               T* __restrict__ d, const double* __restrict__ coef, int64_t nnod) {
-  grid_dep_wait();
+__global__ void k_cheb_first_x(const T* r, const T* __restrict__ dinv, T* x,
+                               T* d, const double* __restrict__ coef, int64_t nnod) {
+  grid_dep_launch();
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   typedef typename V2<T>::T X2;
+  const NodeInv<T> di(dinv, n);
+  const T it = (T)ld_early(coef);
+  grid_dep_sync();
   const X2 rv = reinterpret_cast<const X2*>(r)[n];
   const X2 xv = reinterpret_cast<const X2*>(x)[n];
-  const T it = (T)coef[0];
   X2 dv;
   T z0, z1;
-  bj_apply_t<T>(dinv, n, rv.x, rv.y, z0, z1);
+  di.apply(rv.x, rv.y, z0, z1);
   dv.x = it * z0; dv.y = it * z1;
   reinterpret_cast<X2*>(d)[n] = dv;
   X2 xn;
@@ -542,19 +552,21 @@ __global__ void k_cheb_first_x(const T* __restrict__ r, const T* __restrict__ di
 }
 // d = c1 d + c2 D^-1 r; x += d  (c1, c2 = coef[0], coef[1]; r already holds r - A d_prev)
 template <typename T>
-__global__ void k_cheb_step(const T* __restrict__ r, const T* __restrict__ dinv, T* __restrict__ x,
-                            T* __restrict__ d, const double* __restrict__ coef, int64_t nnod) {
-  grid_dep_wait();
+__global__ void k_cheb_step(const T* r, const T* __restrict__ dinv, T* x,
+                            T* d, const double* __restrict__ coef, int64_t nnod) {
+  grid_dep_launch();
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   typedef typename V2<T>::T X2;
+  const NodeInv<T> di(dinv, n);
+  const T c1 = (T)ld_early(coef), c2 = (T)ld_early(coef + 1);
+  grid_dep_sync();
   const X2 rv = reinterpret_cast<const X2*>(r)[n];
   const X2 dv = reinterpret_cast<const X2*>(d)[n];
   const X2 xv = reinterpret_cast<const X2*>(x)[n];
-  const T c1 = (T)coef[0], c2 = (T)coef[1];
   X2 dn, xn;
   T z0, z1;
-  bj_apply_t<T>(dinv, n, rv.x, rv.y, z0, z1);
+  di.apply(rv.x, rv.y, z0, z1);
   dn.x = c1 * dv.x + c2 * z0; dn.y = c1 * dv.y + c2 * z1;
   xn.x = xv.x + dn.x; xn.y = xv.y + dn.y;
   reinterpret_cast<X2*>(d)[n] = dn;
@@ -562,7 +574,7 @@ __global__ void k_cheb_step(const T* __restrict__ r, const T* __restrict__ dinv,
 }
 // z = D^-1 r (nodal blocks)
 template <typename T>
-__global__ void k_bj(const T* __restrict__ dinv, const T* __restrict__ r, T* __restrict__ z, int64_t nnod) {
+__global__ void k_bj(const T* __restrict__ dinv, const T* r, T* z, int64_t nnod) {
   grid_dep_wait();
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nnod) return;
@@ -710,14 +722,28 @@ __global__ void k_symmetrize(double* __restrict__ A, int n) {
 // x = Inv b, one CTA per row: each thread reads a few entries of the row (all
 // loads in flight at once), then a block reduction.
 template <typename T>
-__global__ void __launch_bounds__(128) k_dense_apply(const double* __restrict__ Inv, const T* __restrict__ b,
-                                                     T* __restrict__ x, int n) {
-  grid_dep_wait();
+__global__ void __launch_bounds__(128) k_dense_apply(const double* __restrict__ Inv, const T* b,
+                                                     T* x, int n) {
+  grid_dep_launch();
   const int row = blockIdx.x;
   const double* a = Inv + (size_t)row * n;
+  // the row is constant during a solve: its first 12 x 128 entries (all of it
+  // up to the default coarse_max) are fetched before the wait
+  constexpr int kPre = 12;
+  double av[kPre];
+#pragma unroll
+  for (int k = 0; k < kPre; ++k) {
+    const int j = threadIdx.x + 128 * k;
+    av[k] = j < n ? ld_stream(a + j) : 0.0;
+  }
+  grid_dep_sync();
   double s = 0.0;
-#pragma unroll 4
-  for (int j = threadIdx.x; j < n; j += 128) s += a[j] * (double)b[j];
+#pragma unroll
+  for (int k = 0; k < kPre; ++k) {
+    const int j = threadIdx.x + 128 * k;
+    if (j < n) s += av[k] * (double)b[j];
+  }
+  for (int j = threadIdx.x + 128 * kPre; j < n; j += 128) s += a[j] * (double)b[j];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   __shared__ double part[4];

@@ -58,7 +58,10 @@ __device__ inline int tile_element(int ncr, int wt) {
 // ye = K_e x_e for element e, with the lattice index of each of its 6 nodes.
 // kL2: read x with ld.global.cg (L2 only), for callers where other CTAs
 // rewrite x during the same kernel.
-template <typename Tm, typename Tv, bool kL2>
+// kDep: the caller is a kernel of the solve chain: the element's matrix, which
+// nothing rewrites during a solve, is fetched before the wait for the
+// predecessor and the nodes are gathered after it.
+template <typename Tm, typename Tv, bool kL2, bool kDep = false>
 __device__ __forceinline__ void element_product(const Tm* __restrict__ K, const Tv* x, int e, int ncr, int A, int B,
                                                 int nd[6], Tv ye[12]) {
   typedef typename KVec<Tm>::V VT;
@@ -67,7 +70,10 @@ __device__ __forceinline__ void element_product(const Tm* __restrict__ K, const 
   const VT* Kb = reinterpret_cast<const VT*>(K + (int64_t)(e >> 5) * (32 * NV * PER)) + (e & 31);
   Tm kk[NV * PER];
 #pragma unroll
-  for (int j = 0; j < NV; ++j) vec_to(Kb[j * 32], kk + j * PER);
+  for (int j = 0; j < NV; ++j) {
+    if (kDep) vec_to(ld_stream(Kb + j * 32), kk + j * PER);
+    else vec_to(Kb[j * 32], kk + j * PER);
+  }
   const int q = e >> 1, t = e & 1;
   const int ir = q % ncr, it = q / ncr;
   const int a0 = 2 * ir, b0 = 2 * it;
@@ -85,6 +91,7 @@ __device__ __forceinline__ void element_product(const Tm* __restrict__ K, const 
   }
   typedef typename V2<Tv>::T X2;
   const X2* x2 = reinterpret_cast<const X2*>(x);
+  if (kDep) grid_dep_sync();
   Tv xe[12];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
@@ -106,12 +113,12 @@ __device__ __forceinline__ void element_product(const Tm* __restrict__ K, const 
 }
 
 // y += K_e x_e for element e (kSub: y -= K_e x_e), scatter-added with atomics.
-template <typename Tm, typename Tv, bool kL2, bool kSub = false>
+template <typename Tm, typename Tv, bool kL2, bool kSub = false, bool kDep = false>
 __device__ __forceinline__ void apply_element(const Tm* __restrict__ K, const Tv* x, Tv* y, int e, int ncr, int A,
                                               int B) {
   int nd[6];
   Tv ye[12];
-  element_product<Tm, Tv, kL2>(K, x, e, ncr, A, B, nd, ye);
+  element_product<Tm, Tv, kL2, kDep>(K, x, e, ncr, A, B, nd, ye);
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     if (kSub) atomic_add2(&y[2 * nd[k]], -ye[2 * k], -ye[2 * k + 1]);
@@ -120,25 +127,25 @@ __device__ __forceinline__ void apply_element(const Tm* __restrict__ K, const Tv
 }
 
 template <typename Tm, typename Tv, bool kSub = false>
-__global__ void __launch_bounds__(256) k_apply_K(const Tm* __restrict__ K, const Tv* __restrict__ x,
-                                                 Tv* __restrict__ y, int nel, int ncr, int A, int B, int wt) {
-  grid_dep_wait();
+__global__ void __launch_bounds__(256) k_apply_K(const Tm* __restrict__ K, const Tv* x,
+                                                 Tv* y, int nel, int ncr, int A, int B, int wt) {
+  grid_dep_launch();
   const int e = tile_element(ncr, wt);
   if (e >= nel) return;
-  apply_element<Tm, Tv, false, kSub>(K, x, y, e, ncr, A, B);
+  apply_element<Tm, Tv, false, kSub, true>(K, x, y, e, ncr, A, B);
 }
 
 // Deterministic form, pass 1: E[(2k + c) nel + e] = (K_e x_e) of local node k,
 // component c (no atomics; k_node_gather sums the nodes in a fixed order).
 template <typename Tm, typename Tv>
-__global__ void __launch_bounds__(256) k_apply_K_elem(const Tm* __restrict__ K, const Tv* __restrict__ x,
-                                                      Tv* __restrict__ E, int nel, int ncr, int A, int B) {
-  grid_dep_wait();
+__global__ void __launch_bounds__(256) k_apply_K_elem(const Tm* __restrict__ K, const Tv* x,
+                                                      Tv* E, int nel, int ncr, int A, int B) {
+  grid_dep_launch();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nel) return;
   int nd[6];
   Tv ye[12];
-  element_product<Tm, Tv, false>(K, x, e, ncr, A, B, nd, ye);
+  element_product<Tm, Tv, false, true>(K, x, e, ncr, A, B, nd, ye);
 #pragma unroll
   for (int d = 0; d < 12; ++d) E[(int64_t)d * nel + e] = ye[d];
 }
@@ -164,7 +171,7 @@ __host__ __device__ constexpr int loc_b(int t, int k) {
 // (i + (pa - loc_a) / 2, j + (pb - loc_b) / 2), theta periodic), so a warp
 // never diverges on them, and neighbouring lanes write neighbouring nodes.
 template <int PA, int PB, typename T, int NC>
-__device__ __forceinline__ void gather_class(const T* __restrict__ E, int i, int j, int ncr, int nct, int64_t nel,
+__device__ __forceinline__ void gather_class(const T* E, int i, int j, int ncr, int nct, int64_t nel,
                                              T s[NC]) {
 #pragma unroll
   for (int c = 0; c < NC; ++c) s[c] = (T)0;
@@ -185,7 +192,7 @@ __device__ __forceinline__ void gather_class(const T* __restrict__ E, int i, int
 }
 
 template <int PA, int PB, typename T, int NC, int MODE>
-__device__ __forceinline__ void gather_node(const T* __restrict__ E, T* __restrict__ y, int i, int j, int ncr, int nct,
+__device__ __forceinline__ void gather_node(const T* E, T* y, int i, int j, int ncr, int nct,
                                             int64_t nel) {
   const int a = 2 * i + PA;
   if (a > 2 * ncr) return;
@@ -202,7 +209,7 @@ __device__ __forceinline__ void gather_node(const T* __restrict__ E, T* __restri
 }
 
 template <typename T, int NC, int MODE>
-__global__ void __launch_bounds__(256) k_node_gather(const T* __restrict__ E, T* __restrict__ y, int ncr, int nct,
+__global__ void __launch_bounds__(256) k_node_gather(const T* E, T* y, int ncr, int nct,
                                                      int64_t nel) {
   grid_dep_wait();
   const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -247,7 +254,7 @@ template void launch_node_gather<float>(const Level&, const float*, float*, int,
 // read it with coalesced loads.
 template <typename T, bool kSub = false>
 __global__ void __launch_bounds__(256) k_apply_K_mf(const T* __restrict__ Dw, const T* __restrict__ tab,
-                                                    const T* __restrict__ x, T* __restrict__ y, int ncr, int nct,
+                                                    const T* x, T* y, int ncr, int nct,
                                                     int A, int B, int pin) {
   grid_dep_wait();
   const int nel = 2 * ncr * nct;
@@ -439,7 +446,7 @@ __device__ inline void element_pdofs_dev(int e, int ncr, int nct, int pressure, 
   else        { pd[0] = v2; pd[1] = v3; pd[2] = v4; }
 }
 
-__global__ void k_apply_G(const double* __restrict__ G, const double* __restrict__ p, double* __restrict__ y,
+__global__ void k_apply_G(const double* __restrict__ G, const double* p, double* y,
                           int nel, int ncr, int nct, int A, int B, int pressure) {
   grid_dep_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -458,7 +465,7 @@ __global__ void k_apply_G(const double* __restrict__ G, const double* __restrict
 
 // Deterministic form of the G apply, pass 1: element e's 12 values of G_e p_e
 // into E[d nel + e] (k_node_gather sums them per node).
-__global__ void k_apply_G_elem(const double* __restrict__ G, const double* __restrict__ p, double* __restrict__ E,
+__global__ void k_apply_G_elem(const double* __restrict__ G, const double* p, double* E,
                                int nel, int ncr, int nct, int pressure) {
   grid_dep_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -472,22 +479,30 @@ __global__ void k_apply_G_elem(const double* __restrict__ G, const double* __res
                              G[(size_t)(24 + d) * nel + e] * p2;
 }
 
-__global__ void k_apply_GT(const double* __restrict__ G, const double* __restrict__ x, double* __restrict__ p,
+__global__ void k_apply_GT(const double* __restrict__ G, const double* x, double* p,
                            int nel, int ncr, int nct, int A, int B, int pressure) {
-  grid_dep_wait();
+  grid_dep_launch();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nel) return;
   int nd[6], pd[3];
+  double g[kGe];   // the element's block is constant during a solve: fetched before the wait
+#pragma unroll
+  for (int k = 0; k < kGe; ++k) g[k] = ld_stream(G + (size_t)k * nel + e);
   element_nodes_dev(e, ncr, A, B, nd);
   element_pdofs_dev(e, ncr, nct, pressure, pd);
+  grid_dep_sync();
   double xe[12];
 #pragma unroll
-  for (int k = 0; k < 6; ++k) { xe[2 * k] = x[2 * nd[k]]; xe[2 * k + 1] = x[2 * nd[k] + 1]; }
+  for (int k = 0; k < 6; ++k) {
+    const double2 v = reinterpret_cast<const double2*>(x)[nd[k]];
+    xe[2 * k] = v.x;
+    xe[2 * k + 1] = v.y;
+  }
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     double s = 0.0;
 #pragma unroll
-    for (int d = 0; d < 12; ++d) s += G[(size_t)(i * 12 + d) * nel + e] * xe[d];
+    for (int d = 0; d < 12; ++d) s += g[i * 12 + d] * xe[d];
     if (pressure == 1) p[pd[i]] = s;
     else atomicAdd(&p[pd[i]], s);
   }
@@ -499,10 +514,10 @@ __global__ void k_apply_GT(const double* __restrict__ G, const double* __restric
 // into a shared-memory copy of those nodes first and then issues one global FP64
 // atomic per node and component (198), since sm_100a has no vector FP64 reduction.
 constexpr int kGWarpNodes = 99;
-__global__ void __launch_bounds__(128) k_apply_G_warp(const double* __restrict__ G, const double* __restrict__ p,
-                                                      double* __restrict__ y, int nel, int ncr, int nct, int A, int B,
+__global__ void __launch_bounds__(128) k_apply_G_warp(const double* __restrict__ G, const double* p,
+                                                      double* y, int nel, int ncr, int nct, int A, int B,
                                                       int pressure) {
-  grid_dep_wait();
+  grid_dep_launch();
   __shared__ double acc[4][2 * kGWarpNodes];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -510,7 +525,11 @@ __global__ void __launch_bounds__(128) k_apply_G_warp(const double* __restrict__
   if (e0 >= nel) return;                          // whole warps past the last element (tail block)
   const int q0 = e0 >> 1, ir0 = q0 % ncr, it = q0 / ncr;
   double* s = acc[w];
+  double g[kGe];   // constant during a solve: fetched before the wait
+#pragma unroll
+  for (int k = 0; k < kGe; ++k) g[k] = ld_stream(G + (size_t)k * nel + e);
   for (int k = lane; k < 2 * kGWarpNodes; k += 32) s[k] = 0.0;
+  grid_dep_sync();
   __syncwarp();
   {
     const int q = e >> 1, t = e & 1;
@@ -530,8 +549,7 @@ __global__ void __launch_bounds__(128) k_apply_G_warp(const double* __restrict__
     }
 #pragma unroll
     for (int d = 0; d < 12; ++d) {
-      const double v = G[(size_t)d * nel + e] * p0 + G[(size_t)(12 + d) * nel + e] * p1 +
-                       G[(size_t)(24 + d) * nel + e] * p2;
+      const double v = g[d] * p0 + g[12 + d] * p1 + g[24 + d] * p2;
       const int k = d >> 1;
       atomicAdd(&s[2 * (la[k] + 33 * lb[k]) + (d & 1)], v);
     }
@@ -577,7 +595,7 @@ void launch_apply_GT(Ctx& c, const double* x, double* p) {
 
 // ---- deterministic reductions ---------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_dot(const T* __restrict__ a, const T* __restrict__ b, int64_t n,
+__global__ void __launch_bounds__(kRedThreads) k_dot(const T* a, const T* b, int64_t n,
                                                      double* partial, unsigned int* counter, double* out) {
   grid_dep_wait();
   double s = 0.0;
@@ -588,7 +606,7 @@ __global__ void __launch_bounds__(kRedThreads) k_dot(const T* __restrict__ a, co
   grid_finish<1>(v, partial, counter, o);
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_sum(const double* __restrict__ a, int64_t n, double* partial,
+__global__ void __launch_bounds__(kRedThreads) k_sum(const double* a, int64_t n, double* partial,
                                                      unsigned int* counter, double* out) {
   grid_dep_wait();
   double s = 0.0;
@@ -600,7 +618,7 @@ __global__ void __launch_bounds__(kRedThreads) k_sum(const double* __restrict__ 
 }
 
 // compensated variants (double-double accumulation) for the Schur-complement loop
-__global__ void __launch_bounds__(kRedThreads) k_dot_c(const double* __restrict__ a, const double* __restrict__ b,
+__global__ void __launch_bounds__(kRedThreads) k_dot_c(const double* a, const double* b,
                                                        int64_t n, double* partial, unsigned int* counter, double* out) {
   grid_dep_wait();
   DD s{0.0, 0.0};
@@ -611,7 +629,7 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_c(const double* __restrict_
   grid_finish_dd<1>(v, partial, counter, o);
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_sum_c(const double* __restrict__ a, int64_t n, double* partial,
+__global__ void __launch_bounds__(kRedThreads) k_sum_c(const double* a, int64_t n, double* partial,
                                                        unsigned int* counter, double* out) {
   grid_dep_wait();
   DD s{0.0, 0.0};

@@ -41,16 +41,16 @@ enum Slot {
 static int nb256(int64_t n) { return (int)div_up(n, 256); }
 
 // ---- outer vector kernels -----------------------------------------------------
-__global__ void k_sub_mean(double* __restrict__ a, int64_t n, const double* __restrict__ sum) {
+__global__ void k_sub_mean(double* a, int64_t n, const double* sum) {
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) a[i] -= *sum / (double)n;
 }
 
 // rlast = r; alpha = rd/qSq; P += alpha q; r -= alpha Sq; sum(r) -> scal[S_SUMR]
-__global__ void __launch_bounds__(kRedThreads) k_schur_update_p(double* __restrict__ P, double* __restrict__ r,
-                                                                 double* __restrict__ rlast, const double* __restrict__ q,
-                                                                 const double* __restrict__ Sq, int64_t n,
+__global__ void __launch_bounds__(kRedThreads) k_schur_update_p(double* P, double* r,
+                                                                 double* rlast, const double* q,
+                                                                 const double* Sq, int64_t n,
                                                                  double* scal, double* partial, unsigned int* counter) {
   grid_dep_wait();
   const double alpha = scal[S_RD] / scal[S_QSQ];
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kRedThreads) k_schur_update_p(double* __restri
   grid_finish_dd<1>(v, partial, counter, o);
 }
 
-__global__ void k_axpy_slot(double* __restrict__ U, const double* __restrict__ z, int64_t n, const double* scal) {
+__global__ void k_axpy_slot(double* U, const double* z, int64_t n, const double* scal) {
   grid_dep_wait();
   const double alpha = scal[S_RD] / scal[S_QSQ];
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -76,8 +76,8 @@ __global__ void k_axpy_slot(double* __restrict__ U, const double* __restrict__ z
 }
 
 // r -= mean(r); d = r*pc; ||r||^2 -> S_RR; (r - rlast).d -> S_BNUM
-__global__ void __launch_bounds__(kRedThreads) k_schur_center(double* __restrict__ r, const double* __restrict__ rlast,
-                                                               const double* __restrict__ pc, double* __restrict__ d,
+__global__ void __launch_bounds__(kRedThreads) k_schur_center(double* r, const double* rlast,
+                                                               const double* __restrict__ pc, double* d,
                                                                int64_t n, double* scal, double* partial,
                                                                unsigned int* counter) {
   grid_dep_wait();
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kRedThreads) k_schur_center(double* __restrict
 }
 
 // Element-block mass preconditioner (discontinuous pressure): d_e = M_e^-1 r_e.
-__global__ void k_mass_blk(const double* __restrict__ r, const double* __restrict__ Minv, double* __restrict__ d,
+__global__ void k_mass_blk(const double* r, const double* __restrict__ Minv, double* d,
                            int nel) {
   grid_dep_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -111,8 +111,8 @@ __global__ void k_mass_blk(const double* __restrict__ r, const double* __restric
 }
 
 // k_schur_center with d = M^-1 r per element block
-__global__ void __launch_bounds__(kRedThreads) k_schur_center_blk(double* __restrict__ r, const double* __restrict__ rlast,
-                                                                   const double* __restrict__ Minv, double* __restrict__ d,
+__global__ void __launch_bounds__(kRedThreads) k_schur_center_blk(double* r, const double* rlast,
+                                                                   const double* __restrict__ Minv, double* d,
                                                                    int nel, double* scal, double* partial,
                                                                    unsigned int* counter) {
   grid_dep_wait();
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kRedThreads) k_schur_center_blk(double* __rest
 }
 
 // q = d + beta q, beta = BNUM / RD; sum(q) -> S_SUMQ (for the next rm0space!)
-__global__ void __launch_bounds__(kRedThreads) k_q_update(double* __restrict__ q, const double* __restrict__ d, int64_t n,
+__global__ void __launch_bounds__(kRedThreads) k_q_update(double* q, const double* d, int64_t n,
                                                            double* scal, double* partial, unsigned int* counter) {
   grid_dep_wait();
   const double beta = scal[S_BNUM] / scal[S_RD];
@@ -156,8 +156,8 @@ __global__ void __launch_bounds__(kRedThreads) k_q_update(double* __restrict__ q
 }
 
 // q -= mean(q); rd = r.d -> S_RD
-__global__ void __launch_bounds__(kRedThreads) k_q_center_rd(double* __restrict__ q, const double* __restrict__ r,
-                                                              const double* __restrict__ d, int64_t n, double* scal,
+__global__ void __launch_bounds__(kRedThreads) k_q_center_rd(double* q, const double* r,
+                                                              const double* d, int64_t n, double* scal,
                                                               double* partial, unsigned int* counter) {
   grid_dep_wait();
   const double m = scal[S_SUMQ] / (double)n;
@@ -171,18 +171,18 @@ __global__ void __launch_bounds__(kRedThreads) k_q_center_rd(double* __restrict_
   grid_finish_dd<1>(v, partial, counter, o);
 }
 
-__global__ void k_mul_into(const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out,
+__global__ void k_mul_into(const double* a, const double* b, double* out,
                            int64_t n) {
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) out[i] = a[i] * b[i];
 }
-__global__ void k_neg(double* __restrict__ a, int64_t n) {
+__global__ void k_neg(double* a, int64_t n) {
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) a[i] = -a[i];
 }
-__global__ void k_add(const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out, int64_t n) {
+__global__ void k_add(const double* a, const double* b, double* out, int64_t n) {
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) out[i] = a[i] + b[i];
@@ -191,8 +191,8 @@ __global__ void k_add(const double* __restrict__ a, const double* __restrict__ b
 // ---- inner PCG kernels (templated on the vector precision) --------------------
 // x += alpha p; r -= alpha Ap; alpha = scal[rz]/scal[pAp]; ||r||^2 -> scal[S_IRR]
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_pcg_update(T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
-                                                             const T* __restrict__ Ap, int64_t n, double* scal, int rz_slot,
+__global__ void __launch_bounds__(kRedThreads) k_pcg_update(T* x, T* r, const T* p,
+                                                             const T* Ap, int64_t n, double* scal, int rz_slot,
                                                              double* partial, unsigned int* counter) {
   grid_dep_wait();
   const double pap = scal[S_PAP];
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_update(T* __restrict__ x, T
 
 // p = z + beta p, beta = scal[new]/scal[old]
 template <typename T>
-__global__ void k_pcg_dir(T* __restrict__ p, const T* __restrict__ z, int64_t n, const double* scal, int new_slot,
+__global__ void k_pcg_dir(T* p, const T* z, int64_t n, const double* scal, int new_slot,
                           int old_slot) {
   grid_dep_wait();
   const double beta = scal[new_slot] / scal[old_slot];
@@ -220,12 +220,12 @@ __global__ void k_pcg_dir(T* __restrict__ p, const T* __restrict__ z, int64_t n,
 }
 
 
-__global__ void k_f32_to_f64(const float* __restrict__ a, double* __restrict__ b, int64_t n) {
+__global__ void k_f32_to_f64(const float* a, double* b, int64_t n) {
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) b[i] = (double)a[i];
 }
-__global__ void k_bj_host_mixed(const float* __restrict__ dinv, const double* __restrict__ r, double* __restrict__ z,
+__global__ void k_bj_host_mixed(const float* __restrict__ dinv, const double* r, double* z,
                                 int64_t nnod) {
   grid_dep_wait();
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -237,18 +237,18 @@ __global__ void k_bj_host_mixed(const float* __restrict__ dinv, const double* __
 }
 
 template <typename T>
-__global__ void k_scale_copy(const double* __restrict__ a, T* __restrict__ b, double s, int64_t n) {
+__global__ void k_scale_copy(const double* a, T* b, double s, int64_t n) {
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) b[i] = (T)(s * a[i]);
 }
 template <typename T>
-__global__ void k_add_scaled(double* __restrict__ z, const T* __restrict__ e, double s, int64_t n) {
+__global__ void k_add_scaled(double* z, const T* e, double s, int64_t n) {
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) z[i] += s * (double)e[i];
 }
-__global__ void k_residual(const double* __restrict__ y, double* __restrict__ Kz, int64_t n) {  // Kz <- y - Kz
+__global__ void k_residual(const double* y, double* Kz, int64_t n) {  // Kz <- y - Kz
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) Kz[i] = y[i] - Kz[i];
@@ -384,7 +384,7 @@ int inner_solve(Ctx& c, const double* y, double* z, const SolveCfg& cfg, InnerSt
 
 // ---- rigid-rotation removal ----------------------------------------------------
 // per element: sum_ip (N . V_el) * r_ip * detJ * w_ip with V = Uth*rho (am) and r*rho (mom)
-__global__ void __launch_bounds__(kRedThreads) k_rot_integrals(const double* __restrict__ U, const double* __restrict__ rho,
+__global__ void __launch_bounds__(kRedThreads) k_rot_integrals(const double* U, const double* __restrict__ rho,
                                                                 const double* __restrict__ th_lat,
                                                                 const double* __restrict__ r_lat, int nel, int ncr, int A,
                                                                 int B, double* scal, double* partial,
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kRedThreads) k_rot_integrals(const double* __r
   grid_finish_dd<2>(v, partial, counter, o);
 }
 
-__global__ void k_rot_remove(double* __restrict__ U, const double* __restrict__ r_lat, int64_t nnod, const double* scal) {
+__global__ void k_rot_remove(double* U, const double* __restrict__ r_lat, int64_t nnod, const double* scal) {
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= nnod) return;
@@ -429,7 +429,7 @@ __global__ void k_rot_remove(double* __restrict__ U, const double* __restrict__ 
 }
 
 // U_cart = TT U per node: [c s; -s c] (StokesSolver.jl:159, :214-241)
-__global__ void k_to_cartesian(const double* __restrict__ U, const double* __restrict__ th, double* __restrict__ Uc,
+__global__ void k_to_cartesian(const double* U, const double* __restrict__ th, double* Uc,
                                int64_t nnod) {
   grid_dep_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(128) k_th_assemble(ThAsmArgs p) {
 // q += A p over elements (q zeroed by the caller)
 __global__ void __launch_bounds__(128) k_th_apply(const double* __restrict__ Ae, const double* __restrict__ x,
                                                   double* __restrict__ y, int nel, int ncr, int64_t A, int64_t B) {
-  grid_dep_wait();
+  grid_dep_sync();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nel) return;
   double a[kThPack];
@@ -203,14 +203,14 @@ __global__ void __launch_bounds__(kRedThreads) k_th_init(const double* __restric
 
 // sets the loop's condition before its first pass
 __global__ void k_th_start(cudaGraphConditionalHandle h, const double* scal) {
-  grid_dep_wait();
+  grid_dep_sync();
   cudaGraphSetConditional(h, (scal[TH_RR] > scal[TH_TOL2] && scal[TH_ITMAX] >= 1.0) ? 1u : 0u);
 }
 
 __global__ void __launch_bounds__(kRedThreads) k_th_pq(const double* __restrict__ pv, const double* __restrict__ q,
                                                        int64_t n, double* scal, double* partial,
                                                        unsigned int* counter) {
-  grid_dep_wait();
+  grid_dep_sync();
   double v[1] = {0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     v[0] += pv[i] * q[i];
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kRedThreads) k_th_update(double* __restrict__ 
                                                            const double* __restrict__ diag, int64_t n, int64_t A,
                                                            int amax, int heated, double* scal, double* partial,
                                                            unsigned int* counter, cudaGraphConditionalHandle h) {
-  grid_dep_wait();
+  grid_dep_sync();
   const double alpha = scal[TH_ALPHA];
   double v[2] = {0.0, 0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kRedThreads) k_th_update(double* __restrict__ 
 
 __global__ void k_th_dir(double* __restrict__ pv, double* __restrict__ q, const double* __restrict__ z, int64_t n,
                          const double* scal) {
-  grid_dep_wait();
+  grid_dep_sync();
   const double beta = scal[TH_BETA];
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) {

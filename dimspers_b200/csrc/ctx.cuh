@@ -75,6 +75,7 @@ struct MGLevel {
   double lmax = 0.0;         // estimate of lambda_max(D^-1 A)
   int degree = 3;            // Chebyshev steps on this level
   double* cheb = nullptr;    // device: [1/theta, -, (c1, c2) per further step]
+  void* S = nullptr;         // node stencils (stencil.cu), level precision; null: element form
   // work vectors (precision of the hierarchy)
   void* x = nullptr;
   void* b = nullptr;

@@ -3,6 +3,7 @@
 // device code.
 #include "assemble.cu"
 #include "ops.cu"
+#include "stencil.cu"
 #include "mg.cu"
 #include "mgtail.cu"
 #include "solver.cu"

@@ -295,7 +295,7 @@ __device__ inline void fine_node_weights(int a, int b, int ncrc, int Ac, int Bc,
 }
 
 // xf += P xc (per fine node, gather); also sets rf = bf (the fine level's
-// residual buffer, from which the next apply subtracts A xf)
+// residual buffer, from which the next apply subtracts A xf) unless rf is null
 template <typename T>
 __global__ void k_prolong_add(const T* xc, T* xf, const T* bf,
                               T* rf, int Af, int Bf, int ncrc, int Ac, int Bc, int pin) {
@@ -315,7 +315,8 @@ __global__ void k_prolong_add(const T* xc, T* xf, const T* bf,
 #pragma unroll
   for (int k = 0; k < 6; ++k) v[k] = xc2[cn[k]];
   X2 xv = reinterpret_cast<const X2*>(xf)[n];
-  const X2 bv = reinterpret_cast<const X2*>(bf)[n];
+  X2 bv = xv;
+  if (rf) bv = reinterpret_cast<const X2*>(bf)[n];
   T s0 = (T)0, s1 = (T)0;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
@@ -325,7 +326,7 @@ __global__ void k_prolong_add(const T* xc, T* xf, const T* bf,
   if (!dof_fixed(a, b, 0, Af - 1, pin)) xv.x += s0;
   if (!dof_fixed(a, b, 1, Af - 1, pin)) xv.y += s1;
   reinterpret_cast<X2*>(xf)[n] = xv;
-  reinterpret_cast<X2*>(rf)[n] = bv;
+  if (rf) reinterpret_cast<X2*>(rf)[n] = bv;
 }
 
 // bc = P^T (r - t) per coarse node (t = null: P^T r; gather over the class
@@ -496,18 +497,6 @@ __global__ void __launch_bounds__(256) k_restrict_tile(const T* r, const T* t,
 // The three kernels compute in the precision of the level (FP32 on the FP32
 // hierarchy) and move each node's pair of components with one 8/16-byte
 // access, all loads issued before the arithmetic.
-template <typename T>
-struct NodeInv {
-  T a, b, c;
-  // D^-1 is constant during a solve: the steps fetch it before their wait
-  __device__ __forceinline__ NodeInv(const T* __restrict__ dinv, int64_t n)
-      : a(ld_early(dinv + 3 * n)), b(ld_early(dinv + 3 * n + 1)), c(ld_early(dinv + 3 * n + 2)) {}
-  __device__ __forceinline__ void apply(T r0, T r1, T& z0, T& z1) const {
-    z0 = a * r0 + b * r1;
-    z1 = b * r0 + c * r1;
-  }
-};
-
 // first step from x = 0: r = b, d = (1/theta) D^-1 b, x = d
 template <typename T>
 __global__ void k_cheb_first(const T* b, const T* __restrict__ dinv, T* x,
@@ -774,7 +763,7 @@ void mg_free(Ctx& c) {
     MGLevel& L = c.mg[l];
     if (l > 0) { cudaFree(L.K64); cudaFree(L.K32); }
     cudaFree(L.dinv64); cudaFree(L.dinv32); cudaFree(L.cheb);
-    cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.d); cudaFree(L.t);
+    cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.d); cudaFree(L.t); cudaFree(L.S);
   }
   c.mg.clear();
   cudaFree(c.coarse_inv);
@@ -952,6 +941,8 @@ static void mg_setup_t(Ctx& c, const MGOptions& o) {
       DP_CUDA(cudaMalloc(prec ? (void**)&L.dinv32 : (void**)&L.dinv64, sizeof(T) * 3 * L.g.nnod));
       DP_CUDA(cudaMalloc(&L.cheb, sizeof(double) * 2 * (kMaxCheb + 1)));
       setup_level_vectors<T>(L);
+      if (l + 1 < c.mg.size() && L.g.nnod <= kStencilMaxNodes)
+        DP_CUDA(cudaMalloc(&L.S, sizeof(T) * stencil_store<T>(L.g.ncr, L.g.nct)));
     }
     c.coarse_n = 2 * c.mg.back().g.nnod;
     if (c.coarse_n <= o.coarse_max) {
@@ -986,6 +977,8 @@ static void mg_setup_t(Ctx& c, const MGOptions& o) {
                                                                       Lc.g.pin);
     DP_LAUNCH_CHECK();
   }
+  for (MGLevel& L : c.mg)
+    if (L.S) launch_stencil_assemble<T>(L.g, level_K<T>(L), (T*)L.S, c.stream);
   // nodal diagonal blocks, eigenvalue estimates and Chebyshev coefficients
   double* diag = nullptr;
   DP_CUDA(cudaMalloc(&diag, sizeof(double) * 3 * c.mg[0].g.nnod));
@@ -1070,6 +1063,40 @@ void mg_setup(Ctx& c, int precision, const MGOptions& o) {
   else mg_setup_t<double>(c, o);
 }
 
+// Levels whose smoother runs on node stencils: those that have them, except
+// with one Chebyshev step (the deferred x update below needs a second one) and
+// with a matrix-free fine level.
+static bool stencil_level(const Ctx& c, const MGLevel& L) {
+  return L.S && L.degree >= 2 && !(&L == &c.mg[0] && (L.g.mfD64 || L.g.mfD32));
+}
+
+// Chebyshev smoothing on node stencils (same recurrence and modes as
+// chebyshev(), r read from b in mode 2).  d alternates between L.d and L.t: a
+// step gathers the old d from neighbours that other threads are replacing.  In
+// mode 2 the first step gathers x, so x gains d_1 together with d_2.
+// Pre-smoothing (modes 0, 1) ends with r = b - A x, the true residual.
+template <typename T>
+static void chebyshev_stencil(Ctx& c, MGLevel& L, const T* b, T* x, int mode) {
+  T* r = (T*)L.r;
+  T* d = (T*)L.d;
+  T* dn = (T*)L.t;
+  const T* S = (const T*)L.S;
+  const T* dinv = level_dinv<T>(L);
+  const T* none = nullptr;
+  if (mode == 0) klaunch(k_cheb_first<T>, tpb(L.g.nnod), 256, 0, c.stream, b, dinv, x, r, d, L.cheb, L.g.nnod);
+  if (mode == 2) launch_stencil_step<ST_FIRST_X, T>(L.g, S, x, b, r, (T*)nullptr, d, dinv, L.cheb, c.stream);
+  for (int k = 1; k < L.degree; ++k) {
+    if (mode == 2 && k == 1)
+      launch_stencil_step<ST_STEP_X, T>(L.g, S, d, none, r, x, dn, dinv, L.cheb + 2 * k, c.stream);
+    else
+      launch_stencil_step<ST_STEP, T>(L.g, S, d, none, r, x, dn, dinv, L.cheb + 2 * k, c.stream);
+    std::swap(d, dn);
+  }
+  if (mode != 2)
+    launch_stencil_step<ST_RESIDUAL, T>(L.g, S, d, none, r, (T*)nullptr, (T*)nullptr, dinv, L.cheb, c.stream);
+  DP_LAUNCH_CHECK();
+}
+
 // Chebyshev smoothing of A x = b on level L.  mode 0: start from x = 0;
 // mode 1: start from x = 0 with the first step already taken (fused into the
 // restriction that produced b); mode 2: start from the given x, with L.r
@@ -1079,6 +1106,10 @@ void mg_setup(Ctx& c, int precision, const MGOptions& o) {
 // On exit r = b - A (x - d_last), i.e. the true residual is r - A d_last.
 template <typename T>
 static void chebyshev(Ctx& c, MGLevel& L, const T* b, T* x, int mode) {
+  if (stencil_level(c, L)) {
+    chebyshev_stencil<T>(c, L, b, x, mode);
+    return;
+  }
   const int64_t nn = L.g.nnod;
   T* r = (T*)L.r; T* d = (T*)L.d;
   const T* dinv = level_dinv<T>(L);
@@ -1127,8 +1158,9 @@ static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool 
   // pre-smoothing, r -= A d_last (the true residual), then restrict it (and take
   // the coarse level's first smoothing step in the same pass unless it is
   // solved densely)
+  const bool st = stencil_level(c, L);   // its pre-smoothing leaves the true residual in r
   chebyshev<T>(c, L, b, x, first_done ? 1 : 0);
-  launch_apply_K_sub<T, T>(L.g, level_K<T>(L), (const T*)L.d, r, c.stream);
+  if (!st) launch_apply_K_sub<T, T>(L.g, level_K<T>(L), (const T*)L.d, r, c.stream);
   const bool fuse = !(l + 2 == c.mg.size() && dense_coarsest);
   // the cluster tail's smoother accumulates A d into t, which starts at zero
   T* tc = (l + 1 == tail_start(c, o)) ? (T*)C.t : nullptr;
@@ -1148,8 +1180,8 @@ static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool 
   }
   DP_LAUNCH_CHECK();
   vcycle<T>(c, l + 1, bc, xc, o, fuse);
-  klaunch(k_prolong_add<T>, tpb(L.g.nnod), 256, 0, c.stream, (const T*)xc, x, b, r, (int)L.g.A(), (int)L.g.B(),
-          C.g.ncr, (int)C.g.A(), (int)C.g.B(), L.g.pin);
+  klaunch(k_prolong_add<T>, tpb(L.g.nnod), 256, 0, c.stream, (const T*)xc, x, b, st ? (T*)nullptr : r, (int)L.g.A(),
+          (int)L.g.B(), C.g.ncr, (int)C.g.A(), (int)C.g.B(), L.g.pin);
   DP_LAUNCH_CHECK();
   chebyshev<T>(c, L, b, x, 2);
 }

@@ -5,6 +5,12 @@
 namespace dp {
 
 constexpr int kMaxCheb = 8;
+// Largest level (lattice nodes) whose smoother runs on node stencils: the
+// 32x256 level (33,280 nodes) and below.  Per inner iteration of the whole
+// solve: 16x128 FP64 80.7 -> 67.5 us, 32x256 103 -> 92.8 us.  Including the
+// 64x512 level (132k nodes, 24 MB of stencils) measured 145 against 140.5 us
+// at 64x512 and no change at 128x1024: there the bytes count, not the launches.
+constexpr int64_t kStencilMaxNodes = 40000;
 
 struct MGOptions {
   int cheb_degree = 3;      // Chebyshev steps per smoothing (each one A-apply)

@@ -449,7 +449,7 @@ void launch_assemble(Ctx& c, int precision, const CartOut* cart) {
   ++g_klaunch;
   k_assemble<<<grid, kAsmThreads, smem, c.stream>>>(a);
   DP_LAUNCH_CHECK();
-  if (a.Fe) launch_node_gather<double>(L, a.Fe, c.F, 2, 2, c.stream);
+  if (a.Fe) launch_node_gather<double>(L, a.Fe, c.F, 2, c.stream);
   if (c.mfT64) {
     ++g_klaunch;
     k_mf_table<<<(int)div_up(2 * L.ncr, 64), 64, 0, c.stream>>>(L.ncr, (int)L.A(), c.theta_lat, c.r_lat, c.mfT64);

@@ -31,7 +31,7 @@ constexpr int kKe = 78;   // packed lower 12x12
 constexpr int kGe = 36;   // 12x3 column-major
 constexpr int kMe = 6;    // packed lower 3x3
 constexpr int kFe = 12;
-constexpr int kDetPerElem = 18;  // deterministic scratch per element: 6 nodes x up to 3 values
+constexpr int kDetPerElem = 12;  // deterministic scratch per element: 6 nodes x 2 values
 constexpr int kMfTab = 84;  // per ring of the matrix-free apply: 6 IPs x (6 dN/dx, 6 dN/dz), 6 x (cos, sin)
 
 enum MatKind { MAT_NONE = 0, MAT_ISO = 1, MAT_FULL = 2, MAT_TI = 3 };
@@ -72,9 +72,8 @@ struct MGLevel {
   float* K32 = nullptr;
   double* dinv64 = nullptr;  // 3*nnod inverse of the 2x2 nodal diagonal blocks (i00, i01, i11)
   float* dinv32 = nullptr;
-  double lmax = 0.0;         // estimate of lambda_max(D^-1 A)
   int degree = 3;            // Chebyshev steps on this level
-  double* cheb = nullptr;    // device: [1/theta, -, (c1, c2) per further step]
+  double* cheb = nullptr;    // device: [1/theta, -, (c1, c2) per further step], then the Lanczos scalars
   void* S = nullptr;         // node stencils (stencil.cu), level precision; null: element form
   // work vectors (precision of the hierarchy)
   void* x = nullptr;
@@ -138,7 +137,7 @@ struct Ctx {
   int mg_degree = 3;            // Chebyshev steps in use
   int64_t mg_coarse_max = -1;   // coarse_max the hierarchy was built for
   int64_t alloc_gen = 0;        // bumped whenever buffers a captured graph may hold are freed
-  double* coarse_inv = nullptr; // coarsest level: work matrix, then its dense inverse (2 n^2)
+  double* coarse_inv = nullptr; // coarsest level: work matrix, its dense inverse (2 n^2), panel inverses
   int64_t coarse_n = 0;
   int64_t* coarse_map = nullptr;// coarsest DOF -> dense index (-1 fixed)
 

@@ -149,115 +149,180 @@ void upload_mg_constants() {
   upload_restriction_table();
 }
 
-// ---- Galerkin coarsening: one thread per (coarse element, packed entry) ------
+// ---- Galerkin coarsening ---------------------------------------------------------
+// K_E = sum over the 4 children of P_f^T K_f P_f, sums in FP64.  A CTA takes 32
+// consecutive coarse cells: the 8 fine elements of each are copied to shared
+// memory once (coalesced, 16-byte groups as they are stored), then each of the
+// 12 warps owns one (coarse type, coarse node l), its lanes the 32 cells: the
+// two columns of node l of K_f P are summed over the packed entries with the
+// 6 weights P[.][l] in registers, then P^T is applied to them.  The coarse
+// elements leave through shared memory as coalesced 16-byte groups.
+// Bound by FP64 FMA and FP32 -> FP64 conversion (6.9 k FMA a coarse element).
+// The form it replaces, a thread per (coarse element, entry), re-read each
+// child entry ~36 times: 10.55 ms for the first coarsening at 512x4096.
 template <typename T>
-__global__ void k_galerkin(const T* __restrict__ Kf, T* __restrict__ Kc, int nelc, int ncrc, int nctc, int nelf,
-                           int ncrf, int pin) {
+struct GalerkinTile {
+  static constexpr int kVec = KVec<T>::n;            // 16-byte groups per element
+  static constexpr int kPer = 16 / sizeof(T);
+  static constexpr int kSlot = kVec * 32 + 2;        // groups per fine slot; +2 keeps the copy free of bank conflicts
+  static constexpr size_t kSmem = 16 * (size_t)(8 * kSlot + 2 * kVec * 32);
+};
+constexpr int kGalThreads = 384;   // 12 warps: (type, node)
+
+template <typename T>
+__global__ void __launch_bounds__(kGalThreads) k_galerkin(const T* __restrict__ Kf, T* __restrict__ Kc, int ncrc,
+                                                          int nctc, int ncrf, int pin) {
+  typedef GalerkinTile<T> G;
+  typedef typename KVec<T>::V VT;
   grid_dep_wait();
-  const int64_t gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (gid >= (int64_t)nelc * kKe) return;
-  const int E = (int)(gid % nelc);
-  const int pidx = (int)(gid / nelc);
-  // decode packed index -> (R, C)
-  int C = 0, off = 0;
-  while (off + (12 - C) <= pidx) { off += 12 - C; ++C; }
-  const int R = C + (pidx - off);
-  const int k = R >> 1, alpha = R & 1, l = C >> 1, beta = C & 1;
-  const int Q = E >> 1, ct = E & 1;
-  const int IR = Q % ncrc, IT = Q / ncrc;
-  double acc = 0.0;
-#pragma unroll
-  for (int ch = 0; ch < 4; ++ch) {
-    const int fr = 2 * IR + c_child.dr[ct][ch], ft = 2 * IT + c_child.dt[ct][ch];
-    const int ef = 2 * (fr + ncrf * ft) + c_child.tf[ct][ch];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const double pik = c_child.P[ct][ch][i][k];
-      if (pik == 0.0) continue;
-      double s = 0.0;
-#pragma unroll
-      for (int j = 0; j < 6; ++j) {
-        const double pjl = c_child.P[ct][ch][j][l];
-        if (pjl == 0.0) continue;
-        const int r = 2 * i + alpha, cc = 2 * j + beta;
-        const int pi = r >= cc ? packed_index12(r, cc) : packed_index12(cc, r);
-        s += pjl * (double)Kf[kidx<T>(pi, ef)];
-      }
-      acc += pik * s;
+  extern __shared__ __align__(16) unsigned char gal_raw[];
+  VT* in = reinterpret_cast<VT*>(gal_raw);          // [fine slot 4 dt + 2 dr + tf][group][cell]
+  VT* out = in + 8 * G::kSlot;                      // [type][group][cell]
+  const int ncell = ncrc * nctc, q0 = blockIdx.x * 32;
+  for (int idx = threadIdx.x; idx < 8 * 32 * G::kVec; idx += kGalThreads) {
+    const int el4 = idx & 127, rest = idx >> 7;      // 4 consecutive fine elements per cell and angular row
+    const int j = rest % G::kVec, dt = rest / G::kVec;
+    const int cell = el4 >> 2, Q = q0 + cell;
+    if (Q < ncell) {
+      const int IR = Q % ncrc, IT = Q / ncrc;
+      const int64_t e = 4 * (int64_t)IR + (el4 & 3) + 2 * (int64_t)ncrf * (2 * IT + dt);
+      in[(4 * dt + (el4 & 3)) * G::kSlot + j * 32 + cell] =
+          reinterpret_cast<const VT*>(Kf)[(e >> 5) * (32 * G::kVec) + j * 32 + (e & 31)];
     }
   }
-  // coarse constraint mask (free slip + optional tangential pin)
-  const int a0 = 2 * IR, b0 = 2 * IT, Bc = 2 * nctc;
-  const int ak = a0 + kLocA_dev(ct, k), al = a0 + kLocA_dev(ct, l);
-  int bk = b0 + kLocB_dev(ct, k), bl = b0 + kLocB_dev(ct, l);
-  if (bk >= Bc) bk -= Bc;
-  if (bl >= Bc) bl -= Bc;
-  const int amax = 2 * ncrc;
-  if (dof_fixed(ak, bk, alpha, amax, pin) || dof_fixed(al, bl, beta, amax, pin)) acc = 0.0;
-  Kc[kidx<T>(pidx, E)] = (T)acc;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int ct = w / 6, l = w - 6 * ct;
+  const int Q = q0 + lane;
+  if (Q < ncell) {
+    double acc[6][2][2];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) acc[k][0][0] = acc[k][0][1] = acc[k][1][0] = acc[k][1][1] = 0.0;
+#pragma unroll 1
+    for (int ch = 0; ch < 4; ++ch) {
+      const VT* src = in + (4 * c_child.dt[ct][ch] + 2 * c_child.dr[ct][ch] + c_child.tf[ct][ch]) * G::kSlot + lane;
+      double wl[6], s[6][2][2];   // wl = P[.][l]; s[i] = the 2x2 block (row node i, column node l) of K_f P
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        wl[i] = c_child.P[ct][ch][i][l];
+        s[i][0][0] = s[i][0][1] = s[i][1][0] = s[i][1][1] = 0.0;
+      }
+#pragma unroll
+      for (int C = 0; C < 12; ++C) {
+#pragma unroll
+        for (int R = C; R < 12; ++R) {
+          const int p = packed_index12(R, C);
+          T kk[G::kPer];
+          vec_to(src[(p / G::kPer) * 32], kk);
+          const double v = (double)kk[p % G::kPer];
+          s[R >> 1][R & 1][C & 1] += v * wl[C >> 1];
+          if (R != C) s[C >> 1][C & 1][R & 1] += v * wl[R >> 1];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+          const double pik = c_child.P[ct][ch][i][k];
+          if (pik == 0.0) continue;   // the same for the whole warp
+          acc[k][0][0] += pik * s[i][0][0];
+          acc[k][0][1] += pik * s[i][0][1];
+          acc[k][1][0] += pik * s[i][1][0];
+          acc[k][1][1] += pik * s[i][1][1];
+        }
+      }
+    }
+    // coarse constraint mask (free slip + optional tangential pin)
+    const int IR = Q % ncrc, IT = Q / ncrc, Bc = 2 * nctc, amax = 2 * ncrc;
+    auto fixed = [&](int k, int comp) {
+      int b = 2 * IT + kLocB_dev(ct, k);
+      if (b >= Bc) b -= Bc;
+      return dof_fixed(2 * IR + kLocA_dev(ct, k), b, comp, amax, pin);
+    };
+    T* o = reinterpret_cast<T*>(out + (size_t)ct * G::kVec * 32 + lane);
+    const bool fl[2] = {fixed(l, 0), fixed(l, 1)};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      if (k < l) continue;
+      const bool fk[2] = {fixed(k, 0), fixed(k, 1)};
+#pragma unroll
+      for (int al = 0; al < 2; ++al) {
+#pragma unroll
+        for (int be = 0; be < 2; ++be) {
+          if (k == l && al < be) continue;
+          const int p = packed_index12(2 * k + al, 2 * l + be);
+          o[(size_t)(p / G::kPer) * 32 * G::kPer + p % G::kPer] = (T)(fk[al] || fl[be] ? 0.0 : acc[k][al][be]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < 2 * 32 * G::kVec; idx += kGalThreads) {
+    const int el2 = idx & 63, j = idx >> 6, cell = el2 >> 1;
+    if (q0 + cell < ncell) {
+      const int64_t E = 2 * (int64_t)q0 + el2;
+      reinterpret_cast<VT*>(Kc)[(E >> 5) * (32 * G::kVec) + j * 32 + (E & 31)] =
+          out[(el2 & 1) * G::kVec * 32 + j * 32 + cell];
+    }
+  }
 }
 
 // ---- nodal 2x2 diagonal blocks and their inverses ----------------------------
-template <typename T>
-__global__ void k_diag_blocks(const T* __restrict__ K, double* __restrict__ diag, int nel, int ncr, int A, int B) {
-  grid_dep_wait();
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nel) return;
-  int nd[6];
-  element_nodes_mg(e, ncr, A, B, nd);
+// Per node: the sum of its 2x2 diagonal blocks over the elements that hold it (a
+// gather in a fixed order, no atomics and no buffer of sums) and the inverse of
+// that block (block = 1) or of its diagonal (block = 0).  Constrained DOFs get
+// zero rows/columns so the smoother never touches them.  One thread per 2x2
+// node block, one node of each parity class, as in k_node_gather.
+template <int PA, int PB, typename T>
+__device__ __forceinline__ void diag_invert_node(const T* __restrict__ K, T* __restrict__ dinv, int i, int j, int ncr,
+                                                 int nct, int pin, int block) {
+  const int a = 2 * i + PA, b = 2 * j + PB;
+  if (a > 2 * ncr) return;
+  double d00 = 0.0, d01 = 0.0, d11 = 0.0;
 #pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    atomicAdd(&diag[3 * nd[k] + 0], (double)K[kidx<T>(packed_index12(2 * k, 2 * k), e)]);
-    atomicAdd(&diag[3 * nd[k] + 1], (double)K[kidx<T>(packed_index12(2 * k + 1, 2 * k), e)]);
-    atomicAdd(&diag[3 * nd[k] + 2], (double)K[kidx<T>(packed_index12(2 * k + 1, 2 * k + 1), e)]);
-  }
-}
-
-// Deterministic form: element e's three block entries at its local node k into
-// E[(3k + c) nel + e], summed per node by k_node_gather.
-template <typename T>
-__global__ void k_diag_blocks_elem(const T* __restrict__ K, double* __restrict__ E, int nel) {
-  grid_dep_wait();
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nel) return;
+  for (int t = 0; t < 2; ++t) {
 #pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    E[(size_t)(3 * k + 0) * nel + e] = (double)K[kidx<T>(packed_index12(2 * k, 2 * k), e)];
-    E[(size_t)(3 * k + 1) * nel + e] = (double)K[kidx<T>(packed_index12(2 * k + 1, 2 * k), e)];
-    E[(size_t)(3 * k + 2) * nel + e] = (double)K[kidx<T>(packed_index12(2 * k + 1, 2 * k + 1), e)];
+    for (int k = 0; k < 6; ++k) {
+      if ((loc_a(t, k) & 1) != PA || (loc_b(t, k) & 1) != PB) continue;   // resolved at compile time
+      const int ir = i + ((PA - loc_a(t, k)) >> 1);
+      int it = j + ((PB - loc_b(t, k)) >> 1);
+      if (ir < 0 || ir >= ncr) continue;
+      if (it < 0) it += nct;
+      const int64_t e = 2 * ((int64_t)ir + (int64_t)ncr * it) + t;
+      d00 += (double)K[kidx<T>(packed_index12(2 * k, 2 * k), e)];
+      d01 += (double)K[kidx<T>(packed_index12(2 * k + 1, 2 * k), e)];
+      d11 += (double)K[kidx<T>(packed_index12(2 * k + 1, 2 * k + 1), e)];
+    }
   }
-}
-
-// Inverse of the nodal block (block = 1) or of its diagonal (block = 0);
-// constrained DOFs get zero rows/columns so the smoother never touches them.
-template <typename T>
-__global__ void k_block_invert(const double* __restrict__ diag, T* __restrict__ dinv, int64_t nnod, int A, int pin,
-                               int block) {
-  grid_dep_wait();
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n >= nnod) return;
-  const int a = (int)(n % A), b = (int)(n / A);
-  const bool f0 = dof_fixed(a, b, 0, A - 1, pin), f1 = dof_fixed(a, b, 1, A - 1, pin);
-  const double d00 = diag[3 * n], d11 = diag[3 * n + 2];
-  double d01 = block ? diag[3 * n + 1] : 0.0;
+  const bool f0 = dof_fixed(a, b, 0, 2 * ncr, pin), f1 = dof_fixed(a, b, 1, 2 * ncr, pin);
+  if (!block) d01 = 0.0;
   double i00 = 0.0, i01 = 0.0, i11 = 0.0;
-  if (f0 || f1 || d01 == 0.0) {
+  const double det = d00 * d11 - d01 * d01;
+  if (f0 || f1 || d01 == 0.0 || !(det > 0.0)) {
     i00 = (!f0 && d00 > 0.0) ? 1.0 / d00 : 0.0;
     i11 = (!f1 && d11 > 0.0) ? 1.0 / d11 : 0.0;
   } else {
-    const double det = d00 * d11 - d01 * d01;
-    if (det > 0.0) {
-      i00 = d11 / det;
-      i01 = -d01 / det;
-      i11 = d00 / det;
-    } else {
-      i00 = d00 > 0.0 ? 1.0 / d00 : 0.0;
-      i11 = d11 > 0.0 ? 1.0 / d11 : 0.0;
-    }
+    i00 = d11 / det;
+    i01 = -d01 / det;
+    i11 = d00 / det;
   }
-  dinv[3 * n] = (T)i00;
-  dinv[3 * n + 1] = (T)i01;
-  dinv[3 * n + 2] = (T)i11;
+  T* o = dinv + 3 * (a + (int64_t)(2 * ncr + 1) * b);
+  o[0] = (T)i00;
+  o[1] = (T)i01;
+  o[2] = (T)i11;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_diag_invert(const T* __restrict__ K, T* __restrict__ dinv, int ncr, int nct,
+                                                     int pin, int block) {
+  grid_dep_wait();
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (q >= (int64_t)(ncr + 1) * nct) return;
+  const int j = (int)(q / (ncr + 1)), i = (int)(q - (int64_t)j * (ncr + 1));
+  diag_invert_node<0, 0, T>(K, dinv, i, j, ncr, nct, pin, block);
+  diag_invert_node<1, 0, T>(K, dinv, i, j, ncr, nct, pin, block);
+  diag_invert_node<0, 1, T>(K, dinv, i, j, ncr, nct, pin, block);
+  diag_invert_node<1, 1, T>(K, dinv, i, j, ncr, nct, pin, block);
 }
 
 template <typename T>
@@ -574,50 +639,37 @@ __global__ void k_bj(const T* __restrict__ dinv, const T* r, T* z, int64_t nnod)
 }
 
 // ---- coarse dense solve --------------------------------------------------------
-template <typename T>
-__global__ void k_dense_assemble(const T* __restrict__ K, double* __restrict__ D, int nel, int ncr, int A, int B, int n) {
-  grid_dep_wait();
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nel) return;
-  int nd[6];
-  element_nodes_mg(e, ncr, A, B, nd);
-  for (int C = 0; C < 12; ++C)
-    for (int R = C; R < 12; ++R) {
-      const double v = (double)K[kidx<T>(packed_index12(R, C), e)];
-      const int gr = 2 * nd[R >> 1] + (R & 1), gc = 2 * nd[C >> 1] + (C & 1);
-      atomicAdd(&D[(size_t)gr * n + gc], v);
-      if (R != C) atomicAdd(&D[(size_t)gc * n + gr], v);
-    }
+// The dense matrix row by row from the elements around each node (the gather of
+// the node stencils: every entry written once, in a fixed order).
+template <int C, int J, typename T>
+__device__ __forceinline__ void dense_entry(const T* __restrict__ K, double* D, int i, int ia, int jb, int ncr, int nct) {
+  constexpr int DA = StencilEntry<C, J>::da, DB = StencilEntry<C, J>::db;
+  const int A = 2 * ncr + 1, B = 2 * nct, a = 2 * ia + (C & 1), b = 2 * jb + (C >> 1);
+  if (a + DA < 0 || a + DA >= A) return;
+  double acc[4];
+  stencil_sum<C, J, T>(K, ia, jb, ncr, nct, acc);
+  int bm = b + DB;
+  bm += bm < 0 ? B : (bm >= B ? -B : 0);
+  const int64_t n = 2 * (int64_t)A * B, row = 2 * (a + (int64_t)A * b), col = 2 * (a + DA + (int64_t)A * bm);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) D[(row + (q >> 1)) * n + col + (q & 1)] = acc[q];
 }
-
-// Deterministic form: one CTA walks the elements in order, its threads taking
-// the 78 packed entries of one element at a time.  The entries of one element
-// land on distinct matrix positions (its 12 DOFs are distinct), so the threads
-// never collide, and every position receives its contributions in element
-// order.  The coarsest level has a few hundred elements.
+template <int C, typename T, int... J>
+__device__ __forceinline__ void dense_rows(const T* __restrict__ K, double* D, int i, int ncr, int nct,
+                                           std::integer_sequence<int, J...>) {
+  const int nA = (C & 1) ? ncr : ncr + 1;
+  const int ia = i % nA, jb = i / nA;
+  (dense_entry<C, J, T>(K, D, i, ia, jb, ncr, nct), ...);
+}
 template <typename T>
-__global__ void __launch_bounds__(128) k_dense_assemble_seq(const T* __restrict__ K, double* __restrict__ D, int nel,
-                                                            int ncr, int A, int B, int n) {
+__global__ void __launch_bounds__(64) k_dense_assemble(const T* __restrict__ K, double* D, int ncr, int nct) {
   grid_dep_wait();
-  const int i = threadIdx.x;
-  int R = 0, C = 0;
-  if (i < kKe) {   // packed entry i -> (R, C), R >= C, column-major lower triangle
-    int c0 = 0, rem = i;
-    while (rem >= 12 - c0) { rem -= 12 - c0; ++c0; }
-    C = c0;
-    R = c0 + rem;
-  }
-  for (int e = 0; e < nel; ++e) {
-    if (i < kKe) {
-      int nd[6];
-      element_nodes_mg(e, ncr, A, B, nd);
-      const double v = (double)K[kidx<T>(packed_index12(R, C), e)];
-      const int gr = 2 * nd[R >> 1] + (R & 1), gc = 2 * nd[C >> 1] + (C & 1);
-      D[(size_t)gr * n + gc] += v;
-      if (R != C) D[(size_t)gc * n + gr] += v;
-    }
-    __syncthreads();
-  }
+  const int c = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= st_nodes(c, ncr, nct)) return;
+  if (c == 0) dense_rows<0, T>(K, D, i, ncr, nct, std::make_integer_sequence<int, st_entries(0)>{});
+  else if (c == 1) dense_rows<1, T>(K, D, i, ncr, nct, std::make_integer_sequence<int, st_entries(1)>{});
+  else if (c == 2) dense_rows<2, T>(K, D, i, ncr, nct, std::make_integer_sequence<int, st_entries(2)>{});
+  else dense_rows<3, T>(K, D, i, ncr, nct, std::make_integer_sequence<int, st_entries(3)>{});
 }
 
 // Identity on the diagonal of fixed (all-zero) rows, so the matrix stays SPD.
@@ -632,9 +684,12 @@ __global__ void k_dense_fix_diag(double* __restrict__ D, int n) {
 // SPD matrix are SPD).  With W = A_KK^-1 and T = A_{:,K} W, the panel step maps A
 // (old) to B (new):
 //   B_KK = W,   B_Kj = W A_Kj,   B_iK = -T_iK,   B_ij = A_ij - T_iK A_Kj
-// (i, j outside K).  After all panels B = A^-1.  Three launches per panel: the
-// pivot-block inverse (one CTA, shared memory), T (one thread per (row, pivot))
-// and the update (one thread per entry, coalesced along rows, ping-pong buffers).
+// (i, j outside K).  After all panels B = A^-1.  One launch per panel: a CTA
+// forms T for its 64 rows, updates its 64x64 tile from the 32 pivot rows (all
+// in shared memory) and, if the tile holds the next pivot block, inverts that
+// for the next launch while the other tiles are still at work.
+// At n = 1152 a panel took 47 us as three launches with every entry's 64
+// operands read through L1.
 constexpr int kGJPanel = 32;
 
 __global__ void __launch_bounds__(kGJPanel * kGJPanel) k_gj_panel_inverse(const double* __restrict__ A,
@@ -659,53 +714,118 @@ __global__ void __launch_bounds__(kGJPanel * kGJPanel) k_gj_panel_inverse(const 
   W[r * kGJPanel + c] = s[r][c];
 }
 
-// T[i][m] = sum_l A[i][k0 + l] W[l][m]  (i < n, m < b; row stride kGJPanel)
-__global__ void k_gj_panel_cols(const double* __restrict__ A, const double* __restrict__ W, double* __restrict__ T,
-                                int n, int k0, int b) {
-  grid_dep_wait();
-  const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)n * kGJPanel) return;
-  const int i = (int)(idx / kGJPanel), m = (int)(idx % kGJPanel);
-  double t = 0.0;
-  if (m < b)
-    for (int l = 0; l < b; ++l) t += A[(size_t)i * n + k0 + l] * W[l * kGJPanel + m];
-  T[idx] = t;
-}
+constexpr int kGJTile = 64;
+constexpr size_t kGJSmem = sizeof(double) * (kGJPanel * kGJPanel + 2 * kGJTile * (kGJPanel + 1) +
+                                             kGJPanel * kGJTile + 2 * kGJPanel * (kGJPanel + 1));
 
-__global__ void k_gj_panel_update(const double* __restrict__ A, double* __restrict__ B, const double* __restrict__ W,
-                                  const double* __restrict__ T, int n, int k0, int b) {
+__global__ void __launch_bounds__(256) k_gj_panel(const double* A, double* B, const double* W, double* Wn, int n,
+                                                  int k0) {
   grid_dep_wait();
-  const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)n * n) return;
-  const int i = (int)(idx / n), j = (int)(idx % n);
-  const bool ik = i >= k0 && i < k0 + b, jk = j >= k0 && j < k0 + b;
-  double v;
-  if (ik && jk) {
-    v = W[(i - k0) * kGJPanel + (j - k0)];
-  } else if (ik) {
-    v = 0.0;
-    for (int m = 0; m < b; ++m) v += W[(i - k0) * kGJPanel + m] * A[(size_t)(k0 + m) * n + j];
-  } else if (jk) {
-    v = -T[(size_t)i * kGJPanel + (j - k0)];
-  } else {
-    v = A[idx];
-    for (int m = 0; m < b; ++m) v -= T[(size_t)i * kGJPanel + m] * A[(size_t)(k0 + m) * n + j];
+  extern __shared__ __align__(16) double gj[];
+  double(*sw)[kGJPanel] = reinterpret_cast<double(*)[kGJPanel]>(gj);
+  double(*sa)[kGJPanel + 1] = reinterpret_cast<double(*)[kGJPanel + 1]>(gj + kGJPanel * kGJPanel);
+  double(*st)[kGJPanel + 1] = sa + kGJTile;
+  double(*sb)[kGJTile] = reinterpret_cast<double(*)[kGJTile]>(&st[kGJTile][0]);
+  double(*sp)[kGJPanel][kGJPanel + 1] = reinterpret_cast<double(*)[kGJPanel][kGJPanel + 1]>(&sb[kGJPanel][0]);
+  const int i0 = blockIdx.y * kGJTile, j0 = blockIdx.x * kGJTile, b = min(kGJPanel, n - k0);
+  for (int q = threadIdx.x; q < kGJPanel * kGJPanel; q += 256) sw[q / kGJPanel][q % kGJPanel] = W[q];
+  for (int q = threadIdx.x; q < kGJTile * kGJPanel; q += 256) {
+    const int r = q / kGJPanel, m = q % kGJPanel;
+    sa[r][m] = (i0 + r < n && m < b) ? A[(size_t)(i0 + r) * n + k0 + m] : 0.0;
   }
-  B[idx] = v;
+  for (int q = threadIdx.x; q < kGJPanel * kGJTile; q += 256) {
+    const int m = q / kGJTile, c = q % kGJTile;
+    sb[m][c] = (j0 + c < n && m < b) ? A[(size_t)(k0 + m) * n + j0 + c] : 0.0;
+  }
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  double v[4][4];   // rows ty + 16 r, columns tx + 16 c of the tile; the rows of K start from zero
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = i0 + ty + 16 * r, j = j0 + tx + 16 * c;
+      const bool ik = i >= k0 && i < k0 + b;
+      v[r][c] = (i < n && j < n && !ik) ? A[(size_t)i * n + j] : 0.0;
+    }
+  __syncthreads();
+  // T rows (-W for the rows of K, which turns the update below into W A_Kj)
+  for (int q = threadIdx.x; q < kGJTile * kGJPanel; q += 256) {
+    const int r = q / kGJPanel, m = q % kGJPanel, i = i0 + r;
+    double t = 0.0;
+    if (i >= k0 && i < k0 + b) {
+      t = -sw[i - k0][m];
+    } else {
+#pragma unroll 8
+      for (int l = 0; l < kGJPanel; ++l) t += sa[r][l] * sw[l][m];
+    }
+    st[r][m] = m < b ? t : 0.0;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int m = 0; m < kGJPanel; ++m) {
+    double t[4], p[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) t[r] = st[ty + 16 * r][m];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) p[c] = sb[m][tx + 16 * c];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) v[r][c] -= t[r] * p[c];
+  }
+  const int k1 = k0 + kGJPanel;   // next pivot block; 32 divides 64, so it lies in one tile
+  const int bn = min(kGJPanel, n - k1);
+  const bool next = bn > 0 && i0 == k1 / kGJTile * kGJTile && j0 == i0;
+  const int off = k1 - i0;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = i0 + ty + 16 * r, j = j0 + tx + 16 * c;
+      if (j >= k0 && j < k0 + b) v[r][c] = -st[ty + 16 * r][j - k0];
+      if (i < n && j < n) B[(size_t)i * n + j] = v[r][c];
+      if (next) {
+        const int pr = ty + 16 * r - off, pc = tx + 16 * c - off;
+        if (pr >= 0 && pr < kGJPanel && pc >= 0 && pc < kGJPanel)
+          sp[0][pr][pc] = (pr < bn && pc < bn) ? v[r][c] : (pr == pc ? 1.0 : 0.0);
+      }
+    }
+  if (!next) return;   // the same for the whole CTA
+  __syncthreads();
+  // Gauss-Jordan on the 32x32 block, ping-pong between two copies
+  for (int k = 0; k < kGJPanel; ++k) {
+    const double(*o)[kGJPanel + 1] = sp[k & 1];
+    double(*w)[kGJPanel + 1] = sp[(k & 1) ^ 1];
+    const double ip = 1.0 / o[k][k];
+#pragma unroll
+    for (int q = threadIdx.x; q < kGJPanel * kGJPanel; q += 256) {
+      const int r = q / kGJPanel, c = q % kGJPanel;
+      double x;
+      if (r == k) x = (c == k) ? ip : o[k][c] * ip;
+      else if (c == k) x = -o[r][k] * ip;
+      else x = o[r][c] - o[r][k] * o[k][c] * ip;
+      w[r][c] = x;
+    }
+    __syncthreads();
+  }
+  for (int q = threadIdx.x; q < kGJPanel * kGJPanel; q += 256) Wn[q] = sp[0][q / kGJPanel][q % kGJPanel];
 }
 
-// A = (A + A^T) / 2 in place (one thread per pair i < j): the inverse of the SPD
-// coarse matrix is symmetric in exact arithmetic; the elimination's rounding is
-// not, and a symmetric coarse solve keeps the V-cycle a symmetric preconditioner.
-__global__ void k_symmetrize(double* __restrict__ A, int n) {
+// out = (A + A^T) / 2: the inverse of the SPD coarse matrix is symmetric in exact
+// arithmetic; the elimination's rounding is not, and a symmetric coarse solve
+// keeps the V-cycle a symmetric preconditioner.  32x32 tiles through shared memory.
+__global__ void __launch_bounds__(256) k_symmetrize(const double* A, double* out, int n) {
   grid_dep_wait();
-  const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)n * n) return;
-  const int i = (int)(idx / n), j = (int)(idx % n);
-  if (i >= j) return;
-  const double v = 0.5 * (A[(size_t)i * n + j] + A[(size_t)j * n + i]);
-  A[(size_t)i * n + j] = v;
-  A[(size_t)j * n + i] = v;
+  __shared__ double s[32][33];
+  const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+  for (int r = ty; r < 32; r += 8)
+    if (j0 + r < n && i0 + tx < n) s[r][tx] = A[(size_t)(j0 + r) * n + i0 + tx];
+  __syncthreads();
+#pragma unroll
+  for (int r = ty; r < 32; r += 8)
+    if (i0 + r < n && j0 + tx < n)
+      out[(size_t)(i0 + r) * n + j0 + tx] = 0.5 * (A[(size_t)(i0 + r) * n + j0 + tx] + s[tx][r]);
 }
 
 // x = Inv b, one CTA per row: each thread reads a few entries of the row (all
@@ -772,131 +892,178 @@ void mg_free(Ctx& c) {
   c.mg_prec = -1;
 }
 
-// Largest eigenvalue of a symmetric tridiagonal matrix (Sturm bisection).
-static double tridiag_lmax(const std::vector<double>& a, const std::vector<double>& b) {
-  const int m = (int)a.size();
-  double lo = 0.0, hi = 0.0;
-  for (int i = 0; i < m; ++i) {
-    const double r = (i > 0 ? std::fabs(b[i - 1]) : 0.0) + (i < m - 1 ? std::fabs(b[i]) : 0.0);
-    hi = std::max(hi, a[i] + r);
-    lo = std::min(lo, a[i] - r);
-  }
-  auto count_below = [&](double x) {
-    int cnt = 0;
-    double d = 1.0;
-    for (int i = 0; i < m; ++i) {
-      d = a[i] - x - (i > 0 ? b[i - 1] * b[i - 1] / d : 0.0);
-      if (d == 0.0) d = 1e-300;
-      if (d < 0) ++cnt;
-    }
-    return cnt;
-  };
-  for (int it = 0; it < 100; ++it) {
-    const double mid = 0.5 * (lo + hi);
-    if (count_below(mid) >= m) hi = mid; else lo = mid;
-  }
-  return hi;
-}
+// ---- smoother bounds -----------------------------------------------------------
+// lambda_max(D^-1 A) from kLanSteps steps of Jacobi-PCG on a pseudo-random start
+// vector: the Lanczos coefficients stay on the device, in the level's table,
+// and one kernel turns those of all levels into Chebyshev coefficients, so the
+// set-up enqueues without waiting for the GPU.
+constexpr int kLanSteps = 10;
+enum LanSlot { LAN_RZ = 0, LAN_PAP = 1, LAN_M = 2, LAN_STOP = 3, LAN_ALPHA = 4, LAN_BETA = LAN_ALPHA + kLanSteps,
+               LAN_COUNT = LAN_BETA + kLanSteps };
+constexpr int kChebCoefs = 2 * (kMaxCheb + 1);   // of a level's table: the coefficients, then the LAN_ slots
 
+// r = deterministic pseudo-random vector (zero on fixed DOFs), p = z = D^-1 r, Ap = 0, r.z
 template <typename T>
-static void apply_level(Ctx& c, MGLevel& L, const T* x, T* y) {
-  launch_apply_K<T, T>(L.g, level_K<T>(L), x, y, c.stream);
-}
-
-template <typename T>
-static void dot_level(Ctx& c, const T* a, const T* b, int64_t n, int slot);
-template <>
-void dot_level<double>(Ctx& c, const double* a, const double* b, int64_t n, int slot) { launch_dot(c, a, b, n, slot); }
-template <>
-void dot_level<float>(Ctx& c, const float* a, const float* b, int64_t n, int slot) { launch_dot_f(c, a, b, n, slot); }
-
-template <typename T>
-__global__ void k_fill_pattern(T* v, int64_t n, int A, int pin) {
-  grid_dep_wait();
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  // deterministic pseudo-random start vector, zero on fixed DOFs
-  uint64_t z = (uint64_t)i * 0x9E3779B97F4A7C15ull + 0x632BE59BD9B4E019ull;
-  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-  z ^= z >> 31;
-  const double u = (double)(z >> 11) * (1.0 / 9007199254740992.0) - 0.5;
-  const int64_t node = i >> 1;
-  const int a = (int)(node % A), b = (int)(node / A);
-  const bool fixed = dof_fixed(a, b, (int)(i & 1), A - 1, pin);
-  v[i] = fixed ? (T)0 : (T)u;
-}
-
-template <typename T>
-__global__ void k_pcg_vec(T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p, const T* __restrict__ Ap,
-                          const T* __restrict__ dinv, T* __restrict__ z, double alpha, int64_t nnod) {
-  grid_dep_wait();
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n >= nnod) return;
-  double rr[2];
+__global__ void __launch_bounds__(kRedThreads) k_lan_start(const T* __restrict__ dinv, T* r, T* p, T* Ap, int64_t nnod,
+                                                           int A, int pin, double* lan, double* partial,
+                                                           unsigned int* counter) {
+  typedef typename V2<T>::T X2;
+  double v[1] = {0.0};
+  for (int64_t n = blockIdx.x * (int64_t)kRedThreads + threadIdx.x; n < nnod; n += (int64_t)gridDim.x * kRedThreads) {
+    const int a = (int)(n % A), b = (int)(n / A);
+    X2 rv, zv;
+    T u[2];
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    x[2 * n + c] += (T)(alpha * (double)p[2 * n + c]);
-    rr[c] = (double)r[2 * n + c] - alpha * (double)Ap[2 * n + c];
-    r[2 * n + c] = (T)rr[c];
+    for (int c = 0; c < 2; ++c) {
+      uint64_t z = (uint64_t)(2 * n + c) * 0x9E3779B97F4A7C15ull + 0x632BE59BD9B4E019ull;
+      z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+      z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+      z ^= z >> 31;
+      u[c] = dof_fixed(a, b, c, A - 1, pin) ? (T)0 : (T)((double)(z >> 11) * (1.0 / 9007199254740992.0) - 0.5);
+    }
+    double z0, z1;
+    bj_apply<T>(dinv, n, (double)u[0], (double)u[1], z0, z1);
+    rv.x = u[0]; rv.y = u[1];
+    zv.x = (T)z0; zv.y = (T)z1;
+    reinterpret_cast<X2*>(r)[n] = rv;
+    reinterpret_cast<X2*>(p)[n] = zv;
+    zv.x = zv.y = (T)0;
+    reinterpret_cast<X2*>(Ap)[n] = zv;
+    v[0] += (double)u[0] * (double)(T)z0 + (double)u[1] * (double)(T)z1;
   }
-  double z0, z1;
-  bj_apply<T>(dinv, n, rr[0], rr[1], z0, z1);
-  z[2 * n] = (T)z0;
-  z[2 * n + 1] = (T)z1;
-}
-template <typename T>
-__global__ void k_xpby(const T* __restrict__ z, T* __restrict__ p, double beta, int64_t n) {
-  grid_dep_wait();
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) p[i] = z[i] + (T)(beta * (double)p[i]);
+  double* o[1] = {lan + LAN_RZ};
+  if (grid_finish<1>(v, partial, counter, o) && threadIdx.x == 0) {
+    lan[LAN_M] = 0.0;
+    lan[LAN_STOP] = lan[LAN_RZ] > 0.0 ? 0.0 : 1.0;
+  }
 }
 
-// lambda_max(D^-1 A) from 10 steps of Jacobi-PCG (Lanczos coefficients).
+// p.Ap; stops the recurrence where it is not positive
 template <typename T>
-static double estimate_lmax(Ctx& c, MGLevel& L) {
-  const int64_t n = 2 * L.g.nnod;
-  T* x = (T*)L.x; T* r = (T*)L.r; T* p = (T*)L.d; T* z = (T*)L.b; T* Ap = (T*)L.t;
+__global__ void __launch_bounds__(kRedThreads) k_lan_pap(const T* p, const T* Ap, int64_t n, double* lan,
+                                                         double* partial, unsigned int* counter) {
+  if (lan[LAN_STOP] != 0.0) return;
+  double v[1] = {0.0};
+  for (int64_t i = blockIdx.x * (int64_t)kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads)
+    v[0] += (double)p[i] * (double)Ap[i];
+  double* o[1] = {lan + LAN_PAP};
+  if (grid_finish<1>(v, partial, counter, o) && threadIdx.x == 0 && !(lan[LAN_PAP] > 0.0)) lan[LAN_STOP] = 1.0;
+}
+
+// r -= alpha Ap; z = D^-1 r; r.z; the last block records alpha and beta
+template <typename T>
+__global__ void __launch_bounds__(kRedThreads) k_lan_update(T* r, const T* Ap, const T* __restrict__ dinv, T* z,
+                                                            int64_t nnod, double* lan, double* partial,
+                                                            unsigned int* counter) {
+  if (lan[LAN_STOP] != 0.0) return;
+  typedef typename V2<T>::T X2;
+  const double rz = lan[LAN_RZ], alpha = rz / lan[LAN_PAP];
+  double v[1] = {0.0};
+  for (int64_t n = blockIdx.x * (int64_t)kRedThreads + threadIdx.x; n < nnod; n += (int64_t)gridDim.x * kRedThreads) {
+    X2 rv = reinterpret_cast<X2*>(r)[n];
+    const X2 av = reinterpret_cast<const X2*>(Ap)[n];
+    const double r0 = (double)rv.x - alpha * (double)av.x, r1 = (double)rv.y - alpha * (double)av.y;
+    double z0, z1;
+    bj_apply<T>(dinv, n, r0, r1, z0, z1);
+    rv.x = (T)r0; rv.y = (T)r1;
+    reinterpret_cast<X2*>(r)[n] = rv;
+    X2 zv;
+    zv.x = (T)z0; zv.y = (T)z1;
+    reinterpret_cast<X2*>(z)[n] = zv;
+    v[0] += (double)rv.x * (double)zv.x + (double)rv.y * (double)zv.y;
+  }
+  // every block has read rz before the ticket of the last one is drawn, so the
+  // result may replace it
+  double* o[1] = {lan + LAN_RZ};
+  if (grid_finish<1>(v, partial, counter, o) && threadIdx.x == 0) {
+    const int m = (int)lan[LAN_M];
+    lan[LAN_ALPHA + m] = alpha;
+    lan[LAN_BETA + m] = lan[LAN_RZ] / rz;
+    lan[LAN_M] = (double)(m + 1);
+    if (!(lan[LAN_RZ] > 0.0)) lan[LAN_STOP] = 1.0;
+  }
+}
+
+// p = z + beta p, Ap = 0
+template <typename T>
+__global__ void k_lan_dir(const T* z, T* p, T* Ap, int64_t n, const double* lan) {
+  if (lan[LAN_STOP] != 0.0) return;
+  const double beta = lan[LAN_BETA + (int)lan[LAN_M] - 1];
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) {
+    p[i] = z[i] + (T)(beta * (double)p[i]);
+    Ap[i] = (T)0;
+  }
+}
+
+template <typename T>
+static void estimate_lmax(Ctx& c, MGLevel& L) {
+  const int64_t nn = L.g.nnod, n = 2 * nn;
+  T* r = (T*)L.r; T* p = (T*)L.d; T* z = (T*)L.b; T* Ap = (T*)L.t;
   const T* dinv = level_dinv<T>(L);
-  DP_CUDA(cudaMemsetAsync(x, 0, sizeof(T) * n, c.stream));
-  klaunch(k_fill_pattern<T>, tpb(n), 256, 0, c.stream, r, n, (int)L.g.A(), L.g.pin);
-  klaunch(k_bj<T>, tpb(L.g.nnod), 256, 0, c.stream, dinv, r, z, L.g.nnod);
-  DP_CUDA(cudaMemcpyAsync(p, z, sizeof(T) * n, cudaMemcpyDeviceToDevice, c.stream));
-  dot_level<T>(c, r, z, n, 20);
-  DP_CUDA(cudaMemcpyAsync(c.h_scal + 20, c.scal + 20, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-  DP_CUDA(cudaStreamSynchronize(c.stream));
-  double rz = c.h_scal[20];
-  std::vector<double> alphas, betas;
-  const int kSteps = 10;
-  for (int k = 0; k < kSteps && rz > 0.0; ++k) {
-    apply_level<T>(c, L, p, Ap);
-    dot_level<T>(c, p, Ap, n, 21);
-    DP_CUDA(cudaMemcpyAsync(c.h_scal + 21, c.scal + 21, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    DP_CUDA(cudaStreamSynchronize(c.stream));
-    const double pAp = c.h_scal[21];
-    if (!(pAp > 0.0)) break;
-    const double alpha = rz / pAp;
-    klaunch(k_pcg_vec<T>, tpb(L.g.nnod), 256, 0, c.stream, x, r, p, Ap, dinv, z, alpha, L.g.nnod);
-    dot_level<T>(c, r, z, n, 20);
-    DP_CUDA(cudaMemcpyAsync(c.h_scal + 20, c.scal + 20, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    DP_CUDA(cudaStreamSynchronize(c.stream));
-    const double rz_new = c.h_scal[20];
-    const double beta = rz_new / rz;
-    alphas.push_back(alpha);
-    betas.push_back(beta);
-    rz = rz_new;
-    if (!(rz > 0.0)) break;
-    klaunch(k_xpby<T>, tpb(n), 256, 0, c.stream, z, p, beta, n);
+  double* lan = L.cheb + kChebCoefs;
+  klaunch(k_lan_start<T>, red_grid(n), kRedThreads, 0, c.stream, dinv, r, p, Ap, nn, (int)L.g.A(), L.g.pin, lan,
+          c.partial, c.counter);
+  for (int k = 0; k < kLanSteps; ++k) {
+    launch_apply_K_acc<T, T>(L.g, level_K<T>(L), p, Ap, c.stream);
+    klaunch(k_lan_pap<T>, red_grid(n), kRedThreads, 0, c.stream, p, Ap, n, lan, c.partial, c.counter);
+    klaunch(k_lan_update<T>, red_grid(n), kRedThreads, 0, c.stream, r, Ap, dinv, z, nn, lan, c.partial, c.counter);
+    if (k + 1 < kLanSteps) klaunch(k_lan_dir<T>, tpb(n), 256, 0, c.stream, z, p, Ap, n, lan);
   }
   DP_LAUNCH_CHECK();
-  const int m = (int)alphas.size();
-  if (m == 0) return 2.0;
-  std::vector<double> a(m), b(std::max(m - 1, 0));
-  for (int j = 0; j < m; ++j) {
-    a[j] = 1.0 / alphas[j] + (j > 0 ? betas[j - 1] / alphas[j - 1] : 0.0);
-    if (j < m - 1) b[j] = std::sqrt(betas[j]) / alphas[j];
+}
+
+// Chebyshev recurrence coefficients on [lo, hi] * lambda_max (three-term form),
+// one warp per level.  lambda_max of the Lanczos tridiagonal matrix by Sturm
+// counts: 32 trial values a round, 12 rounds (33^-12 of the Gershgorin interval).
+struct ChebArgs {
+  double* cheb[16];
+  int degree[16];
+};
+__global__ void __launch_bounds__(32) k_cheb_coefs(ChebArgs args, double frac_lo, double frac_hi) {
+  double* coef = args.cheb[blockIdx.x];
+  const double* lan = coef + kChebCoefs;
+  const int lane = threadIdx.x, m = (int)lan[LAN_M], degree = args.degree[blockIdx.x];
+  double lmax = 2.0;
+  if (m > 0) {
+    double a[kLanSteps], b2[kLanSteps], lo = 0.0, hi = 0.0, left = 0.0;
+    for (int j = 0; j < m; ++j) {
+      a[j] = 1.0 / lan[LAN_ALPHA + j] + (j > 0 ? lan[LAN_BETA + j - 1] / lan[LAN_ALPHA + j - 1] : 0.0);
+      const double b = j < m - 1 ? sqrt(lan[LAN_BETA + j]) / lan[LAN_ALPHA + j] : 0.0;
+      b2[j] = b * b;
+      hi = fmax(hi, a[j] + left + b);
+      lo = fmin(lo, a[j] - left - b);
+      left = b;
+    }
+    for (int round = 0; round < 12; ++round) {
+      const double x = lo + (hi - lo) * ((lane + 1) * (1.0 / 33.0));
+      int cnt = 0;
+      double d = 1.0;
+      for (int j = 0; j < m; ++j) {
+        d = a[j] - x - (j > 0 ? b2[j - 1] / d : 0.0);
+        if (d == 0.0) d = 1e-300;
+        if (d < 0) ++cnt;
+      }
+      const unsigned above = __ballot_sync(0xffffffffu, cnt >= m);   // trial values >= lambda_max
+      const int first = above ? __ffs(above) - 1 : 32;
+      const double xl = __shfl_sync(0xffffffffu, x, first > 0 ? first - 1 : 0);
+      const double xh = __shfl_sync(0xffffffffu, x, first < 32 ? first : 31);
+      if (first > 0) lo = xl;
+      if (first < 32) hi = xh;
+    }
+    lmax = hi;
   }
-  return tridiag_lmax(a, b);
+  if (lane != 0) return;
+  const double lmx = frac_hi * lmax, lmn = frac_lo * lmax;
+  const double theta = 0.5 * (lmx + lmn), delta = 0.5 * (lmx - lmn), sigma = theta / delta;
+  double rho_prev = 1.0 / sigma;
+  coef[0] = 1.0 / theta;
+  for (int k = 1; k < degree; ++k) {
+    const double rho = 1.0 / (2.0 * sigma - rho_prev);
+    coef[2 * k] = rho * rho_prev;
+    coef[2 * k + 1] = 2.0 * rho / delta;
+    rho_prev = rho;
+  }
 }
 
 template <typename T>
@@ -939,17 +1106,21 @@ static void mg_setup_t(Ctx& c, const MGOptions& o) {
         DP_CUDA(cudaMalloc(prec ? (void**)&L.K32 : (void**)&L.K64, sizeof(T) * kstore<T>(L.g.nel)));
       }
       DP_CUDA(cudaMalloc(prec ? (void**)&L.dinv32 : (void**)&L.dinv64, sizeof(T) * 3 * L.g.nnod));
-      DP_CUDA(cudaMalloc(&L.cheb, sizeof(double) * 2 * (kMaxCheb + 1)));
+      DP_CUDA(cudaMalloc(&L.cheb, sizeof(double) * (kChebCoefs + LAN_COUNT)));
+      DP_CUDA(cudaMemsetAsync(L.cheb, 0, sizeof(double) * (kChebCoefs + LAN_COUNT), c.stream));
       setup_level_vectors<T>(L);
       if (l + 1 < c.mg.size() && L.g.nnod <= kStencilMaxNodes)
         DP_CUDA(cudaMalloc(&L.S, sizeof(T) * stencil_store<T>(L.g.ncr, L.g.nct)));
     }
     c.coarse_n = 2 * c.mg.back().g.nnod;
     if (c.coarse_n <= o.coarse_max) {
-      DP_CUDA(cudaMalloc(&c.coarse_inv, sizeof(double) * c.coarse_n * c.coarse_n * 2));
+      DP_CUDA(cudaMalloc(&c.coarse_inv, sizeof(double) * (c.coarse_n * c.coarse_n * 2 + 2 * kGJPanel * kGJPanel)));
     } else {
       c.coarse_n = 0;
     }
+    DP_CUDA(cudaFuncSetAttribute(k_galerkin<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)GalerkinTile<T>::kSmem));
+    DP_CUDA(cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGJSmem));
     c.mg_prec = prec;
     c.mg_coarse_max = o.coarse_max;
   }
@@ -971,90 +1142,55 @@ static void mg_setup_t(Ctx& c, const MGOptions& o) {
   for (size_t l = 1; l < c.mg.size(); ++l) {
     MGLevel& Lf = c.mg[l - 1];
     MGLevel& Lc = c.mg[l];
-    const int64_t nthreads = Lc.g.nel * kKe;
-    klaunch(k_galerkin<T>, (int)div_up(nthreads, 128), 128, 0, c.stream, level_K<T>(Lf), level_K<T>(Lc), (int)Lc.g.nel,
-                                                                      Lc.g.ncr, Lc.g.nct, (int)Lf.g.nel, Lf.g.ncr,
-                                                                      Lc.g.pin);
+    klaunch(k_galerkin<T>, (int)div_up((int64_t)Lc.g.ncr * Lc.g.nct, 32), kGalThreads, GalerkinTile<T>::kSmem,
+            c.stream, level_K<T>(Lf), level_K<T>(Lc), Lc.g.ncr, Lc.g.nct, Lf.g.ncr, Lc.g.pin);
     DP_LAUNCH_CHECK();
   }
   for (MGLevel& L : c.mg)
     if (L.S) launch_stencil_assemble<T>(L.g, level_K<T>(L), (T*)L.S, c.stream);
   // nodal diagonal blocks, eigenvalue estimates and Chebyshev coefficients
-  double* diag = nullptr;
-  DP_CUDA(cudaMalloc(&diag, sizeof(double) * 3 * c.mg[0].g.nnod));
   const int deg = std::max(1, std::min(o.cheb_degree, kMaxCheb));
   const int deg_coarse = o.cheb_degree_coarse > 0 ? std::max(1, std::min(o.cheb_degree_coarse, kMaxCheb)) : deg;
+  ChebArgs ca{};
+  int nsmooth = 0;
   for (size_t l = 0; l < c.mg.size(); ++l) {
     MGLevel& L = c.mg[l];
     L.degree = l == 0 ? deg : deg_coarse;
-    if (L.g.det) {
-      double* E = static_cast<double*>(L.g.det);
-      klaunch(k_diag_blocks_elem<T>, (int)div_up(L.g.nel, 128), 128, 0, c.stream, level_K<T>(L), E, (int)L.g.nel);
-      DP_LAUNCH_CHECK();
-      launch_node_gather<double>(L.g, E, diag, 3, 2, c.stream);
-    } else {
-      DP_CUDA(cudaMemsetAsync(diag, 0, sizeof(double) * 3 * L.g.nnod, c.stream));
-      klaunch(k_diag_blocks<T>, (int)div_up(L.g.nel, 128), 128, 0, c.stream, level_K<T>(L), diag, (int)L.g.nel,
-              L.g.ncr, (int)L.g.A(), (int)L.g.B());
-    }
-    klaunch(k_block_invert<T>, tpb(L.g.nnod), 256, 0, c.stream, diag, level_dinv<T>(L), L.g.nnod, (int)L.g.A(), L.g.pin,
-                                                            o.block_jacobi);
+    klaunch(k_diag_invert<T>, tpb((int64_t)(L.g.ncr + 1) * L.g.nct), 256, 0, c.stream, level_K<T>(L),
+            level_dinv<T>(L), L.g.ncr, L.g.nct, L.g.pin, o.block_jacobi);
     DP_LAUNCH_CHECK();
-    const bool is_coarsest_direct = (l + 1 == c.mg.size()) && c.coarse_n > 0;
-    L.lmax = is_coarsest_direct ? 0.0 : estimate_lmax<T>(c, L);
-    // Chebyshev recurrence coefficients on [lo, hi] * lmax (three-term form)
-    double coef[2 * (kMaxCheb + 1)] = {0.0};
-    if (L.lmax > 0.0) {
-      const double lmx = o.cheb_hi * L.lmax, lmn = o.cheb_lo * L.lmax;
-      const double theta = 0.5 * (lmx + lmn), delta = 0.5 * (lmx - lmn), sigma = theta / delta;
-      double rho_prev = 1.0 / sigma;
-      coef[0] = 1.0 / theta;
-      for (int k = 1; k < L.degree; ++k) {
-        const double rho = 1.0 / (2.0 * sigma - rho_prev);
-        coef[2 * k] = rho * rho_prev;
-        coef[2 * k + 1] = 2.0 * rho / delta;
-        rho_prev = rho;
-      }
-    }
-    DP_CUDA(cudaMemcpyAsync(L.cheb, coef, sizeof(coef), cudaMemcpyHostToDevice, c.stream));
-    DP_CUDA(cudaStreamSynchronize(c.stream));
+    if (l + 1 == c.mg.size() && c.coarse_n > 0) continue;   // solved directly, never smoothed
+    estimate_lmax<T>(c, L);
+    ca.cheb[nsmooth] = L.cheb;
+    ca.degree[nsmooth++] = L.degree;
   }
+  if (nsmooth > 0) klaunch(k_cheb_coefs, nsmooth, 32, 0, c.stream, ca, o.cheb_lo, o.cheb_hi);
+  DP_LAUNCH_CHECK();
   c.mg_degree = deg + 16 * deg_coarse;  // both degrees shape the captured graph
-  DP_CUDA(cudaFree(diag));
   // coarse dense inverse
   if (c.coarse_n > 0) {
     MGLevel& L = c.mg.back();
-    const int n = (int)c.coarse_n;
+    const int n = (int)c.coarse_n, npanel = (int)div_up(n, kGJPanel);
     double* D = c.coarse_inv;
     double* Inv = D + (size_t)n * n;
-    DP_CUDA(cudaMemsetAsync(D, 0, sizeof(double) * n * n, c.stream));
-    if (L.g.det)
-      klaunch(k_dense_assemble_seq<T>, 1, 128, 0, c.stream, level_K<T>(L), D, (int)L.g.nel, L.g.ncr, (int)L.g.A(),
-              (int)L.g.B(), n);
-    else
-      klaunch(k_dense_assemble<T>, (int)div_up(L.g.nel, 128), 128, 0, c.stream, level_K<T>(L), D, (int)L.g.nel,
-              L.g.ncr, (int)L.g.A(), (int)L.g.B(), n);
-    klaunch(k_dense_fix_diag, (int)div_up(n, 256), 256, 0, c.stream, D, n);
-    double* buf[2] = {D, Inv};
-    double* W = nullptr;   // panel inverse (kGJPanel^2) and T (n x kGJPanel)
-    DP_CUDA(cudaMalloc(&W, sizeof(double) * (kGJPanel * kGJPanel + (size_t)n * kGJPanel)));
-    double* Tc = W + kGJPanel * kGJPanel;
-    const int npanel = (int)div_up(n, kGJPanel);
+    double* W = Inv + (size_t)n * n;   // two panel inverses, in turn
+    // ping-pong between D and Inv such that the last panel writes D
+    double* cur = (npanel & 1) ? Inv : D;
+    double* oth = (npanel & 1) ? D : Inv;
+    DP_CUDA(cudaMemsetAsync(cur, 0, sizeof(double) * n * n, c.stream));
+    klaunch(k_dense_assemble<T>, dim3((unsigned)div_up(st_nodes(0, L.g.ncr, L.g.nct), 64), 4), 64, 0, c.stream,
+            level_K<T>(L), cur, L.g.ncr, L.g.nct);
+    klaunch(k_dense_fix_diag, (int)div_up(n, 256), 256, 0, c.stream, cur, n);
+    klaunch(k_gj_panel_inverse, 1, dim3(kGJPanel, kGJPanel), 0, c.stream, cur, W, n, 0, std::min(kGJPanel, n));
+    const unsigned tiles = (unsigned)div_up(n, kGJTile);
     for (int p = 0; p < npanel; ++p) {
-      const int k0 = p * kGJPanel, b = std::min(kGJPanel, n - k0);
-      const double* Aold = buf[p & 1];
-      klaunch(k_gj_panel_inverse, 1, dim3(kGJPanel, kGJPanel), 0, c.stream, Aold, W, n, k0, b);
-      klaunch(k_gj_panel_cols, (int)div_up((int64_t)n * kGJPanel, 256), 256, 0, c.stream, Aold, (const double*)W, Tc,
-              n, k0, b);
-      klaunch(k_gj_panel_update, (int)div_up((int64_t)n * n, 256), 256, 0, c.stream, Aold, buf[(p + 1) & 1],
-              (const double*)W, (const double*)Tc, n, k0, b);
+      klaunch(k_gj_panel, dim3(tiles, tiles), 256, kGJSmem, c.stream, cur, oth,
+              W + (p & 1) * kGJPanel * kGJPanel, W + ((p & 1) ^ 1) * kGJPanel * kGJPanel, n, p * kGJPanel);
+      std::swap(cur, oth);
     }
-    // panel p writes buf[(p + 1) & 1]: for an even panel count the inverse ends in D
-    if (!(npanel & 1)) DP_CUDA(cudaMemcpyAsync(Inv, D, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, c.stream));
-    klaunch(k_symmetrize, (int)div_up((int64_t)n * n, 256), 256, 0, c.stream, Inv, n);
+    const unsigned blk = (unsigned)div_up(n, 32);
+    klaunch(k_symmetrize, dim3(blk, blk), 256, 0, c.stream, D, Inv, n);
     DP_LAUNCH_CHECK();
-    DP_CUDA(cudaStreamSynchronize(c.stream));
-    DP_CUDA(cudaFree(W));
   }
 }
 

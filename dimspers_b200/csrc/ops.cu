@@ -162,19 +162,19 @@ __host__ __device__ constexpr int loc_b(int t, int k) {
 // Deterministic form, pass 2: per lattice node n, the sum of E over the
 // elements that contain it, taken in a fixed order (triangle type t = 0, 1,
 // then local node k = 0..5), so the result is the same bit for bit in every
-// run.  E[(NC k + c) nel + e] holds element e's value c at its local node k.
-// MODE 0: y[NC n + c] += s; 1: y -= s; 2: y = s.
+// run.  E[(2k + c) nel + e] holds element e's component c at its local node k.
+// MODE 0: y[2n + c] += s; 1: y -= s; 2: y = s.
 // One thread owns the 2x2 node block a = 2i + pa, b = 2j + pb (i <= ncr,
 // j < nct): for each parity class (pa, pb) the elements holding the node are
 // fixed at compile time (local node k of type t holds it iff loc_a(t, k) has
 // the parity of a and loc_b(t, k) that of b; the element's cell is then
 // (i + (pa - loc_a) / 2, j + (pb - loc_b) / 2), theta periodic), so a warp
 // never diverges on them, and neighbouring lanes write neighbouring nodes.
-template <int PA, int PB, typename T, int NC>
+template <int PA, int PB, typename T>
 __device__ __forceinline__ void gather_class(const T* E, int i, int j, int ncr, int nct, int64_t nel,
-                                             T s[NC]) {
+                                             T s[2]) {
 #pragma unroll
-  for (int c = 0; c < NC; ++c) s[c] = (T)0;
+  for (int c = 0; c < 2; ++c) s[c] = (T)0;
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
 #pragma unroll
@@ -186,60 +186,51 @@ __device__ __forceinline__ void gather_class(const T* E, int i, int j, int ncr, 
       if (it < 0) it += nct;
       const int64_t e = 2 * ((int64_t)ir + (int64_t)ncr * it) + t;
 #pragma unroll
-      for (int c = 0; c < NC; ++c) s[c] += E[(int64_t)(NC * k + c) * nel + e];
+      for (int c = 0; c < 2; ++c) s[c] += E[(int64_t)(2 * k + c) * nel + e];
     }
   }
 }
 
-template <int PA, int PB, typename T, int NC, int MODE>
+template <int PA, int PB, typename T, int MODE>
 __device__ __forceinline__ void gather_node(const T* E, T* y, int i, int j, int ncr, int nct,
                                             int64_t nel) {
   const int a = 2 * i + PA;
   if (a > 2 * ncr) return;
-  T s[NC];
-  gather_class<PA, PB, T, NC>(E, i, j, ncr, nct, nel, s);
+  T s[2];
+  gather_class<PA, PB, T>(E, i, j, ncr, nct, nel, s);
   const int64_t n = a + (int64_t)(2 * ncr + 1) * (2 * j + PB);
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    T* p = y + NC * n + c;
+  for (int c = 0; c < 2; ++c) {
+    T* p = y + 2 * n + c;
     if (MODE == 0) *p += s[c];
     else if (MODE == 1) *p -= s[c];
     else *p = s[c];
   }
 }
 
-template <typename T, int NC, int MODE>
+template <typename T, int MODE>
 __global__ void __launch_bounds__(256) k_node_gather(const T* E, T* y, int ncr, int nct,
                                                      int64_t nel) {
   grid_dep_wait();
   const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (q >= (int64_t)(ncr + 1) * nct) return;
   const int j = (int)(q / (ncr + 1)), i = (int)(q - (int64_t)j * (ncr + 1));
-  gather_node<0, 0, T, NC, MODE>(E, y, i, j, ncr, nct, nel);
-  gather_node<1, 0, T, NC, MODE>(E, y, i, j, ncr, nct, nel);
-  gather_node<0, 1, T, NC, MODE>(E, y, i, j, ncr, nct, nel);
-  gather_node<1, 1, T, NC, MODE>(E, y, i, j, ncr, nct, nel);
+  gather_node<0, 0, T, MODE>(E, y, i, j, ncr, nct, nel);
+  gather_node<1, 0, T, MODE>(E, y, i, j, ncr, nct, nel);
+  gather_node<0, 1, T, MODE>(E, y, i, j, ncr, nct, nel);
+  gather_node<1, 1, T, MODE>(E, y, i, j, ncr, nct, nel);
 }
 
 template <typename T>
-void launch_node_gather(const Level& L, const T* E, T* y, int nc, int mode, cudaStream_t s) {
+void launch_node_gather(const Level& L, const T* E, T* y, int mode, cudaStream_t s) {
   const int grid = (int)div_up((int64_t)(L.ncr + 1) * L.nct, 256);
-#define DP_GATHER(NC, M) \
-  klaunch(k_node_gather<T, NC, M>, grid, 256, 0, s, E, y, L.ncr, L.nct, (int64_t)L.nel)
-  if (nc == 2) {
-    if (mode == 0) DP_GATHER(2, 0);
-    else if (mode == 1) DP_GATHER(2, 1);
-    else DP_GATHER(2, 2);
-  } else if (nc == 3 && mode == 2) {
-    DP_GATHER(3, 2);
-  } else {
-    throw std::runtime_error("launch_node_gather: unsupported layout");
-  }
-#undef DP_GATHER
+  if (mode == 0) klaunch(k_node_gather<T, 0>, grid, 256, 0, s, E, y, L.ncr, L.nct, (int64_t)L.nel);
+  else if (mode == 1) klaunch(k_node_gather<T, 1>, grid, 256, 0, s, E, y, L.ncr, L.nct, (int64_t)L.nel);
+  else klaunch(k_node_gather<T, 2>, grid, 256, 0, s, E, y, L.ncr, L.nct, (int64_t)L.nel);
   DP_LAUNCH_CHECK();
 }
-template void launch_node_gather<double>(const Level&, const double*, double*, int, int, cudaStream_t);
-template void launch_node_gather<float>(const Level&, const float*, float*, int, int, cudaStream_t);
+template void launch_node_gather<double>(const Level&, const double*, double*, int, cudaStream_t);
+template void launch_node_gather<float>(const Level&, const float*, float*, int, cudaStream_t);
 
 // ---- matrix-free element-by-element K apply (fine level) -------------------------
 // K_e (polar DOFs, constrained rows/columns masked) = sum_ip B0^T Dw_ip B0, with
@@ -375,7 +366,7 @@ static void apply_K_into(const Level& L, const Tm* K, const Tv* x, Tv* y, cudaSt
     klaunch(k_apply_K_elem<Tm, Tv>, (int)div_up(L.nel, 256), 256, 0, s, K, x, E, (int)L.nel, L.ncr, (int)L.A(),
             (int)L.B());
     DP_LAUNCH_CHECK();
-    launch_node_gather<Tv>(L, E, y, 2, kMode, s);
+    launch_node_gather<Tv>(L, E, y, kMode, s);
     return;
   }
   if (kMode == 2) DP_CUDA(cudaMemsetAsync(y, 0, sizeof(Tv) * 2 * L.nnod, s));
@@ -570,7 +561,7 @@ void launch_apply_G(Ctx& c, const double* p, double* y) {
     klaunch(k_apply_G_elem, (int)div_up(L.nel, 128), 128, 0, c.stream, c.Gp, p, E, (int)L.nel, L.ncr, L.nct,
             c.mesh.pressure);
     DP_LAUNCH_CHECK();
-    launch_node_gather<double>(L, E, y, 2, 2, c.stream);
+    launch_node_gather<double>(L, E, y, 2, c.stream);
     return;
   }
   DP_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * 2 * L.nnod, c.stream));

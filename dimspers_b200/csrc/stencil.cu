@@ -100,10 +100,9 @@ __device__ __forceinline__ void st_block(double* S, int64_t base, int j, int n, 
 // order, sums in FP64, one rounding to T.  Blocks that would leave the annulus
 // stay zero.
 template <int C, int J, typename T>
-__device__ __forceinline__ void stencil_entry(const T* __restrict__ K, T* S, int i, int ia, int jb, int ncr, int nct,
-                                              int64_t base, int n) {
+__device__ __forceinline__ void stencil_sum(const T* __restrict__ K, int ia, int jb, int ncr, int nct, double acc[4]) {
   constexpr int PA = C & 1, PB = C >> 1, DA = StencilEntry<C, J>::da, DB = StencilEntry<C, J>::db;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
 #pragma unroll
   for (int ty = 0; ty < 2; ++ty) {
 #pragma unroll
@@ -126,6 +125,13 @@ __device__ __forceinline__ void stencil_entry(const T* __restrict__ K, T* S, int
       }
     }
   }
+}
+
+template <int C, int J, typename T>
+__device__ __forceinline__ void stencil_entry(const T* __restrict__ K, T* S, int i, int ia, int jb, int ncr, int nct,
+                                              int64_t base, int n) {
+  double acc[4];
+  stencil_sum<C, J, T>(K, ia, jb, ncr, nct, acc);
   st_block(S, base, J, n, i, acc);
 }
 

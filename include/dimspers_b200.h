@@ -209,7 +209,7 @@ int dp_assemble(dp_ctx* ctx, int32_t precision);
  * applies in FP32 and FP64, the right-hand side, the multigrid diagonal blocks
  * and the dense coarsest matrix) runs without atomics, as element results
  * summed per node in a fixed order, so repeated solves of the same inputs give
- * the same U, P and iteration counts bit for bit.  Costs 144 bytes of device
+ * the same U, P and iteration counts bit for bit.  Costs 96 bytes of device
  * scratch per element and two passes per apply.  Needs discontinuous
  * pressure and matrix_free = 0.  Switching it on discards the current assembly
  * (call dp_assemble again); on = 0 returns to the atomic scatter.  A dp_batch

@@ -119,6 +119,7 @@ SIGNATURES = {
     "dp_cnn_gradients": (C.c_int, [_P, _P, _P, C.c_int32, C.POINTER(C.c_double)]),
     "dp_cnn_train_step": (C.c_int, [_P, _P, _P, C.c_int32, C.c_float, C.POINTER(C.c_double)]),
     "dp_cnn_inputs": (C.c_int, [_P, _P, C.c_int32, C.c_int32]),
+    "dp_guess_predict": (C.c_int, [_P, _P, _P, _P, C.c_float, C.c_float, C.c_double, _P, _P, _P, C.c_int32]),
     "dp_guess_from_grid": (C.c_int, [_P, _P, C.c_int32, C.c_int32, C.c_double, _P, C.c_int32]),
 }
 

@@ -162,15 +162,14 @@ class LearnedGuess:
         dev = torch.device("cuda", ctx.desc.device)
         self.x = torch.empty((1, 4, net.nrg, net.ntg), dtype=torch.float32, device=dev)
         self.y = torch.empty((1, 1, net.nrg, net.ntg), dtype=torch.float32, device=dev)
-        self.xm = torch.tensor(net.x_mean, device=dev).view(1, 4, 1, 1)
-        self.xs = torch.tensor(net.x_std, device=dev).view(1, 4, 1, 1)
+        self.xm = np.ascontiguousarray(net.x_mean, np.float32)
+        self.xs = np.ascontiguousarray(net.x_std, np.float32)
 
     def predict(self, g, P_out_ptr, mem=DP_MEM_DEVICE):
         """Write the guess for the context's current material into P (device
         pointer by default)."""
-        features(self.ctx, self.x)
-        self.x.sub_(self.xm).div_(self.xs)
-        self.net.forward(self.x, self.y)
-        self.y.mul_(self.net.y_std).add_(self.net.y_mean)
-        self.ctx._chk(lib().dp_guess_from_grid(self.ctx.h, C.c_void_p(self.y.data_ptr()), self.net.nrg, self.net.ntg,
-                                               float(g), C.c_void_p(P_out_ptr), mem))
+        n = self.net
+        self.ctx._chk(lib().dp_guess_predict(self.ctx.h, n.h, C.c_void_p(self.xm.ctypes.data),
+                                             C.c_void_p(self.xs.ctypes.data), float(n.y_mean), float(n.y_std),
+                                             float(g), C.c_void_p(self.x.data_ptr()), C.c_void_p(self.y.data_ptr()),
+                                             C.c_void_p(P_out_ptr), mem))

@@ -388,6 +388,12 @@ int dp_cnn_inputs(dp_ctx* ctx, float* x, int32_t nrg, int32_t ntg);
 /* P = scale * (grid field, bilinear at the element vertices) -> pressure DOFs. */
 int dp_guess_from_grid(dp_ctx* ctx, const float* p_grid, int32_t nrg, int32_t ntg, double scale, double* P,
                        int32_t mem);
+/* The three steps of a guess as one sequence of launches: x (4 x nrg x ntg,
+ * device) = (dp_cnn_inputs - x_mean) / x_std, y (nrg x ntg, device) = network
+ * output * y_std + y_mean (FP32, each operation rounded), P as
+ * dp_guess_from_grid.  x_mean, x_std: 4 host floats. */
+int dp_guess_predict(dp_ctx* ctx, dp_cnn* net, const float* x_mean, const float* x_std, float y_mean, float y_std,
+                     double scale, float* x, float* y, double* P, int32_t mem);
 
 /* Average device time (ms) of one launch of a hot kernel on the context's
  * stream, from CUDA events, after an assembly: which = 0 fine-level A-apply

@@ -27,7 +27,7 @@ Ctx::~Ctx() {
   for (cudaStream_t s : aux)
     if (s) cudaStreamDestroy(s);
   mg_free(*this);
-  cudaFree(theta_lat); cudaFree(r_lat); cudaFree(ref2lat);
+  cudaFree(theta_lat); cudaFree(r_lat);
   cudaFree(eta); cudaFree(C); cudaFree(rho_lat); cudaFree(rho_ref);
   cudaFree(mfD64); cudaFree(mfT64); cudaFree(mfD32); cudaFree(mfT32); cudaFree(det_buf);
   cudaFree(K64); cudaFree(K32); cudaFree(Gp); cudaFree(F); cudaFree(pc); cudaFree(Minv); cudaFree(Fscale);
@@ -35,6 +35,8 @@ Ctx::~Ctx() {
   cudaFree(stress_buf);
   cudaFree(rheo_buf);
   cudaFree(fabric_buf);
+  cudaFree(dem_tab);
+  cudaFreeHost(h_dem);
   if (th_exec) cudaGraphExecDestroy((cudaGraphExec_t)th_exec);
   cudaFree(th_buf);
   cudaFree(scal); cudaFreeHost(h_scal); cudaFree(partial); cudaFree(counter);
@@ -78,18 +80,31 @@ static void dalloc(T** p, size_t n) {
   DP_CUDA(cudaMalloc((void**)p, sizeof(T) * (n ? n : 1)));
 }
 
+// Whether [a, a + na) and [b, b + nb) share memory: device calls whose outputs
+// overlap their inputs go through the staging copies that host arrays take.
+static bool overlap(const double* a, int64_t na, const double* b, int64_t nb) {
+  return a && b && (uintptr_t)a < (uintptr_t)(b + nb) && (uintptr_t)b < (uintptr_t)(a + na);
+}
+
+// The caller's array where the device can read it: itself (device memory), or a
+// copy in `stage` (host memory).
+static const double* staged(Ctx& c, const double* src, double* stage, int64_t n, int mem) {
+  if (mem == DP_MEM_DEVICE) return src;
+  DP_CUDA(cudaMemcpyAsync(stage, src, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream));
+  return stage;
+}
+
 static void upload_eta(Ctx& c, const double* eta_ip, int64_t ld, int mem) {
   const int64_t nel = c.fine.nel;
   if (!eta_ip) throw BadArg("eta_ip is null");
   if (ld < nel) throw BadArg("ld_eta < nel");
-  for (int ip = 0; ip < kNip; ++ip)
-    DP_CUDA(cudaMemcpyAsync(c.eta + ip * nel, eta_ip + ip * ld, sizeof(double) * nel, kind_in(mem), c.stream));
+  DP_CUDA(cudaMemcpy2DAsync(c.eta, sizeof(double) * nel, eta_ip, sizeof(double) * ld, sizeof(double) * nel, kNip,
+                            kind_in(mem), c.stream));
 }
 
 static void upload_rho(Ctx& c, const double* rho, double g, int mem) {
   if (!rho) throw BadArg("rho_node is null");
-  DP_CUDA(cudaMemcpyAsync(c.rho_ref, rho, sizeof(double) * c.fine.nnod, kind_in(mem), c.stream));
-  launch_gather_ref2lat(c, c.rho_ref, c.rho_lat, 1);
+  launch_gather_ref2lat(c, staged(c, rho, c.rho_ref, c.fine.nnod, mem), c.rho_lat, 1);
   c.g = g;
 }
 
@@ -246,16 +261,18 @@ static void deliver_solution(Ctx& c, double* U, double* P, double* Ucart, int me
   double* dU = (double*)c.work[W_U];
   double* dP = (double*)c.work[W_P];
   double* stage = (double*)c.work[W_UC];
-  if (U) {
-    launch_scatter_lat2ref(c, dU, stage, 2);
-    DP_CUDA(cudaMemcpyAsync(U, stage, sizeof(double) * 2 * nn, kind_out(mem), c.stream));
-  }
+  // device arrays are written in place, host arrays through the staging vector
+  auto put = [&](const double* lat, double* out) {
+    launch_scatter_lat2ref(c, lat, mem == DP_MEM_DEVICE ? out : stage, 2);
+    if (mem != DP_MEM_DEVICE)
+      DP_CUDA(cudaMemcpyAsync(out, stage, sizeof(double) * 2 * nn, cudaMemcpyDeviceToHost, c.stream));
+  };
+  if (U) put(dU, U);
   if (P) DP_CUDA(cudaMemcpyAsync(P, dP, sizeof(double) * np, kind_out(mem), c.stream));
   if (Ucart) {
     double* uc = (double*)c.work[W_RES];
     to_cartesian(c, dU, uc);
-    launch_scatter_lat2ref(c, uc, stage, 2);
-    DP_CUDA(cudaMemcpyAsync(Ucart, stage, sizeof(double) * 2 * nn, kind_out(mem), c.stream));
+    put(uc, Ucart);
   }
 }
 
@@ -471,10 +488,8 @@ int dp_ctx_create(const dp_mesh_desc* d, dp_ctx** out) {
     }
     dalloc(&c.theta_lat, nn);
     dalloc(&c.r_lat, nn);
-    dalloc(&c.ref2lat, nn);
     DP_CUDA(cudaMemcpy(c.theta_lat, tl.data(), sizeof(double) * nn, cudaMemcpyHostToDevice));
     DP_CUDA(cudaMemcpy(c.r_lat, rl.data(), sizeof(double) * nn, cudaMemcpyHostToDevice));
-    DP_CUDA(cudaMemcpy(c.ref2lat, c.mesh.ref2lat.data(), sizeof(int64_t) * nn, cudaMemcpyHostToDevice));
     dalloc(&c.eta, kNip * nel);
     dalloc(&c.rho_lat, nn);
     dalloc(&c.rho_ref, nn);
@@ -545,9 +560,8 @@ int dp_set_material(dp_ctx* h, const double* eta_ip, int64_t ld_eta, const doubl
       ensure_C(c, 36 * nel);
       for (int f = 0; f < 6; ++f) {
         if (!C6[f]) throw BadArg("null tensor field");
-        for (int ip = 0; ip < kNip; ++ip)
-          DP_CUDA(cudaMemcpyAsync(c.C + ((size_t)f * 6 + ip) * nel, C6[f] + ip * ld_C, sizeof(double) * nel,
-                                  kind_in(mem), c.stream));
+        DP_CUDA(cudaMemcpy2DAsync(c.C + (size_t)f * 6 * nel, sizeof(double) * nel, C6[f], sizeof(double) * ld_C,
+                                  sizeof(double) * nel, kNip, kind_in(mem), c.stream));
       }
       c.mat_kind = MAT_FULL;
     } else {
@@ -734,22 +748,22 @@ static int apply_common(dp_ctx* h, const double* in, double* out, int32_t mem, i
     double* b = (double*)c.work[W_Z];
     double* stage = (double*)c.work[W_UC];
     double* pbuf = (double*)c.work[W_P];
+    const bool dev = mem == DP_MEM_DEVICE;   // the caller's arrays are read and written in place
+    auto deliver = [&](const double* lat) {
+      launch_scatter_lat2ref(c, lat, dev ? out : stage, 2);
+      if (!dev) DP_CUDA(cudaMemcpyAsync(out, stage, sizeof(double) * 2 * nn, cudaMemcpyDeviceToHost, c.stream));
+    };
     if (which == 0) {  // K
-      DP_CUDA(cudaMemcpyAsync(stage, in, sizeof(double) * 2 * nn, kind_in(mem), c.stream));
-      launch_gather_ref2lat(c, stage, a, 2);
+      launch_gather_ref2lat(c, staged(c, in, stage, 2 * nn, mem), a, 2);
       launch_apply_K<double, double>(c.fine, c.K64, a, b, c.stream);
-      launch_scatter_lat2ref(c, b, stage, 2);
-      DP_CUDA(cudaMemcpyAsync(out, stage, sizeof(double) * 2 * nn, kind_out(mem), c.stream));
+      deliver(b);
     } else if (which == 1) {  // G
-      DP_CUDA(cudaMemcpyAsync(pbuf, in, sizeof(double) * np, kind_in(mem), c.stream));
-      launch_apply_G(c, pbuf, b);
-      launch_scatter_lat2ref(c, b, stage, 2);
-      DP_CUDA(cudaMemcpyAsync(out, stage, sizeof(double) * 2 * nn, kind_out(mem), c.stream));
+      launch_apply_G(c, staged(c, in, pbuf, np, mem), b);
+      deliver(b);
     } else {  // G^T
-      DP_CUDA(cudaMemcpyAsync(stage, in, sizeof(double) * 2 * nn, kind_in(mem), c.stream));
-      launch_gather_ref2lat(c, stage, a, 2);
-      launch_apply_GT(c, a, pbuf);
-      DP_CUDA(cudaMemcpyAsync(out, pbuf, sizeof(double) * np, kind_out(mem), c.stream));
+      launch_gather_ref2lat(c, staged(c, in, stage, 2 * nn, mem), a, 2);
+      launch_apply_GT(c, a, dev ? out : pbuf);
+      if (!dev) DP_CUDA(cudaMemcpyAsync(out, pbuf, sizeof(double) * np, cudaMemcpyDeviceToHost, c.stream));
     }
     DP_CUDA(cudaStreamSynchronize(c.stream));
     return (int)DP_OK;
@@ -817,8 +831,8 @@ int dp_profile_kernel(dp_ctx* h, int32_t which, int32_t reps, int32_t flush_l2, 
     if (reps < 1 || !ms) throw BadArg("reps must be >= 1");
     if (which == 0 && !c.K32) throw BadArg("no FP32 element matrices (assemble with precision 1)");
     if (which == 2 && c.mg.empty()) throw BadArg("no multigrid hierarchy (run a solve first)");
-    if (which == 3 && !c.stress_buf) throw BadArg("no staged post-processor inputs (call dp_stress first)");
-    if (which == 4 && !c.rheo_buf) throw BadArg("no staged viscosity inputs (call dp_viscosity_arrhenius first)");
+    if (which == 3 && !c.stress_called) throw BadArg("no staged post-processor inputs (call dp_stress first)");
+    if (which == 4 && !c.rheo_called) throw BadArg("no staged viscosity inputs (call dp_viscosity_arrhenius first)");
     if (which == 5 && c.fabric_dem[0] == 0)
       throw BadArg("no staged DEM tensor inputs (call dp_anisotropic_tensor first)");
     if (which == 6 && !c.th_buf) throw BadArg("no thermal element blocks (call dp_thermal_step first)");

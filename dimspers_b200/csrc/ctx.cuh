@@ -93,7 +93,6 @@ struct Ctx {
   // geometry
   double* theta_lat = nullptr;  // nnod
   double* r_lat = nullptr;      // nnod
-  int64_t* ref2lat = nullptr;   // nnod
 
   // material
   int mat_kind = MAT_NONE;
@@ -120,11 +119,15 @@ struct Ctx {
   double* Fscale = nullptr;
   void* flush = nullptr;        // L2 flush buffer for cold kernel timings
   double* stress_buf = nullptr; // post-processor staging: eta 7, tensor 42, outputs 56 per element
-  bool stress_tensor = false;   // the staged inputs carry a tensor
-  double* rheo_buf = nullptr;   // viscosity update staging: 4 x 7 per element, 4 per node
-  double* fabric_buf = nullptr; // FSE / DEM tensor staging (fabric_cap doubles)
+  bool stress_tensor = false;   // the last call's inputs carried a tensor
+  bool stress_called = false, rheo_called = false;
+  double* rheo_buf = nullptr;   // viscosity update staging (host arrays): 4 x 7 per element, 3 per node
+  double* fabric_buf = nullptr; // FSE / DEM tensor staging (host arrays; fabric_cap doubles)
   int64_t fabric_cap = 0;
-  int64_t fabric_dem[3] = {0, 0, 0};  // the last staged DEM table: nrows, n_a1a2, sblk (0: none)
+  double* dem_tab = nullptr;    // DEM table of the last tensor call (dem_cap doubles), and its pinned source
+  double* h_dem = nullptr;
+  int64_t dem_cap = 0;
+  int64_t fabric_dem[3] = {0, 0, 0};  // that table's nrows, n_a1a2, sblk (0: none)
   double fabric_w = 0.0;
   double* th_buf = nullptr;     // thermal step: 21 x nel element blocks + 10 nnod vectors
   void* th_exec = nullptr;      // cudaGraphExec_t of the thermal CG loop
@@ -308,6 +311,48 @@ __host__ __device__ inline void element_nodes(int64_t e, int ncr, int64_t A, int
   }
 #pragma unroll
   for (int k = 0; k < 6; ++k) n[k] = a[k] + A * wrapb(b[k], B);
+}
+
+// Reference number of lattice node (a, b).  Vertices are numbered angle by angle;
+// midpoints follow in the order in which the edges (v1 v2), (v2 v4), (v4 v1) of
+// the triangles meet them (edge_connectivity, mesher.jl:349-392): the first
+// angular column of cells adds 4 per cell (theta edge above, diagonal, both
+// radial edges) and one more at the inner wall, the middle ones 3, the last
+// one 2 (its far radial edges are the first column's near ones).  A few integer
+// operations instead of an 8-byte table entry per node.
+__host__ __device__ inline int ref_of_lattice(int a, int b, int ncr, int nct) {
+  const int ia = a >> 1, jb = b >> 1;
+  if (!((a | b) & 1)) return ia + (ncr + 1) * jb;
+  const int nv = (ncr + 1) * nct;
+  if (b & 1) {
+    const int base = jb == 0 ? 0 : 4 * ncr + 1 + (jb - 1) * (3 * ncr + 1);
+    const int per = jb == 0 ? 4 : (jb == nct - 1 ? 2 : 3);
+    return nv + base + per * ia + (a & 1);
+  }
+  if (jb == 0) return nv + 4 * ia + 2;
+  if (jb == 1) return nv + 4 * ia + 3;
+  return nv + 4 * ncr + 1 + (jb - 2) * (3 * ncr + 1) + 3 * ia + 2;
+}
+
+// Lattice (a, b) of the 6 local nodes of element e and their reference numbers.
+__host__ __device__ inline void element_ref_nodes(int e, int ncr, int nct, int n[6]) {
+  const int q = e >> 1, t = e & 1;
+  const int ir = q % ncr, it = q / ncr, a0 = 2 * ir, b0 = 2 * it, b2 = it + 1 == nct ? 0 : b0 + 2;
+  if (t == 0) {
+    n[0] = ref_of_lattice(a0, b0, ncr, nct);
+    n[1] = ref_of_lattice(a0, b2, ncr, nct);
+    n[2] = ref_of_lattice(a0 + 2, b0, ncr, nct);
+    n[3] = ref_of_lattice(a0, b0 + 1, ncr, nct);
+    n[4] = ref_of_lattice(a0 + 1, b0 + 1, ncr, nct);
+    n[5] = ref_of_lattice(a0 + 1, b0, ncr, nct);
+  } else {
+    n[0] = ref_of_lattice(a0, b2, ncr, nct);
+    n[1] = ref_of_lattice(a0 + 2, b2, ncr, nct);
+    n[2] = ref_of_lattice(a0 + 2, b0, ncr, nct);
+    n[3] = ref_of_lattice(a0 + 1, b2, ncr, nct);
+    n[4] = ref_of_lattice(a0 + 2, b0 + 1, ncr, nct);
+    n[5] = ref_of_lattice(a0 + 1, b0 + 1, ncr, nct);
+  }
 }
 
 __host__ __device__ inline void element_pdofs_cont(int64_t e, int ncr, int nct, int64_t p[3]) {

@@ -25,21 +25,27 @@ struct DemDev {
   double w;
 };
 
-// F: 4 doubles per (ip, e) at (ip * nel + e) * 4; out: field-major 6 x n
-// (vx1, vx2, vy1, vy2, a1, a2), n = 6 nel (ip * nel + e).
-__global__ void __launch_bounds__(256) k_fse_ip(const double* __restrict__ F, double* __restrict__ out, int64_t n) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double2 f0 = reinterpret_cast<const double2*>(F)[2 * i];
-  const double2 f1 = reinterpret_cast<const double2*>(F)[2 * i + 1];
+// F: 4 doubles per (ip, e) at (ip * nel + e) * 4, 16-byte aligned; out: the six
+// fields (vx1, vx2, vy1, vy2, a1, a2), 6 columns of ld each.
+struct Fields6 {
+  double* f[6];
+  int64_t ld;
+};
+__global__ void __launch_bounds__(256) k_fse_ip(const double* __restrict__ F, Fields6 out, int nel) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 6 * nel) return;
+  const double2 f0 = reinterpret_cast<const double2*>(F)[2 * (int64_t)i];
+  const double2 f1 = reinterpret_cast<const double2*>(F)[2 * (int64_t)i + 1];
   double vx, vy, l1, l2;
   fse_axes(f0.x, f0.y, f1.x, f1.y, vx, vy, l1, l2);
-  out[i] = vx;
-  out[n + i] = -vy;  // minor axis, perpendicular to the major one
-  out[2 * n + i] = vy;
-  out[3 * n + i] = vx;
-  out[4 * n + i] = sqrt(fabs(l1));
-  out[5 * n + i] = sqrt(fabs(l2));
+  const int ip = i / nel;
+  const int64_t o = ip * out.ld + (i - ip * nel);
+  out.f[0][o] = vx;
+  out.f[1][o] = -vy;  // minor axis, perpendicular to the major one
+  out.f[2][o] = vy;
+  out.f[3][o] = vx;
+  out.f[4][o] = sqrt(fabs(l1));
+  out.f[5][o] = sqrt(fabs(l2));
 }
 
 // argminsorted (anisotropy.jl:110-118), 0-based
@@ -73,18 +79,21 @@ __device__ __forceinline__ void direct_rotation_2d(double cosa, double sina, dou
 
 constexpr int kDemEl = 32;  // elements per CTA: warps 0..5 one IP each, warp 6 the IP-7 mean
 
-// in: field-major 4 x 6 nel (vx1, vy1, r1, r2; ip * nel + e); out: 6 x 7 nel.
-// Every load and store is a coalesced row of an element-fastest matrix.
-__global__ void __launch_bounds__(kDemEl * 7) k_dem_tensor(const double* __restrict__ in, double* __restrict__ out,
-                                                           DemDev d, int nel) {
+// in: vx1, vy1, r1, r2 (6 columns of ld_in each); out: the six tensor fields (7
+// columns of ld each).  Every load and store is a coalesced row of an
+// element-fastest matrix.
+struct DemIn {
+  const double *x, *y, *r1, *r2;
+  int64_t ld;
+};
+__global__ void __launch_bounds__(kDemEl * 7) k_dem_tensor(DemIn in, Fields6 out, DemDev d, int nel) {
   __shared__ double sh[6][6][kDemEl];  // field, ip, element
   const int tx = threadIdx.x, ip = threadIdx.y;
   const int e = blockIdx.x * kDemEl + tx;
   const bool valid = e < nel;
-  const size_t st = (size_t)nel, n6 = 6 * st, n7 = 7 * st;
   if (valid && ip < 6) {
-    const size_t i = (size_t)ip * st + e;
-    const double x = in[i], y = in[n6 + i], r1 = in[2 * n6 + i], r2 = in[3 * n6 + i];
+    const int64_t i = ip * in.ld + e, o = ip * out.ld + e;
+    const double x = in.x[i], y = in.y[i], r1 = in.r1[i], r2 = in.r2[i];
     const int i1 = argmin_sorted(r1, d.b1, d.n1);
     const int64_t i2 = d.perm[argmin_sorted(r2, d.b2, d.sblk)];  // 1-based, checked on the host
     const int64_t row = (int64_t)d.sblk * i1 + i2 - 1;
@@ -96,7 +105,7 @@ __global__ void __launch_bounds__(kDemEl * 7) k_dem_tensor(const double* __restr
     n[2] = jmax(n[2], d.w);
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-      out[k * n7 + i] = n[k];
+      out.f[k][o] = n[k];
       sh[k][ip][tx] = n[k];
     }
   }
@@ -107,15 +116,15 @@ __global__ void __launch_bounds__(kDemEl * 7) k_dem_tensor(const double* __restr
       double acc = 0.0;
 #pragma unroll
       for (int q = 0; q < 6; ++q) acc += sh[k][q][tx];
-      out[k * n7 + 6 * st + e] = acc * (1.0 / 6.0);
+      out.f[k][6 * out.ld + e] = acc * (1.0 / 6.0);
     }
   }
 }
 
-static DemDev staged_dem(Ctx& c, double* tab) {
+static DemDev staged_dem(Ctx& c) {
   DemDev d;
-  d.C = tab;
-  d.b1 = tab + 9 * c.fabric_dem[0];
+  d.C = c.dem_tab;
+  d.b1 = d.C + 9 * c.fabric_dem[0];
   d.b2 = d.b1 + c.fabric_dem[1];
   d.perm = reinterpret_cast<const int64_t*>(d.b2 + c.fabric_dem[2]);
   d.nrows = c.fabric_dem[0];
@@ -125,19 +134,38 @@ static DemDev staged_dem(Ctx& c, double* tab) {
   return d;
 }
 
-static void launch_k_dem_tensor(Ctx& c, const double* in, double* o, const DemDev& d) {
-  const int64_t nel = c.fine.nel;
-  ++g_klaunch;
-  k_dem_tensor<<<(int)div_up(nel, kDemEl), dim3(kDemEl, 7), 0, c.stream>>>(in, o, d, (int)nel);
-  DP_LAUNCH_CHECK();
+// The DEM table to the device as one copy from pinned memory (four copies from
+// pageable memory each wait for their staging).
+static void upload_dem(Ctx& c, const dp_dem& dem) {
+  const int64_t n = 9 * dem.nrows + dem.n_a1a2 + 2 * dem.sblk;
+  if (c.dem_cap < n) {
+    cudaFree(c.dem_tab);
+    cudaFreeHost(c.h_dem);
+    c.dem_tab = c.h_dem = nullptr;
+    c.dem_cap = 0;
+    dalloc(&c.dem_tab, (size_t)n);
+    DP_CUDA(cudaMallocHost((void**)&c.h_dem, sizeof(double) * n));
+    c.dem_cap = n;
+  }
+  c.fabric_dem[0] = dem.nrows;
+  c.fabric_dem[1] = dem.n_a1a2;
+  c.fabric_dem[2] = dem.sblk;
+  c.fabric_w = dem.w;
+  double* h = c.h_dem;   // every call ends with a synchronisation, so the last upload has been read
+  std::memcpy(h, dem.C, sizeof(double) * 9 * dem.nrows);
+  h += 9 * dem.nrows;
+  std::memcpy(h, dem.a1a2_blk, sizeof(double) * dem.n_a1a2);
+  h += dem.n_a1a2;
+  std::memcpy(h, dem.a2a3_blk, sizeof(double) * dem.sblk);
+  std::memcpy(h + dem.sblk, dem.permutation_blk, sizeof(int64_t) * dem.sblk);
+  DP_CUDA(cudaMemcpyAsync(c.dem_tab, c.h_dem, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream));
 }
 
-// k_dem_tensor on the inputs and table staged by the last
-// dp_anisotropic_tensor call (kernel timing)
-void launch_dem_staged(Ctx& c) {
+static void launch_k_dem_tensor(Ctx& c, const DemIn& in, const Fields6& out) {
   const int64_t nel = c.fine.nel;
-  double* in = c.fabric_buf;
-  launch_k_dem_tensor(c, in, in + 24 * nel, staged_dem(c, in + 66 * nel));
+  ++g_klaunch;
+  k_dem_tensor<<<(int)div_up(nel, kDemEl), dim3(kDemEl, 7), 0, c.stream>>>(in, out, staged_dem(c), (int)nel);
+  DP_LAUNCH_CHECK();
 }
 
 static double* fabric_scratch(Ctx& c, int64_t n) {
@@ -146,9 +174,27 @@ static double* fabric_scratch(Ctx& c, int64_t n) {
     c.fabric_buf = nullptr;
     c.fabric_cap = 0;
     dalloc(&c.fabric_buf, (size_t)n);
+    DP_CUDA(cudaMemsetAsync(c.fabric_buf, 0, sizeof(double) * n, c.stream));
     c.fabric_cap = n;
   }
   return c.fabric_buf;
+}
+
+// staging of the tensor lookup: 4 inputs of 6 columns, 6 outputs of 7
+static void dem_staging(Ctx& c, DemIn& in, Fields6& out) {
+  const int64_t nel = c.fine.nel;
+  double* b = fabric_scratch(c, 66 * nel);
+  in = DemIn{b, b + 6 * nel, b + 12 * nel, b + 18 * nel, nel};
+  for (int f = 0; f < 6; ++f) out.f[f] = b + 24 * nel + (int64_t)f * 7 * nel;
+  out.ld = nel;
+}
+
+// k_dem_tensor on the staging buffer and the last call's table (kernel timing)
+void launch_dem_staged(Ctx& c) {
+  DemIn in;
+  Fields6 out;
+  dem_staging(c, in, out);
+  launch_k_dem_tensor(c, in, out);
 }
 
 }  // namespace dp
@@ -165,17 +211,28 @@ extern "C" int dp_fse(dp_ctx* h, const double* F, double* const* fse, int64_t ld
       if (!fse[f]) throw BadArg("null output field");
     const int64_t nel = c.fine.nel, n = 6 * nel;
     if (ld_out < nel) throw BadArg("leading dimension below nel");
-    double* buf = fabric_scratch(c, 4 * n + 6 * n);
-    c.fabric_dem[0] = 0;  // the staged DEM table is overwritten
-    double* dF = buf;
-    double* o = buf + 4 * n;
-    DP_CUDA(cudaMemcpyAsync(dF, F, sizeof(double) * 4 * n, kind_in(mem), c.stream));
+    bool dev = mem == DP_MEM_DEVICE;
+    for (int f = 0; f < 6; ++f) dev = dev && !overlap(fse[f], 5 * ld_out + nel, F, 4 * n);
+    c.fabric_dem[0] = 0;  // the staged inputs of the tensor lookup are overwritten
+    Fields6 out;
+    const double* dF = F;
+    for (int f = 0; f < 6; ++f) out.f[f] = fse[f];
+    out.ld = ld_out;
+    if (!dev || !aligned16(F)) {   // the kernel reads F in 16-byte pairs
+      double* buf = fabric_scratch(c, 10 * n);
+      DP_CUDA(cudaMemcpyAsync(buf, F, sizeof(double) * 4 * n, kind_in(mem), c.stream));
+      dF = buf;
+    }
+    if (!dev) {
+      for (int f = 0; f < 6; ++f) out.f[f] = c.fabric_buf + 4 * n + (int64_t)f * n;
+      out.ld = nel;
+    }
     ++g_klaunch;
-    k_fse_ip<<<(int)div_up(n, 256), 256, 0, c.stream>>>(dF, o, n);
+    k_fse_ip<<<(int)div_up(n, 256), 256, 0, c.stream>>>(dF, out, (int)nel);
     DP_LAUNCH_CHECK();
-    for (int f = 0; f < 6; ++f)
-      DP_CUDA(cudaMemcpy2DAsync(fse[f], sizeof(double) * ld_out, o + (size_t)f * n, sizeof(double) * nel,
-                                sizeof(double) * nel, 6, kind_out(mem), c.stream));
+    for (int f = 0; !dev && f < 6; ++f)
+      DP_CUDA(cudaMemcpy2DAsync(fse[f], sizeof(double) * ld_out, out.f[f], sizeof(double) * nel, sizeof(double) * nel,
+                                6, kind_out(mem), c.stream));
     DP_CUDA(cudaStreamSynchronize(c.stream));
     return (int)DP_OK;
   });
@@ -201,31 +258,25 @@ extern "C" int dp_anisotropic_tensor(dp_ctx* h, const dp_dem* dem, const double*
     if (!std::isfinite(dem->w)) throw BadArg("cut-off w must be finite");
     const int64_t nel = c.fine.nel;
     if (ld_in < nel || ld_out < nel) throw BadArg("leading dimension below nel");
-    const int64_t ntab = 9 * dem->nrows + dem->n_a1a2 + 2 * dem->sblk;
-    double* buf = fabric_scratch(c, 24 * nel + 42 * nel + ntab);
-    double* in = buf;
-    double* o = in + 24 * nel;
-    double* tab = o + 42 * nel;
-    const cudaMemcpyKind kin = kind_in(mem);
-    const double* src[4] = {vx1, vy1, r1, r2};
-    for (int f = 0; f < 4; ++f)
-      DP_CUDA(cudaMemcpy2DAsync(in + (size_t)f * 6 * nel, sizeof(double) * nel, src[f], sizeof(double) * ld_in,
-                                sizeof(double) * nel, 6, kin, c.stream));
-    c.fabric_dem[0] = dem->nrows;
-    c.fabric_dem[1] = dem->n_a1a2;
-    c.fabric_dem[2] = dem->sblk;
-    c.fabric_w = dem->w;
-    const DemDev d = staged_dem(c, tab);
-    DP_CUDA(cudaMemcpyAsync(tab, dem->C, sizeof(double) * 9 * dem->nrows, cudaMemcpyHostToDevice, c.stream));
-    DP_CUDA(cudaMemcpyAsync((void*)d.b1, dem->a1a2_blk, sizeof(double) * dem->n_a1a2, cudaMemcpyHostToDevice,
-                            c.stream));
-    DP_CUDA(cudaMemcpyAsync((void*)d.b2, dem->a2a3_blk, sizeof(double) * dem->sblk, cudaMemcpyHostToDevice,
-                            c.stream));
-    DP_CUDA(cudaMemcpyAsync((void*)d.perm, dem->permutation_blk, sizeof(int64_t) * dem->sblk,
-                            cudaMemcpyHostToDevice, c.stream));
-    launch_k_dem_tensor(c, in, o, d);
+    upload_dem(c, *dem);
+    DemIn in{vx1, vy1, r1, r2, ld_in};
+    Fields6 out;
+    for (int f = 0; f < 6; ++f) out.f[f] = C6_out[f];
+    out.ld = ld_out;
+    bool dev = mem == DP_MEM_DEVICE;
     for (int f = 0; f < 6; ++f)
-      DP_CUDA(cudaMemcpy2DAsync(C6_out[f], sizeof(double) * ld_out, o + (size_t)f * 7 * nel, sizeof(double) * nel,
+      for (const double* a : {vx1, vy1, r1, r2}) dev = dev && !overlap(C6_out[f], 6 * ld_out + nel, a, 5 * ld_in + nel);
+    if (!dev) {
+      dem_staging(c, in, out);
+      const double* src[4] = {vx1, vy1, r1, r2};
+      const double* dst[4] = {in.x, in.y, in.r1, in.r2};
+      for (int f = 0; f < 4; ++f)
+        DP_CUDA(cudaMemcpy2DAsync((void*)dst[f], sizeof(double) * nel, src[f], sizeof(double) * ld_in,
+                                  sizeof(double) * nel, 6, kind_in(mem), c.stream));
+    }
+    launch_k_dem_tensor(c, in, out);
+    for (int f = 0; !dev && f < 6; ++f)
+      DP_CUDA(cudaMemcpy2DAsync(C6_out[f], sizeof(double) * ld_out, out.f[f], sizeof(double) * nel,
                                 sizeof(double) * nel, 7, kind_out(mem), c.stream));
     DP_CUDA(cudaStreamSynchronize(c.stream));
     return (int)DP_OK;

@@ -656,30 +656,43 @@ void launch_sum(Ctx& c, const double* a, int64_t n, int slot) {
 }
 
 // ---- permutations between reference numbering and the lattice -------------
-__global__ void k_gather_ref2lat(const int64_t* __restrict__ ref2lat, const double* __restrict__ ref,
-                                 double* __restrict__ lat, int64_t nnod, int comps) {
-  grid_dep_wait();
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// One thread per lattice node; V = double2 moves both components at once (a
+// caller's array that is only 8-byte aligned takes two scalar accesses).
+template <typename V, int COMPS>
+__global__ void k_gather_ref2lat(const double* ref, double* lat, int nnod, int A, int ncr, int nct) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
-  const int64_t l = ref2lat[n];
-  for (int c = 0; c < comps; ++c) lat[comps * l + c] = ref[comps * n + c];
+  const int b = n / A, m = ref_of_lattice(n - b * A, b, ncr, nct);
+#pragma unroll
+  for (int c = 0; c < COMPS; ++c)
+    reinterpret_cast<V*>(lat)[(size_t)COMPS * n + c] = reinterpret_cast<const V*>(ref)[(size_t)COMPS * m + c];
 }
-__global__ void k_scatter_lat2ref(const int64_t* __restrict__ ref2lat, const double* __restrict__ lat,
-                                  double* __restrict__ ref, int64_t nnod, int comps) {
-  grid_dep_wait();
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+template <typename V, int COMPS>
+__global__ void k_scatter_lat2ref(const double* lat, double* ref, int nnod, int A, int ncr, int nct) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
-  const int64_t l = ref2lat[n];
-  for (int c = 0; c < comps; ++c) ref[comps * n + c] = lat[comps * l + c];
+  const int b = n / A, m = ref_of_lattice(n - b * A, b, ncr, nct);
+#pragma unroll
+  for (int c = 0; c < COMPS; ++c)
+    reinterpret_cast<V*>(ref)[(size_t)COMPS * m + c] = reinterpret_cast<const V*>(lat)[(size_t)COMPS * n + c];
 }
+static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 void launch_gather_ref2lat(Ctx& c, const double* ref, double* lat, int comps) {
-  const int64_t n = c.fine.nnod;
-  klaunch(k_gather_ref2lat, (int)div_up(n, 256), 256, 0, c.stream, c.ref2lat, ref, lat, n, comps);
+  const Level& L = c.fine;
+  const int n = (int)L.nnod, A = (int)L.A(), blocks = (int)div_up(n, 256);
+  g_klaunch += 1;
+  if (comps == 1) k_gather_ref2lat<double, 1><<<blocks, 256, 0, c.stream>>>(ref, lat, n, A, L.ncr, L.nct);
+  else if (aligned16(ref)) k_gather_ref2lat<double2, 1><<<blocks, 256, 0, c.stream>>>(ref, lat, n, A, L.ncr, L.nct);
+  else k_gather_ref2lat<double, 2><<<blocks, 256, 0, c.stream>>>(ref, lat, n, A, L.ncr, L.nct);
   DP_LAUNCH_CHECK();
 }
 void launch_scatter_lat2ref(Ctx& c, const double* lat, double* ref, int comps) {
-  const int64_t n = c.fine.nnod;
-  klaunch(k_scatter_lat2ref, (int)div_up(n, 256), 256, 0, c.stream, c.ref2lat, lat, ref, n, comps);
+  const Level& L = c.fine;
+  const int n = (int)L.nnod, A = (int)L.A(), blocks = (int)div_up(n, 256);
+  g_klaunch += 1;
+  if (comps == 1) k_scatter_lat2ref<double, 1><<<blocks, 256, 0, c.stream>>>(lat, ref, n, A, L.ncr, L.nct);
+  else if (aligned16(ref)) k_scatter_lat2ref<double2, 1><<<blocks, 256, 0, c.stream>>>(lat, ref, n, A, L.ncr, L.nct);
+  else k_scatter_lat2ref<double, 2><<<blocks, 256, 0, c.stream>>>(lat, ref, n, A, L.ncr, L.nct);
   DP_LAUNCH_CHECK();
 }
 

@@ -35,63 +35,79 @@ static void upload_rheology_constants() {
   DP_CUDA(cudaMemcpyToSymbol(c_N6s, N6, sizeof(N6)));
 }
 
-// per-block min of P and max of r -> partial[b], partial[nb + b]
-__global__ void __launch_bounds__(kRedThreads) k_minmax_partial(const double* __restrict__ P, int64_t np,
-                                                                const double* __restrict__ r, int64_t nn,
-                                                                double* __restrict__ partial) {
+// |min P| over the vertices and max r over the nodes, in one launch: the last
+// block to arrive reduces the per-block values (a second launch of one thread
+// over the 1184 pairs took 80 us).
+__global__ void __launch_bounds__(kRedThreads) k_minmax(const double* __restrict__ P, int64_t np,
+                                                        const double* __restrict__ r, int64_t nn, double* partial,
+                                                        unsigned int* counter, double* scal) {
+  __shared__ double smn[kRedThreads / 32], smx[kRedThreads / 32];
+  __shared__ bool last;
   double mn = INFINITY, mx = -INFINITY;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x)
     mn = fmin(mn, P[i]);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nn; i += (int64_t)gridDim.x * blockDim.x)
     mx = fmax(mx, r[i]);
+  auto block_minmax = [&]() {   // in thread 0
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = fmin(mn, __shfl_down_sync(0xffffffffu, mn, o));
-    mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
-  }
-  __shared__ double smn[kRedThreads / 32], smx[kRedThreads / 32];
-  if ((threadIdx.x & 31) == 0) {
-    smn[threadIdx.x >> 5] = mn;
-    smx[threadIdx.x >> 5] = mx;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < kRedThreads / 32; ++w) {
-      mn = fmin(mn, smn[w]);
-      mx = fmax(mx, smx[w]);
+    for (int o = 16; o > 0; o >>= 1) {
+      mn = fmin(mn, __shfl_down_sync(0xffffffffu, mn, o));
+      mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
     }
+    if ((threadIdx.x & 31) == 0) {
+      smn[threadIdx.x >> 5] = mn;
+      smx[threadIdx.x >> 5] = mx;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < kRedThreads / 32; ++w) {
+        mn = fmin(mn, smn[w]);
+        mx = fmax(mx, smx[w]);
+      }
+    }
+  };
+  block_minmax();
+  if (threadIdx.x == 0) {
     partial[blockIdx.x] = mn;
     partial[gridDim.x + blockIdx.x] = mx;
+    __threadfence();
+    last = atomicInc(counter, gridDim.x) == gridDim.x - 1;
   }
-}
-
-__global__ void k_minmax_final(const double* __restrict__ partial, int nb, double* __restrict__ scal) {
-  double mn = INFINITY, mx = -INFINITY;
-  for (int b = 0; b < nb; ++b) {
-    mn = fmin(mn, partial[b]);
-    mx = fmax(mx, partial[nb + b]);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  mn = INFINITY;
+  mx = -INFINITY;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+    mn = fmin(mn, ((volatile double*)partial)[b]);
+    mx = fmax(mx, ((volatile double*)partial)[gridDim.x + b]);
   }
-  scal[S_MINP] = fabs(mn);
-  scal[S_MAXR] = mx;
+  block_minmax();
+  if (threadIdx.x == 0) {
+    scal[S_MINP] = fabs(mn);
+    scal[S_MAXR] = mx;
+    *counter = 0;
+  }
 }
 
 struct ArrheniusArgs {
   double eta0, R, Ea, Va, T0, sphi, cphi, phi;
 };
 
-// T, P (vertex entries; others unused), r: lattice order.  epsII, tauII, coh,
-// eta: nel x 7 element-fastest.
+// T, r (nodes) and P (vertices): reference numbering.  epsII, tauII, coh, eta:
+// nel x 7 element-fastest.  All of them the caller's own arrays when they are on
+// the device.
 __global__ void __launch_bounds__(128) k_viscosity_arrhenius(const double* __restrict__ T, const double* __restrict__ P,
                                                              const double* __restrict__ r,
                                                              const double* __restrict__ epsII,
                                                              const double* __restrict__ tauII,
-                                                             const double* __restrict__ coh, double* __restrict__ eta,
-                                                             const double* __restrict__ scal, ArrheniusArgs law,
-                                                             int nel, int ncr, int A, int B) {
+                                                             const double* __restrict__ coh, double* eta,
+                                                             const double* scal, ArrheniusArgs law, int nel, int ncr,
+                                                             int nct) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nel) return;
-  int64_t nd[6];
-  element_nodes(e, ncr, A, B, nd);
+  int nd[6];
+  element_ref_nodes(e, ncr, nct, nd);
   double Te[6], re[6], Pe[3];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
@@ -99,7 +115,7 @@ __global__ void __launch_bounds__(128) k_viscosity_arrhenius(const double* __res
     re[k] = r[nd[k]];
   }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) Pe[k] = P[nd[k]];
+  for (int k = 0; k < 3; ++k) Pe[k] = P[nd[k]];   // vertices are the first reference numbers
   const double minP = scal[S_MINP], maxr = scal[S_MAXR];
   const size_t st = (size_t)nel;
   for (int ip = 0; ip < 7; ++ip) {
@@ -124,22 +140,38 @@ __global__ void __launch_bounds__(128) k_viscosity_arrhenius(const double* __res
   }
 }
 
-// k_viscosity_arrhenius on the inputs staged by the last dp_viscosity_arrhenius
-// call (kernel timing; eta is updated in place, and a second pass over it
-// writes the same values).
-void launch_viscosity_staged(Ctx& c) {
-  const int64_t nel = c.fine.nel, nn = c.fine.nnod;
-  double* e2 = c.rheo_buf;
-  double* Tl = e2 + 28 * nel;
+static ArrheniusArgs last_law(const Ctx& c) {
   ArrheniusArgs a;
   a.eta0 = c.rheo_law[0]; a.R = c.rheo_law[1]; a.Ea = c.rheo_law[2]; a.Va = c.rheo_law[3];
   a.T0 = c.rheo_law[4]; a.sphi = c.rheo_law[5]; a.cphi = c.rheo_law[6]; a.phi = c.rheo_law[7];
+  return a;
+}
+static void launch_viscosity(Ctx& c, const double* T, const double* P, const double* r, const double* e2,
+                             const double* t2, const double* co, double* et) {
+  const int nel = (int)c.fine.nel;
   ++g_klaunch;
-  k_viscosity_arrhenius<<<(int)div_up(nel, 128), 128, 0, c.stream>>>(Tl, Tl + nn, Tl + 2 * nn, e2, e2 + 7 * nel,
-                                                                      e2 + 14 * nel, e2 + 21 * nel, c.scal, a,
-                                                                      (int)nel, c.fine.ncr, (int)c.fine.A(),
-                                                                      (int)c.fine.B());
+  k_viscosity_arrhenius<<<(int)div_up(nel, 128), 128, 0, c.stream>>>(T, P, r, e2, t2, co, et, c.scal, last_law(c), nel,
+                                                                      c.fine.ncr, c.fine.nct);
   DP_LAUNCH_CHECK();
+}
+// the staging buffer: epsII, tauII, cohesion, eta (7 columns each), T, P, r
+// (zero until host arrays are staged)
+static double* rheo_staging(Ctx& c) {
+  const int64_t n = 28 * c.fine.nel + 3 * c.fine.nnod;
+  if (!c.rheo_buf) {
+    dalloc(&c.rheo_buf, n);
+    DP_CUDA(cudaMemsetAsync(c.rheo_buf, 0, sizeof(double) * n, c.stream));
+  }
+  return c.rheo_buf;
+}
+
+// k_viscosity_arrhenius on the staging buffer (kernel timing; eta is updated in
+// place, and a second pass over it writes the same values).
+void launch_viscosity_staged(Ctx& c) {
+  const int64_t nel = c.fine.nel, nn = c.fine.nnod;
+  double* e2 = rheo_staging(c);
+  double* Ts = e2 + 28 * nel;
+  launch_viscosity(c, Ts, Ts + nn, Ts + 2 * nn, e2, e2 + 7 * nel, e2 + 14 * nel, e2 + 21 * nel);
 }
 
 }  // namespace dp
@@ -166,44 +198,38 @@ extern "C" int dp_viscosity_arrhenius(dp_ctx* h, const dp_arrhenius* law, const 
       DP_CUDA(cudaDeviceSynchronize());  // the copies are on the default stream; ours does not wait on it
       if (c.device >= 0 && c.device < 64) uploaded[c.device] = true;
     }
-    if (!c.rheo_buf) dalloc(&c.rheo_buf, 28 * nel + 4 * nn);
-    double* e2 = c.rheo_buf;
-    double* t2 = e2 + 7 * nel;
-    double* co = t2 + 7 * nel;
-    double* et = co + 7 * nel;
-    double* Tl = et + 7 * nel;
-    double* Pl = Tl + nn;
-    double* rl = Pl + nn;
-    double* stage = rl + nn;  // nnod: reference-numbered input before the permutation
-    const cudaMemcpyKind kin = kind_in(mem);
-    DP_CUDA(cudaMemcpyAsync(e2, epsII, sizeof(double) * 7 * nel, kin, c.stream));
-    DP_CUDA(cudaMemcpyAsync(t2, tauII, sizeof(double) * 7 * nel, kin, c.stream));
-    DP_CUDA(cudaMemcpyAsync(co, cohesion, sizeof(double) * 7 * nel, kin, c.stream));
-    DP_CUDA(cudaMemcpyAsync(et, eta_ip, sizeof(double) * 7 * nel, kin, c.stream));
-    DP_CUDA(cudaMemcpyAsync(stage, T_node, sizeof(double) * nn, kin, c.stream));
-    launch_gather_ref2lat(c, stage, Tl, 1);
-    DP_CUDA(cudaMemcpyAsync(stage, r_node, sizeof(double) * nn, kin, c.stream));
-    launch_gather_ref2lat(c, stage, rl, 1);
-    // vertices are the first nvert nodes of the reference numbering
-    DP_CUDA(cudaMemsetAsync(stage, 0, sizeof(double) * nn, c.stream));
-    DP_CUDA(cudaMemcpyAsync(stage, P_vertex, sizeof(double) * nv, kin, c.stream));
-    launch_gather_ref2lat(c, stage, Pl, 1);
-    // |min P| over the vertices (reference numbering) and max r
+    bool dev = mem == DP_MEM_DEVICE && !overlap(eta_ip, 7 * nel, T_node, nn) &&
+               !overlap(eta_ip, 7 * nel, P_vertex, nv) && !overlap(eta_ip, 7 * nel, r_node, nn);
+    for (const double* a : {epsII, tauII, cohesion}) dev = dev && !overlap(eta_ip, 7 * nel, a, 7 * nel);
+    const double *T = T_node, *P = P_vertex, *r = r_node, *e2 = epsII, *t2 = tauII, *co = cohesion;
+    double* et = eta_ip;
+    if (!dev) {
+      double* s = rheo_staging(c);
+      auto up = [&](double* dst, const double* src, int64_t n) {
+        DP_CUDA(cudaMemcpyAsync(dst, src, sizeof(double) * n, kind_in(mem), c.stream));
+        return dst;
+      };
+      e2 = up(s, epsII, 7 * nel);
+      t2 = up(s + 7 * nel, tauII, 7 * nel);
+      co = up(s + 14 * nel, cohesion, 7 * nel);
+      et = up(s + 21 * nel, eta_ip, 7 * nel);
+      T = up(s + 28 * nel, T_node, nn);
+      P = up(s + 28 * nel + nn, P_vertex, nv);
+      r = up(s + 28 * nel + 2 * nn, r_node, nn);
+    }
     ++g_klaunch;
-    k_minmax_partial<<<kRedBlocks, kRedThreads, 0, c.stream>>>(stage, nv, rl, nn, c.partial);
-    ++g_klaunch;
-    k_minmax_final<<<1, 1, 0, c.stream>>>(c.partial, kRedBlocks, c.scal);
+    k_minmax<<<(int)std::min<int64_t>(kRedBlocks, div_up(nn, 4 * kRedThreads)), kRedThreads, 0, c.stream>>>(
+        P, nv, r, nn, c.partial, c.counter, c.scal);
+    DP_LAUNCH_CHECK();
     ArrheniusArgs a;
     a.eta0 = law->eta0; a.R = law->R; a.Ea = law->Ea; a.Va = law->Va; a.T0 = law->T0; a.phi = law->phi_deg;
     a.sphi = std::sin(law->phi_deg * (3.14159265358979323846 / 180.0));
     a.cphi = std::cos(law->phi_deg * (3.14159265358979323846 / 180.0));
     const double keep[8] = {a.eta0, a.R, a.Ea, a.Va, a.T0, a.sphi, a.cphi, a.phi};
     for (int i = 0; i < 8; ++i) c.rheo_law[i] = keep[i];
-    ++g_klaunch;
-    k_viscosity_arrhenius<<<(int)div_up(nel, 128), 128, 0, c.stream>>>(Tl, Pl, rl, e2, t2, co, et, c.scal, a, (int)nel,
-                                                                        c.fine.ncr, (int)c.fine.A(), (int)c.fine.B());
-    DP_LAUNCH_CHECK();
-    DP_CUDA(cudaMemcpyAsync(eta_ip, et, sizeof(double) * 7 * nel, kind_out(mem), c.stream));
+    c.rheo_called = true;
+    launch_viscosity(c, T, P, r, e2, t2, co, et);
+    if (!dev) DP_CUDA(cudaMemcpyAsync(eta_ip, et, sizeof(double) * 7 * nel, kind_out(mem), c.stream));
     DP_CUDA(cudaStreamSynchronize(c.stream));
     return (int)DP_OK;
   });

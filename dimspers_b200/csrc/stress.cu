@@ -36,35 +36,48 @@ static void upload_stress_constants() {
   DP_CUDA(cudaMemcpyToSymbol(c_dNs, dN, sizeof(dN)));
 }
 
-// U: Cartesian velocity, lattice order, interleaved (ux, uz).  eta: 7*nel
-// (ip-major), C: 42*nel ((field*7 + ip)*nel + e) or null.  out: 56*nel.
-__global__ void __launch_bounds__(128) k_stress(const double* __restrict__ U, const double* __restrict__ theta_lat,
-                                                const double* __restrict__ r_lat, const double* __restrict__ eta,
-                                                const double* __restrict__ C, double* __restrict__ out, int nel,
-                                                int ncr, int A, int B) {
+// The caller's arrays: eta 7 columns of ld_eta, the six tensor fields 7 columns
+// of ld_C each, out 56 columns of nel; U the Cartesian velocity in the reference
+// numbering, interleaved (ux, uz).
+struct StressArgs {
+  const double* U;
+  const double* theta_lat;
+  const double* r_lat;
+  const double* eta;
+  const double* C[6];
+  double* out;
+  int64_t ld_eta, ld_C;
+  int nel, ncr, nct, A, B, tensor, u16;   // u16: U is 16-byte aligned
+};
+
+// Reads and writes the caller's device arrays in place (host arrays are staged):
+// at 256x2048 with a tensor 822 us per call when every array went through a
+// staging copy and U through a permutation pass of its own, of which this
+// kernel was 184 us.
+__global__ void __launch_bounds__(128) k_stress(StressArgs p) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nel) return;
-  const int q = e >> 1, t = e & 1;
-  const int ir = q % ncr, it = q / ncr;
-  const int a0 = 2 * ir, b0 = 2 * it;
-  int aa[6], bb[6];
-  if (t == 0) {
-    aa[0] = a0; aa[1] = a0; aa[2] = a0 + 2; aa[3] = a0; aa[4] = a0 + 1; aa[5] = a0 + 1;
-    bb[0] = b0; bb[1] = b0 + 2; bb[2] = b0; bb[3] = b0 + 1; bb[4] = b0 + 1; bb[5] = b0;
-  } else {
-    aa[0] = a0; aa[1] = a0 + 2; aa[2] = a0 + 2; aa[3] = a0 + 1; aa[4] = a0 + 2; aa[5] = a0 + 1;
-    bb[0] = b0 + 2; bb[1] = b0 + 2; bb[2] = b0; bb[3] = b0 + 2; bb[4] = b0 + 1; bb[5] = b0 + 1;
+  if (e >= p.nel) return;
+  const int A = p.A, B = p.B;
+  const double* __restrict__ theta_lat = p.theta_lat;
+  const double* __restrict__ r_lat = p.r_lat;
+  double ux[6], uz[6];
+  {
+    int m[6];
+    element_ref_nodes(e, p.ncr, p.nct, m);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      if (p.u16) {
+        const double2 v = reinterpret_cast<const double2*>(p.U)[m[k]];
+        ux[k] = v.x;
+        uz[k] = v.y;
+      } else {
+        ux[k] = p.U[2 * (size_t)m[k]];
+        uz[k] = p.U[2 * (size_t)m[k] + 1];
+      }
+    }
   }
   int nd[6];
-  double ux[6], uz[6];
-  const double2* U2 = reinterpret_cast<const double2*>(U);
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    nd[k] = aa[k] + A * (bb[k] >= B ? bb[k] - B : bb[k]);
-    const double2 v = U2[nd[k]];
-    ux[k] = v.x;
-    uz[k] = v.y;
-  }
+  element_nodes_mg(e, p.ncr, A, B, nd);
   // vertex coordinates + fixangles! (Utilities.jl:45-61)
   double th[3], rr[3];
 #pragma unroll
@@ -86,7 +99,7 @@ __global__ void __launch_bounds__(128) k_stress(const double* __restrict__ U, co
   const double invdet = 1.0 / (Jt0 * Jr1 - Jt1 * Jr0);
   const double R21 = rr[1] - rr[0], R31 = rr[2] - rr[0];
   const double T31 = th[2] - th[0], T21 = th[1] - th[0];
-  const size_t st = (size_t)nel;
+  const size_t st = (size_t)p.nel;
   for (int ip = 0; ip < 7; ++ip) {
     const double th_ip = th[0] * c_N3s[ip][0] + th[1] * c_N3s[ip][1] + th[2] * c_N3s[ip][2];
     const double r_ip = rr[0] * c_N3s[ip][0] + rr[1] * c_N3s[ip][1] + rr[2] * c_N3s[ip][2];
@@ -106,12 +119,12 @@ __global__ void __launch_bounds__(128) k_stress(const double* __restrict__ U, co
       duzdx += dx * uz[k];
     }
     const double exz = 0.5 * (duxdz + duzdx);
-    const double et = eta[(size_t)ip * st + e];
+    const double et = __ldg(p.eta + ip * p.ld_eta + e);
     double txx, tzz, txz;
-    if (C) {
-      const double c11 = C[(size_t)(0 * 7 + ip) * st + e] * et, c33 = C[(size_t)(1 * 7 + ip) * st + e] * et;
-      const double c55 = C[(size_t)(2 * 7 + ip) * st + e] * et, c13 = C[(size_t)(3 * 7 + ip) * st + e] * et;
-      const double c15 = C[(size_t)(4 * 7 + ip) * st + e] * et, c35 = C[(size_t)(5 * 7 + ip) * st + e] * et;
+    if (p.tensor) {
+      const size_t i = (size_t)(ip * p.ld_C + e);
+      const double c11 = __ldg(p.C[0] + i) * et, c33 = __ldg(p.C[1] + i) * et, c55 = __ldg(p.C[2] + i) * et;
+      const double c13 = __ldg(p.C[3] + i) * et, c15 = __ldg(p.C[4] + i) * et, c35 = __ldg(p.C[5] + i) * et;
       const double pa = -exx / 3.0 + 2.0 * ezz / 3.0, pb = 2.0 * exx / 3.0 - ezz / 3.0;
       txx = c13 * pa + c11 * pb + c15 * exz;
       tzz = c33 * pa + c13 * pb + c35 * 2.0 * exz;
@@ -121,7 +134,7 @@ __global__ void __launch_bounds__(128) k_stress(const double* __restrict__ U, co
       tzz = et * (-2.0 / 3.0 * exx + 4.0 / 3.0 * ezz);
       txz = et * 2.0 * exz;
     }
-    double* o = out + (size_t)ip * st + e;
+    double* o = p.out + (size_t)ip * st + e;
     const size_t blk = 7 * st;
     o[0 * blk] = exx;
     o[1 * blk] = ezz;
@@ -134,18 +147,37 @@ __global__ void __launch_bounds__(128) k_stress(const double* __restrict__ U, co
   }
 }
 
-// k_stress on the inputs staged by the last dp_stress call (kernel timing).
-void launch_stress_staged(Ctx& c, bool tensor) {
-  const int64_t nel = c.fine.nel;
-  double* eta = c.stress_buf;
-  double* C = eta + 7 * nel;
-  double* o = C + 42 * nel;
+static StressArgs stress_args(Ctx& c, bool tensor) {
+  StressArgs a{};
+  a.theta_lat = c.theta_lat; a.r_lat = c.r_lat;
+  a.nel = (int)c.fine.nel; a.ncr = c.fine.ncr; a.nct = c.fine.nct; a.A = (int)c.fine.A(); a.B = (int)c.fine.B();
+  a.tensor = tensor ? 1 : 0;
+  return a;
+}
+static void launch_stress(Ctx& c, StressArgs a) {
+  a.u16 = aligned16(a.U) ? 1 : 0;
   ++g_klaunch;
-  k_stress<<<(int)div_up(nel, 128), 128, 0, c.stream>>>((const double*)c.work[W_RES], c.theta_lat, c.r_lat, eta,
-                                                         tensor ? C : nullptr, o, (int)nel, c.fine.ncr,
-                                                         (int)c.fine.A(), (int)c.fine.B());
+  k_stress<<<(int)div_up(a.nel, 128), 128, 0, c.stream>>>(a);
   DP_LAUNCH_CHECK();
 }
+// the staging buffer: eta 7, tensor 42, out 56 columns (zero until host arrays are staged)
+static StressArgs staged_stress_args(Ctx& c, bool tensor) {
+  const int64_t nel = c.fine.nel;
+  if (!c.stress_buf) {
+    dalloc(&c.stress_buf, (7 + 42 + 56) * nel);
+    DP_CUDA(cudaMemsetAsync(c.stress_buf, 0, sizeof(double) * (7 + 42 + 56) * nel, c.stream));
+  }
+  StressArgs a = stress_args(c, tensor);
+  a.U = (const double*)c.work[W_UC];
+  a.eta = c.stress_buf;
+  for (int f = 0; f < 6; ++f) a.C[f] = c.stress_buf + (7 + 7 * f) * nel;
+  a.out = c.stress_buf + 49 * nel;
+  a.ld_eta = a.ld_C = nel;
+  return a;
+}
+
+// k_stress on the staging buffer (kernel timing)
+void launch_stress_staged(Ctx& c, bool tensor) { launch_stress(c, staged_stress_args(c, tensor)); }
 
 }  // namespace dp
 
@@ -166,32 +198,32 @@ extern "C" int dp_stress(dp_ctx* h, const double* Ucart, const double* eta_ip, i
       DP_CUDA(cudaDeviceSynchronize());  // the copies are on the default stream; ours does not wait on it
       if (c.device >= 0 && c.device < 64) uploaded[c.device] = true;
     }
-    if (!c.stress_buf) dalloc(&c.stress_buf, (7 + 42 + 56) * nel);
-    double* eta = c.stress_buf;
-    double* C = eta + 7 * nel;
-    double* o = C + 42 * nel;
-    const cudaMemcpyKind kin = kind_in(mem);
-    // nel x 7 column-major (element fastest) -> 7 contiguous columns
-    DP_CUDA(cudaMemcpy2DAsync(eta, sizeof(double) * nel, eta_ip, sizeof(double) * ld_eta, sizeof(double) * nel, 7,
-                              kin, c.stream));
-    if (C6) {
-      for (int f = 0; f < 6; ++f) {
+    if (C6)
+      for (int f = 0; f < 6; ++f)
         if (!C6[f]) throw BadArg("null tensor field");
-        DP_CUDA(cudaMemcpy2DAsync(C + (size_t)f * 7 * nel, sizeof(double) * nel, C6[f], sizeof(double) * ld_C,
-                                  sizeof(double) * nel, 7, kin, c.stream));
-      }
-    }
-    // velocity: reference numbering -> lattice
-    double* stage = (double*)c.work[W_UC];
-    double* ulat = (double*)c.work[W_RES];
-    DP_CUDA(cudaMemcpyAsync(stage, Ucart, sizeof(double) * 2 * nn, kin, c.stream));
-    launch_gather_ref2lat(c, stage, ulat, 2);
-    ++g_klaunch;
-    k_stress<<<(int)div_up(nel, 128), 128, 0, c.stream>>>(ulat, c.theta_lat, c.r_lat, eta, C6 ? C : nullptr, o,
-                                                           (int)nel, c.fine.ncr, (int)c.fine.A(), (int)c.fine.B());
-    DP_LAUNCH_CHECK();
+    c.stress_called = true;
     c.stress_tensor = C6 != nullptr;
-    DP_CUDA(cudaMemcpyAsync(out, o, sizeof(double) * 56 * nel, kind_out(mem), c.stream));
+    bool in_place = mem == DP_MEM_DEVICE && !overlap(out, 56 * nel, Ucart, 2 * nn) &&
+                    !overlap(out, 56 * nel, eta_ip, 6 * ld_eta + nel);
+    for (int f = 0; C6 && f < 6; ++f) in_place = in_place && !overlap(out, 56 * nel, C6[f], 6 * ld_C + nel);
+    if (in_place) {
+      StressArgs a = stress_args(c, C6 != nullptr);
+      a.U = Ucart; a.eta = eta_ip; a.out = out;
+      a.ld_eta = ld_eta; a.ld_C = ld_C;
+      for (int f = 0; C6 && f < 6; ++f) a.C[f] = C6[f];
+      launch_stress(c, a);
+    } else {
+      const StressArgs a = staged_stress_args(c, C6 != nullptr);
+      // nel x 7 column-major (element fastest) -> 7 contiguous columns
+      DP_CUDA(cudaMemcpy2DAsync((void*)a.eta, sizeof(double) * nel, eta_ip, sizeof(double) * ld_eta,
+                                sizeof(double) * nel, 7, kind_in(mem), c.stream));
+      for (int f = 0; C6 && f < 6; ++f)
+        DP_CUDA(cudaMemcpy2DAsync((void*)a.C[f], sizeof(double) * nel, C6[f], sizeof(double) * ld_C,
+                                  sizeof(double) * nel, 7, kind_in(mem), c.stream));
+      DP_CUDA(cudaMemcpyAsync((void*)a.U, Ucart, sizeof(double) * 2 * nn, kind_in(mem), c.stream));
+      launch_stress(c, a);
+      DP_CUDA(cudaMemcpyAsync(out, a.out, sizeof(double) * 56 * nel, kind_out(mem), c.stream));
+    }
     DP_CUDA(cudaStreamSynchronize(c.stream));
     return (int)DP_OK;
   });

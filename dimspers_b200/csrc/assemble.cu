@@ -1,4 +1,4 @@
-// Element assembly of the Stokes blocks on the device, one element per thread.
+// Element assembly of the Stokes blocks on the device, three warps per 32 elements.
 //
 // Follows src/Stokes/StokesSolver.jl:
 //   _fill_R_J!            :522-541  linear (theta, r) Jacobian of the 3 vertices
@@ -16,10 +16,16 @@
 // The lumped pressure preconditioner 1/rowsum(M) (IterativeSolvers.jl:238-240)
 // is produced in the same pass.
 //
-// The 132 per-element accumulators live in shared memory (one column per
-// thread, conflict-free), which keeps the register count low enough for
-// several CTAs per SM; assembly runs once per solve and is FP64 throughout
-// (the refined path stores a rounded FP32 copy of Ke).
+// A CTA takes 32 elements, a lane each.  Its three warps first share the
+// integration points (geometry, sincos, D: 15 values per element and IP to
+// shared memory) and the nodal rotations, then warp w sums the columns of the
+// local nodes w and 5 - w (7 of the 21 node-pair blocks) over the IPs in
+// registers, rotates and masks them, and hands them to shared memory, from
+// where the packed matrix leaves in 16-byte groups.  FP64 throughout (the
+// refined path stores a rounded FP32 copy of Ke).
+// Bound by FP64 issue and the 1.4-1.7 kB an element reads and writes.  The form
+// it replaces, one thread per element with 132 accumulators in shared memory,
+// moved 25 kB an element through shared memory: 968 us at 256x2048.
 #include "kernels.cuh"
 
 namespace dp {
@@ -96,38 +102,278 @@ struct AsmArgs {
   CartOut cart;
 };
 
-constexpr int kAsmThreads = 64;
-constexpr int kAcc = kKe + kGe + kMe + kFe;  // 132
+constexpr int kAsmEl = 32, kAsmThreads = 96;
+// per element and IP in shared memory
+enum AsmVal { AV_IX0, AV_IX1, AV_IZ0, AV_IZ1, AV_OM, AV_S, AV_C, AV_OMFG, AV_W3, AV_D11, AV_D22, AV_D33, AV_D12, AV_D13,
+              AV_D23, AV_COUNT };
+constexpr int kAsmGeo = 6 * AV_COUNT * kAsmEl;      // doubles
+
+// Integration point ip of element e to shared memory.
+__device__ __forceinline__ void asm_point(const AsmArgs& p, double* geo, int ip, int e, const double th[3],
+                                          const double rr[3], const double rho[3], double detJ, const double Cel[6],
+                                          double qc, double qs) {
+  const double R31 = rr[2] - rr[0], R21 = rr[1] - rr[0];
+  const double T31 = th[2] - th[0], T21 = th[1] - th[0];
+  const double th_ip = th[0] * c_N3[ip][0] + th[1] * c_N3[ip][1] + th[2] * c_N3[ip][2];
+  const double r_ip = rr[0] * c_N3[ip][0] + rr[1] * c_N3[ip][1] + rr[2] * c_N3[ip][2];
+  const double dens = rho[0] * c_N3[ip][0] + rho[1] * c_N3[ip][1] + rho[2] * c_N3[ip][2];
+  const double visc = p.eta[(size_t)ip * p.nel + e];
+  const double fg = p.g * dens;
+  double s, c;
+  sincos(th_ip, &s, &c);
+  const double inv = 1.0 / r_ip / detJ;
+  const double om = r_ip * detJ * c_w[ip];
+  // D (Voigt xx, zz, xz), symmetric: d11 d12 d13 / d22 d23 / d33
+  double d11, d12, d13, d22, d23, d33;
+  if (p.mat_kind == MAT_ISO) {
+    d11 = d22 = (4.0 / 3.0) * visc;
+    d12 = (-2.0 / 3.0) * visc;
+    d33 = visc;
+    d13 = d23 = 0.0;
+  } else {
+    double cc[6];
+    if (p.mat_kind == MAT_FULL) {
+#pragma unroll
+      for (int f = 0; f < 6; ++f) cc[f] = p.C[((size_t)f * 6 + ip) * p.nel + e];
+    } else {
+#pragma unroll
+      for (int f = 0; f < 6; ++f) cc[f] = Cel[f];
+    }
+    d11 = cc[0] * visc; d22 = cc[1] * visc; d33 = cc[2] * visc;
+    d12 = cc[3] * visc; d13 = cc[4] * visc; d23 = cc[5] * visc;
+  }
+  if (p.mfD) {
+    // om * Q^T D Q, Q = [c^2 s^2 cs; s^2 c^2 -cs; -2cs 2cs c^2-s^2]
+    const double cc2 = qc * qc, ss2 = qs * qs, cs = qc * qs;
+    const double Q[3][3] = {{cc2, ss2, cs}, {ss2, cc2, -cs}, {-2.0 * cs, 2.0 * cs, cc2 - ss2}};
+    const double Dm[3][3] = {{d11, d12, d13}, {d12, d22, d23}, {d13, d23, d33}};
+    double M[3][3];
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 3; ++j) M[i][j] = Dm[i][0] * Q[0][j] + Dm[i][1] * Q[1][j] + Dm[i][2] * Q[2][j];
+    double R[3][3];
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 3; ++j) R[i][j] = Q[0][i] * M[0][j] + Q[1][i] * M[1][j] + Q[2][i] * M[2][j];
+    const size_t st = (size_t)p.nel;
+    double* o = p.mfD + (size_t)(ip * 6) * st + e;
+    o[0 * st] = om * R[0][0];
+    o[1 * st] = om * R[0][1];
+    o[2 * st] = om * R[0][2];
+    o[3 * st] = om * R[1][1];
+    o[4 * st] = om * R[1][2];
+    o[5 * st] = om * R[2][2];
+  }
+  double* v = geo + (size_t)ip * AV_COUNT * kAsmEl;
+  v[AV_IX0 * kAsmEl] = (R31 * c - T31 * s * r_ip) * inv;
+  v[AV_IX1 * kAsmEl] = (-R21 * c + T21 * s * r_ip) * inv;
+  v[AV_IZ0 * kAsmEl] = (-R31 * s - T31 * c * r_ip) * inv;
+  v[AV_IZ1 * kAsmEl] = (R21 * s + T21 * c * r_ip) * inv;
+  v[AV_OM * kAsmEl] = om;
+  v[AV_S * kAsmEl] = s;
+  v[AV_C * kAsmEl] = c;
+  v[AV_OMFG * kAsmEl] = om * fg;
+  v[AV_W3 * kAsmEl] = om / visc;
+  v[AV_D11 * kAsmEl] = d11;
+  v[AV_D22 * kAsmEl] = d22;
+  v[AV_D33 * kAsmEl] = d33;
+  v[AV_D12 * kAsmEl] = d12;
+  v[AV_D13 * kAsmEl] = d13;
+  v[AV_D23 * kAsmEl] = d23;
+}
+
+// Sums of local node I over the IPs: blocks (j, I), j = I..5, of K (k00, k10,
+// k01, k11), its rows of G (component, pressure node) and of the body force.
+template <int I>
+struct AsmNode {
+  double k[6 - I][4], g[2][3], f[2];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int j = 0; j < 6 - I; ++j) k[j][0] = k[j][1] = k[j][2] = k[j][3] = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) g[0][i] = g[1][i] = 0.0;
+    f[0] = f[1] = 0.0;
+  }
+  __device__ __forceinline__ void add(const double* v, int ip, const double dx[6], const double dz[6]) {
+    const double om = v[AV_OM * kAsmEl];
+    const double d11 = v[AV_D11 * kAsmEl], d22 = v[AV_D22 * kAsmEl], d33 = v[AV_D33 * kAsmEl];
+    const double d12 = v[AV_D12 * kAsmEl], d13 = v[AV_D13 * kAsmEl], d23 = v[AV_D23 * kAsmEl];
+    // omega * D * B columns: DBx = D (dx, 0, dz), DBz = D (0, dz, dx)
+    const double x = om * dx[I], z = om * dz[I];
+    const double bx0 = d11 * x + d13 * z, bx1 = d12 * x + d23 * z, bx2 = d13 * x + d33 * z;
+    const double bz0 = d12 * z + d13 * x, bz1 = d22 * z + d23 * x, bz2 = d23 * z + d33 * x;
+#pragma unroll
+    for (int j = I; j < 6; ++j) {
+      k[j - I][0] += dx[j] * bx0 + dz[j] * bx2;
+      k[j - I][1] += dz[j] * bx1 + dx[j] * bx2;
+      if (j > I) k[j - I][2] += dx[j] * bz0 + dz[j] * bz2;
+      k[j - I][3] += dz[j] * bz1 + dx[j] * bz2;
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double tt = om * c_N3[ip][i];
+      g[0][i] += tt * dx[I];
+      g[1][i] += tt * dz[I];
+    }
+    const double cte = v[AV_OMFG * kAsmEl] * c_N[ip][I];
+    f[0] += v[AV_S * kAsmEl] * cte;
+    f[1] += v[AV_C * kAsmEl] * cte;
+  }
+  // Cartesian reference-layout outputs
+  __device__ __forceinline__ void cartesian(const CartOut& o, int e) const {
+    if (o.Ke) {
+#pragma unroll
+      for (int j = I; j < 6; ++j) {
+        o.Ke[(size_t)e * kKe + packed_index12(2 * j, 2 * I)] = k[j - I][0];
+        o.Ke[(size_t)e * kKe + packed_index12(2 * j + 1, 2 * I)] = k[j - I][1];
+        if (j > I) o.Ke[(size_t)e * kKe + packed_index12(2 * j, 2 * I + 1)] = k[j - I][2];
+        o.Ke[(size_t)e * kKe + packed_index12(2 * j + 1, 2 * I + 1)] = k[j - I][3];
+      }
+    }
+    if (o.Ge) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        o.Ge[(size_t)e * kGe + i * 12 + 2 * I] = g[0][i];
+        o.Ge[(size_t)e * kGe + i * 12 + 2 * I + 1] = g[1][i];
+      }
+    }
+    if (o.Fb) {
+      o.Fb[(size_t)e * kFe + 2 * I] = f[0];
+      o.Fb[(size_t)e * kFe + 2 * I + 1] = f[1];
+    }
+  }
+  // rotation to polar DOFs (TT_k = [c s; -s c] per node, StokesSolver.jl:214-241)
+  // and constraint mask; K to the staging area (entry p of element lane at
+  // [p / 2][lane][p % 2]), G and F to global memory.  rot: (cos, sin) per node.
+  __device__ __forceinline__ void polar(const AsmArgs& p, double* stage, const double* rot, unsigned fixr, unsigned fixt,
+                                        int e, int lane, int node, bool live) const {
+    const double ci = rot[(2 * I) * kAsmEl], si = rot[(2 * I + 1) * kAsmEl];
+    const bool fri = fixr >> I & 1, fti = fixt >> I & 1;
+#pragma unroll
+    for (int j = I; j < 6; ++j) {
+      const double cj = rot[(2 * j) * kAsmEl], sj = rot[(2 * j + 1) * kAsmEl];
+      const double k00 = k[j - I][0], k10 = k[j - I][1], k11 = k[j - I][3], k01 = j > I ? k[j - I][2] : k10;
+      // M1 = K_ji T_i, then T_j^T M1
+      const double m00 = k00 * ci - k01 * si, m01 = k00 * si + k01 * ci;
+      const double m10 = k10 * ci - k11 * si, m11 = k10 * si + k11 * ci;
+      double r00 = cj * m00 - sj * m10, r01 = cj * m01 - sj * m11;
+      double r10 = sj * m00 + cj * m10, r11 = sj * m01 + cj * m11;
+      const bool frj = fixr >> j & 1, ftj = fixt >> j & 1;
+      if (fri) { r01 = 0.0; r11 = 0.0; }
+      if (frj) { r10 = 0.0; r11 = 0.0; }
+      if (fti) { r00 = 0.0; r10 = 0.0; }
+      if (ftj) { r00 = 0.0; r01 = 0.0; }
+      auto put = [&](int q, double v) { stage[(q >> 1) * 2 * kAsmEl + 2 * lane + (q & 1)] = v; };
+      put(packed_index12(2 * j, 2 * I), r00);
+      put(packed_index12(2 * j + 1, 2 * I), r10);
+      put(packed_index12(2 * j + 1, 2 * I + 1), r11);
+      if (j > I) put(packed_index12(2 * j, 2 * I + 1), r01);
+    }
+    if (!live) return;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      p.Gp[(size_t)(i * 12 + 2 * I) * p.nel + e] = fti ? 0.0 : ci * g[0][i] - si * g[1][i];
+      p.Gp[(size_t)(i * 12 + 2 * I + 1) * p.nel + e] = fri ? 0.0 : si * g[0][i] + ci * g[1][i];
+    }
+    const double f0 = ci * f[0] - si * f[1], f1 = si * f[0] + ci * f[1];
+    if (p.Fe) {
+      p.Fe[(size_t)(2 * I) * p.nel + e] = fti ? 0.0 : f0;
+      p.Fe[(size_t)(2 * I + 1) * p.nel + e] = fri ? 0.0 : f1;
+    } else {
+      if (!fti) atomicAdd(&p.F[2 * (size_t)node], f0);
+      if (!fri) atomicAdd(&p.F[2 * (size_t)node + 1], f1);
+    }
+  }
+};
+
+// Columns of the nodes W and 5 - W (and, for W = 0, the pressure mass block).
+template <int W>
+__device__ __forceinline__ void asm_columns(const AsmArgs& p, const double* geo, double* stage, const double* rot,
+                                            unsigned fixr, unsigned fixt, const int nd[6], int e, int lane,
+                                            bool live) {
+  AsmNode<W> n0;
+  AsmNode<5 - W> n1;
+  double m[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // Me packed lower 3x3: (0,0),(1,0),(2,0),(1,1),(2,1),(2,2)
+  n0.zero();
+  n1.zero();
+#pragma unroll 1
+  for (int ip = 0; ip < 6; ++ip) {
+    const double* v = geo + (size_t)ip * AV_COUNT * kAsmEl + lane;
+    const double ix0 = v[AV_IX0 * kAsmEl], ix1 = v[AV_IX1 * kAsmEl];
+    const double iz0 = v[AV_IZ0 * kAsmEl], iz1 = v[AV_IZ1 * kAsmEl];
+    double dx[6], dz[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      dx[k] = ix0 * c_dN[ip][0][k] + ix1 * c_dN[ip][1][k];
+      dz[k] = iz0 * c_dN[ip][0][k] + iz1 * c_dN[ip][1][k];
+    }
+    n0.add(v, ip, dx, dz);
+    n1.add(v, ip, dx, dz);
+    if (W == 0) {
+      const double w3 = v[AV_W3 * kAsmEl];
+      const double* NP = c_N3[ip];
+      m[0] += w3 * NP[0] * NP[0];
+      m[1] += w3 * NP[1] * NP[0];
+      m[2] += w3 * NP[2] * NP[0];
+      m[3] += w3 * NP[1] * NP[1];
+      m[4] += w3 * NP[2] * NP[1];
+      m[5] += w3 * NP[2] * NP[2];
+    }
+  }
+  if (live) {
+    n0.cartesian(p.cart, e);
+    n1.cartesian(p.cart, e);
+  }
+  n0.polar(p, stage, rot, fixr, fixt, e, lane, nd[W], live);
+  n1.polar(p, stage, rot, fixr, fixt, e, lane, nd[5 - W], live);
+  if (W != 0 || !live) return;
+  if (p.cart.Me)
+    for (int i = 0; i < kMe; ++i) p.cart.Me[(size_t)e * kMe + i] = m[i];
+  // lumped mass rows
+  const double m00 = m[0], m10 = m[1], m20 = m[2], m11 = m[3], m21 = m[4], m22 = m[5];
+  const double row[3] = {m00 + m10 + m20, m10 + m11 + m21, m20 + m21 + m22};
+  if (p.pressure == 1) {
+    for (int i = 0; i < 3; ++i) p.pcsum[3 * (size_t)e + i] = 1.0 / row[i];
+    // exact inverse of the symmetric 3x3 element block M_e (the whole of M for
+    // discontinuous pressure), packed (00, 10, 20, 11, 21, 22)
+    const double c00 = m11 * m22 - m21 * m21, c10 = -(m10 * m22 - m21 * m20), c20 = m10 * m21 - m11 * m20;
+    const double c11 = m00 * m22 - m20 * m20, c21 = -(m00 * m21 - m10 * m20), c22 = m00 * m11 - m10 * m10;
+    const double det = m00 * c00 + m10 * c10 + m20 * c20;
+    const double id = 1.0 / det;
+    p.Minv[(size_t)0 * p.nel + e] = c00 * id;
+    p.Minv[(size_t)1 * p.nel + e] = c10 * id;
+    p.Minv[(size_t)2 * p.nel + e] = c20 * id;
+    p.Minv[(size_t)3 * p.nel + e] = c11 * id;
+    p.Minv[(size_t)4 * p.nel + e] = c21 * id;
+    p.Minv[(size_t)5 * p.nel + e] = c22 * id;
+  } else {
+    int64_t pd[3];
+    element_pdofs_cont(e, p.ncr, p.nct, pd);
+    for (int i = 0; i < 3; ++i) atomicAdd(&p.pcsum[pd[i]], row[i]);
+  }
+}
 
 __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs p) {
-  extern __shared__ double sm[];
-  const int tid = threadIdx.x;
-  const int e = blockIdx.x * kAsmThreads + tid;
-  if (e >= p.nel) return;  // no block-level synchronisation below
-  double* acc = sm + tid;
-#define ACC(i) acc[(i) * kAsmThreads]
-  for (int i = 0; i < kAcc; ++i) ACC(i) = 0.0;
+  __shared__ double geo[kAsmGeo];
+  __shared__ __align__(16) double stage[kKe * kAsmEl];   // packed matrices, 16-byte groups
+  __shared__ double rot_s[12 * kAsmEl];   // (cos, sin) of the 6 nodes
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool live = blockIdx.x * kAsmEl + lane < p.nel;
+  const int e = live ? blockIdx.x * kAsmEl + lane : p.nel - 1;   // idle lanes repeat the last element, unwritten
 
   // lattice nodes of the element
   const int q = e >> 1, t = e & 1;
   const int ir = q % p.ncr, it = q / p.ncr;
-  int na[6], nb[6];
-  {
-    const int a0 = 2 * ir, b0 = 2 * it;
-    if (t == 0) {
-      const int aa[6] = {a0, a0, a0 + 2, a0, a0 + 1, a0 + 1};
-      const int bb[6] = {b0, b0 + 2, b0, b0 + 1, b0 + 1, b0};
-      for (int k = 0; k < 6; ++k) { na[k] = aa[k]; nb[k] = bb[k]; }
-    } else {
-      const int aa[6] = {a0, a0 + 2, a0 + 2, a0 + 1, a0 + 2, a0 + 1};
-      const int bb[6] = {b0 + 2, b0 + 2, b0, b0 + 2, b0 + 1, b0 + 1};
-      for (int k = 0; k < 6; ++k) { na[k] = aa[k]; nb[k] = bb[k]; }
-    }
-  }
   int nd[6];
+  unsigned fixr = 0, fixt = 0;   // u_r / u_theta constrained, a bit per node
+  const int amax = 2 * p.ncr;
 #pragma unroll
-  for (int k = 0; k < 6; ++k) nd[k] = na[k] + p.A * (nb[k] >= p.B ? nb[k] - p.B : nb[k]);
-
+  for (int k = 0; k < 6; ++k) {
+    const int a = 2 * ir + (t ? loc_a(1, k) : loc_a(0, k));
+    int b = 2 * it + (t ? loc_b(1, k) : loc_b(0, k));
+    if (b >= p.B) b -= p.B;
+    nd[k] = a + p.A * b;
+    fixr |= dof_fixed(a, b, 1, amax, p.pin) ? 1u << k : 0u;
+    fixt |= dof_fixed(a, b, 0, amax, p.pin) ? 1u << k : 0u;
+  }
   // vertex coordinates + fixangles! (Utilities.jl:45-61)
   double th[3], rr[3], rho[3];
 #pragma unroll
@@ -135,6 +381,22 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs p) {
     th[k] = p.theta_lat[nd[k]];
     rr[k] = p.r_lat[nd[k]];
     rho[k] = p.rho_lat[nd[k]];
+  }
+  // nodal rotations: the six nodes lie on three lattice columns (all nodes of a
+  // column have one angle), one per warp
+  {
+    int n = t ? nd[2] : nd[0];
+    if (w == 1) n = t ? nd[4] : nd[3];
+    if (w == 2) n = t ? nd[0] : nd[1];
+    double s, c;
+    sincos(p.theta_lat[n], &s, &c);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      if ((t ? loc_b(1, k) : loc_b(0, k)) == w) {
+        rot_s[(2 * k) * kAsmEl + lane] = c;
+        rot_s[(2 * k + 1) * kAsmEl + lane] = s;
+      }
+    }
   }
   {
     const double PI = 3.14159265358979323846;
@@ -149,218 +411,41 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs p) {
   const double Jt0 = -th[0] + th[1], Jt1 = -th[0] + th[2];
   const double Jr0 = -rr[0] + rr[1], Jr1 = -rr[0] + rr[2];
   const double detJ = Jt0 * Jr1 - Jt1 * Jr0;
-  const double R31 = rr[2] - rr[0], R21 = rr[1] - rr[0];
-  const double T31 = th[2] - th[0], T21 = th[1] - th[0];
 
-  double Cel[6];
+  double Cel[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   if (p.mat_kind == MAT_TI) ti_tensor(p.C[e], p.C[p.nel + e], p.C[2 * p.nel + e], Cel);
 
   // matrix-free form: the element is its ring's reference element (it = 0)
   // rotated by phi = theta(v0) - theta(v0 of the reference); its polar operator
   // is sum_ip om B0^T (Q^T D Q) B0 with Q the engineering-strain rotation by phi
   double qc = 1.0, qs = 0.0;
-  const size_t emf = (size_t)e;
   if (p.mfD) {
     const int bref = (t == 0) ? 0 : 2;            // vertex 0 of the reference element
     sincos(th[0] - p.theta_lat[2 * ir + p.A * bref], &qs, &qc);
   }
-
-  for (int ip = 0; ip < 6; ++ip) {
-    const double th_ip = th[0] * c_N3[ip][0] + th[1] * c_N3[ip][1] + th[2] * c_N3[ip][2];
-    const double r_ip = rr[0] * c_N3[ip][0] + rr[1] * c_N3[ip][1] + rr[2] * c_N3[ip][2];
-    const double dens = rho[0] * c_N3[ip][0] + rho[1] * c_N3[ip][1] + rho[2] * c_N3[ip][2];
-    const double visc = p.eta[(size_t)ip * p.nel + e];
-    const double fg = p.g * dens;
-    double s, c;
-    sincos(th_ip, &s, &c);
-    const double inv = 1.0 / r_ip / detJ;
-    const double ix0 = (R31 * c - T31 * s * r_ip) * inv;
-    const double ix1 = (-R21 * c + T21 * s * r_ip) * inv;
-    const double iz0 = (-R31 * s - T31 * c * r_ip) * inv;
-    const double iz1 = (R21 * s + T21 * c * r_ip) * inv;
-    const double om = r_ip * detJ * c_w[ip];
-    double dx[6], dz[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      dx[k] = ix0 * c_dN[ip][0][k] + ix1 * c_dN[ip][1][k];
-      dz[k] = iz0 * c_dN[ip][0][k] + iz1 * c_dN[ip][1][k];
-    }
-    // D (Voigt xx, zz, xz), symmetric: d11 d12 d13 / d22 d23 / d33
-    double d11, d12, d13, d22, d23, d33;
-    if (p.mat_kind == MAT_ISO) {
-      d11 = d22 = (4.0 / 3.0) * visc;
-      d12 = (-2.0 / 3.0) * visc;
-      d33 = visc;
-      d13 = d23 = 0.0;
-    } else {
-      double cc[6];
-      if (p.mat_kind == MAT_FULL) {
-#pragma unroll
-        for (int f = 0; f < 6; ++f) cc[f] = p.C[((size_t)f * 6 + ip) * p.nel + e];
-      } else {
-#pragma unroll
-        for (int f = 0; f < 6; ++f) cc[f] = Cel[f];
-      }
-      d11 = cc[0] * visc; d22 = cc[1] * visc; d33 = cc[2] * visc;
-      d12 = cc[3] * visc; d13 = cc[4] * visc; d23 = cc[5] * visc;
-    }
-    if (p.mfD) {
-      // om * Q^T D Q, Q = [c^2 s^2 cs; s^2 c^2 -cs; -2cs 2cs c^2-s^2]
-      const double cc2 = qc * qc, ss2 = qs * qs, cs = qc * qs;
-      const double Q[3][3] = {{cc2, ss2, cs}, {ss2, cc2, -cs}, {-2.0 * cs, 2.0 * cs, cc2 - ss2}};
-      const double Dm[3][3] = {{d11, d12, d13}, {d12, d22, d23}, {d13, d23, d33}};
-      double M[3][3];
-      for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) M[i][j] = Dm[i][0] * Q[0][j] + Dm[i][1] * Q[1][j] + Dm[i][2] * Q[2][j];
-      double R[3][3];
-      for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) R[i][j] = Q[0][i] * M[0][j] + Q[1][i] * M[1][j] + Q[2][i] * M[2][j];
-      const size_t st = (size_t)p.nel;
-      double* o = p.mfD + (size_t)(ip * 6) * st + emf;
-      o[0 * st] = om * R[0][0];
-      o[1 * st] = om * R[0][1];
-      o[2 * st] = om * R[0][2];
-      o[3 * st] = om * R[1][1];
-      o[4 * st] = om * R[1][2];
-      o[5 * st] = om * R[2][2];
-    }
-    // omega * D * B columns: DBx_i = D (dx_i, 0, dz_i), DBz_i = D (0, dz_i, dx_i)
-    double bx0[6], bx1[6], bx2[6], bz0[6], bz1[6], bz2[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const double x = om * dx[i], z = om * dz[i];
-      bx0[i] = d11 * x + d13 * z; bx1[i] = d12 * x + d23 * z; bx2[i] = d13 * x + d33 * z;
-      bz0[i] = d12 * z + d13 * x; bz1[i] = d22 * z + d23 * x; bz2[i] = d23 * z + d33 * x;
-    }
-    // Ke lower packed: column 2i rows (2j, 2j+1) j>=i; column 2i+1 rows 2j (j>i), 2j+1 (j>=i)
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-#pragma unroll
-      for (int j = i; j < 6; ++j) {
-        ACC(packed_index12(2 * j, 2 * i)) += dx[j] * bx0[i] + dz[j] * bx2[i];
-        ACC(packed_index12(2 * j + 1, 2 * i)) += dz[j] * bx1[i] + dx[j] * bx2[i];
-        if (j > i) ACC(packed_index12(2 * j, 2 * i + 1)) += dx[j] * bz0[i] + dz[j] * bz2[i];
-        ACC(packed_index12(2 * j + 1, 2 * i + 1)) += dz[j] * bz1[i] + dx[j] * bz2[i];
-      }
-    }
-    // Ge (12x3 column-major)
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const double tt = om * c_N3[ip][i];
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        ACC(kKe + i * 12 + 2 * k) += tt * dx[k];
-        ACC(kKe + i * 12 + 2 * k + 1) += tt * dz[k];
-      }
-    }
-    // Me packed lower 3x3: (0,0),(1,0),(2,0),(1,1),(2,1),(2,2)
-    {
-      const double w3 = om / visc;
-      const double* NP = c_N3[ip];
-      ACC(kKe + kGe + 0) += w3 * NP[0] * NP[0];
-      ACC(kKe + kGe + 1) += w3 * NP[1] * NP[0];
-      ACC(kKe + kGe + 2) += w3 * NP[2] * NP[0];
-      ACC(kKe + kGe + 3) += w3 * NP[1] * NP[1];
-      ACC(kKe + kGe + 4) += w3 * NP[2] * NP[1];
-      ACC(kKe + kGe + 5) += w3 * NP[2] * NP[2];
-    }
-    // Fb
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      const double cte = om * fg * c_N[ip][k];
-      ACC(kKe + kGe + kMe + 2 * k) += s * cte;
-      ACC(kKe + kGe + kMe + 2 * k + 1) += c * cte;
-    }
-  }
-
-  // optional Cartesian reference-layout outputs (column-major 78 x nel etc.)
-  if (p.cart.Ke) for (int i = 0; i < kKe; ++i) p.cart.Ke[(size_t)e * kKe + i] = ACC(i);
-  if (p.cart.Ge) for (int i = 0; i < kGe; ++i) p.cart.Ge[(size_t)e * kGe + i] = ACC(kKe + i);
-  if (p.cart.Me) for (int i = 0; i < kMe; ++i) p.cart.Me[(size_t)e * kMe + i] = ACC(kKe + kGe + i);
-  if (p.cart.Fb) for (int i = 0; i < kFe; ++i) p.cart.Fb[(size_t)e * kFe + i] = ACC(kKe + kGe + kMe + i);
-
-  // rotation to polar DOFs: TT_k = [c s; -s c] per node (StokesSolver.jl:214-241)
-  double cs[6], sn[6];
-  bool fixed[6], fixt[6];  // u_r / u_theta constrained
-  const int amax = 2 * p.ncr;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    sincos(p.theta_lat[nd[k]], &sn[k], &cs[k]);
-    const int bk = nb[k] >= p.B ? nb[k] - p.B : nb[k];
-    fixed[k] = dof_fixed(na[k], bk, 1, amax, p.pin);
-    fixt[k] = dof_fixed(na[k], bk, 0, amax, p.pin);
-  }
-  // K: block (j,i) -> T_j^T K_ji T_i, written to packed lower
-  for (int i = 0; i < 6; ++i) {
-    for (int j = i; j < 6; ++j) {
-      double k00 = ACC(packed_index12(2 * j, 2 * i));
-      double k10 = ACC(packed_index12(2 * j + 1, 2 * i));
-      double k11 = ACC(packed_index12(2 * j + 1, 2 * i + 1));
-      double k01 = (j > i) ? ACC(packed_index12(2 * j, 2 * i + 1)) : k10;
-      // M1 = K_ji T_i
-      const double m00 = k00 * cs[i] - k01 * sn[i], m01 = k00 * sn[i] + k01 * cs[i];
-      const double m10 = k10 * cs[i] - k11 * sn[i], m11 = k10 * sn[i] + k11 * cs[i];
-      // T_j^T M1
-      double r00 = cs[j] * m00 - sn[j] * m10, r01 = cs[j] * m01 - sn[j] * m11;
-      double r10 = sn[j] * m00 + cs[j] * m10, r11 = sn[j] * m01 + cs[j] * m11;
-      if (fixed[i]) { r01 = 0.0; r11 = 0.0; }
-      if (fixed[j]) { r10 = 0.0; r11 = 0.0; }
-      if (fixt[i]) { r00 = 0.0; r10 = 0.0; }
-      if (fixt[j]) { r00 = 0.0; r01 = 0.0; }
-      ACC(packed_index12(2 * j, 2 * i)) = r00;
-      ACC(packed_index12(2 * j + 1, 2 * i)) = r10;
-      ACC(packed_index12(2 * j + 1, 2 * i + 1)) = r11;
-      if (j > i) ACC(packed_index12(2 * j, 2 * i + 1)) = r01;
-    }
-  }
+#pragma unroll 1
+  for (int ip = w; ip < 6; ip += 3) asm_point(p, geo + lane, ip, e, th, rr, rho, detJ, Cel, qc, qs);
+  __syncthreads();
+  if (w == 0) asm_columns<0>(p, geo, stage, rot_s + lane, fixr, fixt, nd, e, lane, live);
+  else if (w == 1) asm_columns<1>(p, geo, stage, rot_s + lane, fixr, fixt, nd, e, lane, live);
+  else asm_columns<2>(p, geo, stage, rot_s + lane, fixr, fixt, nd, e, lane, live);
+  __syncthreads();
+  // packed matrices out in 16-byte groups (the padding behind the last element is left alone)
+  const int64_t blk = blockIdx.x;
   if (p.K64)
-    for (int i = 0; i < kKe; ++i) p.K64[kidx64(i, e)] = ACC(i);
+    for (int idx = threadIdx.x; idx < 39 * kAsmEl; idx += kAsmThreads)
+      if (blockIdx.x * kAsmEl + (idx & 31) < p.nel)
+        reinterpret_cast<double2*>(p.K64)[blk * (39 * kAsmEl) + idx] = reinterpret_cast<const double2*>(stage)[idx];
   if (p.K32)
-    for (int i = 0; i < kKe; ++i) p.K32[kidx32(i, e)] = (float)ACC(i);
-  // G rows and F: T_k^T applied per node, wall u_r rows zeroed
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const double gx = ACC(kKe + i * 12 + 2 * k), gz = ACC(kKe + i * 12 + 2 * k + 1);
-      p.Gp[(size_t)(i * 12 + 2 * k) * p.nel + e] = fixt[k] ? 0.0 : cs[k] * gx - sn[k] * gz;
-      p.Gp[(size_t)(i * 12 + 2 * k + 1) * p.nel + e] = fixed[k] ? 0.0 : sn[k] * gx + cs[k] * gz;
+    for (int idx = threadIdx.x; idx < 20 * kAsmEl; idx += kAsmThreads) {
+      const int j = idx >> 5, el = idx & 31;
+      if (blockIdx.x * kAsmEl + el >= p.nel) continue;
+      const double2 u = reinterpret_cast<const double2*>(stage)[(2 * j) * kAsmEl + el];
+      double2 v = make_double2(0.0, 0.0);      // entries 78 and 79 do not exist
+      if (j < 19) v = reinterpret_cast<const double2*>(stage)[(2 * j + 1) * kAsmEl + el];
+      reinterpret_cast<float4*>(p.K32)[blk * (20 * kAsmEl) + idx] =
+          make_float4((float)u.x, (float)u.y, (float)v.x, (float)v.y);
     }
-    const double fx = ACC(kKe + kGe + kMe + 2 * k), fz = ACC(kKe + kGe + kMe + 2 * k + 1);
-    if (p.Fe) {
-      p.Fe[(size_t)(2 * k) * p.nel + e] = fixt[k] ? 0.0 : cs[k] * fx - sn[k] * fz;
-      p.Fe[(size_t)(2 * k + 1) * p.nel + e] = fixed[k] ? 0.0 : sn[k] * fx + cs[k] * fz;
-    } else {
-      if (!fixt[k]) atomicAdd(&p.F[2 * (size_t)nd[k]], cs[k] * fx - sn[k] * fz);
-      if (!fixed[k]) atomicAdd(&p.F[2 * (size_t)nd[k] + 1], sn[k] * fx + cs[k] * fz);
-    }
-  }
-  // lumped mass rows
-  {
-    const double m00 = ACC(kKe + kGe + 0), m10 = ACC(kKe + kGe + 1), m20 = ACC(kKe + kGe + 2);
-    const double m11 = ACC(kKe + kGe + 3), m21 = ACC(kKe + kGe + 4), m22 = ACC(kKe + kGe + 5);
-    const double row[3] = {m00 + m10 + m20, m10 + m11 + m21, m20 + m21 + m22};
-    if (p.pressure == 1) {
-      for (int i = 0; i < 3; ++i) p.pcsum[3 * (size_t)e + i] = 1.0 / row[i];
-      // exact inverse of the symmetric 3x3 element block M_e (the whole of M for
-      // discontinuous pressure), packed (00, 10, 20, 11, 21, 22)
-      const double c00 = m11 * m22 - m21 * m21, c10 = -(m10 * m22 - m21 * m20), c20 = m10 * m21 - m11 * m20;
-      const double c11 = m00 * m22 - m20 * m20, c21 = -(m00 * m21 - m10 * m20), c22 = m00 * m11 - m10 * m10;
-      const double det = m00 * c00 + m10 * c10 + m20 * c20;
-      const double id = 1.0 / det;
-      p.Minv[(size_t)0 * p.nel + e] = c00 * id;
-      p.Minv[(size_t)1 * p.nel + e] = c10 * id;
-      p.Minv[(size_t)2 * p.nel + e] = c20 * id;
-      p.Minv[(size_t)3 * p.nel + e] = c11 * id;
-      p.Minv[(size_t)4 * p.nel + e] = c21 * id;
-      p.Minv[(size_t)5 * p.nel + e] = c22 * id;
-    } else {
-      int64_t pd[3];
-      element_pdofs_cont(e, p.ncr, p.nct, pd);
-      for (int i = 0; i < 3; ++i) atomicAdd(&p.pcsum[pd[i]], row[i]);
-    }
-  }
-#undef ACC
 }
 
 // Per ring (ir, t) of the matrix-free apply (ring = 2 ir + t): the reference
@@ -437,17 +522,10 @@ void launch_assemble(Ctx& c, int precision, const CartOut* cart) {
   a.Fe = static_cast<double*>(L.det);
   a.mfD = c.mfD64;
   if (cart) a.cart = *cart;
-  const size_t smem = sizeof(double) * kAcc * kAsmThreads;
-  static bool attr_set = false;
-  if (!attr_set) {
-    DP_CUDA(cudaFuncSetAttribute(k_assemble, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
-  }
   if (!a.Fe) DP_CUDA(cudaMemsetAsync(c.F, 0, sizeof(double) * 2 * L.nnod, c.stream));
   if (c.mesh.pressure == 0) DP_CUDA(cudaMemsetAsync(c.pc, 0, sizeof(double) * c.mesh.npres, c.stream));
-  const int grid = (int)div_up(L.nel, kAsmThreads);
   ++g_klaunch;
-  k_assemble<<<grid, kAsmThreads, smem, c.stream>>>(a);
+  k_assemble<<<(int)div_up(L.nel, kAsmEl), kAsmThreads, 0, c.stream>>>(a);
   DP_LAUNCH_CHECK();
   if (a.Fe) launch_node_gather<double>(L, a.Fe, c.F, 2, c.stream);
   if (c.mfT64) {

@@ -313,6 +313,15 @@ __host__ __device__ inline void element_nodes(int64_t e, int ncr, int64_t A, int
   for (int k = 0; k < 6; ++k) n[k] = a[k] + A * wrapb(b[k], B);
 }
 
+// Local node k of triangle type t sits at lattice offset (kLocA, kLocB) from
+// its cell origin (2 ir, 2 it): the node order of element_product.
+__host__ __device__ constexpr int loc_a(int t, int k) {
+  return t == 0 ? (k == 2 ? 2 : (k >= 4 ? 1 : 0)) : (k == 0 ? 0 : (k == 3 || k == 5 ? 1 : 2));
+}
+__host__ __device__ constexpr int loc_b(int t, int k) {
+  return t == 0 ? (k == 1 ? 2 : (k == 3 || k == 4 ? 1 : 0)) : (k == 2 ? 0 : (k >= 4 ? 1 : 2));
+}
+
 // Reference number of lattice node (a, b).  Vertices are numbered angle by angle;
 // midpoints follow in the order in which the edges (v1 v2), (v2 v4), (v4 v1) of
 // the triangles meet them (edge_connectivity, mesher.jl:349-392): the first

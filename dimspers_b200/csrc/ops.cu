@@ -150,15 +150,6 @@ __global__ void __launch_bounds__(256) k_apply_K_elem(const Tm* __restrict__ K, 
   for (int d = 0; d < 12; ++d) E[(int64_t)d * nel + e] = ye[d];
 }
 
-// Local node k of triangle type t sits at lattice offset (kLocA, kLocB) from
-// its cell origin (2 ir, 2 it): the node order of element_product.
-__host__ __device__ constexpr int loc_a(int t, int k) {
-  return t == 0 ? (k == 2 ? 2 : (k >= 4 ? 1 : 0)) : (k == 0 ? 0 : (k == 3 || k == 5 ? 1 : 2));
-}
-__host__ __device__ constexpr int loc_b(int t, int k) {
-  return t == 0 ? (k == 1 ? 2 : (k == 3 || k == 4 ? 1 : 0)) : (k == 2 ? 0 : (k >= 4 ? 1 : 2));
-}
-
 // Deterministic form, pass 2: per lattice node n, the sum of E over the
 // elements that contain it, taken in a fixed order (triangle type t = 0, 1,
 // then local node k = 0..5), so the result is the same bit for bit in every

@@ -93,6 +93,8 @@ struct AsmArgs {
   double g;
   double* K64;         // 78*nel (may be null)
   float* K32;          // 78*nel (may be null)
+  double* R64;         // reduced matrices, 56*nel (with R32, or null)
+  float* R32;
   double* Gp;          // 36*nel
   double* F;           // 2*nnod, accumulated with atomics (zeroed by caller)
   double* Fe;          // deterministic mode: element RHS, Fe[(2k + c) nel + e] (F then by k_node_gather)
@@ -106,7 +108,8 @@ constexpr int kAsmEl = 32, kAsmThreads = 96;
 // per element and IP in shared memory
 enum AsmVal { AV_IX0, AV_IX1, AV_IZ0, AV_IZ1, AV_OM, AV_S, AV_C, AV_OMFG, AV_W3, AV_D11, AV_D22, AV_D33, AV_D12, AV_D13,
               AV_D23, AV_COUNT };
-constexpr int kAsmGeo = 6 * AV_COUNT * kAsmEl;      // doubles
+constexpr int kAsmGeo = 6 * AV_COUNT * kAsmEl;      // doubles; the reduced matrices (56 x 32) reuse it
+static_assert(kRed * kAsmEl <= kAsmGeo, "staging of the reduced matrices does not fit");
 
 // Integration point ip of element e to shared memory.
 __device__ __forceinline__ void asm_point(const AsmArgs& p, double* geo, int ip, int e, const double th[3],
@@ -180,6 +183,13 @@ __device__ __forceinline__ void asm_point(const AsmArgs& p, double* geo, int ip,
   v[AV_D23 * kAsmEl] = d23;
 }
 
+// Slot of local node k in the reduced matrix of an element of type t, -1 for the
+// reference node (the diagonal midpoint); see reduced_product in ops.cu.
+__host__ __device__ constexpr int red_slot(int t, int k) { return k < 4 ? k : (k == (t == 0 ? 4 : 5) ? -1 : 4); }
+
+// Every warp of the CTA, from wherever it stands in its own instance of asm_columns.
+__device__ __forceinline__ void asm_barrier() { asm volatile("bar.sync 1, 96;" ::: "memory"); }
+
 // Sums of local node I over the IPs: blocks (j, I), j = I..5, of K (k00, k10,
 // k01, k11), its rows of G (component, pressure node) and of the body force.
 template <int I>
@@ -243,8 +253,9 @@ struct AsmNode {
   // rotation to polar DOFs (TT_k = [c s; -s c] per node, StokesSolver.jl:214-241)
   // and constraint mask; K to the staging area (entry p of element lane at
   // [p / 2][lane][p % 2]), G and F to global memory.  rot: (cos, sin) per node.
-  __device__ __forceinline__ void polar(const AsmArgs& p, double* stage, const double* rot, unsigned fixr, unsigned fixt,
-                                        int e, int lane, int node, bool live) const {
+  // red: staging of the reduced matrix (unmasked, same form), or null.
+  __device__ __forceinline__ void polar(const AsmArgs& p, double* stage, double* red, const double* rot, unsigned fixr,
+                                        unsigned fixt, int e, int lane, int node, bool live) const {
     const double ci = rot[(2 * I) * kAsmEl], si = rot[(2 * I + 1) * kAsmEl];
     const bool fri = fixr >> I & 1, fti = fixt >> I & 1;
 #pragma unroll
@@ -256,6 +267,19 @@ struct AsmNode {
       const double m10 = k10 * ci - k11 * si, m11 = k10 * si + k11 * ci;
       double r00 = cj * m00 - sj * m10, r01 = cj * m01 - sj * m11;
       double r10 = sj * m00 + cj * m10, r11 = sj * m01 + cj * m11;
+      if (red) {
+        const int t = e & 1, si = red_slot(t, I), sj = red_slot(t, j);   // local order is slot order: sj >= si
+        if (si >= 0 && sj >= 0) {
+          auto put = [&](int R, int C, double v) {
+            const int q = packed_index10(R, C);
+            red[(q >> 1) * 2 * kAsmEl + 2 * lane + (q & 1)] = v;
+          };
+          put(2 * sj, 2 * si, r00);
+          put(2 * sj + 1, 2 * si, r10);
+          put(2 * sj + 1, 2 * si + 1, r11);
+          if (j > I) put(2 * sj, 2 * si + 1, r01);
+        }
+      }
       const bool frj = fixr >> j & 1, ftj = fixt >> j & 1;
       if (fri) { r01 = 0.0; r11 = 0.0; }
       if (frj) { r10 = 0.0; r11 = 0.0; }
@@ -286,7 +310,7 @@ struct AsmNode {
 
 // Columns of the nodes W and 5 - W (and, for W = 0, the pressure mass block).
 template <int W>
-__device__ __forceinline__ void asm_columns(const AsmArgs& p, const double* geo, double* stage, const double* rot,
+__device__ __forceinline__ void asm_columns(const AsmArgs& p, double* geo, double* stage, const double* rot,
                                             unsigned fixr, unsigned fixt, const int nd[6], int e, int lane,
                                             bool live) {
   AsmNode<W> n0;
@@ -322,8 +346,13 @@ __device__ __forceinline__ void asm_columns(const AsmArgs& p, const double* geo,
     n0.cartesian(p.cart, e);
     n1.cartesian(p.cart, e);
   }
-  n0.polar(p, stage, rot, fixr, fixt, e, lane, nd[W], live);
-  n1.polar(p, stage, rot, fixr, fixt, e, lane, nd[5 - W], live);
+  double* red = nullptr;
+  if (p.R64) {   // the same for the whole grid
+    asm_barrier();   // every warp has read the integration points: their space takes the reduced matrices
+    red = geo;
+  }
+  n0.polar(p, stage, red, rot, fixr, fixt, e, lane, nd[W], live);
+  n1.polar(p, stage, red, rot, fixr, fixt, e, lane, nd[5 - W], live);
   if (W != 0 || !live) return;
   if (p.cart.Me)
     for (int i = 0; i < kMe; ++i) p.cart.Me[(size_t)e * kMe + i] = m[i];
@@ -352,7 +381,7 @@ __device__ __forceinline__ void asm_columns(const AsmArgs& p, const double* geo,
 }
 
 __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs p) {
-  __shared__ double geo[kAsmGeo];
+  __shared__ __align__(16) double geo[kAsmGeo];
   __shared__ __align__(16) double stage[kKe * kAsmEl];   // packed matrices, 16-byte groups
   __shared__ double rot_s[12 * kAsmEl];   // (cos, sin) of the 6 nodes
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -446,6 +475,22 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs p) {
       reinterpret_cast<float4*>(p.K32)[blk * (20 * kAsmEl) + idx] =
           make_float4((float)u.x, (float)u.y, (float)v.x, (float)v.y);
     }
+  if (p.R64) {
+    // entry 55 does not exist
+    for (int idx = threadIdx.x; idx < 28 * kAsmEl; idx += kAsmThreads) {
+      double2 u = reinterpret_cast<const double2*>(geo)[idx];
+      if (idx >= 27 * kAsmEl) u.y = 0.0;
+      if (blockIdx.x * kAsmEl + (idx & 31) < p.nel) reinterpret_cast<double2*>(p.R64)[blk * (28 * kAsmEl) + idx] = u;
+    }
+    for (int idx = threadIdx.x; idx < 14 * kAsmEl; idx += kAsmThreads) {
+      const int j = idx >> 5, el = idx & 31;
+      if (blockIdx.x * kAsmEl + el >= p.nel) continue;
+      const double2 u = reinterpret_cast<const double2*>(geo)[(2 * j) * kAsmEl + el];
+      const double2 v = reinterpret_cast<const double2*>(geo)[(2 * j + 1) * kAsmEl + el];
+      reinterpret_cast<float4*>(p.R32)[blk * (14 * kAsmEl) + idx] =
+          make_float4((float)u.x, (float)u.y, (float)v.x, j == 13 ? 0.f : (float)v.y);
+    }
+  }
 }
 
 // Per ring (ir, t) of the matrix-free apply (ring = 2 ir + t): the reference
@@ -518,6 +563,11 @@ void launch_assemble(Ctx& c, int precision, const CartOut* cart) {
   a.eta = c.eta; a.C = c.C; a.g = c.g;
   a.K64 = c.K64;
   a.K32 = precision >= 1 ? c.K32 : nullptr;
+  a.R64 = precision >= 1 ? c.R64 : nullptr;
+  a.R32 = precision >= 1 ? c.R32 : nullptr;
+  // the reduced matrices are current after an assembly that writes them, and only then
+  c.fine.red64 = a.R64;
+  c.fine.red32 = a.R32;
   a.Gp = c.Gp; a.F = c.F; a.pcsum = c.pc; a.Minv = c.Minv;
   a.Fe = static_cast<double*>(L.det);
   a.mfD = c.mfD64;

@@ -30,7 +30,7 @@ Ctx::~Ctx() {
   cudaFree(theta_lat); cudaFree(r_lat);
   cudaFree(eta); cudaFree(C); cudaFree(rho_lat); cudaFree(rho_ref);
   cudaFree(mfD64); cudaFree(mfT64); cudaFree(mfD32); cudaFree(mfT32); cudaFree(det_buf);
-  cudaFree(K64); cudaFree(K32); cudaFree(Gp); cudaFree(F); cudaFree(pc); cudaFree(Minv); cudaFree(Fscale);
+  cudaFree(K64); cudaFree(K32); cudaFree(R64); cudaFree(R32); cudaFree(Gp); cudaFree(F); cudaFree(pc); cudaFree(Minv); cudaFree(Fscale);
   cudaFree(flush);
   cudaFree(stress_buf);
   cudaFree(rheo_buf);
@@ -166,15 +166,6 @@ static SolveCfg make_cfg(const dp_solve_opts* o) {
   return cfg;
 }
 
-// FP32 copy of the packed FP64 element matrices (the layouts differ)
-__global__ void k_f64_to_f32(const double* a, float* b, int64_t nel) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= nel * kKe) return;
-  const int64_t e = i % nel;
-  const int p = (int)(i / nel);
-  b[kidx32(p, e)] = (float)a[kidx64(p, e)];
-}
-
 // FP32 copy of the operator when a mode needs it, then the multigrid values
 // (Galerkin operators, smoother bounds, coarse inverse) for the current assembly.
 static void check_solve_cfg(const Ctx& c, const SolveCfg& cfg) {
@@ -186,17 +177,31 @@ static void check_solve_cfg(const Ctx& c, const SolveCfg& cfg) {
   if (c.fine.det && cfg.matrix_free) throw BadArg("matrix_free applies scatter with atomics: not in deterministic mode");
 }
 
-// FP32 copy of the assembled operator (once per assembly) for the FP32 modes.
+// Storage of the refined path: FP32 copies of the element matrices and the
+// reduced matrices in both precisions.
+static void alloc_refined(Ctx& c) {
+  const int64_t nel = c.fine.nel;
+  if (!c.K32) {
+    dalloc(&c.K32, kstore<float>(nel));
+    DP_CUDA(cudaMemsetAsync(c.K32, 0, sizeof(float) * kstore<float>(nel), c.stream));
+  }
+  if (!c.R64) {
+    dalloc(&c.R64, rstore<double>(nel));
+    DP_CUDA(cudaMemsetAsync(c.R64, 0, sizeof(double) * rstore<double>(nel), c.stream));
+  }
+  if (!c.R32) {
+    dalloc(&c.R32, rstore<float>(nel));
+    DP_CUDA(cudaMemsetAsync(c.R32, 0, sizeof(float) * rstore<float>(nel), c.stream));
+  }
+}
+
+// The refined path's matrices, where the last assembly was an FP64 one (which does
+// not write them): the same material assembled again.
 static void ensure_k32(Ctx& c, const SolveCfg& cfg) {
   if (cfg.precision >= 1 && c.assembled == 0) {
-    if (!c.K32) {
-      dalloc(&c.K32, kstore<float>(c.fine.nel));
-      DP_CUDA(cudaMemsetAsync(c.K32, 0, sizeof(float) * kstore<float>(c.fine.nel), c.stream));
-    }
-    const int64_t n = kKe * c.fine.nel;
-    ++g_klaunch;
-    k_f64_to_f32<<<(int)div_up(n, 256), 256, 0, c.stream>>>(c.K64, c.K32, c.fine.nel);
-    DP_LAUNCH_CHECK();
+    alloc_refined(c);
+    launch_assemble(c, 1, nullptr);
+    c.mf32_stale = true;
     c.assembled = 1;
   }
 }
@@ -213,6 +218,11 @@ static void set_fine_apply(Ctx& c, const SolveCfg& cfg) {
   c.fine.warps_t = cfg.mg.apply_warps_t;
   c.fine.mfD64 = c.fine.mfT64 = nullptr;
   c.fine.mfD32 = c.fine.mfT32 = nullptr;
+  // FP64 solves read the packed matrices whatever the last assembly wrote, so
+  // which buffers a captured solve holds depends on its options alone
+  const bool red = cfg.precision >= 1 && !cfg.matrix_free;
+  c.fine.red64 = red ? c.R64 : nullptr;
+  c.fine.red32 = red ? c.R32 : nullptr;
   if (!cfg.matrix_free) return;
   if (!c.mfD64) {
     // first matrix-free solve on this context: allocate the data and assemble
@@ -221,6 +231,8 @@ static void set_fine_apply(Ctx& c, const SolveCfg& cfg) {
     dalloc(&c.mfT64, (int64_t)kMfTab * 2 * c.fine.ncr);
     const int keep = c.assembled;
     launch_assemble(c, c.assembled >= 1 ? 1 : 0, nullptr);
+    c.fine.red64 = nullptr;
+    c.fine.red32 = nullptr;
     c.assembled = keep;
     c.mf32_stale = true;
   }
@@ -628,10 +640,7 @@ int dp_assemble(dp_ctx* h, int32_t precision) {
     DP_CUDA(cudaSetDevice(c.device));
     if (c.mat_kind == MAT_NONE) throw BadArg("material not set");
     if (precision < 0 || precision > 2) throw BadArg("precision must be 0, 1 or 2");
-    if (precision >= 1 && !c.K32) {
-      dalloc(&c.K32, kstore<float>(c.fine.nel));
-      DP_CUDA(cudaMemset(c.K32, 0, sizeof(float) * kstore<float>(c.fine.nel)));
-    }
+    if (precision >= 1) alloc_refined(c);
     launch_assemble(c, precision, nullptr);  // also refreshes the matrix-free data once enabled
     c.mf32_stale = true;
     c.assembled = precision;

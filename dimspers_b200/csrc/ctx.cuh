@@ -52,6 +52,10 @@ struct Level {
   const double* mfT64 = nullptr;
   const float* mfD32 = nullptr;
   const float* mfT32 = nullptr;
+  // Reduced element matrices of the fine level (55 of the 78 entries, ops.cu).
+  // Null: the applies read the packed ones.
+  const double* red64 = nullptr;
+  const float* red32 = nullptr;
   // Deterministic mode: scratch for per-element results (kDetPerElem values per
   // element, level precision), summed per node in a fixed order by
   // k_node_gather instead of scatter-added with atomics.  Null: atomics.
@@ -106,6 +110,8 @@ struct Ctx {
   int assembled = -1;           // precision of the last assembly, -1 = none
   double* K64 = nullptr;        // 78*nel
   float* K32 = nullptr;         // 78*nel (refined path)
+  double* R64 = nullptr;        // reduced element matrices (refined path, written with K32)
+  float* R32 = nullptr;
   double* mfD64 = nullptr;      // 36*nel: matrix-free apply data (written by every assembly)
   double* mfT64 = nullptr;      // kMfTab*2*ncr
   float* mfD32 = nullptr;       // FP32 copies for the FP32 levels
@@ -406,6 +412,13 @@ __host__ __device__ inline int64_t kidx64(int p, int64_t e) {
 __host__ __device__ inline int64_t kidx32(int p, int64_t e) {
   return (e >> 5) * (32 * 80) + (int64_t)(p >> 2) * 128 + (e & 31) * 4 + (p & 3);
 }
+// Reduced element matrices: 55 entries padded to 56, 28 double2 / 14 float4 groups.
+constexpr int kRed = 56;
+// packed lower-column-major index of the 10x10 reduced matrix entry (R >= C)
+__host__ __device__ constexpr int packed_index10(int R, int C) { return C * 10 - (C * (C - 1)) / 2 + (R - C); }
+template <typename T>
+inline int64_t rstore(int64_t nel) { return kpad(nel) * kRed; }
+
 template <typename T>
 __host__ __device__ inline int64_t kidx(int p, int64_t e);
 template <>

@@ -1132,10 +1132,14 @@ static void mg_setup_t(Ctx& c, const MGOptions& o) {
     L.g.det = c.fine.det;   // one scratch (sized for the fine level) serves every level in turn
     L.g.mfD64 = L.g.mfT64 = nullptr;
     L.g.mfD32 = L.g.mfT32 = nullptr;
+    L.g.red64 = nullptr;
+    L.g.red32 = nullptr;
   }
   // the fine level applies matrix-free when the fine context level does
   c.mg[0].g.mfD64 = c.fine.mfD64;
   c.mg[0].g.mfT64 = c.fine.mfT64;
+  c.mg[0].g.red64 = c.fine.red64;
+  c.mg[0].g.red32 = c.fine.red32;
   c.mg[0].g.mfD32 = c.fine.mfD32;
   c.mg[0].g.mfT32 = c.fine.mfT32;
   // Galerkin coarse operators

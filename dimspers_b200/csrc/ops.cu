@@ -223,6 +223,141 @@ void launch_node_gather(const Level& L, const T* E, T* y, int mode, cudaStream_t
 template void launch_node_gather<double>(const Level&, const double*, double*, int, cudaStream_t);
 template void launch_node_gather<float>(const Level&, const float*, float*, int, cudaStream_t);
 
+// ---- reduced element matrices (fine level) ------------------------------------------
+// A rigid translation strains no element, so the unmasked K_e (12x12) annihilates
+// the two translations and is determined by the 10x10 block of five nodes: with
+// the cell's diagonal midpoint as the sixth, reference node (never on a wall)
+// and rel_k = u_k - (the polar components at node k of the translation with
+// u_ref at the reference node),
+//   f = K' rel,  y_k = f_k,  y_ref = -sum_k (the same rotation)^T f_k.
+// The reference node lies on the cell's middle lattice column, the others one
+// column to either side or on it, so the rotation is by 0 or +-pi/nct, one
+// (cos, sin) pair for the mesh.  55 entries are read instead of 78: 224 B
+// (FP32) and 448 B (FP64) an element instead of 320 and 624.  The constraint
+// mask, which the packed matrices carry, is applied to x before and y after
+// (elements at the walls only).
+// Slots 0..4 are the local nodes in order without the reference one.
+template <typename T>
+struct RVec {
+  typedef typename KVec<T>::V V;
+  static constexpr int n = kRed * sizeof(T) / 16, per = 16 / sizeof(T);
+};
+
+// y_s (slots 0..4, then the reference node 5) = K_e x of element e and the nodes' lattice
+// indices; the matrix is fetched before the wait for the predecessor.
+template <typename T>
+__device__ __forceinline__ void reduced_product(const T* __restrict__ R, const T* x, int e, int ncr, int A, int B,
+                                                int pin, T ch, T sh, int nd[6], T y[12]) {
+  typedef typename V2<T>::T X2;
+  T kk[kRed];
+  {
+    const typename RVec<T>::V* p =
+        reinterpret_cast<const typename RVec<T>::V*>(R) + (int64_t)(e >> 5) * (32 * RVec<T>::n) + (e & 31);
+#pragma unroll
+    for (int j = 0; j < RVec<T>::n; ++j) vec_to(ld_stream(p + j * 32), kk + j * RVec<T>::per);
+  }
+  const int q = e >> 1, t = e & 1;
+  const int ir = q % ncr, it = q / ncr;
+  const int a0 = 2 * ir, b0 = 2 * it, b2 = b0 + 2 >= B ? 0 : b0 + 2;
+  // t = 0: (0,0) (0,2) (2,0) (0,1) (1,0); t = 1: (0,2) (2,2) (2,0) (1,2) (2,1); both (1,1)
+  nd[0] = a0 + A * (t ? b2 : b0);
+  nd[1] = a0 + (t ? 2 : 0) + A * b2;
+  nd[2] = a0 + 2 + A * b0;
+  nd[3] = a0 + (t ? 1 : 0) + A * (t ? b2 : b0 + 1);
+  nd[4] = a0 + (t ? 2 : 1) + A * (t ? b0 + 1 : b0);
+  nd[5] = a0 + 1 + A * (b0 + 1);
+  // constrained DOFs: u_r of the slots on a wall, u_theta of the pinned node
+  const bool in = ir == 0, out = ir == ncr - 1;
+  bool fr[5], ft[5];
+  fr[0] = in;
+  fr[1] = t ? out : in;
+  fr[2] = out;
+  fr[3] = !t && in;
+  fr[4] = t && out;
+#pragma unroll
+  for (int s = 0; s < 5; ++s) ft[s] = pin && out && nd[s] == 2 * ncr;
+  grid_dep_sync();
+  const X2* x2 = reinterpret_cast<const X2*>(x);
+  X2 v[6];
+#pragma unroll
+  for (int s = 0; s < 6; ++s) v[s] = x2[nd[s]];
+  // the translation of the reference node one column up (p) and down (m)
+  const T px = ch * v[5].x - sh * v[5].y, py = sh * v[5].x + ch * v[5].y;
+  const T mx = ch * v[5].x + sh * v[5].y, my = ch * v[5].y - sh * v[5].x;
+  const T sx[5] = {t ? px : mx, px, mx, t ? px : v[5].x, t ? v[5].x : mx};
+  const T sy[5] = {t ? py : my, py, my, t ? py : v[5].y, t ? v[5].y : my};
+  T rel[10];
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    rel[2 * s] = (ft[s] ? (T)0 : v[s].x) - sx[s];
+    rel[2 * s + 1] = (fr[s] ? (T)0 : v[s].y) - sy[s];
+    y[2 * s] = y[2 * s + 1] = (T)0;
+  }
+#pragma unroll
+  for (int C = 0; C < 10; ++C) {
+#pragma unroll
+    for (int Rr = C; Rr < 10; ++Rr) {
+      const T kv = kk[packed_index10(Rr, C)];
+      y[Rr] += kv * rel[C];
+      if (Rr != C) y[C] += kv * rel[Rr];
+    }
+  }
+  // column sums: up (slot 1, and 0 and 3 for t = 1), down (slot 2, and 0 and 4 for t = 0), middle
+  const T ux = y[2] + (t ? y[0] + y[6] : (T)0), uy = y[3] + (t ? y[1] + y[7] : (T)0);
+  const T dx = y[4] + (t ? (T)0 : y[0] + y[8]), dy = y[5] + (t ? (T)0 : y[1] + y[9]);
+  const T cx = t ? y[8] : y[6], cy = t ? y[9] : y[7];
+  y[10] = -(cx + ch * (ux + dx) + sh * (uy - dy));
+  y[11] = -(cy + ch * (uy + dy) + sh * (dx - ux));
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    if (ft[s]) y[2 * s] = (T)0;
+    if (fr[s]) y[2 * s + 1] = (T)0;
+  }
+}
+
+template <typename T, bool kSub>
+__global__ void __launch_bounds__(256) k_apply_R(const T* __restrict__ R, const T* x, T* y, int nel, int ncr, int A,
+                                                 int B, int wt, int pin, T ch, T sh) {
+  grid_dep_launch();
+  const int e = tile_element(ncr, wt);
+  if (e >= nel) return;
+  int nd[6];
+  T ye[12];
+  reduced_product<T>(R, x, e, ncr, A, B, pin, ch, sh, nd, ye);
+#pragma unroll
+  for (int s = 0; s < 6; ++s) {
+    if (kSub) atomic_add2(&y[2 * nd[s]], -ye[2 * s], -ye[2 * s + 1]);
+    else atomic_add2(&y[2 * nd[s]], ye[2 * s], ye[2 * s + 1]);
+  }
+}
+
+// Deterministic form, pass 1 (as k_apply_K_elem): slot 4 is local node 5 for type 0
+// and 4 for type 1, the reference node the other one.
+template <typename T>
+__global__ void __launch_bounds__(256) k_apply_R_elem(const T* __restrict__ R, const T* x, T* E, int nel, int ncr,
+                                                      int A, int B, int pin, T ch, T sh) {
+  grid_dep_launch();
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nel) return;
+  int nd[6];
+  T ye[12];
+  reduced_product<T>(R, x, e, ncr, A, B, pin, ch, sh, nd, ye);
+  const int t = e & 1;
+#pragma unroll
+  for (int s = 0; s < 6; ++s) {
+    const int k = s < 4 ? s : ((s == 4) == (t == 0) ? 5 : 4);
+    E[(int64_t)(2 * k) * nel + e] = ye[2 * s];
+    E[(int64_t)(2 * k + 1) * nel + e] = ye[2 * s + 1];
+  }
+}
+
+template <typename T>
+static inline const T* red_data(const Level& L);
+template <>
+inline const double* red_data<double>(const Level& L) { return L.red64; }
+template <>
+inline const float* red_data<float>(const Level& L) { return L.red32; }
+
 // ---- matrix-free element-by-element K apply (fine level) -------------------------
 // K_e (polar DOFs, constrained rows/columns masked) = sum_ip B0^T Dw_ip B0, with
 // B0 = B_cart(ref) T(ref) of the ring's reference element (it = 0) and Dw_ip =
@@ -352,6 +487,16 @@ static void apply_tile(const Level& L, int& blocks, int& threads, int& wt) {
 template <int kMode, typename Tm, typename Tv>
 static void apply_K_into(const Level& L, const Tm* K, const Tv* x, Tv* y, cudaStream_t s) {
   constexpr bool kSub = kMode == 1;
+  const Tv* R = std::is_same<Tm, Tv>::value ? red_data<Tv>(L) : nullptr;
+  const double h = 3.14159265358979323846 / L.nct;   // half a cell
+  if (L.det && R) {
+    Tv* E = static_cast<Tv*>(L.det);
+    klaunch(k_apply_R_elem<Tv>, (int)div_up(L.nel, 256), 256, 0, s, R, x, E, (int)L.nel, L.ncr, (int)L.A(),
+            (int)L.B(), L.pin, (Tv)std::cos(h), (Tv)std::sin(h));
+    DP_LAUNCH_CHECK();
+    launch_node_gather<Tv>(L, E, y, kMode, s);
+    return;
+  }
   if (L.det) {
     Tv* E = static_cast<Tv*>(L.det);
     klaunch(k_apply_K_elem<Tm, Tv>, (int)div_up(L.nel, 256), 256, 0, s, K, x, E, (int)L.nel, L.ncr, (int)L.A(),
@@ -369,6 +514,12 @@ static void apply_K_into(const Level& L, const Tm* K, const Tv* x, Tv* y, cudaSt
   }
   int blocks, threads, wt;
   apply_tile(L, blocks, threads, wt);
+  if (R) {
+    klaunch(k_apply_R<Tv, kSub>, blocks, threads, 0, s, R, x, y, (int)L.nel, L.ncr, (int)L.A(), (int)L.B(), wt, L.pin,
+            (Tv)std::cos(h), (Tv)std::sin(h));
+    DP_LAUNCH_CHECK();
+    return;
+  }
   klaunch(k_apply_K<Tm, Tv, kSub>, blocks, threads, 0, s, K, x, y, (int)L.nel, L.ncr, (int)L.A(), (int)L.B(), wt);
   DP_LAUNCH_CHECK();
 }

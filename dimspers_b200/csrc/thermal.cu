@@ -17,16 +17,22 @@
 // unpreconditioned GMRES) with the reference's stopping test ||r|| <= atol +
 // rtol ||b|| (Krylov.jl's defaults sqrt(eps)), captured once per context as a
 // CUDA graph whose WHILE node is continued or ended by the last block of the
-// update kernel: per iteration k_th_apply (q = A p), k_th_pq (alpha),
-// k_th_update (x, r, z, beta and the stop test), k_th_dir (p, q = 0).
+// update kernel.  An iteration is two launches: k_th_apply forms p = z + beta p
+// while it gathers it (p alternates between two buffers), q += A p and p.q;
+// k_th_update x, r, z, beta, the stop test, and q = 0 for the next one.  A pass
+// of a WHILE body costs ~10 us of its own, so a body holds kThUnroll
+// iterations; those after the stopping test return at once.
+// Gathering rows of A per node instead of elements (no atomics, 92 instead of 84
+// bytes of matrix per node) measured 16-20 us per apply at 128x1024 against 9:
+// each neighbour value is fetched 2 x 11.5 times instead of 2 x 3.
 #include "kernels.cuh"
 #include "reduce.cuh"
 
 namespace dp {
 
 // scalar-table slots of the thermal loop
-enum ThSlot { TH_RZ = 48, TH_PQ = 49, TH_ALPHA = 50, TH_BETA = 51, TH_RR = 52, TH_TOL2 = 53, TH_IT = 54,
-              TH_ITMAX = 55, TH_BB = 56, TH_RZN = 57 };
+enum ThSlot { TH_RZ = 48, TH_ALPHA = 50, TH_BETA = 51, TH_RR = 52, TH_TOL2 = 53, TH_IT = 54,
+              TH_ITMAX = 55, TH_BB = 56, TH_RZN = 57, TH_STOP = 58 };
 
 __constant__ double c_w7[7];  // 7-point weights x 0.5 (Quadrature.jl:109-138)
 
@@ -46,27 +52,32 @@ __device__ __forceinline__ bool th_fixed(int64_t n, int64_t A, int amax, int hea
 struct ThAsmArgs {
   const double* theta_lat;
   const double* r_lat;
-  const double* rho_lat;
-  const double* Told;  // lattice
-  const double* Tbc;   // lattice: wall values, 0 inside
+  const double* rho;   // nodal density, reference numbering
+  const double* Told;  // reference numbering
   double* Ae;          // 21 x nel
   double* diag;        // nnod
   double* b;           // nnod
-  double K, Cp, dt;
-  int nel, ncr, A, B;
+  double K, Cp, dt, Ttop, Tbot;
+  int nel, ncr, nct, A, B, heated;
 };
+
+// prescribed value of a node on a wall, 0 inside
+__device__ __forceinline__ double th_wall(int a, int amax, int heated, double Ttop, double Tbot) {
+  return a == amax ? Ttop : ((heated && a == 0) ? Tbot : 0.0);
+}
 
 __global__ void __launch_bounds__(128) k_th_assemble(ThAsmArgs p) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= p.nel) return;
-  int64_t nd[6];
-  element_nodes(e, p.ncr, p.A, p.B, nd);
+  int nd[6], nref[6];
+  element_nodes_mg(e, p.ncr, p.A, p.B, nd);
+  element_ref_nodes(e, p.ncr, p.nct, nref);
   double th[3], rr[3], rho[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     th[k] = p.theta_lat[nd[k]];
     rr[k] = p.r_lat[nd[k]];
-    rho[k] = p.rho_lat[nd[k]];
+    rho[k] = p.rho[nref[k]];
   }
   {
     const double PI = 3.14159265358979323846;
@@ -79,7 +90,7 @@ __global__ void __launch_bounds__(128) k_th_assemble(ThAsmArgs p) {
   }
   // J = dN3ds * [theta r]: rows (dN/dxi, dN/deta) = (-1, 1, 0), (-1, 0, 1)
   const double J1 = -th[0] + th[1], J2 = -th[0] + th[2], J3 = -rr[0] + rr[1], J4 = -rr[0] + rr[2];
-  const double detJ = J1 * J4 - J2 * J3;
+  const double detJ = J1 * J4 - J2 * J3, invdet = 1.0 / detJ;
   const double R21 = rr[1] - rr[0], R31 = rr[2] - rr[0];
   const double T31 = th[2] - th[0], T21 = th[1] - th[0];
   double Ke[kThPack], Me[kThPack];
@@ -97,8 +108,8 @@ __global__ void __launch_bounds__(128) k_th_assemble(ThAsmArgs p) {
     double dx[6], dz[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-      dx[k] = (a11 * c_dNs[ip][0][k] + a12 * c_dNs[ip][1][k]) / detJ;
-      dz[k] = (a21 * c_dNs[ip][0][k] + a22 * c_dNs[ip][1][k]) / detJ;
+      dx[k] = (a11 * c_dNs[ip][0][k] + a12 * c_dNs[ip][1][k]) * invdet;
+      dz[k] = (a21 * c_dNs[ip][0][k] + a22 * c_dNs[ip][1][k]) * invdet;
     }
     const double om = r_ip * detJ * c_w7[ip];
     const double wk = p.K * om, wm = om * rho_ip * p.Cp;
@@ -115,8 +126,8 @@ __global__ void __launch_bounds__(128) k_th_assemble(ThAsmArgs p) {
   double to[6], tb[6];
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
-    to[i] = p.Told[nd[i]];
-    tb[i] = p.Tbc[nd[i]];
+    to[i] = p.Told[nref[i]];
+    tb[i] = th_wall(nd[i] % p.A, 2 * p.ncr, p.heated, p.Ttop, p.Tbot);
   }
   double be[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   const size_t st = (size_t)p.nel;
@@ -140,22 +151,42 @@ __global__ void __launch_bounds__(128) k_th_assemble(ThAsmArgs p) {
   for (int i = 0; i < 6; ++i) atomicAdd(&p.b[nd[i]], be[i]);
 }
 
-// q += A p over elements (q zeroed by the caller)
-__global__ void __launch_bounds__(128) k_th_apply(const double* __restrict__ Ae, const double* __restrict__ x,
-                                                  double* __restrict__ y, int nel, int ncr, int64_t A, int64_t B) {
-  grid_dep_sync();
+// p.q is added up in kThSlots scalars (a warp each, by index) that the update sums.
+// kThUnroll is even, so which of the two p buffers an iteration of the body
+// reads is known when it is captured.
+constexpr int kThSlots = 128, kThUnroll = 4;
+struct ThVecs {
+  const double* Ae;
+  const double* diag;
+  double *x, *r, *z, *q, *slots;
+  double *po, *pn;   // p before and after the iteration
+};
+
+// p' = z + beta p, q += A p' and p'.q over elements.  The type-0 element of a cell
+// also stores p' for the cell's 2x2 nodes (the outer wall's nodes are fixed: p
+// stays 0 there).
+__global__ void __launch_bounds__(128) k_th_apply(ThVecs v, const double* scal, int nel, int ncr, int A, int B) {
+  grid_dep_launch();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nel) return;
-  double a[kThPack];
-  const size_t st = (size_t)nel;
+  const bool live = e < nel;
+  const int ec = live ? e : nel - 1;
+  double a[kThPack];   // constant during the step: fetched before the wait
 #pragma unroll
-  for (int k = 0; k < kThPack; ++k) a[k] = Ae[(size_t)k * st + e];
-  int64_t nd[6];
-  element_nodes(e, ncr, A, B, nd);
-  double xv[6], yv[6];
+  for (int k = 0; k < kThPack; ++k) a[k] = ld_stream(v.Ae + (size_t)k * nel + ec);
+  int nd[6];
+  element_nodes_mg(ec, ncr, A, B, nd);
+  grid_dep_sync();
+  const double stop = scal[TH_STOP], beta = scal[TH_BETA];
+  double zv[6], xv[6], yv[6];
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
-    xv[i] = x[nd[i]];
+    zv[i] = v.z[nd[i]];
+    xv[i] = v.po[nd[i]];
+  }
+  if (stop != 0.0) return;   // the same for the whole grid
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    xv[i] = zv[i] + beta * xv[i];
     yv[i] = 0.0;
   }
   int k = 0;
@@ -167,150 +198,173 @@ __global__ void __launch_bounds__(128) k_th_apply(const double* __restrict__ Ae,
       if (j != i) yv[j] += a[k] * xv[i];
     }
   }
+  double d = 0.0;
+  if (live) {
 #pragma unroll
-  for (int i = 0; i < 6; ++i) atomicAdd(&y[nd[i]], yv[i]);
+    for (int i = 0; i < 6; ++i) {
+      atomicAdd(&v.q[nd[i]], yv[i]);
+      d += xv[i] * yv[i];
+    }
+    if (!(e & 1)) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+        if (i != 1 && i != 2) v.pn[nd[i]] = xv[i];   // local nodes 0, 3, 4, 5: the cell's own 2x2 block
+    }
+  }
+  d = warp_sum(d);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&v.slots[(4 * blockIdx.x + (threadIdx.x >> 5)) % kThSlots], d);
 }
 
-// r = b (free), 0 (walls); z = r / diag; p = z; x = 0; q = 0; sums r.z and b.b
-__global__ void __launch_bounds__(kRedThreads) k_th_init(const double* __restrict__ b, const double* __restrict__ diag,
-                                                         double* __restrict__ x, double* __restrict__ r,
-                                                         double* __restrict__ z, double* __restrict__ pv,
-                                                         double* __restrict__ q, int64_t n, int64_t A, int amax,
-                                                         int heated, double* scal, double* partial,
+// r = b (free), 0 (walls); z = r / diag; x = p = 0; sums r.z and b.b; p.q slots zeroed
+__global__ void __launch_bounds__(kRedThreads) k_th_init(const double* __restrict__ b, ThVecs v, int64_t n, int64_t A,
+                                                         int amax, int heated, double* scal, double* partial,
                                                          unsigned int* counter, double rtol, double atol, int itmax) {
-  double v[2] = {0.0, 0.0};
+  double s[2] = {0.0, 0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const bool fx = th_fixed(i, A, amax, heated);
     const double ri = fx ? 0.0 : b[i];
-    const double zi = fx ? 0.0 : ri / diag[i];
-    x[i] = 0.0;
-    r[i] = ri;
-    z[i] = zi;
-    pv[i] = zi;
-    q[i] = 0.0;
-    v[0] += ri * zi;
-    v[1] += ri * ri;
+    const double zi = fx ? 0.0 : ri / v.diag[i];
+    v.x[i] = 0.0;
+    v.r[i] = ri;
+    v.z[i] = zi;
+    v.po[i] = 0.0;
+    v.pn[i] = 0.0;
+    v.q[i] = 0.0;
+    s[0] += ri * zi;
+    s[1] += ri * ri;
   }
+  if (blockIdx.x == 0 && threadIdx.x < kThSlots) v.slots[threadIdx.x] = 0.0;
   double* outs[2] = {scal + TH_RZ, scal + TH_BB};
-  if (grid_finish<2>(v, partial, counter, outs) && threadIdx.x == 0) {
+  if (grid_finish<2>(s, partial, counter, outs) && threadIdx.x == 0) {
     const double tol = atol + rtol * sqrt(scal[TH_BB]);
     scal[TH_TOL2] = tol * tol;
     scal[TH_RR] = scal[TH_BB];
+    scal[TH_BETA] = 0.0;
+    scal[TH_ALPHA] = 0.0;
     scal[TH_IT] = 0.0;
+    scal[TH_STOP] = 0.0;
     scal[TH_ITMAX] = (double)itmax;
   }
 }
 
 // sets the loop's condition before its first pass
 __global__ void k_th_start(cudaGraphConditionalHandle h, const double* scal) {
-  grid_dep_sync();
+  grid_dep_wait();
   cudaGraphSetConditional(h, (scal[TH_RR] > scal[TH_TOL2] && scal[TH_ITMAX] >= 1.0) ? 1u : 0u);
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_th_pq(const double* __restrict__ pv, const double* __restrict__ q,
-                                                       int64_t n, double* scal, double* partial,
-                                                       unsigned int* counter) {
-  grid_dep_sync();
-  double v[1] = {0.0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v[0] += pv[i] * q[i];
-  double* outs[1] = {scal + TH_PQ};
-  if (grid_finish<1>(v, partial, counter, outs) && threadIdx.x == 0) scal[TH_ALPHA] = scal[TH_RZ] / scal[TH_PQ];
-}
-
-__global__ void __launch_bounds__(kRedThreads) k_th_update(double* __restrict__ x, double* __restrict__ r,
-                                                           double* __restrict__ z, const double* __restrict__ pv,
-                                                           const double* __restrict__ q,
-                                                           const double* __restrict__ diag, int64_t n, int64_t A,
-                                                           int amax, int heated, double* scal, double* partial,
-                                                           unsigned int* counter, cudaGraphConditionalHandle h) {
-  grid_dep_sync();
-  const double alpha = scal[TH_ALPHA];
-  double v[2] = {0.0, 0.0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    if (th_fixed(i, A, amax, heated)) continue;
-    x[i] += alpha * pv[i];
-    const double ri = r[i] - alpha * q[i];
-    const double zi = ri / diag[i];
-    r[i] = ri;
-    z[i] = zi;
-    v[0] += ri * zi;
-    v[1] += ri * ri;
+// x += alpha p; r -= alpha q; z = r / diag; beta and the stop test.  Two nodes per
+// thread and access (the node count is even), all loads issued first.
+__global__ void __launch_bounds__(kRedThreads) k_th_update(ThVecs v, int64_t n, int A, int amax, int heated,
+                                                           double* scal, double* partial, unsigned int* counter,
+                                                           cudaGraphConditionalHandle h) {
+  grid_dep_wait();
+  if (scal[TH_STOP] != 0.0) return;   // the same for the whole grid
+  double pq = 0.0;
+#pragma unroll
+  for (int k = 0; k < kThSlots / 32; ++k) pq += v.slots[(threadIdx.x & 31) + 32 * k];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) pq += __shfl_xor_sync(0xffffffffu, pq, o);
+  const double alpha = scal[TH_RZ] / pq;
+  const double* p = v.pn;
+  double s[2] = {0.0, 0.0};
+  for (int64_t i = 2 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); i < n;
+       i += 2 * (int64_t)gridDim.x * blockDim.x) {
+    const double2 pv = *reinterpret_cast<const double2*>(p + i), qv = *reinterpret_cast<const double2*>(v.q + i);
+    const double2 dv = *reinterpret_cast<const double2*>(v.diag + i);
+    double2 xv = *reinterpret_cast<const double2*>(v.x + i), rv = *reinterpret_cast<const double2*>(v.r + i);
+    double2 zv = make_double2(0.0, 0.0);
+    const int a0 = (int)(i % A), a1 = a0 + 1 == A ? 0 : a0 + 1;
+    if (!(a0 == amax || (heated && a0 == 0))) {
+      xv.x += alpha * pv.x;
+      rv.x -= alpha * qv.x;
+      zv.x = rv.x / dv.x;
+    }
+    if (!(a1 == amax || (heated && a1 == 0))) {
+      xv.y += alpha * pv.y;
+      rv.y -= alpha * qv.y;
+      zv.y = rv.y / dv.y;
+    }
+    *reinterpret_cast<double2*>(v.x + i) = xv;
+    *reinterpret_cast<double2*>(v.r + i) = rv;
+    *reinterpret_cast<double2*>(v.z + i) = zv;
+    *reinterpret_cast<double2*>(v.q + i) = make_double2(0.0, 0.0);   // the next apply adds to it
+    s[0] += rv.x * zv.x + rv.y * zv.y;
+    s[1] += rv.x * rv.x + rv.y * rv.y;
   }
   double* outs[2] = {scal + TH_RZN, scal + TH_RR};
-  if (grid_finish<2>(v, partial, counter, outs) && threadIdx.x == 0) {
+  if (!grid_finish<2>(s, partial, counter, outs)) return;
+  // the last block: every other one has read the slots
+  if (threadIdx.x < kThSlots) v.slots[threadIdx.x] = 0.0;
+  if (threadIdx.x == 0) {
+    scal[TH_ALPHA] = alpha;
     scal[TH_BETA] = scal[TH_RZN] / scal[TH_RZ];
     scal[TH_RZ] = scal[TH_RZN];
     const double it = scal[TH_IT] + 1.0;
     scal[TH_IT] = it;
     const double rr = scal[TH_RR];
-    const bool go = isfinite(rr) && isfinite(scal[TH_ALPHA]) && rr > scal[TH_TOL2] && it < scal[TH_ITMAX];
+    const bool go = isfinite(rr) && isfinite(alpha) && rr > scal[TH_TOL2] && it < scal[TH_ITMAX];
+    if (!go) scal[TH_STOP] = 1.0;   // the body's remaining iterations return at once
     cudaGraphSetConditional(h, go ? 1u : 0u);
   }
 }
 
-__global__ void k_th_dir(double* __restrict__ pv, double* __restrict__ q, const double* __restrict__ z, int64_t n,
-                         const double* scal) {
-  grid_dep_sync();
-  const double beta = scal[TH_BETA];
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) {
-    pv[i] = z[i] + beta * pv[i];
-    q[i] = 0.0;
-  }
-}
-
-// T = x + Tbc (free: x, walls: the prescribed value)
-__global__ void k_th_finish(const double* __restrict__ x, const double* __restrict__ Tbc, double* __restrict__ T,
-                            int64_t n) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) T[i] = x[i] + Tbc[i];
-}
-
-// Tbc: lattice wall values
-__global__ void k_th_bc(double* __restrict__ Tbc, int64_t n, int64_t A, int amax, int heated, double Ttop,
-                        double Tbot) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// T (reference numbering) = x (free) or the prescribed value (walls)
+__global__ void k_th_finish(const double* __restrict__ x, double* __restrict__ T, int n, int A, int ncr, int nct,
+                            int heated, double Ttop, double Tbot) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int a = (int)(i % A);
-  Tbc[i] = a == amax ? Ttop : ((heated && a == 0) ? Tbot : 0.0);
+  const int b = i / A, a = i - b * A;
+  T[ref_of_lattice(a, b, ncr, nct)] = x[i] + th_wall(a, 2 * ncr, heated, Ttop, Tbot);
 }
 
-// thermal work vectors, nnod each, after the 21 x nel element blocks
-enum ThVec { TV_TOLD = 0, TV_TBC, TV_DIAG, TV_B, TV_X, TV_R, TV_Z, TV_P, TV_Q, TV_STAGE, TV_COUNT };
+// thermal work vectors, nnod each, after the 21 x nel element blocks and the slots
+enum ThVec { TV_DIAG = 0, TV_B, TV_X, TV_R, TV_Z, TV_P0, TV_P1, TV_Q, TV_T, TV_RHO, TV_COUNT };
 
-static double* th_vec(Ctx& c, int k) { return c.th_buf + kThPack * c.fine.nel + (size_t)k * c.fine.nnod; }
+static double* th_slots(Ctx& c) { return c.th_buf + kThPack * c.fine.nel; }
+static double* th_vec(Ctx& c, int k) { return th_slots(c) + kThSlots + (size_t)k * c.fine.nnod; }
+static int64_t th_doubles(const Ctx& c) {
+  return kThPack * c.fine.nel + kThSlots + (int64_t)TV_COUNT * c.fine.nnod;
+}
+// of the k-th iteration of a body
+static ThVecs th_vecs(Ctx& c, int k) {
+  return ThVecs{c.th_buf,         th_vec(c, TV_DIAG), th_vec(c, TV_X),  th_vec(c, TV_R), th_vec(c, TV_Z),
+                th_vec(c, TV_Q), th_slots(c),        th_vec(c, k & 1 ? TV_P1 : TV_P0),
+                th_vec(c, k & 1 ? TV_P0 : TV_P1)};
+}
+static void th_launch_apply(Ctx& c, int k, cudaStream_t s) {
+  const Level& L = c.fine;
+  klaunch(k_th_apply, (int)div_up(L.nel, 128), 128, 0, s, th_vecs(c, k), (const double*)c.scal, (int)L.nel, L.ncr,
+          (int)L.A(), (int)L.B());
+  DP_LAUNCH_CHECK();
+}
 
 static void th_emit_loop(Ctx& c, int heated) {
   const Level& L = c.fine;
   const int64_t n = L.nnod;
   const int amax = 2 * L.ncr;
-  double *x = th_vec(c, TV_X), *r = th_vec(c, TV_R), *z = th_vec(c, TV_Z), *pv = th_vec(c, TV_P),
-         *q = th_vec(c, TV_Q), *dg = th_vec(c, TV_DIAG);
   cudaGraphConditionalHandle h = new_handle(c.stream);
   klaunch(k_th_start, 1, 1, 0, c.stream, h, (const double*)c.scal);
   DP_LAUNCH_CHECK();
   cudaGraph_t body = add_while(c.stream, h);
   cudaStream_t aux = c.aux[0];
   DP_CUDA(cudaStreamBeginCaptureToGraph(aux, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-  klaunch(k_th_apply, (int)div_up(L.nel, 128), 128, 0, aux, (const double*)c.th_buf, (const double*)pv, q, (int)L.nel,
-          L.ncr, L.A(), L.B());
-  klaunch(k_th_pq, red_grid(n), kRedThreads, 0, aux, (const double*)pv, (const double*)q, n, c.scal, c.partial,
-          c.counter);
-  klaunch(k_th_update, red_grid(n), kRedThreads, 0, aux, x, r, z, (const double*)pv, (const double*)q,
-          (const double*)dg, n, L.A(), amax, heated, c.scal, c.partial, c.counter, h);
-  klaunch(k_th_dir, (int)div_up(n, 256), 256, 0, aux, pv, q, (const double*)z, n, (const double*)c.scal);
+  for (int k = 0; k < kThUnroll; ++k) {
+    th_launch_apply(c, k, aux);
+    // a pair of nodes per thread, as long as the grid stays within the partial buffer
+    klaunch(k_th_update, (int)std::min<int64_t>(kRedBlocks, div_up(n / 2, kRedThreads)), kRedThreads, 0, aux,
+            th_vecs(c, k), n, (int)L.A(), amax, heated, c.scal, c.partial, c.counter, h);
+  }
   DP_LAUNCH_CHECK();
   cudaGraph_t out = nullptr;
   DP_CUDA(cudaStreamEndCapture(aux, &out));
 }
 
+// the apply kernel on the last step's blocks and vectors (kernel timing: with the
+// stop flag down; what it adds to q and the slots is zeroed by the next step)
 void launch_th_apply_staged(Ctx& c) {
-  const Level& L = c.fine;
-  ++g_klaunch;
-  k_th_apply<<<(int)div_up(L.nel, 128), 128, 0, c.stream>>>(c.th_buf, th_vec(c, TV_P), th_vec(c, TV_Q), (int)L.nel,
-                                                             L.ncr, L.A(), L.B());
-  DP_LAUNCH_CHECK();
+  DP_CUDA(cudaMemsetAsync(c.scal + TH_STOP, 0, sizeof(double), c.stream));
+  th_launch_apply(c, 0, c.stream);
 }
 
 }  // namespace dp
@@ -351,36 +405,26 @@ extern "C" int dp_thermal_step(dp_ctx* h, const dp_thermal_opts* o, const double
       DP_CUDA(cudaDeviceSynchronize());  // the copies are on the default stream; ours does not wait on it
       if (c.device >= 0 && c.device < 64) uploaded[c.device] = true;
     }
-    if (!c.th_buf) dalloc(&c.th_buf, kThPack * nel + TV_COUNT * nn);
+    if (!c.th_buf) dalloc(&c.th_buf, th_doubles(c));
     const int heated = o->heated ? 1 : 0;
     const int amax = 2 * L.ncr;
-    double* Told = th_vec(c, TV_TOLD);
-    double* Tbc = th_vec(c, TV_TBC);
-    double* dg = th_vec(c, TV_DIAG);
     double* b = th_vec(c, TV_B);
-    double* stage = th_vec(c, TV_STAGE);
-    const cudaMemcpyKind kin = kind_in(mem);
-    DP_CUDA(cudaMemcpyAsync(stage, T, sizeof(double) * nn, kin, c.stream));
-    launch_gather_ref2lat(c, stage, Told, 1);
-    DP_CUDA(cudaMemcpyAsync(stage, rho_node, sizeof(double) * nn, kin, c.stream));
-    double* rho = th_vec(c, TV_X);  // x is initialised by k_th_init after the assembly
-    launch_gather_ref2lat(c, stage, rho, 1);
-    ++g_klaunch;
-    k_th_bc<<<(int)div_up(nn, 256), 256, 0, c.stream>>>(Tbc, nn, L.A(), amax, heated, o->Ttop, o->Tbot);
-    DP_CUDA(cudaMemsetAsync(dg, 0, sizeof(double) * nn, c.stream));
-    DP_CUDA(cudaMemsetAsync(b, 0, sizeof(double) * nn, c.stream));
+    double* Tdev = mem == DP_MEM_DEVICE ? T : th_vec(c, TV_T);
+    static_assert(TV_B == TV_DIAG + 1, "diag and b are zeroed together");
+    DP_CUDA(cudaMemsetAsync(th_vec(c, TV_DIAG), 0, sizeof(double) * 2 * nn, c.stream));
     ThAsmArgs a;
-    a.theta_lat = c.theta_lat; a.r_lat = c.r_lat; a.rho_lat = rho; a.Told = Told; a.Tbc = Tbc;
-    a.Ae = c.th_buf; a.diag = dg; a.b = b; a.K = o->K; a.Cp = o->Cp; a.dt = o->dt;
-    a.nel = (int)nel; a.ncr = L.ncr; a.A = (int)L.A(); a.B = (int)L.B();
+    a.theta_lat = c.theta_lat; a.r_lat = c.r_lat;
+    a.rho = staged(c, rho_node, th_vec(c, TV_RHO), nn, mem);
+    a.Told = staged(c, T, Tdev, nn, mem);
+    a.Ae = c.th_buf; a.diag = th_vec(c, TV_DIAG); a.b = b; a.K = o->K; a.Cp = o->Cp; a.dt = o->dt; a.Ttop = o->Ttop; a.Tbot = o->Tbot;
+    a.nel = (int)nel; a.ncr = L.ncr; a.nct = L.nct; a.A = (int)L.A(); a.B = (int)L.B(); a.heated = heated;
     ++g_klaunch;
     k_th_assemble<<<(int)div_up(nel, 128), 128, 0, c.stream>>>(a);
     DP_LAUNCH_CHECK();
     const int itmax = o->itmax > 0 ? o->itmax : (int)std::min<int64_t>(nn, INT32_MAX);
     ++g_klaunch;
-    k_th_init<<<red_grid(nn), kRedThreads, 0, c.stream>>>(b, dg, th_vec(c, TV_X), th_vec(c, TV_R), th_vec(c, TV_Z),
-                                                        th_vec(c, TV_P), th_vec(c, TV_Q), nn, L.A(), amax, heated,
-                                                        c.scal, c.partial, c.counter, o->rtol, o->atol, itmax);
+    k_th_init<<<red_grid(nn), kRedThreads, 0, c.stream>>>(b, th_vecs(c, 0), nn, L.A(), amax, heated, c.scal, c.partial,
+                                                        c.counter, o->rtol, o->atol, itmax);
     DP_LAUNCH_CHECK();
     // the CG loop: one graph per context and wall configuration
     if (!c.th_exec || c.th_heated != heated) {
@@ -411,10 +455,11 @@ extern "C" int dp_thermal_step(dp_ctx* h, const dp_thermal_opts* o, const double
     }
     DP_CUDA(cudaGraphLaunch((cudaGraphExec_t)c.th_exec, c.stream));
     ++g_klaunch;
-    k_th_finish<<<(int)div_up(nn, 256), 256, 0, c.stream>>>(th_vec(c, TV_X), Tbc, stage, nn);
+    k_th_finish<<<(int)div_up(nn, 256), 256, 0, c.stream>>>(th_vec(c, TV_X), Tdev, (int)nn, (int)L.A(), L.ncr, L.nct,
+                                                          heated, o->Ttop, o->Tbot);
     DP_LAUNCH_CHECK();
-    launch_scatter_lat2ref(c, stage, Told, 1);
-    DP_CUDA(cudaMemcpyAsync(T, Told, sizeof(double) * nn, kind_out(mem), c.stream));
+    if (mem != DP_MEM_DEVICE)
+      DP_CUDA(cudaMemcpyAsync(T, Tdev, sizeof(double) * nn, cudaMemcpyDeviceToHost, c.stream));
     DP_CUDA(cudaMemcpyAsync(c.h_scal, c.scal, sizeof(double) * 64, cudaMemcpyDeviceToHost, c.stream));
     DP_CUDA(cudaStreamSynchronize(c.stream));
     const double it = c.h_scal[TH_IT];

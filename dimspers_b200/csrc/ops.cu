@@ -112,13 +112,90 @@ __device__ __forceinline__ void element_product(const Tm* __restrict__ K, const 
   }
 }
 
+// Scatter of a warp's element results, with what its elements add to the same node
+// summed by shuffles first.  The 32 elements are 16 consecutive cells (of one or
+// more lattice columns): the two triangles of a cell share 3 nodes, neighbouring
+// cells of a column 3, which leaves 6 node updates per cell instead of 12.  All
+// lanes of the warp call it; e0 is the lane's element (idle lanes: >= nel).
+// v: NC values per node in cell order -- type 0: (0,0) (0,2) (2,0) (0,1) (1,0)
+// (1,1), type 1: (0,2) (2,2) (2,0) (1,2) (2,1) (1,1) -- and nd their lattice indices.
+// The FP64 applies were bound by these updates (one 8-byte atomic per value):
+// 512x4096 reduced FP64 apply 414 -> 323 us (0.99 of HBM), FP32 176 -> 163 us.
+template <typename T, int NC, bool kSub>
+__device__ __forceinline__ void cell_scatter(T (&v)[6 * NC], const int nd[6], T* y, int e0, int nel, int ncr) {
+  const bool live = e0 < nel;
+  if (!live) {
+#pragma unroll
+    for (int d = 0; d < 6 * NC; ++d) v[d] = (T)0;
+  }
+  const int lane = threadIdx.x & 31, t = e0 & 1, ir = (e0 >> 1) % ncr;
+  const bool from_prev = live && lane >= 2 && ir > 0;
+  // otherwise the next cell of the column takes this cell's outer nodes
+  const bool keep = lane >= 30 || ir == ncr - 1 || (e0 | 1) + 2 >= nel;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    // within the cell: type 0 takes (2,0) and (1,1), type 1 takes (0,2)
+    const T o = __shfl_xor_sync(0xffffffffu, t ? v[2 * NC + c] : v[NC + c], 1);
+    const T m = __shfl_xor_sync(0xffffffffu, v[5 * NC + c], 1);
+    if (t) {
+      v[c] += o;
+    } else {
+      v[2 * NC + c] += o;
+      v[5 * NC + c] += m;
+    }
+    // from the previous cell: its (2,0) and (2,2) are this one's (0,0) and (0,2), its (2,1) the (0,1)
+    const T a = __shfl_up_sync(0xffffffffu, t ? v[NC + c] : v[2 * NC + c], 2);
+    const T b = __shfl_up_sync(0xffffffffu, v[4 * NC + c], 1);
+    if (from_prev) {
+      v[c] += a;
+      if (!t) v[3 * NC + c] += b;
+    }
+  }
+  if (!live) return;
+  auto put = [&](int s) {
+    if (NC == 2) {
+      if (kSub) atomic_add2(&y[2 * nd[s]], -v[2 * s], -v[2 * s + NC - 1]);
+      else atomic_add2(&y[2 * nd[s]], v[2 * s], v[2 * s + NC - 1]);
+    } else {
+      atomicAdd(&y[nd[s]], v[s]);
+    }
+  };
+  put(0);
+  put(3);
+  if (t) {
+    if (keep) {
+      put(1);
+      put(4);
+    }
+  } else {
+    put(4);
+    put(5);
+    if (keep) put(2);
+  }
+}
+
+// The last two local nodes of a type-0 element in cell order (see cell_scatter).
+template <typename T, int NC>
+__device__ __forceinline__ void to_cell_order(T (&v)[6 * NC], int nd[6], int e) {
+  if (e & 1) return;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const T h = v[4 * NC + c];
+    v[4 * NC + c] = v[5 * NC + c];
+    v[5 * NC + c] = h;
+  }
+  const int h = nd[4];
+  nd[4] = nd[5];
+  nd[5] = h;
+}
+
 // y += K_e x_e for element e (kSub: y -= K_e x_e), scatter-added with atomics.
-template <typename Tm, typename Tv, bool kL2, bool kSub = false, bool kDep = false>
+template <typename Tm, typename Tv, bool kL2, bool kSub = false>
 __device__ __forceinline__ void apply_element(const Tm* __restrict__ K, const Tv* x, Tv* y, int e, int ncr, int A,
                                               int B) {
   int nd[6];
   Tv ye[12];
-  element_product<Tm, Tv, kL2, kDep>(K, x, e, ncr, A, B, nd, ye);
+  element_product<Tm, Tv, kL2>(K, x, e, ncr, A, B, nd, ye);
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     if (kSub) atomic_add2(&y[2 * nd[k]], -ye[2 * k], -ye[2 * k + 1]);
@@ -130,9 +207,12 @@ template <typename Tm, typename Tv, bool kSub = false>
 __global__ void __launch_bounds__(256) k_apply_K(const Tm* __restrict__ K, const Tv* x,
                                                  Tv* y, int nel, int ncr, int A, int B, int wt) {
   grid_dep_launch();
-  const int e = tile_element(ncr, wt);
-  if (e >= nel) return;
-  apply_element<Tm, Tv, false, kSub, true>(K, x, y, e, ncr, A, B);
+  const int e0 = tile_element(ncr, wt), e = min(e0, nel - 1);   // idle lanes follow the last element, adding nothing
+  int nd[6];
+  Tv ye[12];
+  element_product<Tm, Tv, false, true>(K, x, e, ncr, A, B, nd, ye);
+  to_cell_order<Tv, 2>(ye, nd, e);
+  cell_scatter<Tv, 2, kSub>(ye, nd, y, e0, nel, ncr);
 }
 
 // Deterministic form, pass 1: E[(2k + c) nel + e] = (K_e x_e) of local node k,
@@ -319,16 +399,11 @@ template <typename T, bool kSub>
 __global__ void __launch_bounds__(256) k_apply_R(const T* __restrict__ R, const T* x, T* y, int nel, int ncr, int A,
                                                  int B, int wt, int pin, T ch, T sh) {
   grid_dep_launch();
-  const int e = tile_element(ncr, wt);
-  if (e >= nel) return;
+  const int e0 = tile_element(ncr, wt), e = min(e0, nel - 1);
   int nd[6];
   T ye[12];
   reduced_product<T>(R, x, e, ncr, A, B, pin, ch, sh, nd, ye);
-#pragma unroll
-  for (int s = 0; s < 6; ++s) {
-    if (kSub) atomic_add2(&y[2 * nd[s]], -ye[2 * s], -ye[2 * s + 1]);
-    else atomic_add2(&y[2 * nd[s]], ye[2 * s], ye[2 * s + 1]);
-  }
+  cell_scatter<T, 2, kSub>(ye, nd, y, e0, nel, ncr);
 }
 
 // Deterministic form, pass 1 (as k_apply_K_elem): slot 4 is local node 5 for type 0
@@ -579,21 +654,23 @@ __device__ inline void element_pdofs_dev(int e, int ncr, int nct, int pressure, 
   else        { pd[0] = v2; pd[1] = v3; pd[2] = v4; }
 }
 
-__global__ void k_apply_G(const double* __restrict__ G, const double* p, double* y,
-                          int nel, int ncr, int nct, int A, int B, int pressure) {
-  grid_dep_wait();
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nel) return;
+__global__ void __launch_bounds__(128) k_apply_G(const double* __restrict__ G, const double* p, double* y, int nel,
+                                                 int ncr, int nct, int A, int B, int pressure) {
+  grid_dep_launch();
+  const int e0 = blockIdx.x * blockDim.x + threadIdx.x, e = min(e0, nel - 1);
+  double g[kGe];   // the element's block is constant during a solve: fetched before the wait
+#pragma unroll
+  for (int k = 0; k < kGe; ++k) g[k] = ld_stream(G + (size_t)k * nel + e);
   int nd[6], pd[3];
   element_nodes_dev(e, ncr, A, B, nd);
   element_pdofs_dev(e, ncr, nct, pressure, pd);
+  grid_dep_sync();
   const double p0 = p[pd[0]], p1 = p[pd[1]], p2 = p[pd[2]];
+  double v[12];
 #pragma unroll
-  for (int d = 0; d < 12; ++d) {
-    const double v = G[(size_t)d * nel + e] * p0 + G[(size_t)(12 + d) * nel + e] * p1 +
-                     G[(size_t)(24 + d) * nel + e] * p2;
-    atomicAdd(&y[2 * nd[d >> 1] + (d & 1)], v);
-  }
+  for (int d = 0; d < 12; ++d) v[d] = g[d] * p0 + g[12 + d] * p1 + g[24 + d] * p2;
+  to_cell_order<double, 2>(v, nd, e);
+  cell_scatter<double, 2, false>(v, nd, y, e0, nel, ncr);
 }
 
 // Deterministic form of the G apply, pass 1: element e's 12 values of G_e p_e
@@ -641,61 +718,6 @@ __global__ void k_apply_GT(const double* __restrict__ G, const double* x, double
   }
 }
 
-// y = G p with the scatter pre-summed per warp: with ncr a multiple of 16 the 32
-// elements of a warp are the two triangles of 16 consecutive cells of one theta
-// column, which share 33 x 3 = 99 lattice nodes.  The warp adds its 384 values
-// into a shared-memory copy of those nodes first and then issues one global FP64
-// atomic per node and component (198), since sm_100a has no vector FP64 reduction.
-constexpr int kGWarpNodes = 99;
-__global__ void __launch_bounds__(128) k_apply_G_warp(const double* __restrict__ G, const double* p,
-                                                      double* y, int nel, int ncr, int nct, int A, int B,
-                                                      int pressure) {
-  grid_dep_launch();
-  __shared__ double acc[4][2 * kGWarpNodes];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  const int e0 = e - lane;                        // first element of the warp (nel is a multiple of 32)
-  if (e0 >= nel) return;                          // whole warps past the last element (tail block)
-  const int q0 = e0 >> 1, ir0 = q0 % ncr, it = q0 / ncr;
-  double* s = acc[w];
-  double g[kGe];   // constant during a solve: fetched before the wait
-#pragma unroll
-  for (int k = 0; k < kGe; ++k) g[k] = ld_stream(G + (size_t)k * nel + e);
-  for (int k = lane; k < 2 * kGWarpNodes; k += 32) s[k] = 0.0;
-  grid_dep_sync();
-  __syncwarp();
-  {
-    const int q = e >> 1, t = e & 1;
-    const int ir = q % ncr;
-    int pd[3];
-    element_pdofs_dev(e, ncr, nct, pressure, pd);
-    const double p0 = p[pd[0]], p1 = p[pd[1]], p2 = p[pd[2]];
-    // local lattice offsets (a relative to 2 ir0, b relative to 2 it) of the 6 nodes
-    const int la0 = 2 * (ir - ir0);
-    int la[6], lb[6];
-    if (t == 0) {
-      la[0] = la0; la[1] = la0; la[2] = la0 + 2; la[3] = la0; la[4] = la0 + 1; la[5] = la0 + 1;
-      lb[0] = 0; lb[1] = 2; lb[2] = 0; lb[3] = 1; lb[4] = 1; lb[5] = 0;
-    } else {
-      la[0] = la0; la[1] = la0 + 2; la[2] = la0 + 2; la[3] = la0 + 1; la[4] = la0 + 2; la[5] = la0 + 1;
-      lb[0] = 2; lb[1] = 2; lb[2] = 0; lb[3] = 2; lb[4] = 1; lb[5] = 1;
-    }
-#pragma unroll
-    for (int d = 0; d < 12; ++d) {
-      const double v = g[d] * p0 + g[12 + d] * p1 + g[24 + d] * p2;
-      const int k = d >> 1;
-      atomicAdd(&s[2 * (la[k] + 33 * lb[k]) + (d & 1)], v);
-    }
-  }
-  __syncwarp();
-  for (int k = lane; k < kGWarpNodes; k += 32) {
-    const int a = 2 * ir0 + k % 33, bl = 2 * it + k / 33;
-    const int64_t n = a + (int64_t)A * (bl >= B ? bl - B : bl);
-    atomicAdd(&y[2 * n], s[2 * k]);
-    atomicAdd(&y[2 * n + 1], s[2 * k + 1]);
-  }
-}
-
 void launch_apply_G(Ctx& c, const double* p, double* y) {
   const Level& L = c.fine;
   if (L.det) {
@@ -707,14 +729,8 @@ void launch_apply_G(Ctx& c, const double* p, double* y) {
     return;
   }
   DP_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * 2 * L.nnod, c.stream));
-  if (L.ncr % 16 == 0) {
-    // nel = 2 ncr nct is then a multiple of 32 and every warp is whole
-    klaunch(k_apply_G_warp, (int)div_up(L.nel, 128), 128, 0, c.stream, c.Gp, p, y, (int)L.nel, L.ncr, L.nct,
-            (int)L.A(), (int)L.B(), c.mesh.pressure);
-  } else {
-    klaunch(k_apply_G, (int)div_up(L.nel, 128), 128, 0, c.stream, c.Gp, p, y, (int)L.nel, L.ncr, L.nct, (int)L.A(),
-            (int)L.B(), c.mesh.pressure);
-  }
+  klaunch(k_apply_G, (int)div_up(L.nel, 128), 128, 0, c.stream, c.Gp, p, y, (int)L.nel, L.ncr, L.nct, (int)L.A(),
+          (int)L.B(), c.mesh.pressure);
   DP_LAUNCH_CHECK();
 }
 

@@ -201,16 +201,15 @@ __global__ void __launch_bounds__(128) k_th_apply(ThVecs v, const double* scal, 
   double d = 0.0;
   if (live) {
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      atomicAdd(&v.q[nd[i]], yv[i]);
-      d += xv[i] * yv[i];
-    }
+    for (int i = 0; i < 6; ++i) d += xv[i] * yv[i];
     if (!(e & 1)) {
 #pragma unroll
       for (int i = 0; i < 6; ++i)
         if (i != 1 && i != 2) v.pn[nd[i]] = xv[i];   // local nodes 0, 3, 4, 5: the cell's own 2x2 block
     }
   }
+  to_cell_order<double, 1>(yv, nd, ec);
+  cell_scatter<double, 1, false>(yv, nd, v.q, e, nel, ncr);
   d = warp_sum(d);
   if ((threadIdx.x & 31) == 0) atomicAdd(&v.slots[(4 * blockIdx.x + (threadIdx.x >> 5)) % kThSlots], d);
 }

@@ -360,9 +360,11 @@ __device__ inline void fine_node_weights(int a, int b, int ncrc, int Ac, int Bc,
 }
 
 // xf += P xc (per fine node, gather); also sets rf = bf (the fine level's
-// residual buffer, from which the next apply subtracts A xf) unless rf is null
+// residual buffer, from which the next apply subtracts A xf) unless rf is null.
+// d1 (and d2) given: xf holds the last step of the pre-smoothing only, and the
+// smoothed x is (d1 + d2) + xf.
 template <typename T>
-__global__ void k_prolong_add(const T* xc, T* xf, const T* bf,
+__global__ void k_prolong_add(const T* xc, T* xf, const T* d1, const T* d2, const T* bf,
                               T* rf, int Af, int Bf, int ncrc, int Ac, int Bc, int pin) {
   grid_dep_launch();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -380,6 +382,16 @@ __global__ void k_prolong_add(const T* xc, T* xf, const T* bf,
 #pragma unroll
   for (int k = 0; k < 6; ++k) v[k] = xc2[cn[k]];
   X2 xv = reinterpret_cast<const X2*>(xf)[n];
+  if (d1) {
+    X2 u = reinterpret_cast<const X2*>(d1)[n];
+    if (d2) {
+      const X2 w2 = reinterpret_cast<const X2*>(d2)[n];
+      u.x += w2.x;
+      u.y += w2.y;
+    }
+    xv.x = u.x + xv.x;
+    xv.y = u.y + xv.y;
+  }
   X2 bv = xv;
   if (rf) bv = reinterpret_cast<const X2*>(bf)[n];
   T s0 = (T)0, s1 = (T)0;
@@ -462,7 +474,7 @@ __global__ void __launch_bounds__(256) k_restrict_g(const T* r, const T* t, T* b
     if (tc) { tc[2 * n] = (T)0; tc[2 * n + 1] = (T)0; }
     rc[2 * n] = (T)b0; rc[2 * n + 1] = (T)b1;
     dc[2 * n] = (T)(it * z0); dc[2 * n + 1] = (T)(it * z1);
-    xc[2 * n] = (T)(it * z0); xc[2 * n + 1] = (T)(it * z1);
+    if (xc) { xc[2 * n] = (T)(it * z0); xc[2 * n + 1] = (T)(it * z1); }
   }
 }
 
@@ -550,19 +562,24 @@ __global__ void __launch_bounds__(256) k_restrict_tile(const T* r, const T* t,
     }
     reinterpret_cast<X2*>(rc)[n] = bv;
     reinterpret_cast<X2*>(dc)[n] = dv;
-    reinterpret_cast<X2*>(xc)[n] = dv;
+    if (xc) reinterpret_cast<X2*>(xc)[n] = dv;
   }
 }
 
 // ---- Chebyshev smoother vector steps (per node, coefficients read from device) --
 // The residual r lives in one buffer that the applies between the steps update
-// in place (r -= A d, launch_apply_K_sub), so a step reads r, d, x and the
-// block inverse and writes only d and x: no accumulator is zeroed, re-read or
-// subtracted (52 instead of 76 bytes per FP32 node).
-// The three kernels compute in the precision of the level (FP32 on the FP32
+// in place (r -= A d, launch_apply_K_sub).  With 2 or 3 steps (the default 3)
+// the steps only form the d_k, each in a buffer of its own, and x is put
+// together where it is next needed anyway: by the prolongation after the
+// pre-smoothing (whose last d lies in x) and by the last post-smoothing step.
+// That moves 272 instead of 328 bytes per FP32 node and V-cycle: the FP32
+// V-cycle takes 2250 instead of 2330 us at 512x4096 and 174 instead of 186 at
+// 64x512, within 1 % of the same at 128x1024.
+// The kernels compute in the precision of the level (FP32 on the FP32
 // hierarchy) and move each node's pair of components with one 8/16-byte
 // access, all loads issued before the arithmetic.
-// first step from x = 0: r = b, d = (1/theta) D^-1 b, x = d
+
+// first step from x = 0: r = b, d = (1/theta) D^-1 b (x = d unless x is null)
 template <typename T>
 __global__ void k_cheb_first(const T* b, const T* __restrict__ dinv, T* x,
                              T* r, T* d, const double* __restrict__ coef, int64_t nnod) {
@@ -580,9 +597,9 @@ __global__ void k_cheb_first(const T* b, const T* __restrict__ dinv, T* x,
   dv.x = it * z0; dv.y = it * z1;
   reinterpret_cast<X2*>(r)[n] = bv;
   reinterpret_cast<X2*>(d)[n] = dv;
-  reinterpret_cast<X2*>(x)[n] = dv;
+  if (x) reinterpret_cast<X2*>(x)[n] = dv;
 }
-// first step from a given x (r = b - Ax on entry): d = (1/theta) D^-1 r, x += d
+// first step from a given x (r = b - Ax on entry): d = (1/theta) D^-1 r (x += d unless x is null)
 template <typename T>
 __global__ void k_cheb_first_x(const T* r, const T* __restrict__ dinv, T* x,
                                T* d, const double* __restrict__ coef, int64_t nnod) {
@@ -594,20 +611,24 @@ __global__ void k_cheb_first_x(const T* r, const T* __restrict__ dinv, T* x,
   const T it = (T)ld_early(coef);
   grid_dep_sync();
   const X2 rv = reinterpret_cast<const X2*>(r)[n];
-  const X2 xv = reinterpret_cast<const X2*>(x)[n];
+  X2 xv;
+  if (x) xv = reinterpret_cast<const X2*>(x)[n];
   X2 dv;
   T z0, z1;
   di.apply(rv.x, rv.y, z0, z1);
   dv.x = it * z0; dv.y = it * z1;
   reinterpret_cast<X2*>(d)[n] = dv;
-  X2 xn;
-  xn.x = xv.x + dv.x; xn.y = xv.y + dv.y;
-  reinterpret_cast<X2*>(x)[n] = xn;
+  if (!x) return;
+  xv.x += dv.x; xv.y += dv.y;
+  reinterpret_cast<X2*>(x)[n] = xv;
 }
-// d = c1 d + c2 D^-1 r; x += d  (c1, c2 = coef[0], coef[1]; r already holds r - A d_prev)
-template <typename T>
-__global__ void k_cheb_step(const T* r, const T* __restrict__ dinv, T* x,
-                            T* d, const double* __restrict__ coef, int64_t nnod) {
+// d_new = c1 d + c2 D^-1 r  (c1, c2 = coef[0], coef[1]; r already holds r - A d)
+// CH_IN_PLACE: d = d_new, x += d_new;  CH_NEXT: dn = d_new;
+// CH_LAST: x = ((x + e) + d) + d_new, e the step before d (null: none)
+enum ChebStep { CH_IN_PLACE, CH_NEXT, CH_LAST };
+template <int MODE, typename T>
+__global__ void k_cheb_step(const T* r, const T* __restrict__ dinv, T* x, T* d, T* dn, const T* e,
+                            const double* __restrict__ coef, int64_t nnod) {
   grid_dep_launch();
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nnod) return;
@@ -617,14 +638,24 @@ __global__ void k_cheb_step(const T* r, const T* __restrict__ dinv, T* x,
   grid_dep_sync();
   const X2 rv = reinterpret_cast<const X2*>(r)[n];
   const X2 dv = reinterpret_cast<const X2*>(d)[n];
-  const X2 xv = reinterpret_cast<const X2*>(x)[n];
-  X2 dn, xn;
+  X2 xv, ev;
+  if (MODE != CH_NEXT) xv = reinterpret_cast<const X2*>(x)[n];
+  if (MODE == CH_LAST && e) ev = reinterpret_cast<const X2*>(e)[n];
+  X2 nv;
   T z0, z1;
   di.apply(rv.x, rv.y, z0, z1);
-  dn.x = c1 * dv.x + c2 * z0; dn.y = c1 * dv.y + c2 * z1;
-  xn.x = xv.x + dn.x; xn.y = xv.y + dn.y;
-  reinterpret_cast<X2*>(d)[n] = dn;
-  reinterpret_cast<X2*>(x)[n] = xn;
+  nv.x = c1 * dv.x + c2 * z0; nv.y = c1 * dv.y + c2 * z1;
+  if (MODE == CH_IN_PLACE) reinterpret_cast<X2*>(d)[n] = nv;
+  if (MODE == CH_NEXT) {
+    reinterpret_cast<X2*>(dn)[n] = nv;
+    return;
+  }
+  if (MODE == CH_LAST) {
+    if (e) { xv.x += ev.x; xv.y += ev.y; }
+    xv.x += dv.x; xv.y += dv.y;
+  }
+  xv.x += nv.x; xv.y += nv.y;
+  reinterpret_cast<X2*>(x)[n] = xv;
 }
 // z = D^-1 r (nodal blocks)
 template <typename T>
@@ -1237,33 +1268,59 @@ static void chebyshev_stencil(Ctx& c, MGLevel& L, const T* b, T* x, int mode) {
   DP_LAUNCH_CHECK();
 }
 
+// Levels whose x is put together late (see the vector steps above); not the
+// coarsest, which has no prolongation to complete it.
+static bool late_x(const Ctx& c, const MGLevel& L) {
+  return !stencil_level(c, L) && (L.degree == 2 || L.degree == 3) && &L != &c.mg.back();
+}
+
 // Chebyshev smoothing of A x = b on level L.  mode 0: start from x = 0;
 // mode 1: start from x = 0 with the first step already taken (fused into the
 // restriction that produced b); mode 2: start from the given x, with L.r
 // holding b on entry (the prolongation copies it there).  The recurrence
 // coefficients live in L.cheb on the device, so this sequence is the same for
 // every assembly and is captured once into the solve graph.
-// On exit r = b - A (x - d_last), i.e. the true residual is r - A d_last.
+// On exit of modes 0 and 1 r = b - A (x - d_last), i.e. the true residual is
+// r - A d_last; returns d_last, which for late_x levels lies in x (x itself is
+// then L.d (+ L.t) + x, completed by the prolongation).
 template <typename T>
-static void chebyshev(Ctx& c, MGLevel& L, const T* b, T* x, int mode) {
+static const T* chebyshev(Ctx& c, MGLevel& L, const T* b, T* x, int mode) {
   if (stencil_level(c, L)) {
     chebyshev_stencil<T>(c, L, b, x, mode);
-    return;
+    return nullptr;
   }
   const int64_t nn = L.g.nnod;
-  T* r = (T*)L.r; T* d = (T*)L.d;
+  T* r = (T*)L.r;
+  T* d = (T*)L.d;
   const T* dinv = level_dinv<T>(L);
+  const bool late = late_x(c, L);
+  const T* none = nullptr;
   if (mode == 0) {
-    klaunch(k_cheb_first<T>, tpb(nn), 256, 0, c.stream, b, dinv, x, r, d, L.cheb, nn);
+    klaunch(k_cheb_first<T>, tpb(nn), 256, 0, c.stream, b, dinv, late ? (T*)nullptr : x, r, d, L.cheb, nn);
   } else if (mode == 2) {
     launch_apply_K_sub<T, T>(L.g, level_K<T>(L), x, r, c.stream);
-    klaunch(k_cheb_first_x<T>, tpb(nn), 256, 0, c.stream, (const T*)r, dinv, x, d, L.cheb, nn);
+    klaunch(k_cheb_first_x<T>, tpb(nn), 256, 0, c.stream, (const T*)r, dinv, late ? (T*)nullptr : x, d, L.cheb, nn);
   }
+  const T* before = nullptr;   // the step before d (late form)
   for (int k = 1; k < L.degree; ++k) {
-    launch_apply_K_sub<T, T>(L.g, level_K<T>(L), d, r, c.stream);
-    klaunch(k_cheb_step<T>, tpb(nn), 256, 0, c.stream, (const T*)r, dinv, x, d, L.cheb + 2 * k, nn);
+    launch_apply_K_sub<T, T>(L.g, level_K<T>(L), (const T*)d, r, c.stream);
+    const double* coef = L.cheb + 2 * k;
+    if (!late) {
+      klaunch(k_cheb_step<CH_IN_PLACE, T>, tpb(nn), 256, 0, c.stream, (const T*)r, dinv, x, d, (T*)nullptr, none, coef,
+              nn);
+    } else if (mode == 2 && k + 1 == L.degree) {
+      klaunch(k_cheb_step<CH_LAST, T>, tpb(nn), 256, 0, c.stream, (const T*)r, dinv, x, d, (T*)nullptr, before, coef,
+              nn);
+    } else {
+      T* dn = k + 1 == L.degree ? x : (T*)L.t;
+      klaunch(k_cheb_step<CH_NEXT, T>, tpb(nn), 256, 0, c.stream, (const T*)r, dinv, (T*)nullptr, d, dn, none, coef,
+              nn);
+      before = d;
+      d = dn;
+    }
   }
   DP_LAUNCH_CHECK();
+  return d;
 }
 
 // first_done: the level's first pre-smoothing step was fused into the restriction.
@@ -1299,28 +1356,32 @@ static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool 
   // the coarse level's first smoothing step in the same pass unless it is
   // solved densely)
   const bool st = stencil_level(c, L);   // its pre-smoothing leaves the true residual in r
-  chebyshev<T>(c, L, b, x, first_done ? 1 : 0);
-  if (!st) launch_apply_K_sub<T, T>(L.g, level_K<T>(L), (const T*)L.d, r, c.stream);
+  const T* d_last = chebyshev<T>(c, L, b, x, first_done ? 1 : 0);
+  if (!st) launch_apply_K_sub<T, T>(L.g, level_K<T>(L), d_last, r, c.stream);
   const bool fuse = !(l + 2 == c.mg.size() && dense_coarsest);
   // the cluster tail's smoother accumulates A d into t, which starts at zero
   T* tc = (l + 1 == tail_start(c, o)) ? (T*)C.t : nullptr;
   const int nA0 = (int)((C.g.A() + 1) >> 1);  // coarse nodes per parity class (upper bound)
+  // a coarse level that puts its x together late does not read it before the prolongation from below
+  T* xc1 = late_x(c, C) && l + 1 != tail_start(c, o) ? nullptr : xc;
   // the tiled form needs whole tiles along theta (its patch then wraps at most once)
   const bool small = C.g.nnod < 32768 || C.g.B() % kRTile != 0;
   if (small) {
     dim3 grid((unsigned)div_up(4 * (int64_t)nA0 * (C.g.B() >> 1), 256), 4);
     klaunch(k_restrict_g<T, 4>, grid, 256, 0, c.stream, (const T*)r, (const T*)nullptr, bc, (int)L.g.A(),
-            (int)L.g.B(), (int)C.g.A(), (int)C.g.B(), C.g.pin, fuse ? 1 : 0, (const T*)level_dinv<T>(C), xc, (T*)C.r,
+            (int)L.g.B(), (int)C.g.A(), (int)C.g.B(), C.g.pin, fuse ? 1 : 0, (const T*)level_dinv<T>(C), xc1, (T*)C.r,
             (T*)C.d, tc, (const double*)C.cheb);
   } else {
     dim3 grid((unsigned)div_up(C.g.A(), kRTile), (unsigned)div_up(C.g.B(), kRTile));
     klaunch(k_restrict_tile<T>, grid, 256, 0, c.stream, (const T*)r, (const T*)nullptr, bc, (int)L.g.A(),
-            (int)L.g.B(), (int)C.g.A(), (int)C.g.B(), C.g.pin, fuse ? 1 : 0, (const T*)level_dinv<T>(C), xc,
+            (int)L.g.B(), (int)C.g.A(), (int)C.g.B(), C.g.pin, fuse ? 1 : 0, (const T*)level_dinv<T>(C), xc1,
             (T*)C.r, (T*)C.d, tc, (const double*)C.cheb);
   }
   DP_LAUNCH_CHECK();
   vcycle<T>(c, l + 1, bc, xc, o, fuse);
-  klaunch(k_prolong_add<T>, tpb(L.g.nnod), 256, 0, c.stream, (const T*)xc, x, b, st ? (T*)nullptr : r, (int)L.g.A(),
+  klaunch(k_prolong_add<T>, tpb(L.g.nnod), 256, 0, c.stream, (const T*)xc, x,
+          late_x(c, L) ? (const T*)L.d : (const T*)nullptr,
+          late_x(c, L) && L.degree == 3 ? (const T*)L.t : (const T*)nullptr, b, st ? (T*)nullptr : r, (int)L.g.A(),
           (int)L.g.B(), C.g.ncr, (int)C.g.A(), (int)C.g.B(), L.g.pin);
   DP_LAUNCH_CHECK();
   chebyshev<T>(c, L, b, x, 2);

@@ -52,3 +52,14 @@ def test_stencil_smoother_degrees(degree):
     U, P = _solve(16, 128, 0, cheb_degree=degree)
     Ut, Pt = _solve(16, 128, 0, cheb_degree=degree, matrix_free=1, mg_tail=1 << 20)
     assert rel(U, Ut) < 2.2e-11 and rel(P, Pt) < 2.2e-11
+
+
+@pytest.mark.parametrize("degree", [2, 3])
+@pytest.mark.parametrize("nr,nt", [(140, 292), (128, 640)])
+def test_late_x_smoother(nr, nt, degree):
+    """Levels too large for stencils put x together after the smoothing (degrees 2 and 3): two such
+    levels, reached by either form of the restriction, against the cluster tail's step-by-step x.
+    (140, 292) halves once only, so that its coarsest level is smoothed too."""
+    U, P = _solve(nr, nt, 0, cheb_degree=degree)
+    Ut, Pt = _solve(nr, nt, 0, cheb_degree=degree, matrix_free=1, mg_tail=1 << 20)
+    assert rel(U, Ut) < 2.2e-11 and rel(P, Pt) < 2.2e-11

@@ -359,6 +359,10 @@ __device__ inline void fine_node_weights(int a, int b, int ncrc, int Ac, int Bc,
   }
 }
 
+}  // namespace dp
+#include "halo.cu"
+namespace dp {
+
 // xf += P xc (per fine node, gather); also sets rf = bf (the fine level's
 // residual buffer, from which the next apply subtracts A xf) unless rf is null.
 // d1 (and d2) given: xf holds the last step of the pre-smoothing only, and the
@@ -1323,6 +1327,14 @@ static const T* chebyshev(Ctx& c, MGLevel& L, const T* b, T* x, int mode) {
   return d;
 }
 
+// Levels smoothed by whole passes (halo.cu): stencils, the default degree, small enough.
+template <typename T>
+static bool halo_level(const Ctx& c, size_t l, const MGOptions& o) {
+  const MGLevel& L = c.mg[l];
+  return l + 1 < c.mg.size() && l < tail_start(c, o) && stencil_level(c, L) && L.degree == kHaloDegree &&
+         halo_fits<T>(L.g);
+}
+
 // first_done: the level's first pre-smoothing step was fused into the restriction.
 template <typename T>
 static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool first_done) {
@@ -1354,11 +1366,18 @@ static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool 
   T* xc = (T*)C.x;
   // pre-smoothing, r -= A d_last (the true residual), then restrict it (and take
   // the coarse level's first smoothing step in the same pass unless it is
-  // solved densely)
+  // solved densely or smoothed by whole passes)
   const bool st = stencil_level(c, L);   // its pre-smoothing leaves the true residual in r
-  const T* d_last = chebyshev<T>(c, L, b, x, first_done ? 1 : 0);
-  if (!st) launch_apply_K_sub<T, T>(L.g, level_K<T>(L), d_last, r, c.stream);
-  const bool fuse = !(l + 2 == c.mg.size() && dense_coarsest);
+  const bool halo = halo_level<T>(c, l, o);
+  const unsigned halo_threads = 32 * halo_warps(L.g.ncr);
+  if (halo) {   // the smoothed x goes to L.d
+    klaunch(k_halo_down<T>, (unsigned)L.g.nct, halo_threads, 0, c.stream, (const T*)L.S, b, r, (T*)L.d,
+            level_dinv<T>(L), (const double*)L.cheb, L.g.ncr, L.g.nct);
+  } else {
+    const T* d_last = chebyshev<T>(c, L, b, x, first_done ? 1 : 0);
+    if (!st) launch_apply_K_sub<T, T>(L.g, level_K<T>(L), d_last, r, c.stream);
+  }
+  const bool fuse = !(l + 2 == c.mg.size() && dense_coarsest) && !halo_level<T>(c, l + 1, o);
   // the cluster tail's smoother accumulates A d into t, which starts at zero
   T* tc = (l + 1 == tail_start(c, o)) ? (T*)C.t : nullptr;
   const int nA0 = (int)((C.g.A() + 1) >> 1);  // coarse nodes per parity class (upper bound)
@@ -1379,6 +1398,13 @@ static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool 
   }
   DP_LAUNCH_CHECK();
   vcycle<T>(c, l + 1, bc, xc, o, fuse);
+  if (halo) {
+    klaunch(k_halo_up<T>, (unsigned)L.g.nct, halo_threads, 0, c.stream, (const T*)L.S, b, (const T*)xc, (const T*)L.d,
+            x, level_dinv<T>(L), (const double*)L.cheb, L.g.ncr, L.g.nct, C.g.ncr, (int)C.g.A(), (int)C.g.B(),
+            L.g.pin);
+    DP_LAUNCH_CHECK();
+    return;
+  }
   klaunch(k_prolong_add<T>, tpb(L.g.nnod), 256, 0, c.stream, (const T*)xc, x,
           late_x(c, L) ? (const T*)L.d : (const T*)nullptr,
           late_x(c, L) && L.degree == 3 ? (const T*)L.t : (const T*)nullptr, b, st ? (T*)nullptr : r, (int)L.g.A(),

@@ -63,3 +63,13 @@ def test_late_x_smoother(nr, nt, degree):
     U, P = _solve(nr, nt, 0, cheb_degree=degree)
     Ut, Pt = _solve(nr, nt, 0, cheb_degree=degree, matrix_free=1, mg_tail=1 << 20)
     assert rel(U, Ut) < 2.2e-11 and rel(P, Pt) < 2.2e-11
+
+
+@pytest.mark.parametrize("precision,tol", [(0, 2.2e-11), (1, 2e-4)])
+@pytest.mark.parametrize("nr,nt", [(2, 8), (2, 148), (16, 148), (18, 148), (20, 148), (20, 152), (22, 40)])
+def test_whole_pass_smoother_edges(nr, nt, precision, tol):
+    """The edges of the levels smoothed by whole passes: the fewest cells either way, the radial counts
+    that fill a block in FP64 (16) and FP32 (20) and the next ones, one wave of blocks and more."""
+    U, P = _solve(nr, nt, precision)
+    Ut, Pt = _solve(nr, nt, precision, matrix_free=1, mg_tail=1 << 20)
+    assert rel(U, Ut) < tol and rel(P, Pt) < tol

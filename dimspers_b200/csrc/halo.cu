@@ -208,13 +208,18 @@ __global__ void __launch_bounds__(halo_max_threads<T>()) k_halo_up(const T* S, c
   const NodeInv<T> di(dinv, row.node);
   const T it = (T)ld_early(coef), c1 = (T)ld_early(coef + 2), c2 = (T)ld_early(coef + 3),
           e1 = (T)ld_early(coef + 4), e2 = (T)ld_early(coef + 5);
+  const HaloNode nd(min(t, kHaloCols * A - 1), A, 2 * nct);
+  int cn[6];
+  float w[6];   // dyadic fractions, exact in FP32
+  {
+    double wd[6];
+    fine_node_weights(nd.a, nd.b, ncrc, Ac, Bc, cn, wd);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) w[k] = (float)wd[k];
+  }
   grid_dep_sync();
   X2 rv = reinterpret_cast<const X2*>(b)[row.node];
   if (t < kHaloCols * A) {
-    const HaloNode nd(t, A, 2 * nct);
-    int cn[6];
-    double w[6];
-    fine_node_weights(nd.a, nd.b, ncrc, Ac, Bc, cn, w);
     X2 v = reinterpret_cast<const X2*>(xp)[nd.n];
     T s0 = (T)0, s1 = (T)0;
 #pragma unroll

@@ -410,54 +410,70 @@ __global__ void k_prolong_add(const T* xc, T* xf, const T* d1, const T* d2, cons
   if (rf) reinterpret_cast<X2*>(rf)[n] = bv;
 }
 
-// bc = P^T (r - t) per coarse node (t = null: P^T r; gather over the class
-// stencil); constrained DOFs of either level are excluded.  blockIdx.y is the parity class, so the
-// stencil reads are uniform across a warp (constant-cache broadcast), and the
-// stencil loop is unrolled with its loads predicated rather than branched, so
-// a thread keeps several gathers in flight.
+// bc = P^T r per coarse node (gather over the class stencil); constrained DOFs
+// of either level are excluded.  blockIdx.y is the parity class.  Four lanes
+// gather for one coarse node, at most 7 taps each, and add up by shuffles.
+// The gather is a chain of two short latencies behind a launch; what took most
+// of it was the table (each lane of four reads its own entry of constant
+// memory, so a read is four), which now happens before the wait together with
+// D^-1: an inner iteration with 2 (16x128) to 3 (32x256) of these launches takes
+// 56.9 and 78.3 us instead of 59.2 and 81.1 (including the same for the
+// weights in k_halo_up).
 // first != 0 also takes the coarse level's first Chebyshev step from x = 0
-// (the work of k_cheb_first): rc = bc, dc = xc = coef[0] D^-1 bc, and tc = 0
-// when tc is given (the cluster tail's levels accumulate into t).
-template <typename T, int LPN>
-__global__ void __launch_bounds__(256) k_restrict_g(const T* r, const T* t, T* bc,
-                                                    int Af, int Bf, int Ac, int Bc, int pin, int first,
-                                                    const T* __restrict__ dinv_c, T* xc, T* rc,
-                                                    T* dc, T* tc,
-                                                    const double* __restrict__ coef_c) {
-  grid_dep_wait();
+// (the work of k_cheb_first): rc = bc, dc = xc = coef[0] D^-1 bc (no xc if it is
+// null), and tc = 0 when tc is given (the cluster tail's levels accumulate into t).
+template <typename T>
+__global__ void __launch_bounds__(256) k_restrict_g(const T* r, T* bc, int Af, int Bf, int Ac, int Bc, int pin,
+                                                    int first, const T* dinv_c, T* xc, T* rc, T* dc, T* tc,
+                                                    const double* coef_c) {
+  grid_dep_launch();
+  constexpr int LPN = 4, PER = (kRTaps + LPN - 1) / LPN;
   const int cls = blockIdx.y;
   const int pa = cls & 1, pb = cls >> 1;
   const int nA = (Ac - pa + 1) >> 1;  // coarse a = pa, pa + 2, ... <= Ac - 1
-  // LPN lanes per coarse node, each gathering every LPN-th tap (LPN = 4 on
-  // small levels: <= 7 taps per lane, all in flight; LPN = 1 on large levels,
-  // where the grid alone keeps the memory system busy), combined by shuffles
   const int gidx = blockIdx.x * blockDim.x + threadIdx.x;
   const int idx = gidx / LPN, sub = gidx % LPN;
   const bool live = idx < nA * (Bc >> 1);
   const int ac = live ? 2 * (idx % nA) + pa : pa, bcn = live ? 2 * (idx / nA) + pb : pb;
+  const int n = ac + Ac * bcn;
   typedef typename V2<T>::T X2;
-  const X2* r2 = reinterpret_cast<const X2*>(r);
-  const X2* t2 = reinterpret_cast<const X2*>(t);
   const int m = live ? c_rtab.n[cls] : 0;
-  double s0 = 0.0, s1 = 0.0;
-#pragma unroll 8
-  for (int j = sub; j < m; j += LPN) {
-    const int jj = j;
+  int f[PER];
+  float w0[PER], w1[PER];   // dyadic fractions, exact in FP32
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int j = sub + LPN * q, jj = j < m ? j : 0;
     const int a = 2 * ac + c_rtab.da[cls][jj];
     int b = 2 * bcn + c_rtab.db[cls][jj];
     b += (b < 0) ? Bf : 0;
     b -= (b >= Bf) ? Bf : 0;
-    const bool in = a >= 0 && a < Af;
-    const int f = in ? a + Af * b : 0;
-    const X2 rv = r2[f];
-    X2 tv;
-    if (t2) tv = t2[f];
-    else { tv.x = (T)0; tv.y = (T)0; }
-    const double w = c_rtab.w[cls][jj];
-    const double w0 = (in && !dof_fixed(a, b, 0, Af - 1, pin)) ? w : 0.0;
-    const double w1 = (in && !dof_fixed(a, b, 1, Af - 1, pin)) ? w : 0.0;
-    s0 += w0 * ((double)rv.x - (double)tv.x);
-    s1 += w1 * ((double)rv.y - (double)tv.y);
+    const bool in = j < m && a >= 0 && a < Af;
+    const float w = (float)c_rtab.w[cls][jj];
+    f[q] = in ? a + Af * b : -1;
+    w0[q] = dof_fixed(a, b, 0, Af - 1, pin) ? 0.f : w;
+    w1[q] = dof_fixed(a, b, 1, Af - 1, pin) ? 0.f : w;
+  }
+  T da = (T)0, db = (T)0, dd = (T)0;
+  double it = 0.0;
+  if (first) {
+    da = ld_early(dinv_c + 3 * (int64_t)n);
+    db = ld_early(dinv_c + 3 * (int64_t)n + 1);
+    dd = ld_early(dinv_c + 3 * (int64_t)n + 2);
+    it = ld_early(coef_c);
+  }
+  grid_dep_sync();
+  const X2* r2 = reinterpret_cast<const X2*>(r);
+  X2 rv[PER];
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    rv[q].x = rv[q].y = (T)0;
+    if (f[q] >= 0) rv[q] = r2[f[q]];
+  }
+  double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    s0 += (double)w0[q] * (double)rv[q].x;
+    s1 += (double)w1[q] * (double)rv[q].y;
   }
   // every lane of the warp takes part in the shuffles (dead lanes add zeros)
 #pragma unroll
@@ -466,24 +482,27 @@ __global__ void __launch_bounds__(256) k_restrict_g(const T* r, const T* t, T* b
     s1 += __shfl_xor_sync(0xffffffffu, s1, o);
   }
   if (!live || sub != 0) return;
-  const int n = ac + Ac * bcn;
+  X2 v;
   const double b0 = dof_fixed(ac, bcn, 0, Ac - 1, pin) ? 0.0 : s0;
   const double b1 = dof_fixed(ac, bcn, 1, Ac - 1, pin) ? 0.0 : s1;
-  bc[2 * n] = (T)b0;
-  bc[2 * n + 1] = (T)b1;
+  v.x = (T)b0;
+  v.y = (T)b1;
+  reinterpret_cast<X2*>(bc)[n] = v;
   if (first) {
-    const double it = coef_c[0];
-    double z0, z1;
-    bj_apply<T>(dinv_c, n, b0, b1, z0, z1);
-    if (tc) { tc[2 * n] = (T)0; tc[2 * n + 1] = (T)0; }
-    rc[2 * n] = (T)b0; rc[2 * n + 1] = (T)b1;
-    dc[2 * n] = (T)(it * z0); dc[2 * n + 1] = (T)(it * z1);
-    if (xc) { xc[2 * n] = (T)(it * z0); xc[2 * n + 1] = (T)(it * z1); }
+    reinterpret_cast<X2*>(rc)[n] = v;
+    v.x = (T)(it * ((double)da * b0 + (double)db * b1));
+    v.y = (T)(it * ((double)db * b0 + (double)dd * b1));
+    reinterpret_cast<X2*>(dc)[n] = v;
+    if (xc) reinterpret_cast<X2*>(xc)[n] = v;
+    if (tc) {
+      v.x = v.y = (T)0;
+      reinterpret_cast<X2*>(tc)[n] = v;
+    }
   }
 }
 
 // Tiled form of the same restriction for the large levels.  One CTA = 16 x 16
-// coarse nodes; the fine values r - t of the CTA's stencil footprint (a 39 x 39
+// coarse nodes; the fine values r of the CTA's stencil footprint (a 39 x 39
 // patch of fine nodes, constrained fine DOFs zeroed) are read from global
 // memory once into shared memory, and each coarse node gathers its class
 // stencil from there (the gather form reads every fine value ~4 times through
@@ -493,8 +512,7 @@ __global__ void __launch_bounds__(256) k_restrict_g(const T* r, const T* t, T* b
 constexpr int kRTile = 16;
 constexpr int kRPatch = 2 * (kRTile - 1) + 1 + 8;   // 39: stencil offsets reach 4 fine nodes each way
 template <typename T>
-__global__ void __launch_bounds__(256) k_restrict_tile(const T* r, const T* t,
-                                                       T* bc, int Af, int Bf, int Ac, int Bc, int pin,
+__global__ void __launch_bounds__(256) k_restrict_tile(const T* r, T* bc, int Af, int Bf, int Ac, int Bc, int pin,
                                                        int first, const T* __restrict__ dinv_c, T* xc,
                                                        T* rc, T* dc, T* tc,
                                                        const double* __restrict__ coef_c) {
@@ -504,7 +522,6 @@ __global__ void __launch_bounds__(256) k_restrict_tile(const T* r, const T* t,
   const int ac0 = blockIdx.x * kRTile, bc0 = blockIdx.y * kRTile;
   const int fa0 = 2 * ac0 - 4, fb0 = 2 * bc0 - 4;
   const X2* r2 = reinterpret_cast<const X2*>(r);
-  const X2* t2 = reinterpret_cast<const X2*>(t);
   for (int k = threadIdx.x; k < kRPatch * kRPatch; k += blockDim.x) {
     const int la = k % kRPatch, lb = k / kRPatch;
     const int a = fa0 + la;
@@ -516,12 +533,7 @@ __global__ void __launch_bounds__(256) k_restrict_tile(const T* r, const T* t,
     v.y = (T)0;
     if (a >= 0 && a < Af) {
       const int64_t f = a + (int64_t)Af * b;
-      X2 rv = r2[f];
-      if (t2) {
-        const X2 tv = t2[f];
-        rv.x -= tv.x;
-        rv.y -= tv.y;
-      }
+      const X2 rv = r2[f];
       if (!dof_fixed(a, b, 0, Af - 1, pin)) v.x = rv.x;
       if (!dof_fixed(a, b, 1, Af - 1, pin)) v.y = rv.y;
     }
@@ -1387,12 +1399,12 @@ static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool 
   const bool small = C.g.nnod < 32768 || C.g.B() % kRTile != 0;
   if (small) {
     dim3 grid((unsigned)div_up(4 * (int64_t)nA0 * (C.g.B() >> 1), 256), 4);
-    klaunch(k_restrict_g<T, 4>, grid, 256, 0, c.stream, (const T*)r, (const T*)nullptr, bc, (int)L.g.A(),
+    klaunch(k_restrict_g<T>, grid, 256, 0, c.stream, (const T*)r, bc, (int)L.g.A(),
             (int)L.g.B(), (int)C.g.A(), (int)C.g.B(), C.g.pin, fuse ? 1 : 0, (const T*)level_dinv<T>(C), xc1, (T*)C.r,
             (T*)C.d, tc, (const double*)C.cheb);
   } else {
     dim3 grid((unsigned)div_up(C.g.A(), kRTile), (unsigned)div_up(C.g.B(), kRTile));
-    klaunch(k_restrict_tile<T>, grid, 256, 0, c.stream, (const T*)r, (const T*)nullptr, bc, (int)L.g.A(),
+    klaunch(k_restrict_tile<T>, grid, 256, 0, c.stream, (const T*)r, bc, (int)L.g.A(),
             (int)L.g.B(), (int)C.g.A(), (int)C.g.B(), C.g.pin, fuse ? 1 : 0, (const T*)level_dinv<T>(C), xc1,
             (T*)C.r, (T*)C.d, tc, (const double*)C.cheb);
   }

@@ -25,6 +25,7 @@ template <typename Tm, typename Tv>
 void launch_apply_K_acc(const Level& L, const Tm* K, const Tv* x, Tv* y, cudaStream_t s);   // y += K x
 template <typename Tm, typename Tv>
 void launch_apply_K_sub(const Level& L, const Tm* K, const Tv* x, Tv* y, cudaStream_t s);   // y -= K x
+bool launch_apply_K_dot(const Level& L, const double* x, double* y, double* dot, cudaStream_t s);
 // Deterministic mode: per node, y (mode 0: +=, 1: -=, 2: =) the sum over its
 // elements, in a fixed order, of E[(2 k + c) nel + e]
 template <typename T>

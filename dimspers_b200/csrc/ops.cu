@@ -327,7 +327,7 @@ struct RVec {
 // indices; the matrix is fetched before the wait for the predecessor.
 template <typename T>
 __device__ __forceinline__ void reduced_product(const T* __restrict__ R, const T* x, int e, int ncr, int A, int B,
-                                                int pin, T ch, T sh, int nd[6], T y[12]) {
+                                                int pin, T ch, T sh, int nd[6], T y[12], T* xy = nullptr) {
   typedef typename V2<T>::T X2;
   T kk[kRed];
   {
@@ -382,6 +382,12 @@ __device__ __forceinline__ void reduced_product(const T* __restrict__ R, const T
       if (Rr != C) y[C] += kv * rel[Rr];
     }
   }
+  if (xy) {   // x_e . K_e x_e, from the values relative to the reference node
+    T s = (T)0;
+#pragma unroll
+    for (int C = 0; C < 10; ++C) s += rel[C] * y[C];
+    *xy = s;
+  }
   // column sums: up (slot 1, and 0 and 3 for t = 1), down (slot 2, and 0 and 4 for t = 0), middle
   const T ux = y[2] + (t ? y[0] + y[6] : (T)0), uy = y[3] + (t ? y[1] + y[7] : (T)0);
   const T dx = y[4] + (t ? (T)0 : y[0] + y[8]), dy = y[5] + (t ? (T)0 : y[1] + y[9]);
@@ -395,15 +401,29 @@ __device__ __forceinline__ void reduced_product(const T* __restrict__ R, const T
   }
 }
 
-template <typename T, bool kSub>
+// kDot: also adds x . K x to *dot, one atomic per block (each element's share is
+// non-negative and known here, so the solver needs no pass over x and y for it).
+template <typename T, bool kSub, bool kDot = false>
 __global__ void __launch_bounds__(256) k_apply_R(const T* __restrict__ R, const T* x, T* y, int nel, int ncr, int A,
-                                                 int B, int wt, int pin, T ch, T sh) {
+                                                 int B, int wt, int pin, T ch, T sh, double* dot) {
   grid_dep_launch();
   const int e0 = tile_element(ncr, wt), e = min(e0, nel - 1);
   int nd[6];
   T ye[12];
-  reduced_product<T>(R, x, e, ncr, A, B, pin, ch, sh, nd, ye);
+  T xy;
+  reduced_product<T>(R, x, e, ncr, A, B, pin, ch, sh, nd, ye, kDot ? &xy : nullptr);
   cell_scatter<T, 2, kSub>(ye, nd, y, e0, nel, ncr);
+  if (kDot) {
+    __shared__ double part[8];
+    const double s = warp_sum(e0 < nel ? (double)xy : 0.0);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
+      atomicAdd(dot, t);
+    }
+  }
 }
 
 // Deterministic form, pass 1 (as k_apply_K_elem): slot 4 is local node 5 for type 0
@@ -591,7 +611,7 @@ static void apply_K_into(const Level& L, const Tm* K, const Tv* x, Tv* y, cudaSt
   apply_tile(L, blocks, threads, wt);
   if (R) {
     klaunch(k_apply_R<Tv, kSub>, blocks, threads, 0, s, R, x, y, (int)L.nel, L.ncr, (int)L.A(), (int)L.B(), wt, L.pin,
-            (Tv)std::cos(h), (Tv)std::sin(h));
+            (Tv)std::cos(h), (Tv)std::sin(h), (double*)nullptr);
     DP_LAUNCH_CHECK();
     return;
   }
@@ -613,6 +633,19 @@ void launch_apply_K_acc(const Level& L, const Tm* K, const Tv* x, Tv* y, cudaStr
 }
 template void launch_apply_K_acc<double, double>(const Level&, const double*, const double*, double*, cudaStream_t);
 template void launch_apply_K_acc<float, float>(const Level&, const float*, const float*, float*, cudaStream_t);
+
+// y += K x and *dot += x . K x on the reduced element matrices; false (nothing
+// done) where the level has none or runs without atomics.
+bool launch_apply_K_dot(const Level& L, const double* x, double* y, double* dot, cudaStream_t s) {
+  if (!L.red64 || L.det || mf_data<double>(L)) return false;
+  const double h = 3.14159265358979323846 / L.nct;
+  int blocks, threads, wt;
+  apply_tile(L, blocks, threads, wt);
+  klaunch(k_apply_R<double, false, true>, blocks, threads, 0, s, L.red64, x, y, (int)L.nel, L.ncr, (int)L.A(),
+          (int)L.B(), wt, L.pin, std::cos(h), std::sin(h), dot);
+  DP_LAUNCH_CHECK();
+  return true;
+}
 
 // y -= K x: the smoother keeps its residual in y and lets the apply update it
 // in place (no accumulator to zero and re-read)

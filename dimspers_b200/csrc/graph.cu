@@ -58,8 +58,9 @@ __device__ inline double inner_rtol_now(const DevCtl* ctl, const double* scal, i
 }
 
 __global__ void k_in_init(cudaGraphConditionalHandle h, DevCtl* ctl, const double* scal, int yy_slot, int irr_slot,
-                          double* scal_w, int fp32, int relax) {
+                          double* scal_w, int fp32, int relax, int rzn_slot) {
   grid_dep_wait();
+  scal_w[rzn_slot] = 0.0;   // the V-cycle's last kernel may accumulate r . z there
   const double yy = scal[yy_slot];
   const double rt = fp32 ? ctl->inner_rtol32 : inner_rtol_now(ctl, scal, relax);
   const double tol2 = rt * rt * yy;
@@ -272,17 +273,32 @@ __global__ void __launch_bounds__(kRedThreads) k_rz_f32(const float* z32, const 
   grid_finish<1>(v, partial, counter, o);
 }
 
+template <typename H, typename X2>
+__device__ __forceinline__ void first_step(const FirstStep<H>& f, int64_t i, X2 b) {
+  const NodeInv<H> di(f.dinv, i);
+  const H it = (H)ld_early(f.coef);
+  H z0, z1;
+  di.apply(b.x, b.y, z0, z1);
+  reinterpret_cast<X2*>(f.r)[i] = b;
+  b.x = it * z0;
+  b.y = it * z1;
+  reinterpret_cast<X2*>(f.d)[i] = b;
+  reinterpret_cast<X2*>(f.x)[i] = b;
+}
+
 // x += alpha p; r -= alpha Ap; ||r||^2 (alpha = rz / pAp from the table); the
 // last block also takes the loop's stopping decision: continue while
 // ||r||^2 > tol^2 ||b||^2 and it < inner_itmax.  r32 != null (FP64 Krylov on
 // the FP32 hierarchy): also writes the next V-cycle's input r / ||b||.
-template <typename T>
+// first.dinv != null: takes the next V-cycle's first smoother step as well, for
+// which it has the input in registers.
+template <typename T, typename H>
 __global__ void __launch_bounds__(kRedThreads) k_pcg_upd_check(T* x, T* r,
                                                                 const T* p, const T* Ap,
                                                                 int64_t nnod, double* scal, int rz, int rzn, int pap,
                                                                 int irr, double* partial, unsigned int* counter,
                                                                 cudaGraphConditionalHandle h, DevCtl* ctl, int fp32,
-                                                                float* r32, int yy) {
+                                                                float* r32, int yy, FirstStep<H> first) {
   grid_dep_wait();
   const double inv_s = r32 ? 1.0 / sqrt(scal[yy]) : 0.0;
   // a non-positive or non-finite p.Ap (breakdown, e.g. an FP32 operator that
@@ -302,7 +318,16 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_upd_check(T* x, T* r,
     rv.y = (T)r1;
     reinterpret_cast<X2*>(x)[i] = xv;
     reinterpret_cast<X2*>(r)[i] = rv;
-    if (r32) reinterpret_cast<float2*>(r32)[i] = make_float2((float)(inv_s * r0), (float)(inv_s * r1));
+    typename V2<H>::T bv;
+    if (std::is_same<T, H>::value) {
+      bv.x = (H)r0;
+      bv.y = (H)r1;
+    } else {
+      bv.x = (H)(inv_s * r0);
+      bv.y = (H)(inv_s * r1);
+      if (r32) reinterpret_cast<float2*>(r32)[i] = make_float2((float)bv.x, (float)bv.y);
+    }
+    if (first.dinv) first_step(first, i, bv);
     s += r0 * r0;
     s += r1 * r1;
   }
@@ -314,6 +339,7 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_upd_check(T* x, T* r,
     if (fp32) { it = ++ctl->in32_it; tol2 = ctl->in32_tol2; ctl->in32_total += 1; }
     else { it = ++ctl->in_it; tol2 = ctl->in_tol2; ctl->in_total += 1; }
     scal[rz] = scal[rzn];
+    scal[rzn] = 0.0;   // every block has read it
     const double rr = scal[irr];
     const bool go = ok && isfinite(rr) && rr > tol2 && it < ctl->inner_itmax;
     cudaGraphSetConditional(h, go ? 1u : 0u);
@@ -417,25 +443,43 @@ static void emit_pcg(Ctx& c, const SolveCfg& cfg, const T* Kmat, const T* b, T* 
   float* r32 = (float*)c.work[W_F_R];
   float* z32 = (float*)c.work[W_F_Z];
   if (mixed) klaunch(k_r_to_f32, g_nb(n), 256, 0, c.stream, (const double*)b, r32, c.scal, YY, n);
+  // the update kernel takes the V-cycle's first smoother step; the loop's first
+  // iteration gets it here
+  FirstStep<float> first32;
+  FirstStep<T> first;
+  if (cfg.inner_pc == 0) {
+    if (mixed) first32 = mg_first_step<float>(c, z32, cfg.mg);
+    else first = mg_first_step<T>(c, z, cfg.mg);
+    if (first32.dinv) launch_first_step<float>(c, r32, first32);
+    if (first.dinv) launch_first_step<T>(c, r, first);
+  }
+  // r . z from the V-cycle's last kernel (an atomic per block, so not in the deterministic mode)
+  RzOut rzo;
+  rzo.r = (const double*)r;
+  rzo.yy = mixed ? c.scal + YY : nullptr;
+  rzo.out = c.scal + RZN;
+  const RzOut* want_rz = f32 || L.det ? nullptr : &rzo;
   cudaGraphConditionalHandle h = new_handle(c.stream);
-  klaunch(k_in_init, 1, 1, 0, c.stream, h, ctl, c.scal, YY, IRR, c.scal, f32 ? 1 : 0, relax);
+  klaunch(k_in_init, 1, 1, 0, c.stream, h, ctl, c.scal, YY, IRR, c.scal, f32 ? 1 : 0, relax, RZN);
   DP_LAUNCH_CHECK();
   cudaGraph_t body = add_while(c.stream, h);
   const int* itp = f32 ? &ctl->in32_it : &ctl->in_it;
   capture_body(c, body, depth, f32 ? B_PCG32 : B_PCG64, [&] {
+    bool have_rz = false;
     if (cfg.inner_pc == 0) {
       if (f32) {
-        mg_apply_f(c, (const float*)r, (float*)z, cfg.mg);
+        mg_apply_f(c, (const float*)r, (float*)z, cfg.mg, first.dinv != nullptr);
       } else if (mixed) {
-        mg_apply_f(c, r32, z32, cfg.mg);
+        have_rz = mg_apply_f(c, r32, z32, cfg.mg, first32.dinv != nullptr, want_rz);
       } else {
-        mg_apply(c, (const double*)r, (double*)z, cfg.mg);
+        have_rz = mg_apply(c, (const double*)r, (double*)z, cfg.mg, first.dinv != nullptr, want_rz);
       }
     } else {
       if (c.mg_prec == 1) klaunch(k_bj_mixed<float, T>, g_nb(L.nnod), 256, 0, c.stream, c.mg[0].dinv32, r, z, L.nnod);
       else klaunch(k_bj_mixed<double, T>, g_nb(L.nnod), 256, 0, c.stream, c.mg[0].dinv64, r, z, L.nnod);
     }
-    if (mixed)
+    if (have_rz) {
+    } else if (mixed)
       klaunch(k_rz_f32, red_grid(n), kRedThreads, 0, c.stream, (const float*)z32, (const double*)r, c.scal, YY, RZN, n / 2,
               c.partial, c.counter);
     else if (f32) launch_dot_f(c, (const float*)r, (const float*)z, n, RZN);
@@ -454,8 +498,12 @@ static void emit_pcg(Ctx& c, const SolveCfg& cfg, const T* Kmat, const T* b, T* 
       if (f32) launch_dot_f(c, (const float*)p, (const float*)Ap, n, PAP);
       else launch_dot(c, (const double*)p, (const double*)Ap, n, PAP);
     }
-    klaunch(k_pcg_upd_check<T>, red_grid(n), kRedThreads, 0, c.stream, x, r, p, Ap, n / 2, c.scal, RZ, RZN, PAP, IRR,
-            c.partial, c.counter, h, ctl, f32 ? 1 : 0, mixed ? r32 : (float*)nullptr, YY);
+    if (mixed)
+      klaunch(k_pcg_upd_check<T, float>, red_grid(n), kRedThreads, 0, c.stream, x, r, p, Ap, n / 2, c.scal, RZ, RZN,
+              PAP, IRR, c.partial, c.counter, h, ctl, 0, r32, YY, first32);
+    else
+      klaunch(k_pcg_upd_check<T, T>, red_grid(n), kRedThreads, 0, c.stream, x, r, p, Ap, n / 2, c.scal, RZ, RZN, PAP,
+              IRR, c.partial, c.counter, h, ctl, f32 ? 1 : 0, (float*)nullptr, YY, first);
     DP_LAUNCH_CHECK();
   });
 }
@@ -679,9 +727,9 @@ void profile_inner_vector_kernels(Ctx& c) {
           (int)G_RZN, n / 2, c.partial, c.counter);
   klaunch(k_pcg_dir_f32z, g_nb(n / 2), 256, 0, c.stream, p, (const float*)z32, Ap, n / 2, c.scal, (int)G_IRR,
           (int)G_RZN, (int)G_RZ, (int)S_TMP, (const int*)&ctl->in_it);
-  klaunch(k_pcg_upd_check<double>, red_grid(n), kRedThreads, 0, c.stream, x, r, (const double*)p,
+  klaunch(k_pcg_upd_check<double, float>, red_grid(n), kRedThreads, 0, c.stream, x, r, (const double*)p,
           (const double*)Ap, n / 2, c.scal, (int)G_RZ, (int)G_RZN, (int)G_PAP, (int)G_IRR, c.partial, c.counter,
-          (cudaGraphConditionalHandle)0, (DevCtl*)nullptr, 0, r32, (int)G_IRR);
+          (cudaGraphConditionalHandle)0, (DevCtl*)nullptr, 0, r32, (int)G_IRR, FirstStep<float>());
   DP_LAUNCH_CHECK();
 }
 

@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(halo_max_threads<T>()) k_halo_down(const T* S,
 template <typename T>
 __global__ void __launch_bounds__(halo_max_threads<T>()) k_halo_up(const T* S, const T* b, const T* xc, const T* xp,
                                                                    T* x, const T* dinv, const double* coef, int ncr,
-                                                                   int nct, int ncrc, int Ac, int Bc, int pin) {
+                                                                   int nct, int ncrc, int Ac, int Bc, int pin,
+                                                                   RzOut rz) {
   grid_dep_launch();
   typedef typename V2<T>::T X2;
   __shared__ X2 sm[2][kHaloCols * kHaloMaxA];
@@ -255,14 +256,22 @@ __global__ void __launch_bounds__(halo_max_threads<T>()) k_halo_up(const T* S, c
     if (row.store && on2) sm[0][row.own] = d;
   }
   __syncthreads();
+  double share = 0.0;
   const bool on3 = row.off == 0 || row.off == 1;
   if (__any_sync(0xffffffffu, on3)) {
     row.subtract(sm[0], rv.x, rv.y);
     di.apply(rv.x, rv.y, z0, z1);
     xv.x += e1 * d.x + e2 * z0;
     xv.y += e1 * d.y + e2 * z1;
-    if (row.store && on3) reinterpret_cast<X2*>(x)[row.node] = xv;
+    if (row.store && on3) {
+      reinterpret_cast<X2*>(x)[row.node] = xv;
+      if (rz.out) {
+        const double2 rr = reinterpret_cast<const double2*>(rz.r)[row.node];
+        share = rr.x * (double)xv.x + rr.y * (double)xv.y;
+      }
+    }
   }
+  if (rz.out) block_add(rz.yy ? sqrt(*rz.yy) * share : share, rz.out);
 }
 
 }  // namespace dp

@@ -1263,7 +1263,7 @@ static bool stencil_level(const Ctx& c, const MGLevel& L) {
 // mode 2 the first step gathers x, so x gains d_1 together with d_2.
 // Pre-smoothing (modes 0, 1) ends with r = b - A x, the true residual.
 template <typename T>
-static void chebyshev_stencil(Ctx& c, MGLevel& L, const T* b, T* x, int mode) {
+static bool chebyshev_stencil(Ctx& c, MGLevel& L, const T* b, T* x, int mode, const RzOut* rz = nullptr) {
   T* r = (T*)L.r;
   T* d = (T*)L.d;
   T* dn = (T*)L.t;
@@ -1272,16 +1272,23 @@ static void chebyshev_stencil(Ctx& c, MGLevel& L, const T* b, T* x, int mode) {
   const T* none = nullptr;
   if (mode == 0) klaunch(k_cheb_first<T>, tpb(L.g.nnod), 256, 0, c.stream, b, dinv, x, r, d, L.cheb, L.g.nnod);
   if (mode == 2) launch_stencil_step<ST_FIRST_X, T>(L.g, S, x, b, r, (T*)nullptr, d, dinv, L.cheb, c.stream);
+  bool summed = false;
   for (int k = 1; k < L.degree; ++k) {
-    if (mode == 2 && k == 1)
-      launch_stencil_step<ST_STEP_X, T>(L.g, S, d, none, r, x, dn, dinv, L.cheb + 2 * k, c.stream);
-    else
-      launch_stencil_step<ST_STEP, T>(L.g, S, d, none, r, x, dn, dinv, L.cheb + 2 * k, c.stream);
+    const double* coef = L.cheb + 2 * k;
+    if (mode == 2 && k == 1) {
+      launch_stencil_step<ST_STEP_X, T>(L.g, S, d, none, r, x, dn, dinv, coef, c.stream);
+    } else if (rz && k + 1 == L.degree) {
+      launch_stencil_step<ST_STEP_RZ, T>(L.g, S, d, none, r, x, dn, dinv, coef, c.stream, *rz);
+      summed = true;
+    } else {
+      launch_stencil_step<ST_STEP, T>(L.g, S, d, none, r, x, dn, dinv, coef, c.stream);
+    }
     std::swap(d, dn);
   }
   if (mode != 2)
     launch_stencil_step<ST_RESIDUAL, T>(L.g, S, d, none, r, (T*)nullptr, (T*)nullptr, dinv, L.cheb, c.stream);
   DP_LAUNCH_CHECK();
+  return summed;
 }
 
 // Levels whose x is put together late (see the vector steps above); not the
@@ -1348,11 +1355,13 @@ static bool halo_level(const Ctx& c, size_t l, const MGOptions& o) {
 }
 
 // first_done: the level's first pre-smoothing step was fused into the restriction.
+// rz (fine level): see mg.cuh; returns whether the last kernel took it.
 template <typename T>
-static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool first_done) {
+static bool vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool first_done,
+                   const RzOut* rz = nullptr) {
   if (l == tail_start(c, o)) {
     launch_vcycle_tail<T>(c, l, b, x, first_done, o);
-    return;
+    return false;
   }
   MGLevel& L = c.mg[l];
   const bool dense_coarsest = c.coarse_n > 0;
@@ -1370,7 +1379,7 @@ static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool 
         chebyshev<T>(c, L, b, x, 2);
       }
     }
-    return;
+    return false;
   }
   MGLevel& C = c.mg[l + 1];
   T* r = (T*)L.r;
@@ -1413,19 +1422,46 @@ static void vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool 
   if (halo) {
     klaunch(k_halo_up<T>, (unsigned)L.g.nct, halo_threads, 0, c.stream, (const T*)L.S, b, (const T*)xc, (const T*)L.d,
             x, level_dinv<T>(L), (const double*)L.cheb, L.g.ncr, L.g.nct, C.g.ncr, (int)C.g.A(), (int)C.g.B(),
-            L.g.pin);
+            L.g.pin, rz ? *rz : RzOut());
     DP_LAUNCH_CHECK();
-    return;
+    return rz != nullptr;
   }
   klaunch(k_prolong_add<T>, tpb(L.g.nnod), 256, 0, c.stream, (const T*)xc, x,
           late_x(c, L) ? (const T*)L.d : (const T*)nullptr,
           late_x(c, L) && L.degree == 3 ? (const T*)L.t : (const T*)nullptr, b, st ? (T*)nullptr : r, (int)L.g.A(),
           (int)L.g.B(), C.g.ncr, (int)C.g.A(), (int)C.g.B(), L.g.pin);
   DP_LAUNCH_CHECK();
-  chebyshev<T>(c, L, b, x, 2);
+  if (!st) rz = nullptr;
+  return st ? chebyshev_stencil<T>(c, L, b, x, 2, rz) : (chebyshev<T>(c, L, b, x, 2), false);
 }
 
-void mg_apply(Ctx& c, const double* b, double* x, const MGOptions& o) { vcycle<double>(c, 0, b, x, o, false); }
-void mg_apply_f(Ctx& c, const float* b, float* x, const MGOptions& o) { vcycle<float>(c, 0, b, x, o, false); }
+bool mg_apply(Ctx& c, const double* b, double* x, const MGOptions& o, bool first_done, const RzOut* rz) {
+  return vcycle<double>(c, 0, b, x, o, first_done, rz);
+}
+bool mg_apply_f(Ctx& c, const float* b, float* x, const MGOptions& o, bool first_done, const RzOut* rz) {
+  return vcycle<float>(c, 0, b, x, o, first_done, rz);
+}
+
+template <typename T>
+FirstStep<T> mg_first_step(Ctx& c, T* x, const MGOptions& o) {
+  FirstStep<T> f;
+  if (c.mg.size() < 2 || tail_start(c, o) == 0 || !stencil_level(c, c.mg[0]) || halo_level<T>(c, 0, o)) return f;
+  MGLevel& L = c.mg[0];
+  f.dinv = level_dinv<T>(L);
+  f.r = (T*)L.r;
+  f.d = (T*)L.d;
+  f.x = x;
+  f.coef = L.cheb;
+  return f;
+}
+template FirstStep<float> mg_first_step<float>(Ctx&, float*, const MGOptions&);
+template FirstStep<double> mg_first_step<double>(Ctx&, double*, const MGOptions&);
+template <typename T>
+void launch_first_step(Ctx& c, const T* b, const FirstStep<T>& f) {
+  const int64_t nn = c.fine.nnod;
+  klaunch(k_cheb_first<T>, tpb(nn), 256, 0, c.stream, b, f.dinv, f.x, f.r, f.d, f.coef, nn);
+}
+template void launch_first_step<float>(Ctx&, const float*, const FirstStep<float>&);
+template void launch_first_step<double>(Ctx&, const double*, const FirstStep<double>&);
 
 }  // namespace dp

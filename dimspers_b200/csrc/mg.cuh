@@ -49,8 +49,36 @@ __host__ __device__ inline void element_nodes_mg(int e, int ncr, int A, int B, i
 void upload_mg_constants();
 void mg_setup(Ctx& c, int precision, const MGOptions& o);
 void mg_free(Ctx& c);
-void mg_apply(Ctx& c, const double* b, double* x, const MGOptions& o);
-void mg_apply_f(Ctx& c, const float* b, float* x, const MGOptions& o);
+// first_done: the caller has taken the fine level's first smoother step (mg_first_step).
+// rz given: the cycle's last kernel also adds r . s x to *rz->out (s = sqrt(*rz->yy), 1 without
+// yy; r in FP64) if it is of a kind that can (the passes and steps on stencils, whose few blocks
+// make few atomics; on larger levels the launch saved is below 1 % of the iteration); returns
+// whether it does.  An inner iteration takes 52.4 instead of 55.6 us at 16x128, and with the
+// first step fused as well 69.7 instead of 72.7 at 32x256.
+struct RzOut {
+  const double* r = nullptr;
+  const double* yy = nullptr;
+  double* out = nullptr;
+};
+bool mg_apply(Ctx& c, const double* b, double* x, const MGOptions& o, bool first_done = false,
+              const RzOut* rz = nullptr);
+bool mg_apply_f(Ctx& c, const float* b, float* x, const MGOptions& o, bool first_done = false,
+                const RzOut* rz = nullptr);
+// The fine level's first smoother step from x = 0 for b: r = b, d = coef[0] D^-1 b,
+// x = d, for a kernel that has b in registers anyway.  On fine levels with
+// stencils only: a launch of 2 us is 3 % of an inner iteration at 32x256, while
+// on larger levels the step is as fast in a launch of its own (64x512: 116.7
+// fused, 116.4 us apart).
+template <typename T>
+struct FirstStep {
+  const T* dinv = nullptr;   // null: the cycle takes the step itself
+  T *r = nullptr, *d = nullptr, *x = nullptr;
+  const double* coef = nullptr;
+};
+template <typename T>
+FirstStep<T> mg_first_step(Ctx& c, T* x, const MGOptions& o);
+template <typename T>
+void launch_first_step(Ctx& c, const T* b, const FirstStep<T>& f);
 
 // The small levels as one thread-block-cluster kernel (mgtail.cu): first level
 // it covers, and its launcher (V-cycle of levels l0.. with b, x of level l0).

@@ -15,6 +15,8 @@
 #include <utility>
 
 #include "kernels.cuh"
+#include "mg.cuh"
+#include "reduce.cuh"
 
 namespace dp {
 
@@ -164,6 +166,7 @@ enum StepMode {
   ST_STEP = 0,      // r -= A v; d = c1 v + c2 D^-1 r; x += d           (v = the previous d)
   ST_STEP_X = 1,    // the same with x += v first (the step after ST_FIRST_X)
   ST_RESIDUAL = 2,  // r -= A v
+  ST_STEP_RZ = 4,   // ST_STEP, then *rz.out += rz.r . s x
   ST_FIRST_X = 3,   // r = b - A v; d = (1/theta) D^-1 r                 (v = x, which gains d in the next step)
 };
 
@@ -178,6 +181,19 @@ struct NodeInv {
     z1 = b * r0 + c * r1;
   }
 };
+
+// Adds the block's sum of v to *out (every thread of the block takes part).
+__device__ __forceinline__ void block_add(double v, double* out) {
+  __shared__ double part[32];
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
+    atomicAdd(out, t);
+  }
+}
 
 // Offsets of entry sub * PER + Q of a class-C row, as selects between
 // compile-time values (a table lookup by lane would serialise the warp).  Past
@@ -197,10 +213,11 @@ __device__ __forceinline__ bool lane_entry(int sub, int& da, int& db) {
   return sub * PER + Q < NE;
 }
 
+// returns the node's share of the sum of ST_STEP_RZ, without its scale
 template <int C, int MODE, typename T>
-__device__ __forceinline__ void smooth_node(const T* __restrict__ S, const T* v, const T* b, T* r, T* x, T* d,
+__device__ __forceinline__ double smooth_node(const T* __restrict__ S, const T* v, const T* b, T* r, T* x, T* d,
                                             const T* __restrict__ dinv, const double* __restrict__ coef, int blk,
-                                            int ncr, int nct) {
+                                            int ncr, int nct, const double* rr) {
   typedef typename V2<T>::T X2;
   constexpr int NE = st_entries(C), LN = st_lanes(C), PER = (NE + LN - 1) / LN, NPW = 32 / LN;
   constexpr int PA = C & 1, PB = C >> 1;
@@ -236,7 +253,8 @@ __device__ __forceinline__ void smooth_node(const T* __restrict__ S, const T* v,
   const NodeInv<T> di(dinv, n);
   T c1 = (T)0, c2 = (T)0;
   if (MODE == ST_FIRST_X) c2 = (T)ld_early(coef);
-  if (MODE == ST_STEP || MODE == ST_STEP_X) { c1 = (T)ld_early(coef); c2 = (T)ld_early(coef + 1); }
+  constexpr bool kStep = MODE == ST_STEP || MODE == ST_STEP_X || MODE == ST_STEP_RZ;
+  if (kStep) { c1 = (T)ld_early(coef); c2 = (T)ld_early(coef + 1); }
   grid_dep_sync();
   const X2* v2 = reinterpret_cast<const X2*>(v);
   X2 vn[PER];
@@ -246,7 +264,9 @@ __device__ __forceinline__ void smooth_node(const T* __restrict__ S, const T* v,
   const X2 rv = reinterpret_cast<const X2*>(MODE == ST_FIRST_X ? b : r)[n];
   X2 xv;
   xv.x = xv.y = (T)0;
-  if (MODE == ST_STEP || MODE == ST_STEP_X) xv = reinterpret_cast<const X2*>(x)[n];
+  double2 rrv = make_double2(0.0, 0.0);
+  if (MODE == ST_STEP_RZ) rrv = reinterpret_cast<const double2*>(rr)[n];
+  if (kStep) xv = reinterpret_cast<const X2*>(x)[n];
   T s0 = (T)0, s1 = (T)0;
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
@@ -260,12 +280,12 @@ __device__ __forceinline__ void smooth_node(const T* __restrict__ S, const T* v,
     s0 += __shfl_xor_sync(0xffffffffu, s0, o);
     s1 += __shfl_xor_sync(0xffffffffu, s1, o);
   }
-  if (!live || sub != 0) return;
+  if (!live || sub != 0) return 0.0;
   X2 rn;
   rn.x = rv.x - s0;
   rn.y = rv.y - s1;
   reinterpret_cast<X2*>(r)[n] = rn;
-  if (MODE == ST_RESIDUAL) return;
+  if (MODE == ST_RESIDUAL) return 0.0;
   T z0, z1;
   di.apply(rn.x, rn.y, z0, z1);
   X2 dn;
@@ -283,7 +303,9 @@ __device__ __forceinline__ void smooth_node(const T* __restrict__ S, const T* v,
     xv.y += dn.y;
     reinterpret_cast<X2*>(x)[n] = xv;
   }
+  if (MODE == ST_STEP_RZ) return rrv.x * (double)xv.x + rrv.y * (double)xv.y;   // nobody reads d again
   reinterpret_cast<X2*>(d)[n] = dn;
+  return 0.0;
 }
 
 // CTAs [0, nb0) take class 0, the next nb1 class 1, and so on.
@@ -292,28 +314,30 @@ template <int MODE, typename T>
 __global__ void __launch_bounds__(kStThreads) k_stencil_step(const T* __restrict__ S, const T* v, const T* b, T* r,
                                                              T* x, T* d, const T* __restrict__ dinv,
                                                              const double* __restrict__ coef, int ncr, int nct,
-                                                             int nb0, int nb1, int nb2) {
+                                                             int nb0, int nb1, int nb2, RzOut rz) {
   grid_dep_launch();
   int blk = blockIdx.x;
+  double s;
   if (blk < nb0) {
-    smooth_node<0, MODE, T>(S, v, b, r, x, d, dinv, coef, blk, ncr, nct);
+    s = smooth_node<0, MODE, T>(S, v, b, r, x, d, dinv, coef, blk, ncr, nct, rz.r);
   } else if ((blk -= nb0) < nb1) {
-    smooth_node<1, MODE, T>(S, v, b, r, x, d, dinv, coef, blk, ncr, nct);
+    s = smooth_node<1, MODE, T>(S, v, b, r, x, d, dinv, coef, blk, ncr, nct, rz.r);
   } else if ((blk -= nb1) < nb2) {
-    smooth_node<2, MODE, T>(S, v, b, r, x, d, dinv, coef, blk, ncr, nct);
+    s = smooth_node<2, MODE, T>(S, v, b, r, x, d, dinv, coef, blk, ncr, nct, rz.r);
   } else {
-    smooth_node<3, MODE, T>(S, v, b, r, x, d, dinv, coef, blk - nb2, ncr, nct);
+    s = smooth_node<3, MODE, T>(S, v, b, r, x, d, dinv, coef, blk - nb2, ncr, nct, rz.r);
   }
+  if (MODE == ST_STEP_RZ) block_add(rz.yy ? sqrt(*rz.yy) * s : s, rz.out);
 }
 
 template <int MODE, typename T>
 static void launch_stencil_step(const Level& g, const T* S, const T* v, const T* b, T* r, T* x, T* d, const T* dinv,
-                                const double* coef, cudaStream_t s) {
+                                const double* coef, cudaStream_t s, const RzOut& rz = RzOut()) {
   int nb[4];
   for (int c = 0; c < 4; ++c)
     nb[c] = (int)div_up((int64_t)st_nodes(c, g.ncr, g.nct) * st_lanes(c), kStThreads);
   klaunch(k_stencil_step<MODE, T>, nb[0] + nb[1] + nb[2] + nb[3], kStThreads, 0, s, S, v, b, r, x, d, dinv, coef,
-          g.ncr, g.nct, nb[0], nb[1], nb[2]);
+          g.ncr, g.nct, nb[0], nb[1], nb[2], rz);
 }
 
 template <typename T>

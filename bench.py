@@ -504,18 +504,18 @@ def run_ours(args, rank, world, local):
     w.ctx.assemble(1)
     ms_cold = ctx.profile_kernel(0, reps=20, flush_l2=True)
     ms_warm = ctx.profile_kernel(0, reps=50)
-    alg_bytes = nel * 78 * 4 + nnod * 2 * 4 * 2
+    alg_bytes = nel * 56 * 4 + nnod * 2 * 4 * 2   # 55 reduced entries in 14 float4
     pk, pk_kind = peaks()
     achieved = alg_bytes / (ms_cold * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "k_apply_K<float,float> (fine level)", "achieved": achieved,
+    roofline = {"bound": "hbm", "kernel": "k_apply_R<float> (fine level)", "achieved": achieved,
                 "peak": pk, "peak_kind": pk_kind, "unit": "GB/s", "frac": achieved / pk,
                 "traffic": traffic_from_profiles(args.nr, args.nt), "algorithmic_bytes": alg_bytes,
                 "ms_per_launch": ms_cold, "ms_per_launch_warm_l2": ms_warm,
                 "achieved_warm_l2": alg_bytes / (ms_warm * 1e-3) / 1e9}
     w.ctx.assemble(0)
     ms64_apply = ctx.profile_kernel(1, reps=20, flush_l2=True)
-    alg64 = nel * 78 * 8 + nnod * 2 * 8 * 2
-    roofline["fp64_apply"] = {"kernel": "k_apply_K<double,double> (fine level)", "ms_per_launch": ms64_apply,
+    alg64 = nel * 56 * 8 + nnod * 2 * 8 * 2
+    roofline["fp64_apply"] = {"kernel": "k_apply_R<double> (fine level)", "ms_per_launch": ms64_apply,
                               "achieved": alg64 / (ms64_apply * 1e-3) / 1e9,
                               "frac": alg64 / (ms64_apply * 1e-3) / 1e9 / pk}
 
@@ -534,7 +534,7 @@ def run_ours(args, rank, world, local):
                    "fast_arm": fast, "plain_arm": PLAIN,
                    "parallelism": f"replicas x{world}", "e2e_steps": e2e_steps,
                    "l2": "inputs larger than L2: every step re-assembles and streams the element blocks "
-                         f"({nel * 78 * 4 / 1e9:.2f} GB FP32 + {nel * 78 * 8 / 1e9:.2f} GB FP64; L2 is 126 MB)"},
+                         f"({nel * 56 * 4 / 1e9:.2f} GB FP32 + {nel * 56 * 8 / 1e9:.2f} GB FP64; L2 is 126 MB)"},
         "outer_iterations": last["iterations"], "inner_iterations": last["inner_iterations"],
         "iterations": {"outer": spread(r["iterations"] for r in allreps),
                        "inner": spread(r["inner_iterations"] for r in allreps),
@@ -553,7 +553,7 @@ def run_ours(args, rank, world, local):
     }
     try:   # the whole solve against the HBM roofline, from a per-kernel byte model
         sb = solve_bytes_model(args.nr, args.nt, last["iterations"], last["inner_iterations"], args.pressure,
-                               FAST["cheb_degree"])
+                               FAST["cheb_degree"], reduced=True)
         sgbs = sb / (ms_per_step * 1e-3) / 1e9
         line["solve_model"] = {"bytes_per_solve": sb, "achieved": sgbs, "unit": "GB/s", "frac": sgbs / pk,
                                "note": "algorithmic bytes of every kernel of one fast solve (bench.solve_bytes_model)"}
@@ -575,17 +575,21 @@ def run_ours(args, rank, world, local):
         print(json.dumps(line), flush=True)
 
 
-def solve_bytes_model(nr, nt, outer, inner, pressure="discontinuous", cheb_degree=3, coarse_max=1536):
+def solve_bytes_model(nr, nt, outer, inner, pressure="discontinuous", cheb_degree=3, coarse_max=1536, reduced=False):
     """Algorithmic HBM bytes of one fast-path solve (FP64 Krylov, FP32 multigrid
     V-cycle per inner iteration): every kernel's reads and writes once, from
-    the measured iteration counts.  Per-kernel figures (the kernel table):
-    FP32 apply 312 B/element + 16 B/node; FP64 apply 624 B/element + 48 B/node;
-    Chebyshev vector steps 52 B/node, first steps 44 B/node (on the coarse
-    levels the first is fused into the restriction); restriction 8 B/fine node
-    + 44 B/coarse node; prolongation 32 B/fine node; dense coarsest n^2 x 8 B; inner PCG
-    vector passes 108 B/DOF; outer: G and G^T 288 B/element + vectors, the
-    fused Schur update (5 N_P + 2 N_U) x 8 B and its dots; assembly and
-    set-up excluded."""
+    the measured iteration counts; assembly and set-up excluded.
+
+    reduced=False: packed 78-entry element matrices on every level and separate
+    vector passes (312 / 624 B/element FP32 / FP64 + 16 / 48 B/node per apply;
+    328 B/node of smoother, restriction and prolongation passes; 108 B/DOF of
+    Krylov vector passes), the form that earlier figures are stated in.
+    reduced=True, what the default path moves: 55-entry matrices on the fine
+    level (224 / 448 B/element), node stencils up to 40,000 nodes (184 B/node),
+    272 B/node of smoother passes, 92 B/DOF of Krylov passes.
+    Both: dense coarsest n^2 x 8 B; outer: G and G^T 288 B/element + vectors,
+    the fused Schur update (5 N_P + 2 N_U) x 8 B and its dots."""
+    fine32, fine64, krylov = (224.0, 448.0, 92.0) if reduced else (312.0, 624.0, 108.0)
     levels = []
     r_, t_ = nr, nt
     while True:
@@ -600,14 +604,18 @@ def solve_bytes_model(nr, nt, outer, inner, pressure="discontinuous", cheb_degre
             vcycle += (2 * nnod) ** 2 * 8.0
             break
         cn = levels[i + 1][1]
-        vcycle += 2 * cheb_degree * (312.0 * nel + 16.0 * nnod)          # smoothing and residual applies
-        vcycle += (44.0 if i == 0 else 0.0) * nnod + 44.0 * nnod         # first steps (pre on the top level, post)
-        vcycle += 2 * (cheb_degree - 1) * 52.0 * nnod                    # Chebyshev vector steps
-        vcycle += 8.0 * nnod + 44.0 * cn + 32.0 * nnod                   # restriction, prolongation
+        matrix = (fine32 if i == 0 else 312.0) * nel + 16.0 * nnod
+        if reduced and nnod <= 40000:
+            matrix = 184.0 * nnod + 16.0 * nnod
+        first, first_x, step, last, prolong, coarse = (36, 28, 36, 52, 48, 36) if reduced else (44, 44, 52, 52, 32, 44)
+        vcycle += 2 * cheb_degree * matrix                                     # smoothing and residual applies
+        vcycle += (first if i == 0 else 0.0) * nnod + first_x * nnod           # first steps (pre on the top level, post)
+        vcycle += (2 * cheb_degree - 3) * step * nnod + last * nnod            # the other steps; the last one writes x
+        vcycle += 8.0 * nnod + coarse * cn + prolong * nnod                    # restriction, prolongation
     nel, nnod = levels[0]
     n_u = 2 * nnod
     n_p = 3 * nel if pressure == "discontinuous" else (nr + 1) * nt
-    per_inner = vcycle + 624.0 * nel + 48.0 * nnod + 108.0 * n_u
+    per_inner = vcycle + fine64 * nel + 48.0 * nnod + krylov * n_u
     per_outer = 2 * (288.0 * nel + 16.0 * nnod + 8.0 * n_p) + (5 * n_p + 2 * n_u) * 8.0 + 4 * 16.0 * n_p
     return inner * per_inner + outer * per_outer
 

@@ -202,6 +202,9 @@ struct CudaError {
 // what no kernel of the solve writes -- element blocks, D^-1, coefficients --
 // and then wait), so a launch with or without the attribute computes the same
 // thing; without the attribute the wait returns at once.
+// Fetching before the wait, and waiting after the launch of the successor, took
+// an inner iteration from 114 to 103 us at 32x256, 340 to 304 at 128x1024 and
+// 3529 to 3314 at 512x4096 when it came in.
 // A kernel completes only after its own wait returned, so waiting for the
 // direct predecessor covers all earlier ones.  Pointers to data that a
 // predecessor writes carry no __restrict__ here: the compiler may move a load

@@ -19,14 +19,13 @@ device):
   apply64  one fine-level FP64 A-apply
   vcycle   one FP32 multigrid V-cycle from the fine level (after a solve built
            the hierarchy): Chebyshev steps, restriction, prolongation, dense
-           coarsest, the coarse-level applies
+           coarsest, the coarse-level applies, stencil steps, whole passes
   solve32  assembly (FP32 blocks) and one host-driven fast solve of 2 outer
            iterations: Galerkin levels, Gauss-Jordan coarse inverse, the
            FP64 Krylov kernels, G and G^T, the compensated Schur kernels
   solve64  the same in FP64 with the lumped Schur preconditioner
   det      solve32 in deterministic mode: the element-result kernels of the
-           applies, right-hand side and diagonal blocks, the per-node gathers,
-           the sequential dense coarse assembly
+           applies and the right-hand side, the per-node gathers
   inner    the graph solve's inner-iteration vector kernels (launched outside
            the graph: ncu cannot look inside conditional graph nodes)
   post     stress post-processor, viscosity update, FSE, DEM tensor lookup,

@@ -86,11 +86,25 @@ static bool overlap(const double* a, int64_t na, const double* b, int64_t nb) {
   return a && b && (uintptr_t)a < (uintptr_t)(b + nb) && (uintptr_t)b < (uintptr_t)(a + na);
 }
 
-// The caller's array where the device can read it: itself (device memory), or a
-// copy in `stage` (host memory).
+// Whether a kernel may work on the caller's array where it lies: memory of this GPU
+// (or managed), aligned as its type.  What only a copy can reach (another GPU's
+// memory, pinned host memory, a buffer at an odd address) takes the staging copies of
+// host arrays; a host address handed over as device memory, which a copy refuses and
+// a kernel would fault on, is refused here.  The query takes 50 ns.
+static bool in_place(int device, const void* p, int mem, size_t align = sizeof(double)) {
+  if (mem != DP_MEM_DEVICE) return false;
+  cudaPointerAttributes a;
+  DP_CUDA(cudaPointerGetAttributes(&a, p));
+  if (a.type == cudaMemoryTypeUnregistered) throw BadArg("an array passed as device memory is host memory");
+  return ((uintptr_t)p & (align - 1)) == 0 &&
+         (a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeDevice && a.device == device));
+}
+
+// The caller's array where the device can read it: itself (in_place), or a copy in
+// `stage`.
 static const double* staged(Ctx& c, const double* src, double* stage, int64_t n, int mem) {
-  if (mem == DP_MEM_DEVICE) return src;
-  DP_CUDA(cudaMemcpyAsync(stage, src, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream));
+  if (in_place(c.device, src, mem)) return src;
+  DP_CUDA(cudaMemcpyAsync(stage, src, sizeof(double) * n, kind_in(mem), c.stream));
   return stage;
 }
 
@@ -275,9 +289,9 @@ static void deliver_solution(Ctx& c, double* U, double* P, double* Ucart, int me
   double* stage = (double*)c.work[W_UC];
   // device arrays are written in place, host arrays through the staging vector
   auto put = [&](const double* lat, double* out) {
-    launch_scatter_lat2ref(c, lat, mem == DP_MEM_DEVICE ? out : stage, 2);
-    if (mem != DP_MEM_DEVICE)
-      DP_CUDA(cudaMemcpyAsync(out, stage, sizeof(double) * 2 * nn, cudaMemcpyDeviceToHost, c.stream));
+    const bool dev = in_place(c.device, out, mem);
+    launch_scatter_lat2ref(c, lat, dev ? out : stage, 2);
+    if (!dev) DP_CUDA(cudaMemcpyAsync(out, stage, sizeof(double) * 2 * nn, kind_out(mem), c.stream));
   };
   if (U) put(dU, U);
   if (P) DP_CUDA(cudaMemcpyAsync(P, dP, sizeof(double) * np, kind_out(mem), c.stream));
@@ -757,10 +771,10 @@ static int apply_common(dp_ctx* h, const double* in, double* out, int32_t mem, i
     double* b = (double*)c.work[W_Z];
     double* stage = (double*)c.work[W_UC];
     double* pbuf = (double*)c.work[W_P];
-    const bool dev = mem == DP_MEM_DEVICE;   // the caller's arrays are read and written in place
+    const bool dev = in_place(c.device, out, mem);
     auto deliver = [&](const double* lat) {
       launch_scatter_lat2ref(c, lat, dev ? out : stage, 2);
-      if (!dev) DP_CUDA(cudaMemcpyAsync(out, stage, sizeof(double) * 2 * nn, cudaMemcpyDeviceToHost, c.stream));
+      if (!dev) DP_CUDA(cudaMemcpyAsync(out, stage, sizeof(double) * 2 * nn, kind_out(mem), c.stream));
     };
     if (which == 0) {  // K
       launch_gather_ref2lat(c, staged(c, in, stage, 2 * nn, mem), a, 2);
@@ -772,7 +786,7 @@ static int apply_common(dp_ctx* h, const double* in, double* out, int32_t mem, i
     } else {  // G^T
       launch_gather_ref2lat(c, staged(c, in, stage, 2 * nn, mem), a, 2);
       launch_apply_GT(c, a, dev ? out : pbuf);
-      if (!dev) DP_CUDA(cudaMemcpyAsync(out, pbuf, sizeof(double) * np, cudaMemcpyDeviceToHost, c.stream));
+      if (!dev) DP_CUDA(cudaMemcpyAsync(out, pbuf, sizeof(double) * np, kind_out(mem), c.stream));
     }
     DP_CUDA(cudaStreamSynchronize(c.stream));
     return (int)DP_OK;

@@ -709,8 +709,8 @@ static void cnn_forward(Cnn& n, cudaStream_t s, const float* x, float* y, int nb
   n.act[0] = const_cast<float*>(x);
   for (int l = 0; l < n.L; ++l) {
     const bool last = l == n.L - 1;
-    // straight into the caller's y where its 16-byte stores allow it
-    float* out = last && y && ((uintptr_t)y & 15) == 0 ? y : n.act[l + 1];
+    // straight into the caller's y where the kernel's 16-byte stores can reach it
+    float* out = last && y && in_place(n.device, y, DP_MEM_DEVICE, 16) ? y : n.act[l + 1];
     if (tc_ok(n)) {
       conv_tc(n, s, n.act[l], n.wk + n.wkoff[2 * l], n.param + n.boff[l], nullptr, out, n.cin_of(l), n.cout_of(l),
               n.dil[l], 1, last ? 0 : 1, nb, last ? affine : 0, scale, shift);
@@ -983,13 +983,12 @@ static void launch_cnn_inputs(Ctx& c, float* x, int nrg, int ntg, const CnnNorm&
 // scale * grid field -> pressure DOFs in P (host or device)
 static void launch_guess_prolong(Ctx& c, const float* pg, int nrg, int ntg, double scale, double* P, int mem) {
   if (nrg != c.fine.ncr / 2 + 1 || ntg != c.fine.nct / 2) throw BadArg("grid must be (ncr/2+1) x (nct/2)");
-  double* dP = mem == DP_MEM_DEVICE ? P : (double*)c.work[W_P];
+  double* dP = in_place(c.device, P, mem) ? P : (double*)c.work[W_P];
   ++g_klaunch;
   k_guess_prolong<<<(int)div_up(c.fine.nel, 256), 256, 0, c.stream>>>(pg, nrg, ntg, scale, c.fine.ncr, c.fine.nct,
                                                                       c.mesh.pressure, dP, (int)c.fine.nel);
   DP_LAUNCH_CHECK();
-  if (mem != DP_MEM_DEVICE)
-    DP_CUDA(cudaMemcpyAsync(P, dP, sizeof(double) * c.mesh.npres, cudaMemcpyDeviceToHost, c.stream));
+  if (dP != P) DP_CUDA(cudaMemcpyAsync(P, dP, sizeof(double) * c.mesh.npres, kind_out(mem), c.stream));
 }
 
 int dp_cnn_inputs(dp_ctx* h, float* x, int32_t nrg, int32_t ntg) {

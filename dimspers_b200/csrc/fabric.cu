@@ -211,8 +211,9 @@ extern "C" int dp_fse(dp_ctx* h, const double* F, double* const* fse, int64_t ld
       if (!fse[f]) throw BadArg("null output field");
     const int64_t nel = c.fine.nel, n = 6 * nel;
     if (ld_out < nel) throw BadArg("leading dimension below nel");
-    bool dev = mem == DP_MEM_DEVICE;
-    for (int f = 0; f < 6; ++f) dev = dev && !overlap(fse[f], 5 * ld_out + nel, F, 4 * n);
+    bool dev = in_place(c.device, F, mem);
+    for (int f = 0; f < 6; ++f)
+      dev = dev && in_place(c.device, fse[f], mem) && !overlap(fse[f], 5 * ld_out + nel, F, 4 * n);
     c.fabric_dem[0] = 0;  // the staged inputs of the tensor lookup are overwritten
     Fields6 out;
     const double* dF = F;
@@ -263,7 +264,9 @@ extern "C" int dp_anisotropic_tensor(dp_ctx* h, const dp_dem* dem, const double*
     Fields6 out;
     for (int f = 0; f < 6; ++f) out.f[f] = C6_out[f];
     out.ld = ld_out;
-    bool dev = mem == DP_MEM_DEVICE;
+    bool dev = true;
+    for (const double* a : {vx1, vy1, r1, r2}) dev = dev && in_place(c.device, a, mem);
+    for (int f = 0; f < 6; ++f) dev = dev && in_place(c.device, C6_out[f], mem);
     for (int f = 0; f < 6; ++f)
       for (const double* a : {vx1, vy1, r1, r2}) dev = dev && !overlap(C6_out[f], 6 * ld_out + nel, a, 5 * ld_in + nel);
     if (!dev) {

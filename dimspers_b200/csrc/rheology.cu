@@ -198,9 +198,14 @@ extern "C" int dp_viscosity_arrhenius(dp_ctx* h, const dp_arrhenius* law, const 
       DP_CUDA(cudaDeviceSynchronize());  // the copies are on the default stream; ours does not wait on it
       if (c.device >= 0 && c.device < 64) uploaded[c.device] = true;
     }
-    bool dev = mem == DP_MEM_DEVICE && !overlap(eta_ip, 7 * nel, T_node, nn) &&
-               !overlap(eta_ip, 7 * nel, P_vertex, nv) && !overlap(eta_ip, 7 * nel, r_node, nn);
-    for (const double* a : {epsII, tauII, cohesion}) dev = dev && !overlap(eta_ip, 7 * nel, a, 7 * nel);
+    bool dev = in_place(c.device, eta_ip, mem);
+    auto readable = [&](const double* a, int64_t n) {
+      dev = dev && in_place(c.device, a, mem) && !overlap(eta_ip, 7 * nel, a, n);
+    };
+    readable(T_node, nn);
+    readable(P_vertex, nv);
+    readable(r_node, nn);
+    for (const double* a : {epsII, tauII, cohesion}) readable(a, 7 * nel);
     const double *T = T_node, *P = P_vertex, *r = r_node, *e2 = epsII, *t2 = tauII, *co = cohesion;
     double* et = eta_ip;
     if (!dev) {

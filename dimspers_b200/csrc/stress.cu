@@ -203,10 +203,11 @@ extern "C" int dp_stress(dp_ctx* h, const double* Ucart, const double* eta_ip, i
         if (!C6[f]) throw BadArg("null tensor field");
     c.stress_called = true;
     c.stress_tensor = C6 != nullptr;
-    bool in_place = mem == DP_MEM_DEVICE && !overlap(out, 56 * nel, Ucart, 2 * nn) &&
-                    !overlap(out, 56 * nel, eta_ip, 6 * ld_eta + nel);
-    for (int f = 0; C6 && f < 6; ++f) in_place = in_place && !overlap(out, 56 * nel, C6[f], 6 * ld_C + nel);
-    if (in_place) {
+    bool dev = in_place(c.device, out, mem) && in_place(c.device, Ucart, mem) && in_place(c.device, eta_ip, mem) &&
+               !overlap(out, 56 * nel, Ucart, 2 * nn) && !overlap(out, 56 * nel, eta_ip, 6 * ld_eta + nel);
+    for (int f = 0; C6 && f < 6; ++f)
+      dev = dev && in_place(c.device, C6[f], mem) && !overlap(out, 56 * nel, C6[f], 6 * ld_C + nel);
+    if (dev) {
       StressArgs a = stress_args(c, C6 != nullptr);
       a.U = Ucart; a.eta = eta_ip; a.out = out;
       a.ld_eta = ld_eta; a.ld_C = ld_C;

@@ -408,13 +408,14 @@ extern "C" int dp_thermal_step(dp_ctx* h, const dp_thermal_opts* o, const double
     const int heated = o->heated ? 1 : 0;
     const int amax = 2 * L.ncr;
     double* b = th_vec(c, TV_B);
-    double* Tdev = mem == DP_MEM_DEVICE ? T : th_vec(c, TV_T);
+    double* Tdev = in_place(c.device, T, mem) ? T : th_vec(c, TV_T);
     static_assert(TV_B == TV_DIAG + 1, "diag and b are zeroed together");
     DP_CUDA(cudaMemsetAsync(th_vec(c, TV_DIAG), 0, sizeof(double) * 2 * nn, c.stream));
     ThAsmArgs a;
     a.theta_lat = c.theta_lat; a.r_lat = c.r_lat;
     a.rho = staged(c, rho_node, th_vec(c, TV_RHO), nn, mem);
-    a.Told = staged(c, T, Tdev, nn, mem);
+    a.Told = Tdev;
+    if (Tdev != T) DP_CUDA(cudaMemcpyAsync(Tdev, T, sizeof(double) * nn, kind_in(mem), c.stream));
     a.Ae = c.th_buf; a.diag = th_vec(c, TV_DIAG); a.b = b; a.K = o->K; a.Cp = o->Cp; a.dt = o->dt; a.Ttop = o->Ttop; a.Tbot = o->Tbot;
     a.nel = (int)nel; a.ncr = L.ncr; a.nct = L.nct; a.A = (int)L.A(); a.B = (int)L.B(); a.heated = heated;
     ++g_klaunch;
@@ -457,8 +458,7 @@ extern "C" int dp_thermal_step(dp_ctx* h, const dp_thermal_opts* o, const double
     k_th_finish<<<(int)div_up(nn, 256), 256, 0, c.stream>>>(th_vec(c, TV_X), Tdev, (int)nn, (int)L.A(), L.ncr, L.nct,
                                                           heated, o->Ttop, o->Tbot);
     DP_LAUNCH_CHECK();
-    if (mem != DP_MEM_DEVICE)
-      DP_CUDA(cudaMemcpyAsync(T, Tdev, sizeof(double) * nn, cudaMemcpyDeviceToHost, c.stream));
+    if (Tdev != T) DP_CUDA(cudaMemcpyAsync(T, Tdev, sizeof(double) * nn, kind_out(mem), c.stream));
     DP_CUDA(cudaMemcpyAsync(c.h_scal, c.scal, sizeof(double) * 64, cudaMemcpyDeviceToHost, c.stream));
     DP_CUDA(cudaStreamSynchronize(c.stream));
     const double it = c.h_scal[TH_IT];

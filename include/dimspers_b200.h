@@ -42,6 +42,9 @@ typedef enum { DP_PRESSURE_CONTINUOUS = 0, DP_PRESSURE_DISCONTINUOUS = 1 } dp_pr
  * residual, updates and dot products stay FP64.  FP32_IR: classic iterative
  * refinement, an FP32 PCG inside an FP64 residual / correction loop. */
 typedef enum { DP_PREC_FP64 = 0, DP_PREC_FP32_REFINED = 1, DP_PREC_FP32_IR = 2 } dp_precision;
+/* Where a call's arrays lie.  Device arrays of the context's GPU are read and
+ * written in place; what only a copy can reach (another GPU's memory, an address
+ * that is no multiple of 8) is staged; host memory is refused. */
 typedef enum { DP_MEM_HOST = 0, DP_MEM_DEVICE = 1 } dp_memory;
 typedef enum { DP_INNER_MG = 0, DP_INNER_JACOBI = 1 } dp_inner_pc;
 

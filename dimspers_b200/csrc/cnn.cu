@@ -853,9 +853,11 @@ int dp_cnn_create(int32_t nrg, int32_t ntg, int32_t channels, int32_t layers, co
     DP_CUDA(cudaMalloc(&n.grad, sizeof(float) * off));
     DP_CUDA(cudaMalloc(&n.adam_m, sizeof(float) * off));
     DP_CUDA(cudaMalloc(&n.adam_v, sizeof(float) * off));
-    DP_CUDA(cudaMemset(n.param, 0, sizeof(float) * off));
-    DP_CUDA(cudaMemset(n.adam_m, 0, sizeof(float) * off));
-    DP_CUDA(cudaMemset(n.adam_v, 0, sizeof(float) * off));
+    // zeroed on the network's own stream, which dp_cnn_set_params writes them on and
+    // which does not wait for the default stream
+    DP_CUDA(cudaMemsetAsync(n.param, 0, sizeof(float) * off, n.stream));
+    DP_CUDA(cudaMemsetAsync(n.adam_m, 0, sizeof(float) * off, n.stream));
+    DP_CUDA(cudaMemsetAsync(n.adam_v, 0, sizeof(float) * off, n.stream));
     const int64_t plane = (int64_t)nrg * ntg;
     n.act.assign(layers + 1, nullptr);
     for (int l = 0; l < layers; ++l) DP_CUDA(cudaMalloc(&n.act[l + 1], sizeof(float) * max_batch * n.cout_of(l) * plane));
@@ -868,12 +870,13 @@ int dp_cnn_create(int32_t nrg, int32_t ntg, int32_t channels, int32_t layers, co
       wtot += wk_elems(n.cin_of(k / 2), n.cout_of(k / 2), k & 1);   // a multiple of 8 elements: 16-byte aligned
     }
     DP_CUDA(cudaMalloc(&n.wk, sizeof(__nv_bfloat16) * wtot));
-    DP_CUDA(cudaMemset(n.wk, 0, sizeof(__nv_bfloat16) * wtot));     // the operands of zero weights
+    DP_CUDA(cudaMemsetAsync(n.wk, 0, sizeof(__nv_bfloat16) * wtot, n.stream));   // the operands of zero weights
     DP_CUDA(cudaMalloc(&n.partial, sizeof(double) * 4 * kRedBlocks));
     DP_CUDA(cudaMalloc(&n.counter, sizeof(unsigned int)));
-    DP_CUDA(cudaMemset(n.counter, 0, sizeof(unsigned int)));
+    DP_CUDA(cudaMemsetAsync(n.counter, 0, sizeof(unsigned int), n.stream));
     DP_CUDA(cudaMalloc(&n.loss, sizeof(double)));
     DP_CUDA(cudaMallocHost(&n.h_loss, sizeof(double)));
+    DP_CUDA(cudaStreamSynchronize(n.stream));   // dp_guess_predict reads the weights on the context's stream
     return (int)DP_OK;
   });
   if (st != DP_OK) {

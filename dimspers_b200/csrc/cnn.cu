@@ -32,7 +32,7 @@ struct Cnn {
   int bf16 = 1;                 // 1: BF16 tensor-core convolutions (FP32 accumulate), 0: FP32 CUDA cores
   __nv_bfloat16* wk = nullptr;  // BF16 B operands of every layer, forward then data gradient (refreshed with the weights)
   std::vector<int64_t> wkoff;   // per layer: forward, data gradient
-  float* wpart = nullptr;       // partial sums of the weight gradient (allocated by the first backward pass)
+  float* wpart = nullptr;       // partial sums of the weight gradient
   int dil[kCnnMaxLayers];
   int bmax = 0;
   cudaStream_t stream = nullptr;
@@ -663,13 +663,25 @@ static void refresh_weights(Cnn& n, cudaStream_t s) {
   DP_LAUNCH_CHECK();
 }
 
+// CTAs of a weight gradient, and the floats of a layer's partial sums: kShare sets
+// (BwTile) for each
+static int bw_ctas(const Cnn& n, int nb) {
+  return (int)std::min<int64_t>(kBwCtas, (int64_t)nb * n.nrg * div_up(n.ntg, kBwTj));
+}
+static int64_t bw_part_floats(const Cnn& n, int l) {
+  const int cin = n.cin_of(l), cout = n.cout_of(l), groups = cout / std::min(cout, 8);
+  return (int64_t)bw_ctas(n, n.bmax) * (4 / groups) * (cout * cin * 9 + cout);
+}
+static_assert(BwTile<8, 16>::kShare == 2 && BwTile<4, 1>::kShare == 4 && BwTile<32, 32>::kShare == 1 &&
+              BwTile<8, 16>::kSet == 16 * 8 * 9 + 16, "bw_part_floats follows BwTile");
+
 template <int CIN, int COUT>
 static void conv_bwd_w_t(Cnn& n, int l, const float* X, const float* dY, int nb) {
   typedef BwTile<CIN, COUT> T;
   const size_t smem = T::smem(n.dil[l]);
   if (smem > 48 * 1024)
     DP_CUDA(cudaFuncSetAttribute(k_conv_bwd_w<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int ctas = (int)std::min<int64_t>(kBwCtas, (int64_t)nb * n.nrg * div_up(n.ntg, kBwTj));
+  const int ctas = bw_ctas(n, nb);
   ++g_klaunch;
   k_conv_bwd_w<CIN, COUT><<<ctas, 128, smem, n.stream>>>(X, dY, n.wpart, nb, n.nrg, n.ntg, n.dil[l]);
   ++g_klaunch;
@@ -738,10 +750,6 @@ static void cnn_fwd_bwd(Cnn& n, const float* x, const float* t, int nb) {
   ++g_klaunch;
   k_mse<<<red_grid(nout), kRedThreads, 0, n.stream>>>(n.act[n.L], t, g, nout, n.partial, n.counter, n.loss);
   DP_LAUNCH_CHECK();
-  if (!n.wpart) {
-    // sets of sums: at most kBwCtas CTAs, 32 x 32 channels (or, with fewer output channels, more but smaller sets)
-    DP_CUDA(cudaMalloc(&n.wpart, sizeof(float) * kBwCtas * (size_t)(32 * 32 * 9 + 32)));
-  }
   for (int l = n.L - 1; l >= 0; --l) {
     const int cin = n.cin_of(l), cout = n.cout_of(l);
     conv_bwd_w(n, l, n.act[l], g, nb);
@@ -864,6 +872,9 @@ int dp_cnn_create(int32_t nrg, int32_t ntg, int32_t channels, int32_t layers, co
     const int64_t gmax = (int64_t)max_batch * std::max(channels, 4) * plane;
     DP_CUDA(cudaMalloc(&n.dbuf0, sizeof(float) * gmax));
     DP_CUDA(cudaMalloc(&n.dbuf1, sizeof(float) * gmax));
+    int64_t part = 0;
+    for (int l = 0; l < layers; ++l) part = std::max(part, bw_part_floats(n, l));
+    DP_CUDA(cudaMalloc(&n.wpart, sizeof(float) * part));
     int64_t wtot = 0;
     for (int k = 0; k < 2 * layers; ++k) {
       n.wkoff.push_back(wtot);

@@ -20,3 +20,21 @@ def test_weights_set_while_the_default_stream_is_busy():
         torch.cuda.synchronize()
         assert np.array_equal(net.get_params(), p)
         net.close()
+
+
+def test_the_first_training_step_allocates_nothing():
+    import torch
+
+    from dimspers_b200.learned import GuessNet
+    x = torch.randn((2, 4, 65, 128), device="cuda")
+    t = torch.randn((2, 1, 65, 128), device="cuda")
+    free = []
+    for _ in range(2):                     # the first network's step also loads the kernels
+        net = GuessNet(65, 128, 32, 4, (1, 2, 4, 1), 2)
+        net.init_params(0)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        net.train_step(x, t, 1e-3)
+        free.append(before - torch.cuda.mem_get_info()[0])
+        net.close()
+    assert free[1] == 0

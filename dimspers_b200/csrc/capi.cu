@@ -854,10 +854,12 @@ int dp_profile_kernel(dp_ctx* h, int32_t which, int32_t reps, int32_t flush_l2, 
     if (reps < 1 || !ms) throw BadArg("reps must be >= 1");
     if (which == 0 && !c.K32) throw BadArg("no FP32 element matrices (assemble with precision 1)");
     if (which == 2 && c.mg.empty()) throw BadArg("no multigrid hierarchy (run a solve first)");
-    if (which == 3 && !c.stress_called) throw BadArg("no staged post-processor inputs (call dp_stress first)");
-    if (which == 4 && !c.rheo_called) throw BadArg("no staged viscosity inputs (call dp_viscosity_arrhenius first)");
-    if (which == 5 && c.fabric_dem[0] == 0)
-      throw BadArg("no staged DEM tensor inputs (call dp_anisotropic_tensor first)");
+    if (which == 3 && !c.stress_staged)
+      throw BadArg("no staged post-processor inputs (call dp_stress with host arrays first)");
+    if (which == 4 && !c.rheo_staged)
+      throw BadArg("no staged viscosity inputs (call dp_viscosity_arrhenius with host arrays first)");
+    if (which == 5 && !c.dem_staged)
+      throw BadArg("no staged DEM tensor inputs (call dp_anisotropic_tensor with host arrays first)");
     if (which == 6 && !c.th_buf) throw BadArg("no thermal element blocks (call dp_thermal_step first)");
     if (which < 0 || which > 7) throw BadArg("which must be 0..7");
     const int64_t n = 2 * c.fine.nnod;

@@ -125,15 +125,15 @@ struct Ctx {
   double* Fscale = nullptr;
   void* flush = nullptr;        // L2 flush buffer for cold kernel timings
   double* stress_buf = nullptr; // post-processor staging: eta 7, tensor 42, outputs 56 per element
-  bool stress_tensor = false;   // the last call's inputs carried a tensor
-  bool stress_called = false, rheo_called = false;
+  bool stress_tensor = false;   // its inputs carry a tensor
+  bool stress_staged = false, rheo_staged = false, dem_staged = false;   // the staging holds a call's inputs
   double* rheo_buf = nullptr;   // viscosity update staging (host arrays): 4 x 7 per element, 3 per node
   double* fabric_buf = nullptr; // FSE / DEM tensor staging (host arrays; fabric_cap doubles)
   int64_t fabric_cap = 0;
   double* dem_tab = nullptr;    // DEM table of the last tensor call (dem_cap doubles), and its pinned source
   double* h_dem = nullptr;
   int64_t dem_cap = 0;
-  int64_t fabric_dem[3] = {0, 0, 0};  // that table's nrows, n_a1a2, sblk (0: none)
+  int64_t fabric_dem[3] = {0, 0, 0};  // that table's nrows, n_a1a2, sblk
   double fabric_w = 0.0;
   double* th_buf = nullptr;     // thermal step: 21 x nel element blocks + 10 nnod vectors
   void* th_exec = nullptr;      // cudaGraphExec_t of the thermal CG loop

@@ -143,9 +143,12 @@ static void upload_dem(Ctx& c, const dp_dem& dem) {
     cudaFreeHost(c.h_dem);
     c.dem_tab = c.h_dem = nullptr;
     c.dem_cap = 0;
+    const bool staged_inputs = c.dem_staged;
+    c.dem_staged = false;   // there is no table should an allocation fail
     dalloc(&c.dem_tab, (size_t)n);
     DP_CUDA(cudaMallocHost((void**)&c.h_dem, sizeof(double) * n));
     c.dem_cap = n;
+    c.dem_staged = staged_inputs;
   }
   c.fabric_dem[0] = dem.nrows;
   c.fabric_dem[1] = dem.n_a1a2;
@@ -173,8 +176,8 @@ static double* fabric_scratch(Ctx& c, int64_t n) {
     cudaFree(c.fabric_buf);
     c.fabric_buf = nullptr;
     c.fabric_cap = 0;
+    c.dem_staged = false;
     dalloc(&c.fabric_buf, (size_t)n);
-    DP_CUDA(cudaMemsetAsync(c.fabric_buf, 0, sizeof(double) * n, c.stream));
     c.fabric_cap = n;
   }
   return c.fabric_buf;
@@ -189,7 +192,7 @@ static void dem_staging(Ctx& c, DemIn& in, Fields6& out) {
   out.ld = nel;
 }
 
-// k_dem_tensor on the staging buffer and the last call's table (kernel timing)
+// k_dem_tensor on the inputs of the last staged call and the last call's table (kernel timing)
 void launch_dem_staged(Ctx& c) {
   DemIn in;
   Fields6 out;
@@ -214,13 +217,13 @@ extern "C" int dp_fse(dp_ctx* h, const double* F, double* const* fse, int64_t ld
     bool dev = in_place(c.device, F, mem);
     for (int f = 0; f < 6; ++f)
       dev = dev && in_place(c.device, fse[f], mem) && !overlap(fse[f], 5 * ld_out + nel, F, 4 * n);
-    c.fabric_dem[0] = 0;  // the staged inputs of the tensor lookup are overwritten
     Fields6 out;
     const double* dF = F;
     for (int f = 0; f < 6; ++f) out.f[f] = fse[f];
     out.ld = ld_out;
     if (!dev || !aligned16(F)) {   // the kernel reads F in 16-byte pairs
       double* buf = fabric_scratch(c, 10 * n);
+      c.dem_staged = false;        // the tensor lookup's staged inputs are overwritten
       DP_CUDA(cudaMemcpyAsync(buf, F, sizeof(double) * 4 * n, kind_in(mem), c.stream));
       dF = buf;
     }
@@ -276,6 +279,7 @@ extern "C" int dp_anisotropic_tensor(dp_ctx* h, const dp_dem* dem, const double*
       for (int f = 0; f < 4; ++f)
         DP_CUDA(cudaMemcpy2DAsync((void*)dst[f], sizeof(double) * nel, src[f], sizeof(double) * ld_in,
                                   sizeof(double) * nel, 6, kind_in(mem), c.stream));
+      c.dem_staged = true;
     }
     launch_k_dem_tensor(c, in, out);
     for (int f = 0; !dev && f < 6; ++f)

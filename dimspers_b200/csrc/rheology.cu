@@ -155,18 +155,14 @@ static void launch_viscosity(Ctx& c, const double* T, const double* P, const dou
   DP_LAUNCH_CHECK();
 }
 // the staging buffer: epsII, tauII, cohesion, eta (7 columns each), T, P, r
-// (zero until host arrays are staged)
 static double* rheo_staging(Ctx& c) {
-  const int64_t n = 28 * c.fine.nel + 3 * c.fine.nnod;
-  if (!c.rheo_buf) {
-    dalloc(&c.rheo_buf, n);
-    DP_CUDA(cudaMemsetAsync(c.rheo_buf, 0, sizeof(double) * n, c.stream));
-  }
+  if (!c.rheo_buf) dalloc(&c.rheo_buf, 28 * c.fine.nel + 3 * c.fine.nnod);
   return c.rheo_buf;
 }
 
-// k_viscosity_arrhenius on the staging buffer (kernel timing; eta is updated in
-// place, and a second pass over it writes the same values).
+// k_viscosity_arrhenius on the inputs of the last staged call, with the last
+// call's law and extremes (kernel timing; eta is updated in place, and a second
+// pass over it writes the same values).
 void launch_viscosity_staged(Ctx& c) {
   const int64_t nel = c.fine.nel, nn = c.fine.nnod;
   double* e2 = rheo_staging(c);
@@ -221,6 +217,7 @@ extern "C" int dp_viscosity_arrhenius(dp_ctx* h, const dp_arrhenius* law, const 
       T = up(s + 28 * nel, T_node, nn);
       P = up(s + 28 * nel + nn, P_vertex, nv);
       r = up(s + 28 * nel + 2 * nn, r_node, nn);
+      c.rheo_staged = true;
     }
     ++g_klaunch;
     k_minmax<<<(int)std::min<int64_t>(kRedBlocks, div_up(nn, 4 * kRedThreads)), kRedThreads, 0, c.stream>>>(
@@ -232,7 +229,6 @@ extern "C" int dp_viscosity_arrhenius(dp_ctx* h, const dp_arrhenius* law, const 
     a.cphi = std::cos(law->phi_deg * (3.14159265358979323846 / 180.0));
     const double keep[8] = {a.eta0, a.R, a.Ea, a.Va, a.T0, a.sphi, a.cphi, a.phi};
     for (int i = 0; i < 8; ++i) c.rheo_law[i] = keep[i];
-    c.rheo_called = true;
     launch_viscosity(c, T, P, r, e2, t2, co, et);
     if (!dev) DP_CUDA(cudaMemcpyAsync(eta_ip, et, sizeof(double) * 7 * nel, kind_out(mem), c.stream));
     DP_CUDA(cudaStreamSynchronize(c.stream));

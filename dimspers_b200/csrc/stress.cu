@@ -160,13 +160,10 @@ static void launch_stress(Ctx& c, StressArgs a) {
   k_stress<<<(int)div_up(a.nel, 128), 128, 0, c.stream>>>(a);
   DP_LAUNCH_CHECK();
 }
-// the staging buffer: eta 7, tensor 42, out 56 columns (zero until host arrays are staged)
+// the staging buffer: eta 7, tensor 42, out 56 columns
 static StressArgs staged_stress_args(Ctx& c, bool tensor) {
   const int64_t nel = c.fine.nel;
-  if (!c.stress_buf) {
-    dalloc(&c.stress_buf, (7 + 42 + 56) * nel);
-    DP_CUDA(cudaMemsetAsync(c.stress_buf, 0, sizeof(double) * (7 + 42 + 56) * nel, c.stream));
-  }
+  if (!c.stress_buf) dalloc(&c.stress_buf, (7 + 42 + 56) * nel);
   StressArgs a = stress_args(c, tensor);
   a.U = (const double*)c.work[W_UC];
   a.eta = c.stress_buf;
@@ -176,7 +173,7 @@ static StressArgs staged_stress_args(Ctx& c, bool tensor) {
   return a;
 }
 
-// k_stress on the staging buffer (kernel timing)
+// k_stress on the inputs of the last staged call (kernel timing)
 void launch_stress_staged(Ctx& c, bool tensor) { launch_stress(c, staged_stress_args(c, tensor)); }
 
 }  // namespace dp
@@ -201,8 +198,6 @@ extern "C" int dp_stress(dp_ctx* h, const double* Ucart, const double* eta_ip, i
     if (C6)
       for (int f = 0; f < 6; ++f)
         if (!C6[f]) throw BadArg("null tensor field");
-    c.stress_called = true;
-    c.stress_tensor = C6 != nullptr;
     bool dev = in_place(c.device, out, mem) && in_place(c.device, Ucart, mem) && in_place(c.device, eta_ip, mem) &&
                !overlap(out, 56 * nel, Ucart, 2 * nn) && !overlap(out, 56 * nel, eta_ip, 6 * ld_eta + nel);
     for (int f = 0; C6 && f < 6; ++f)
@@ -222,6 +217,8 @@ extern "C" int dp_stress(dp_ctx* h, const double* Ucart, const double* eta_ip, i
         DP_CUDA(cudaMemcpy2DAsync((void*)a.C[f], sizeof(double) * nel, C6[f], sizeof(double) * ld_C,
                                   sizeof(double) * nel, 7, kind_in(mem), c.stream));
       DP_CUDA(cudaMemcpyAsync((void*)a.U, Ucart, sizeof(double) * 2 * nn, kind_in(mem), c.stream));
+      c.stress_staged = true;
+      c.stress_tensor = C6 != nullptr;
       launch_stress(c, a);
       DP_CUDA(cudaMemcpyAsync(out, a.out, sizeof(double) * 56 * nel, kind_out(mem), c.stream));
     }

@@ -354,8 +354,9 @@ class StokesContext:
 
     def profile_kernel(self, which, reps=50, flush_l2=False):
         """Average ms per launch: 0 FP32 A-apply, 1 FP64 A-apply, 2 V-cycle,
-        3 stress post-processor, 4 viscosity update, 5 DEM tensor lookup, 6
-        thermal apply (last call's inputs), 7 the graph solve's inner-iteration
+        3 stress post-processor, 4 viscosity update, 5 DEM tensor lookup
+        (inputs of the last call with host arrays), 6 thermal apply (last
+        call's blocks), 7 the graph solve's inner-iteration
         vector kernels launched outside the graph (for profilers);
         flush_l2 times each launch alone after overwriting 256 MB (cold L2)."""
         ms = C.c_double(0.0)

@@ -842,6 +842,7 @@ namespace dp {
 void launch_stress_staged(Ctx& c, bool tensor);
 void launch_viscosity_staged(Ctx& c);
 void launch_dem_staged(Ctx& c);
+void th_clear_stop(Ctx& c);
 void launch_th_apply_staged(Ctx& c);
 }
 
@@ -884,6 +885,7 @@ int dp_profile_kernel(dp_ctx* h, int32_t which, int32_t reps, int32_t flush_l2, 
       else if (c.mg_prec == 1) mg_apply_f(c, x32, y32, MGOptions());
       else mg_apply(c, x64, y64, MGOptions());
     };
+    if (which == 6) th_clear_stop(c);
     once();
     cudaEvent_t e0, e1;
     DP_CUDA(cudaEventCreate(&e0));

@@ -359,12 +359,11 @@ static void th_emit_loop(Ctx& c, int heated) {
   DP_CUDA(cudaStreamEndCapture(aux, &out));
 }
 
-// the apply kernel on the last step's blocks and vectors (kernel timing: with the
-// stop flag down; what it adds to q and the slots is zeroed by the next step)
-void launch_th_apply_staged(Ctx& c) {
-  DP_CUDA(cudaMemsetAsync(c.scal + TH_STOP, 0, sizeof(double), c.stream));
-  th_launch_apply(c, 0, c.stream);
-}
+// Kernel timing: the apply on the last step's blocks and vectors, after the stop
+// flag that the step left was taken down (the apply does not raise it; what it adds
+// to q and the slots is zeroed by the next step).
+void th_clear_stop(Ctx& c) { DP_CUDA(cudaMemsetAsync(c.scal + TH_STOP, 0, sizeof(double), c.stream)); }
+void launch_th_apply_staged(Ctx& c) { th_launch_apply(c, 0, c.stream); }
 
 }  // namespace dp
 

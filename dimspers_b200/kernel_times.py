@@ -103,8 +103,9 @@ def thermal(nr, nt):
     T, rho, dt = inputs_thermal(c.mesh, nr, np.random.default_rng(0))
     Tn, it, rel = c.thermal_step(T, rho, dt)
     call = _best_ms(lambda: c.thermal_step(T, rho, dt), reps=5)
+    # per node z and the old p read, the new p written, q read and written
     rec = _line("k_th_apply", size, c.profile_kernel(6, 50), c.profile_kernel(6, 10, True),
-                c.nel * 21 * 8 + c.nnod * 3 * 8, np.isfinite(Tn).all(), dt=dt, iterations=it, relres=rel,
+                c.nel * 21 * 8 + c.nnod * 5 * 8, np.isfinite(Tn).all(), dt=dt, iterations=it, relres=rel,
                 step_ms=call, call_ms=call)
     c.close()
     return [rec]

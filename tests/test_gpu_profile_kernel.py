@@ -60,3 +60,24 @@ def test_staged_kernels_are_timed_on_a_calls_inputs_or_refused():
         c.fse(F)                          # staged over the tensor lookup's inputs
         with pytest.raises(Exception, match="host arrays"):
             c.profile_kernel(5, 1)
+
+
+def test_timed_region_holds_the_kernel_alone():
+    """What the GPU runs in a call with 3 + 1 launches of the thermal apply: as many kernels, and no
+    more copies or memsets than the call's set-up has whatever the launches."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with StokesContext(16, 128, "continuous") as c:
+        T, rho, dt = KT.inputs_thermal(c.mesh, 16, np.random.default_rng(0))
+        c.thermal_step(T, rho, dt)
+        c.profile_kernel(6, 1)
+        seen = {}
+        for reps in (1, 3):
+            torch.cuda.synchronize()
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                c.profile_kernel(6, reps)
+                torch.cuda.synchronize()
+            names = [e.name for e in prof.events()]
+            seen[reps] = (sum("k_th_apply" in k for k in names), sum("emset" in k for k in names))
+    assert seen[1][0] == 2 and seen[3][0] == 4
+    assert seen[1][1] == seen[3][1] > 0

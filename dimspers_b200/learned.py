@@ -162,13 +162,29 @@ class LearnedGuess:
         dev = torch.device("cuda", ctx.desc.device)
         self.x = torch.empty((1, 4, net.nrg, net.ntg), dtype=torch.float32, device=dev)
         self.y = torch.empty((1, 1, net.nrg, net.ntg), dtype=torch.float32, device=dev)
-        self.xm = np.ascontiguousarray(net.x_mean, np.float32)
-        self.xs = np.ascontiguousarray(net.x_std, np.float32)
+        stats = [np.asarray(v).reshape(4) for v in (net.x_mean, net.x_std)]
+        self.xm, self.xs = (np.ascontiguousarray(v, np.float32) for v in stats)
+        # statistics that FP32 does not hold are applied in their own precision
+        self.wide = None
+        if any(not np.array_equal(v, f) for v, f in zip(stats, (self.xm, self.xs))):
+            self.wide = [torch.tensor(v, device=dev).view(1, 4, 1, 1) for v in stats]
 
     def predict(self, g, P_out_ptr, mem=DP_MEM_DEVICE):
         """Write the guess for the context's current material into P (device
         pointer by default)."""
         n = self.net
+        if self.wide:
+            import torch
+            done = torch.cuda.current_stream(self.x.device).synchronize   # the library's streams do not wait for torch's
+            features(self.ctx, self.x)
+            self.x.sub_(self.wide[0]).div_(self.wide[1])
+            done()
+            n.forward(self.x, self.y)
+            self.y.mul_(n.y_std).add_(n.y_mean)
+            done()
+            self.ctx._chk(lib().dp_guess_from_grid(self.ctx.h, C.c_void_p(self.y.data_ptr()), n.nrg, n.ntg, float(g),
+                                                   C.c_void_p(P_out_ptr), mem))
+            return
         self.ctx._chk(lib().dp_guess_predict(self.ctx.h, n.h, C.c_void_p(self.xm.ctypes.data),
                                              C.c_void_p(self.xs.ctypes.data), float(n.y_mean), float(n.y_std),
                                              float(g), C.c_void_p(self.x.data_ptr()), C.c_void_p(self.y.data_ptr()),

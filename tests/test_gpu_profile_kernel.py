@@ -81,3 +81,23 @@ def test_timed_region_holds_the_kernel_alone():
             seen[reps] = (sum("k_th_apply" in k for k in names), sum("emset" in k for k in names))
     assert seen[1][0] == 2 and seen[3][0] == 4
     assert seen[1][1] == seen[3][1] > 0
+
+
+def test_fp64_apply_of_the_benchmark_is_the_kernel_it_names():
+    import sys
+
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    sys.path.insert(0, ROOT)
+    import bench
+    with StokesContext(16, 128, "discontinuous") as c:
+        m = inputs.make_material(c.mesh, "aniso", seed=4)
+        c.set_material(m.eta_ip, m.rho, m.g, m.C6)
+        c.assemble(1)
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            rec = bench.fp64_apply_roofline(c, c.nel, c.nnod, 6546.2)
+            torch.cuda.synchronize()
+    named = rec["kernel"].split(" ")[0].rstrip(">")          # k_apply_R<double
+    applies = [e.name for e in prof.events() if "k_apply_" in e.name]
+    assert len(applies) == 21 and all(named in k for k in applies), (named, set(applies))

@@ -254,8 +254,6 @@ __global__ void k_bj_mixed(const Td* __restrict__ dinv, const Tv* r, Tv* z, int6
   z[2 * n + 1] = (Tv)z1;
 }
 
-// x += alpha p; r -= alpha Ap; alpha = rzn/pAp; ||r||^2 -> irr
-
 // rz = r . z with z = ||b|| z32 (the V-cycle ran on r / ||b||); z itself is
 // never stored: k_pcg_dir_f32z reads z32 again
 __global__ void __launch_bounds__(kRedThreads) k_rz_f32(const float* z32, const double* r,
@@ -458,12 +456,12 @@ static void emit_pcg(Ctx& c, const SolveCfg& cfg, const T* Kmat, const T* b, T* 
     if (first32.dinv) launch_first_step<float>(c, r32, first32);
     if (first.dinv) launch_first_step<T>(c, r, first);
   }
-  // r . z from the V-cycle's last kernel (an atomic per block, so not in the deterministic mode)
+  // r . z from the V-cycle's last kernel, where it sums it
   RzOut rzo;
   rzo.r = (const double*)r;
   rzo.yy = mixed ? c.scal + YY : nullptr;
   rzo.out = c.scal + RZN;
-  const RzOut* want_rz = f32 || L.det ? nullptr : &rzo;
+  const RzOut* want_rz = f32 ? nullptr : &rzo;
   cudaGraphConditionalHandle h = new_handle(c.stream);
   klaunch(k_in_init, 1, 1, 0, c.stream, h, ctl, c.scal, YY, IRR, c.scal, f32 ? 1 : 0, relax, RZN);
   DP_LAUNCH_CHECK();

@@ -1383,6 +1383,7 @@ static bool vcycle(Ctx& c, size_t l, const T* b, T* x, const MGOptions& o, bool 
     return false;
   }
   MGLevel& L = c.mg[l];
+  if (L.g.det) rz = nullptr;   // an atomic per block: the sum would depend on scheduling
   const bool dense_coarsest = c.coarse_n > 0;
   if (l + 1 == c.mg.size()) {
     if (dense_coarsest) {

@@ -52,8 +52,8 @@ void mg_free(Ctx& c);
 // first_done: the caller has taken the fine level's first smoother step (mg_first_step).
 // rz given: the cycle's last kernel also adds r . s x to *rz->out (s = sqrt(*rz->yy), 1 without
 // yy; r in FP64) if it is of a kind that can (the passes and steps on stencils, whose few blocks
-// make few atomics; on larger levels the launch saved is below 1 % of the iteration); returns
-// whether it does.  An inner iteration takes 52.4 instead of 55.6 us at 16x128, and with the
+// make few atomics; on larger levels the launch saved is below 1 % of the iteration) and the mode
+// is not deterministic; returns whether it does.  An inner iteration takes 52.4 instead of 55.6 us at 16x128, and with the
 // first step fused as well 69.7 instead of 72.7 at 32x256.
 struct RzOut {
   const double* r = nullptr;

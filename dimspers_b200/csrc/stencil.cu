@@ -8,7 +8,8 @@
 // 19 for a vertex (parity class 0) and 9 for the midpoints (classes 1..3), so
 // a node's row of A d is a gather, the smoother's update of r, d and x follows
 // in the same thread, and a step is one launch without atomics.  Its result
-// does not depend on scheduling, so the deterministic mode uses it as it is.
+// does not depend on scheduling, so the deterministic mode uses it as it is
+// (but for ST_STEP_RZ, whose sum takes an atomic per block: not in that mode).
 // The price is 184 bytes of matrix per FP32 node where the element form has
 // 156, which is why large levels keep the element form (kStencilMaxNodes).
 #pragma once

@@ -32,7 +32,7 @@ struct Cnn {
   int bf16 = 1;                 // 1: BF16 tensor-core convolutions (FP32 accumulate), 0: FP32 CUDA cores
   __nv_bfloat16* wk = nullptr;  // BF16 B operands of every layer, forward then data gradient (refreshed with the weights)
   std::vector<int64_t> wkoff;   // per layer: forward, data gradient
-  float* wpart = nullptr;       // partial sums of the weight gradient
+  float* wpart = nullptr;       // partial sums of the weight gradient (in dbuf0's allocation)
   int dil[kCnnMaxLayers];
   int bmax = 0;
   cudaStream_t stream = nullptr;
@@ -46,7 +46,7 @@ struct Cnn {
   float* adam_v = nullptr;
   int64_t step = 0;
   std::vector<float*> act;   // act[0] = input (external), act[l+1] = output of layer l
-  float* dbuf0 = nullptr;    // gradient buffers (max size)
+  float* dbuf0 = nullptr;    // gradient buffers (max size), one allocation
   float* dbuf1 = nullptr;
   double* partial = nullptr;
   unsigned int* counter = nullptr;
@@ -57,7 +57,7 @@ struct Cnn {
   ~Cnn() {
     cudaFree(param); cudaFree(grad); cudaFree(adam_m); cudaFree(adam_v);
     for (size_t i = 1; i < act.size(); ++i) cudaFree(act[i]);
-    cudaFree(dbuf0); cudaFree(dbuf1); cudaFree(partial); cudaFree(counter); cudaFree(loss); cudaFree(wk); cudaFree(wpart);
+    cudaFree(dbuf0); cudaFree(partial); cudaFree(counter); cudaFree(loss); cudaFree(wk);
     cudaFreeHost(h_loss);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -869,12 +869,14 @@ int dp_cnn_create(int32_t nrg, int32_t ntg, int32_t channels, int32_t layers, co
     const int64_t plane = (int64_t)nrg * ntg;
     n.act.assign(layers + 1, nullptr);
     for (int l = 0; l < layers; ++l) DP_CUDA(cudaMalloc(&n.act[l + 1], sizeof(float) * max_batch * n.cout_of(l) * plane));
-    const int64_t gmax = (int64_t)max_batch * std::max(channels, 4) * plane;
-    DP_CUDA(cudaMalloc(&n.dbuf0, sizeof(float) * gmax));
-    DP_CUDA(cudaMalloc(&n.dbuf1, sizeof(float) * gmax));
+    // both gradient buffers and the weight gradient's workspace: an allocation costs
+    // ~0.35 ms whatever its size
+    const int64_t gmax = div_up((int64_t)max_batch * std::max(channels, 4) * plane, 64) * 64;   // 256-byte steps
     int64_t part = 0;
     for (int l = 0; l < layers; ++l) part = std::max(part, bw_part_floats(n, l));
-    DP_CUDA(cudaMalloc(&n.wpart, sizeof(float) * part));
+    DP_CUDA(cudaMalloc(&n.dbuf0, sizeof(float) * (2 * gmax + part)));
+    n.dbuf1 = n.dbuf0 + gmax;
+    n.wpart = n.dbuf1 + gmax;
     int64_t wtot = 0;
     for (int k = 0; k < 2 * layers; ++k) {
       n.wkoff.push_back(wtot);

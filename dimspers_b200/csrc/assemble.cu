@@ -23,9 +23,11 @@
 // registers, rotates and masks them, and hands them to shared memory, from
 // where the packed matrix leaves in 16-byte groups.  FP64 throughout (the
 // refined path stores a rounded FP32 copy of Ke).
-// Bound by FP64 issue and the 1.4-1.7 kB an element reads and writes.  The form
-// it replaces, one thread per element with 132 accumulators in shared memory,
-// moved 25 kB an element through shared memory: 968 us at 256x2048.
+// Bound by FP64 issue and by the 1.0-1.4 kB an element reads and writes (2.0-2.3
+// on the refined path, which adds the FP32 copy and the reduced matrices to the
+// packed ones): 0.58 and 0.72 ms at 256x2048.  The form it replaces, one thread
+// per element with 132 accumulators in shared memory, moved 25 kB an element
+// through shared memory: 968 us.
 #include "kernels.cuh"
 
 namespace dp {

@@ -7,9 +7,13 @@ namespace dp {
 constexpr int kMaxCheb = 8;
 // Largest level (lattice nodes) whose smoother runs on node stencils: the
 // 32x256 level (33,280 nodes) and below.  Per inner iteration of the whole
-// solve: 16x128 FP64 80.7 -> 67.5 us, 32x256 103 -> 92.8 us.  Including the
-// 64x512 level (132k nodes, 24 MB of stencils) measured 145 against 140.5 us
-// at 64x512 and no change at 128x1024: there the bytes count, not the launches.
+// solve when they came in: 16x128 FP64 80.7 -> 67.5 us, 32x256 103 -> 92.8 us.
+// On larger fine levels the bytes (184 a node against 112 of the reduced element
+// matrices) weigh more than the launches; fast path, element form -> stencils on the fine level too:
+// 42k nodes (36x288) 89.5 -> 84.7 us, 52k (40x320) 100.2 -> 97.7, 74k (48x384)
+// 93.8 -> 89.0, 101k (56x448) 115.0 -> 114.3, 132k (64x512) 112.7 -> 116.4.
+// The two meet near 100k nodes; the line is below that, at the largest level of
+// the meshes that halve down from the benchmark's.
 constexpr int64_t kStencilMaxNodes = 40000;
 
 struct MGOptions {

@@ -400,19 +400,20 @@ int dp_guess_predict(dp_ctx* ctx, dp_cnn* net, const float* x_mean, const float*
 
 /* Average device time (ms) of one launch of a hot kernel on the context's
  * stream, from CUDA events, after an assembly: which = 0 fine-level A-apply
- * FP32, 1 fine-level A-apply FP64, 2 one multigrid V-cycle (precision of the
- * last solve), 3 the stress post-processor on the inputs of the last
- * dp_stress call that was staged, 4 the viscosity update on those of the last
- * dp_viscosity_arrhenius call that was, 5 the DEM tensor lookup on those of the
- * last dp_anisotropic_tensor call that was, 6 the thermal element-by-element apply
- * (A p of the last dp_thermal_step's blocks), 7 the vector kernels of one
- * inner iteration of the graph solve launched outside the graph (for
- * profilers; the event time includes their zeroing).  Calls with
- * host arrays stage copies of them; calls with device arrays work on those in
- * place, so 3 to 5 return DP_BAD_ARG until a call with host arrays was made (5:
- * and again after a staged dp_fse, which uses the same space).  flush_l2 = 0: `reps` back-to-back launches (warm L2);
- * 1: a 256 MB buffer is read before each launch and each launch is timed
- * alone (cold L2, DRAM-bound figure). */
+ * FP32, 1 fine-level A-apply FP64 (on the reduced matrices after a refined
+ * assembly, on the packed ones after an FP64 one), 2 one multigrid V-cycle
+ * (precision of the last solve), 3 the stress post-processor on the inputs of
+ * the last dp_stress call that was staged, 4 the viscosity update on those of
+ * the last dp_viscosity_arrhenius call that was, 5 the DEM tensor lookup on
+ * those of the last dp_anisotropic_tensor call that was, 6 the thermal
+ * element-by-element apply (A p of the last dp_thermal_step's blocks), 7 the
+ * vector kernels of one inner iteration of the graph solve launched outside the
+ * graph (for profilers; the event time includes their zeroing).  Calls with host
+ * arrays stage copies of them; calls with device arrays work on those in place,
+ * so 3 to 5 return DP_BAD_ARG until a call with host arrays was made (5: and
+ * again after a staged dp_fse, which uses the same space).  flush_l2 = 0: `reps`
+ * back-to-back launches (warm L2); 1: a 256 MB buffer is read before each launch
+ * and each launch is timed alone (cold L2, DRAM-bound figure). */
 int dp_profile_kernel(dp_ctx* ctx, int32_t which, int32_t reps, int32_t flush_l2, double* ms_per_launch);
 
 #ifdef __cplusplus
